@@ -317,3 +317,43 @@ def tolerance(case):
         return {"rel": 1e-5 if case["out"] == "f32" else 2e-4, "max": 2e-3}
     # Integer sums and operations rounded one by one in a fixed order: the bytes are the contract.
     return "exact"
+
+
+def _activated(x, act):
+    if act == "relu":
+        return x.clamp_min(0)
+    if act == "gelu":
+        return 0.5 * x * (1 + torch.tanh(math.sqrt(2.0 / math.pi) * (x + 0.044715 * x ** 3)))
+    return x * torch.sigmoid(x) if act == "silu" else x
+
+
+def exact(case, seed):
+    """The floating destinations of the products in 64 bits; whole-number results are compared byte for byte instead."""
+    c, op = case, case["op"]
+    if op not in ("linear", "matmul", "q4_1") or c["out"] not in _DTYPE:
+        return None
+    state = prepare(case, seed)
+    a = state["a"].double()
+    if op == "q4_1":
+        if c["packed"]:
+            state["w"] = _q4_1_blocks(_gen(seed), c["n"], c["k"])
+        blocks = state["w"].view(c["n"], -1, 20)
+        d, low = (blocks[:, :, i:i + 2].contiguous().view(torch.float16).double() for i in (0, 2))
+        nibbles = torch.cat([blocks[:, :, 4:] & 15, blocks[:, :, 4:] >> 4], dim=2).double()
+        w = (d * nibbles + low).reshape(c["n"], c["k"])
+        return _activated(a @ w.t(), c["act"])
+    kw = state["kw"]
+    if op == "matmul":
+        return a @ state["w"].double().transpose(-1, -2) * (kw["scale_a"] * kw["scale_w"])
+
+    def column(v):
+        return v.double().unsqueeze(1) if isinstance(v, torch.Tensor) else v
+
+    if c["packed"]:
+        g = _gen(seed)
+        w, scale_w = _s8(g, c["n"], c["k"]), _scales(g, c["n"])
+        zp_w = state["packed"].zp_w
+    else:
+        w, scale_w, zp_w = state["w"], kw["scale_w"], kw["zp_w"]
+    x = (a - column(kw.get("zp_a", 0))) @ (w.double() - column(zp_w)).t()
+    return _activated(x * column(kw["scale_a"]) * scale_w.double() + kw["bias"].double(), c["act"])
