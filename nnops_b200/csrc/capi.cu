@@ -9,6 +9,7 @@
 #include <cstring>
 #include <mutex>
 
+#include "gemm_i8_umma_batched.cuh"
 #include "internal.cuh"
 #include "ptx.cuh"
 
@@ -367,7 +368,7 @@ static I8SplitPlan i8_split_plan(const nnb200_gemm_i8_args* a)
     return plan;
 }
 
-// The part of the caller's workspace that serves the split, or null when it is absent, too small or misaligned.
+// The part of the caller's workspace, that serves the split, or null when it is absent, too small or misaligned.
 static void* i8_split_scratch(const nnb200_gemm_i8_args* a, size_t required, size_t split_bytes)
 {
     if (split_bytes == 0 || a->workspace == nullptr || a->workspace_bytes < required + split_bytes ||
@@ -410,27 +411,28 @@ int nnb200_gemm_i8_engine(const nnb200_gemm_i8_args* a)
     return i8_engine_with_workspace(a, nullptr);
 }
 
-int nnb200_gemm_i8(const nnb200_gemm_i8_args* a, void* stream_v)
+// Whether a batched call goes out as one launch of the tile kernel, and its strides.
+static bool i8_batched_call(const nnb200_gemm_i8_args* a, const DeviceInfo& dev, I8Batch* b)
 {
-    if (!valid_i8_args(a)) {
-        return NNB200_INVALID_ARGUMENT;
+    if ((a->force_engine != NNB200_ENGINE_AUTO && a->force_engine != NNB200_ENGINE_UMMA) || sharded_out(a)) {
+        return false;
     }
-    if (a->m == 0 || a->n == 0 || a->batch == 0) {
-        return NNB200_OK;
-    }
-    const DeviceInfo* dev = current_device_info();
-    if (dev == nullptr) {
-        return NNB200_INTERNAL;
-    }
-    if (dev->cc_major != 10) {
-        return NNB200_UNSUPPORTED;  // sm_100a only: there is no other code path
-    }
-    cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+    b->count = a->batch;
+    b->a_stride = a->a_batch_stride;
+    b->w_stride = a->w_batch_stride;
+    b->out_stride = a->out_batch_stride;
+    b->ra_step = 0;
+    b->rw_step = 0;
+    // Products whose outputs overlap keep the order of one launch after another.
+    const bool apart = (a->out_batch_stride >= (a->m - 1) * a->ldc + a->n) ||
+                       (a->out_batch_stride >= a->n && a->out_batch_stride * (a->batch - 1) + a->n <= a->ldc);
+    return apart && umma_i8_batched_supported(problem_of(a, 0), *b, dev);
+}
+
+// One call's kernels.
+static int run_gemm_i8(const nnb200_gemm_i8_args* a, const DeviceInfo* dev, cudaStream_t stream)
+{
     const bool comp = needs_compensation(a);
-    const size_t need = nnb200_gemm_i8_min_workspace_bytes(a);
-    if (need > 0 && (a->workspace == nullptr || a->workspace_bytes < need)) {
-        return NNB200_INVALID_ARGUMENT;
-    }
     // The rest of the workspace, when there is enough of it, lets the few-row engine share K
     // among the SMs (and on narrow layers with a long K makes it the engine of choice).
     void* split_scratch = nullptr;
@@ -461,16 +463,26 @@ int nnb200_gemm_i8(const nnb200_gemm_i8_args* a, void* stream_v)
         }
     }
 
+    // A batch of small products goes out as one launch: alone, a product of a few tiles leaves
+    // most SMs idle and the launches follow one another (32 heads of 512 x 128 x 512: 279 us a
+    // call, nearly all of it launches).
+    I8Batch batch;
+    const bool batched = a->batch > 1 && i8_batched_call(a, *dev, &batch);
+
     // Launchability of every batch element is settled before the first launch, so that a
     // refusal leaves the outputs untouched: the generic engine's grid has 65535 rows of 32.
-    for (int64_t b = 0; b < a->batch; ++b) {
+    for (int64_t b = 0; !batched && b < a->batch; ++b) {
         const int e = a->batch == 1 ? engine0 : pick_i8_engine(a, problem_of(a, b));
         if (e == NNB200_ENGINE_GENERIC && (a->m + 31) / 32 > 65535) {
             return NNB200_UNSUPPORTED;
         }
     }
 
-    for (int64_t b = 0; b < a->batch; ++b) {
+    // Sums of an operand that every product shares are taken once.
+    const bool shared_a = a->a_batch_stride == 0;
+    const bool shared_w = a->w_batch_stride == 0;
+    const int64_t launches = batched ? 1 : a->batch;
+    for (int64_t b = 0; b < launches; ++b) {
         const I8Problem p = problem_of(a, b);
         I8Epilogue ep;
         std::memset(&ep, 0, sizeof(ep));
@@ -503,25 +515,40 @@ int nnb200_gemm_i8(const nnb200_gemm_i8_args* a, void* stream_v)
             ep.peer_out[i] = a->peer_out[i];
         }
         if (comp) {
-            uint8_t* ws = static_cast<uint8_t*>(a->workspace) + static_cast<size_t>(b) * (ra_bytes + rw_bytes);
-            int32_t* r_a = reinterpret_cast<int32_t*>(ws);
-            int32_t* r_w = reinterpret_cast<int32_t*>(ws + ra_bytes);
+            uint8_t* ws = static_cast<uint8_t*>(a->workspace);
+            const size_t slot = ra_bytes + rw_bytes;
+            int32_t* r_a = reinterpret_cast<int32_t*>(ws + (shared_a ? 0 : static_cast<size_t>(b) * slot));
+            int32_t* r_w = reinterpret_cast<int32_t*>(ws + (shared_w ? 0 : static_cast<size_t>(b) * slot) + ra_bytes);
             const bool have_rw = a->r_w != nullptr && (a->batch == 1 || a->w_batch_stride == 0);
             // R_a only multiplies weight zero points: without any, the sweep over A is skipped.
             // Likewise R_w only multiplies activation zero points.
             const bool need_ra = a->zp_w_scalar != 0 || (a->zp_w != nullptr && a->zp_w_nonzero != 0);
             const bool need_rw = a->zp_a_scalar != 0 || (a->zp_a != nullptr && a->zp_a_nonzero != 0);
-            const bool sweep_w = need_rw && !have_rw;
-            if (need_ra || sweep_w) {
-                const int st = launch_i8_sums(p, need_ra ? r_a : nullptr, sweep_w ? r_w : nullptr, stream);
-                if (st != NNB200_OK) {
-                    return st;
+            const bool sweep_w = need_rw && !have_rw && !(shared_w && b > 0);
+            const bool sweep_a = need_ra && !(shared_a && b > 0);
+            // A batched call sweeps the operands of all its products here.
+            for (int64_t e = b; e < (batched ? a->batch : b + 1); ++e) {
+                const bool sa = sweep_a && !(shared_a && e > b);
+                const bool sw = sweep_w && !(shared_w && e > b);
+                if (sa || sw) {
+                    const int st = launch_i8_sums(problem_of(a, e), sa ? r_a + (e - b) * (slot / 4) : nullptr,
+                                                  sw ? r_w + (e - b) * (slot / 4) : nullptr, stream);
+                    if (st != NNB200_OK) {
+                        return st;
+                    }
                 }
+            }
+            if (batched) {
+                batch.ra_step = shared_a ? 0 : static_cast<int32_t>(slot / 4);
+                batch.rw_step = shared_w || have_rw ? 0 : static_cast<int32_t>(slot / 4);
             }
             ep.r_a = need_ra ? r_a : nullptr;
             ep.r_w = !need_rw ? nullptr : (have_rw ? a->r_w : r_w);
         }
         int st;
+        if (batched) {
+            return launch_gemm_i8_umma_batched(p, batch, ep, *dev, stream);
+        }
         switch (a->batch == 1 ? engine0 : pick_i8_engine(a, p)) {
         case NNB200_ENGINE_UMMA: st = launch_gemm_i8_umma(p, ep, *dev, stream); break;
         case NNB200_ENGINE_NARROW: st = launch_gemm_i8_narrow(p, ep, *dev, stream); break;
@@ -534,6 +561,29 @@ int nnb200_gemm_i8(const nnb200_gemm_i8_args* a, void* stream_v)
         }
     }
     return NNB200_OK;
+}
+
+int nnb200_gemm_i8(const nnb200_gemm_i8_args* a, void* stream_v)
+{
+    if (!valid_i8_args(a)) {
+        return NNB200_INVALID_ARGUMENT;
+    }
+    if (a->m == 0 || a->n == 0 || a->batch == 0) {
+        return NNB200_OK;
+    }
+    const DeviceInfo* dev = current_device_info();
+    if (dev == nullptr) {
+        return NNB200_INTERNAL;
+    }
+    if (dev->cc_major != 10) {
+        return NNB200_UNSUPPORTED;  // sm_100a only: there is no other code path
+    }
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+    const size_t need = nnb200_gemm_i8_min_workspace_bytes(a);
+    if (need > 0 && (a->workspace == nullptr || a->workspace_bytes < need)) {
+        return NNB200_INVALID_ARGUMENT;
+    }
+    return run_gemm_i8(a, dev, stream);
 }
 
 static bool valid_q4_args(const nnb200_q4_1_args* q)
