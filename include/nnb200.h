@@ -90,7 +90,9 @@ extern "C" {
  * serves, the partial sums and arrival counters with which that engine shares K evenly among
  * all SMs.  Only the first part is required: a workspace of at least
  * nnb200_gemm_i8_min_workspace_bytes() is accepted, and the call then runs with whole tiles
- * per SM (same results, slower when N / 128 does not fill the SMs evenly).
+ * per SM (same results, slower when N / 128 does not fill the SMs evenly).  An operand whose base
+ * or pitch is not a multiple of 16 bytes is, from a size on, copied into aligned rows of the
+ * workspace when there is room; without it the call runs on the generic engine (same results).
  */
 typedef struct nnb200_gemm_i8_args {
     const void* a;
@@ -295,7 +297,10 @@ NNB200_API int nnb200_set_knob(int knob, int value);
 NNB200_API int nnb200_get_knob(int knob);
 
 /* Which engine nnb200_gemm_i8 would run for these arguments (NNB200_ENGINE_*), the workspace the
- * block carries included: with enough of it some few-row calls move to the weights-as-rows engine. */
+ * block carries included: with enough of it some few-row calls move to the weights-as-rows engine.
+ * The answer is for the operands as they lie: a call that this says is NNB200_ENGINE_GENERIC, with the
+ * workspace nnb200_gemm_i8_workspace_bytes asks for, first copies the operands that the tensor-core
+ * engines cannot address into aligned rows and then runs the engine of the copies. */
 NNB200_API int nnb200_gemm_i8_engine(const nnb200_gemm_i8_args* args);
 
 /*

@@ -10,6 +10,7 @@
 #include <mutex>
 
 #include "gemm_i8_umma_batched.cuh"
+#include "i8_realign.cuh"
 #include "internal.cuh"
 #include "ptx.cuh"
 
@@ -368,7 +369,7 @@ static I8SplitPlan i8_split_plan(const nnb200_gemm_i8_args* a)
     return plan;
 }
 
-// The part of the caller's workspace, that serves the split, or null when it is absent, too small or misaligned.
+// The part of the caller's workspace, past the first `required` bytes, that serves the split, or null when it is absent, too small or misaligned.
 static void* i8_split_scratch(const nnb200_gemm_i8_args* a, size_t required, size_t split_bytes)
 {
     if (split_bytes == 0 || a->workspace == nullptr || a->workspace_bytes < required + split_bytes ||
@@ -379,10 +380,10 @@ static void* i8_split_scratch(const nnb200_gemm_i8_args* a, size_t required, siz
 }
 
 // Engine of batch element 0 given the workspace the block carries.
-static int i8_engine_with_workspace(const nnb200_gemm_i8_args* a, void** split_scratch)
+static int i8_engine_with_workspace(const nnb200_gemm_i8_args* a, size_t reserved, void** split_scratch)
 {
     const I8SplitPlan plan = i8_split_plan(a);
-    void* scratch = i8_split_scratch(a, nnb200_gemm_i8_min_workspace_bytes(a), plan.bytes);
+    void* scratch = i8_split_scratch(a, nnb200_gemm_i8_min_workspace_bytes(a) + reserved, plan.bytes);
     if (split_scratch != nullptr) {
         *split_scratch = scratch;
     }
@@ -392,12 +393,99 @@ static int i8_engine_with_workspace(const nnb200_gemm_i8_args* a, void** split_s
     return pick_i8_engine(a, problem_of(a, 0));
 }
 
+// Realigned copies of the operands, for calls that alone their base or row pitch keeps off the
+// tensor-core engines (see i8_realign.cu).
+struct I8AlignPlan {
+    size_t copy_bytes;               // scratch for the copies; 0 = the call is not rerouted
+    I8RealignJob a, w;               // rows == 0: that operand is used as it lies
+    nnb200_gemm_i8_args aligned;     // the call over the copies
+};
+
+// From this many multiply-adds on the copies pay: a copy launch and a tensor-core launch against one of
+// the generic engine take 7.6 / 11.2 us at 2^20.8, 8.4 / 28.5 at 2^25.4, 14.0 / 80.4 at 2^26, 41.8 / 1477 at
+// 2^33 (CUDA-graph timings); a problem of 2^19 is a single short wave of generic tiles.
+static constexpr int64_t kRealignMinMacs = int64_t{1} << 19;
+
+static I8AlignPlan i8_align_plan(const nnb200_gemm_i8_args* a, uint8_t* scratch)
+{
+    I8AlignPlan plan;
+    std::memset(&plan, 0, sizeof(plan));
+    if (a->force_engine != NNB200_ENGINE_AUTO || sharded_out(a) || a->m > INT32_MAX || a->n > INT32_MAX ||
+        a->k > INT32_MAX || static_cast<double>(a->m) * a->n * a->k * a->batch < static_cast<double>(kRealignMinMacs)) {
+        return plan;
+    }
+    for (int64_t b = 0; b < (a->batch < 2 ? 1 : 2); ++b) {
+        // Element 0 tells for base and pitch, element 1 for the batch strides.
+        if (pick_i8_engine(a, problem_of(a, b)) == NNB200_ENGINE_GENERIC) {
+            plan.copy_bytes = 1;
+        }
+    }
+    if (plan.copy_bytes == 0) {
+        return plan;
+    }
+    plan.copy_bytes = 0;
+    plan.aligned = *a;
+    const auto place = [&](const void* base, int64_t rows, int64_t cols, int64_t* pitch, int64_t* batch_stride, const void** moved) {
+        const bool batched = a->batch > 1 && *batch_stride != 0;
+        I8RealignJob job;
+        std::memset(&job, 0, sizeof(job));
+        const bool aligned = (reinterpret_cast<uintptr_t>(base) & 15u) == 0 && (*pitch & 15) == 0 && *pitch >= cols &&
+                             (!batched || (*batch_stride & 15) == 0);
+        if (!aligned) {
+            job.src = static_cast<const uint8_t*>(base);
+            job.rows = rows;
+            job.cols = cols;
+            job.src_pitch = *pitch;
+            job.src_batch = *batch_stride;
+            job.batch = batched ? a->batch : 1;
+            job.dst_pitch = (cols + 15) / 16 * 16;
+            job.dst = scratch + plan.copy_bytes;
+            *moved = job.dst;
+            *pitch = job.dst_pitch;
+            *batch_stride = batched ? rows * job.dst_pitch : 0;
+            plan.copy_bytes += (static_cast<size_t>(job.batch) * static_cast<size_t>(rows * job.dst_pitch) + 255) & ~size_t(255);
+        }
+        return job;
+    };
+    nnb200_gemm_i8_args& q = plan.aligned;
+    plan.a = a->a_stride_k == 1 ? place(a->a, a->m, a->k, &q.a_stride_m, &q.a_batch_stride, &q.a)
+                                : place(a->a, a->k, a->m, &q.a_stride_k, &q.a_batch_stride, &q.a);
+    plan.w = a->w_stride_k == 1 ? place(a->w, a->n, a->k, &q.w_stride_n, &q.w_batch_stride, &q.w)
+                                : place(a->w, a->k, a->n, &q.w_stride_k, &q.w_batch_stride, &q.w);
+    return plan;
+}
+
+// Any 256-byte aligned address will do for a plan that only counts bytes.
+static uint8_t* plan_scratch_stand_in() { return reinterpret_cast<uint8_t*>(uintptr_t(4096)); }
+
 size_t nnb200_gemm_i8_workspace_bytes(const nnb200_gemm_i8_args* a)
 {
     if (!valid_i8_args(a) || a->m == 0 || a->n == 0 || a->batch == 0) {
         return 0;
     }
-    return nnb200_gemm_i8_min_workspace_bytes(a) + i8_split_plan(a).bytes;
+    const size_t least = nnb200_gemm_i8_min_workspace_bytes(a);
+    const I8AlignPlan align = i8_align_plan(a, plan_scratch_stand_in());
+    return least + align.copy_bytes + i8_split_plan(align.copy_bytes > 0 ? &align.aligned : a).bytes;
+}
+
+// Whether the workspace has room for realigned copies where the call wants them; if so *q is the
+// call over the copies (not made yet) and *copies their bytes.
+static bool i8_align_in_workspace(const nnb200_gemm_i8_args* a, I8AlignPlan* plan_out, nnb200_gemm_i8_args* q, size_t* copies)
+{
+    const size_t least = nnb200_gemm_i8_min_workspace_bytes(a);
+    if (a->workspace == nullptr || a->workspace_bytes <= least) {
+        return false;
+    }
+    const I8AlignPlan plan = i8_align_plan(a, static_cast<uint8_t*>(a->workspace) + least);
+    if (plan.copy_bytes == 0 || a->workspace_bytes < least + plan.copy_bytes) {
+        return false;
+    }
+    *q = plan.aligned;
+    *copies = plan.copy_bytes;
+    if (plan_out != nullptr) {
+        *plan_out = plan;
+    }
+    return true;
 }
 
 int nnb200_gemm_i8_engine(const nnb200_gemm_i8_args* a)
@@ -408,7 +496,7 @@ int nnb200_gemm_i8_engine(const nnb200_gemm_i8_args* a)
     if (a->m == 0 || a->n == 0 || a->batch == 0) {
         return pick_i8_engine(a, problem_of(a, 0));
     }
-    return i8_engine_with_workspace(a, nullptr);
+    return i8_engine_with_workspace(a, 0, nullptr);
 }
 
 // Whether a batched call goes out as one launch of the tile kernel, and its strides.
@@ -429,14 +517,17 @@ static bool i8_batched_call(const nnb200_gemm_i8_args* a, const DeviceInfo& dev,
     return apart && umma_i8_batched_supported(problem_of(a, 0), *b, dev);
 }
 
-// One call's kernels.
-static int run_gemm_i8(const nnb200_gemm_i8_args* a, const DeviceInfo* dev, cudaStream_t stream)
+// One call's kernels.  `reserved`: bytes of the workspace between the sums and the optional
+// scratch that belong to somebody else (realigned operands); ra_done / rw_done: the sums are in
+// their place already.
+static int run_gemm_i8(const nnb200_gemm_i8_args* a, const DeviceInfo* dev, cudaStream_t stream, size_t reserved,
+                       bool ra_done, bool rw_done)
 {
     const bool comp = needs_compensation(a);
     // The rest of the workspace, when there is enough of it, lets the few-row engine share K
     // among the SMs (and on narrow layers with a long K makes it the engine of choice).
     void* split_scratch = nullptr;
-    const int engine0 = i8_engine_with_workspace(a, &split_scratch);
+    const int engine0 = i8_engine_with_workspace(a, reserved, &split_scratch);
     const size_t ra_bytes = (static_cast<size_t>(a->m) * 4 + 255) & ~size_t(255);
     const size_t rw_bytes = (static_cast<size_t>(a->n) * 4 + 255) & ~size_t(255);
 
@@ -524,8 +615,8 @@ static int run_gemm_i8(const nnb200_gemm_i8_args* a, const DeviceInfo* dev, cuda
             // Likewise R_w only multiplies activation zero points.
             const bool need_ra = a->zp_w_scalar != 0 || (a->zp_w != nullptr && a->zp_w_nonzero != 0);
             const bool need_rw = a->zp_a_scalar != 0 || (a->zp_a != nullptr && a->zp_a_nonzero != 0);
-            const bool sweep_w = need_rw && !have_rw && !(shared_w && b > 0);
-            const bool sweep_a = need_ra && !(shared_a && b > 0);
+            const bool sweep_w = need_rw && !have_rw && !rw_done && !(shared_w && b > 0);
+            const bool sweep_a = need_ra && !ra_done && !(shared_a && b > 0);
             // A batched call sweeps the operands of all its products here.
             for (int64_t e = b; e < (batched ? a->batch : b + 1); ++e) {
                 const bool sa = sweep_a && !(shared_a && e > b);
@@ -583,7 +674,31 @@ int nnb200_gemm_i8(const nnb200_gemm_i8_args* a, void* stream_v)
     if (need > 0 && (a->workspace == nullptr || a->workspace_bytes < need)) {
         return NNB200_INVALID_ARGUMENT;
     }
-    return run_gemm_i8(a, dev, stream);
+    I8AlignPlan plan;
+    nnb200_gemm_i8_args aligned;
+    size_t copies = 0;
+    if (!i8_align_in_workspace(a, &plan, &aligned, &copies)) {
+        return run_gemm_i8(a, dev, stream, 0, false, false);
+    }
+    // The copy pass takes the row sums along where a row of the copy is a row of the operand.
+    const bool need_ra = a->zp_w_scalar != 0 || (a->zp_w != nullptr && a->zp_w_nonzero != 0);
+    const bool need_rw = (a->zp_a_scalar != 0 || (a->zp_a != nullptr && a->zp_a_nonzero != 0)) &&
+                         !(a->r_w != nullptr && (a->batch == 1 || a->w_batch_stride == 0));
+    const size_t ra_bytes = (static_cast<size_t>(a->m) * 4 + 255) & ~size_t(255);
+    const size_t rw_bytes = (static_cast<size_t>(a->n) * 4 + 255) & ~size_t(255);
+    const bool ra_done = need_ra && plan.a.rows > 0 && a->a_stride_k == 1;
+    const bool rw_done = need_rw && plan.w.rows > 0 && a->w_stride_k == 1;
+    if (ra_done) {
+        plan.a.sums = static_cast<uint8_t*>(a->workspace);
+        plan.a.sums_batch = static_cast<int64_t>(ra_bytes + rw_bytes);
+        plan.a.is_unsigned = a->a_unsigned;
+    }
+    if (rw_done) {
+        plan.w.sums = static_cast<uint8_t*>(a->workspace) + ra_bytes;
+        plan.w.sums_batch = static_cast<int64_t>(ra_bytes + rw_bytes);
+    }
+    const int st = launch_i8_realign(plan.a, plan.w, *dev, stream);
+    return st != NNB200_OK ? st : run_gemm_i8(&aligned, dev, stream, copies, ra_done, rw_done);
 }
 
 static bool valid_q4_args(const nnb200_q4_1_args* q)

@@ -1,4 +1,4 @@
-"""A batch of products in one launch: byte for byte against the oracle."""
+"""A batch of products in one launch, and operands off the 16-byte rule: byte for byte against the oracle."""
 import numpy as np
 import pytest
 import torch
@@ -75,3 +75,19 @@ def test_batch_writes_interleaved_outputs(cuda_device, nnb200_lib):
     got = out.cpu().numpy()
     for b in range(6):
         assert np.array_equal(got[:, b], oracle.gemm_i8(a[b], w[b])), b
+
+
+@pytest.mark.parametrize("case", [
+    # k, offset, pose, batch
+    (2049, 0, "nt", 1), (2050, 1, "nt", 1), (2047, 3, "nt", 1), (2052, 13, "nt", 1), (2048, 5, "nt", 1),
+    (2049, 0, "nn", 1), (2053, 0, "tt", 1), (2048, 7, "tn", 1), (700, 0, "nt", 3), (701, 2, "nn", 3)])
+@pytest.mark.parametrize("zero_points", [False, True])
+def test_operands_off_the_tma_rule(cuda_device, nnb200_lib, case, zero_points):
+    """Sizes from which the operands are copied into aligned rows: odd K, odd bases, each pose, batches."""
+    k, offset, pose, batch = case
+    _check(cuda_device, batch, 257, 301, k, pose=pose, offset=offset, zero_points=zero_points, unsigned=k % 2 == 0, seed=k)
+
+
+@pytest.mark.parametrize("m", [1, 7, 17])
+def test_few_rows_off_the_tma_rule(cuda_device, nnb200_lib, m):
+    _check(cuda_device, 1, m, 9001, 1500 if m > 7 else 15001, zero_points=True, seed=m)
