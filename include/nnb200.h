@@ -332,7 +332,9 @@ typedef struct nnb200_q4_1_args {
     size_t workspace_bytes;
     int32_t force_engine; /* 0 auto, 1 fused tensor-core GEMM, 2 GEMV (best), 3 GEMV on CUDA cores, 4 GEMV with
                              warp MMA after per-weight dequantisation, 5 two-pass GEMM (needs the workspace),
-                             6 GEMV with warp MMA on raw nibbles, scale and minimum applied per block afterwards */
+                             6 GEMV with warp MMA on raw nibbles, scale and minimum applied per block afterwards,
+                             7 weights as the 128-row operand in tensor memory (up to 128 f16 or 64 f32 rows,
+                             the latter with the workspace) */
     int32_t flags;        /* NNB200_Q4_FLAG_* */
     /* Prepacked weights (nnb200_q4_1_pack): when w_dm is not NULL, w_blocks points at the nibble
      * plane -- 16 bytes per block, ldw_blocks still counted in blocks -- and w_dm at the plane of

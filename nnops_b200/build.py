@@ -10,6 +10,7 @@ CPU arithmetic bit for bit.
 from __future__ import annotations
 
 import os
+import re
 import subprocess
 import sys
 from concurrent.futures import ThreadPoolExecutor
@@ -21,8 +22,7 @@ LIB_DIR = PKG / "lib"
 LIB = LIB_DIR / "libnnb200.so"
 NVCC = os.environ.get("NNB200_NVCC", "/usr/local/cuda/bin/nvcc")
 
-SOURCES = ["capi.cu", "gemm_i8_umma.cu", "gemm_i8_umma_batched.cu", "i8_realign.cu", "gemm_i8_simt.cu", "gemm_i8_decode.cu", "gemm_i8_skinny.cu", "q4_1_gemv.cu", "q4_1_gemv_mma.cu", "q4_1_gemv_dsq.cu", "q4_1_gemm_umma.cu", "gemm_f16_umma.cu", "shard_gather.cu", "quant_linear.cu", "prepack.cu", "static_scratch.cu", "mma_peak.cu", "conv2d_i8.cu"]
-HEADERS = ["gemm_i8_umma_tile.cuh", "gemm_i8_umma_batched.cuh", "i8_realign.cuh", "ptx.cuh", "ptx_pair.cuh", "epilogue.cuh", "internal.cuh", "q4_1_common.cuh", "../../include/nnb200.h"]
+SOURCES = ["capi.cu", "gemm_i8_umma.cu", "gemm_i8_umma_batched.cu", "i8_realign.cu", "gemm_i8_simt.cu", "gemm_i8_decode.cu", "gemm_i8_skinny.cu", "q4_1_gemv.cu", "q4_1_gemv_mma.cu", "q4_1_gemv_dsq.cu", "q4_1_gemm_umma.cu", "q4_1_rows_umma.cu", "gemm_f16_umma.cu", "shard_gather.cu", "quant_linear.cu", "prepack.cu", "static_scratch.cu", "mma_peak.cu", "conv2d_i8.cu"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -30,6 +30,17 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
     "--expt-relaxed-constexpr",
 ]
+
+
+def _headers(src: Path, seen: set[Path] | None = None) -> set[Path]:
+    """The project headers ``src`` includes, directly or through others."""
+    seen = set() if seen is None else seen
+    for name in re.findall(r'^#include "([^"]+)"', src.read_text(), re.M):
+        h = (src.parent / name).resolve()
+        if h.exists() and h not in seen:
+            seen.add(h)
+            _headers(h, seen)
+    return seen
 
 
 def _stale(out: Path, deps: list[Path]) -> bool:
@@ -43,13 +54,12 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     LIB_DIR.mkdir(exist_ok=True)
     obj_dir = LIB_DIR / "obj"
     obj_dir.mkdir(exist_ok=True)
-    headers = [CSRC / h for h in HEADERS]
     flags = list(NVCC_FLAGS) + (["-Xptxas", "-v"] if verbose else [])
 
     def compile_one(name: str) -> Path:
         src = CSRC / name
         obj = obj_dir / (name + ".o")
-        if force or _stale(obj, [src, *headers]):
+        if force or _stale(obj, [src, *_headers(src)]):
             r = subprocess.run([NVCC, *flags, "-c", str(src), "-o", str(obj)], capture_output=True, text=True)
             if r.returncode != 0:
                 raise RuntimeError(f"nvcc failed on {name}:\n{r.stdout}\n{r.stderr}")

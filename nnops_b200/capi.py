@@ -18,7 +18,7 @@ ACTIVATIONS = {"none": 0, "relu": 1, "gelu": 2, "sigmoid": 3, "tanh": 4, "leaky_
                "hard_swish": 7, "elu": 8, "relu6": 9}
 ENGINES = {"auto": 0, "umma": 1, "narrow": 2, "generic": 3, "decode": 4, "skinny": 5}
 ENGINE_NAMES = {v: k for k, v in ENGINES.items()}
-Q4_ENGINES = {"auto": 0, "gemm": 1, "gemv": 2, "gemv_simt": 3, "gemv_mma": 4, "gemm_two_pass": 5, "gemv_dsq": 6}
+Q4_ENGINES = {"auto": 0, "gemm": 1, "gemv": 2, "gemv_simt": 3, "gemv_mma": 4, "gemm_two_pass": 5, "gemv_dsq": 6, "rows": 7}
 STATIC_SCRATCH_BYTES = 1 << 20
 # Measurement / test switches (NNB200_KNOB_* in nnb200.h); process-wide, negative = default.
 KNOBS = {"group_m": 0, "i8_bn": 1, "i8_pair": 2, "i8_peer_staging": 3, "f16_pair": 4, "i8_share_k": 5, "q4_gemv": 6,

@@ -13,6 +13,7 @@
 #include "i8_realign.cuh"
 #include "internal.cuh"
 #include "ptx.cuh"
+#include "q4_1_rows_umma.cuh"
 
 namespace nnb200 {
 
@@ -734,12 +735,41 @@ static int64_t two_pass_min_rows(const nnb200_q4_1_args* q)
     return q->a_f16 != 0 ? kTwoPassMinRows : kTwoPassMinRowsF32;
 }
 
+// Weights as the 128-row operand in tensor memory (engine 7), for up to 128 rows as the MMA sees them
+// (f32 rows count twice).  CUDA-graph timings, us, that form against the best other one:
+//   N x K          f16 rows 2        8          16         64         128        f32 rows 1   4          16         64
+//   14336 x 4096   15.6 / 20.7  16 / 23.2  16.0 / 50.5  18.3 / 50.5  25.0 / 51.1   17.6 / 14.1  18 / 49   18.2 / 195  27 / 78
+//   4096 x 4096     8.5 / 6.0    9 / 7.6    9.0 / 49.3  11.3 / 49.3  15.6 / 31.0   10.0 / 6.6   10 / 16   10.5 / 65   16 / 53
+//   1024 x 4096     6.7 / 5.1    7 / 5.5    7.0 / 49.0   8.5 / 49.0  11.3 / 26.0    8.2 / 5.0    8 / 11    8.7 / 44   13 / 48
+//   28672 x 8192   46.2 / 57.8  47 / 67.3  46.8 / 142    55 / 186    84 / 188      48.2 / 38.5  48 / 155  48.5 / 621  86 / 275
+//   4096 x 14336   15.8 / 16.7  16 / 21.7  16.5 / 161    19 / 161   27 / 94        17.6 / 19.1  18 / 49   20 / 191   31 / 169
+// One row stays on the GEMV with deferred scaling; so do 2 to 8 f16 (2 f32) rows on the GEMV while the
+// layer is small, where this form's set-up and the exchange between the CTAs of a cluster weigh most.
+static constexpr int64_t kRowsUmmaMaxRows = 128;
+
+static bool q4_1_wants_rows_umma(const nnb200_q4_1_args* q)
+{
+    const int64_t b_rows = q->a_f16 != 0 ? q->m : 2 * q->m;
+    const bool few = q->m <= (q->a_f16 != 0 ? 8 : 2) && static_cast<double>(q->n) * q->k <= static_cast<double>(1 << 25);
+    const bool chosen = q->force_engine == 0 && q->m >= 2 && b_rows <= kRowsUmmaMaxRows && !few;
+    return (chosen || q->force_engine == 7) && q4_1_rows_umma_supported(*q);
+}
+
+// Scratch for f32 activations as pairs of f16 rows.
+static size_t q4_1_rows_scratch_bytes(const nnb200_q4_1_args* q)
+{
+    return static_cast<size_t>(q->m) * static_cast<size_t>(q->k) * 4;
+}
+
 size_t nnb200_q4_1_workspace_bytes(const nnb200_q4_1_args* q)
 {
     if (!valid_q4_args(q) || q->m == 0 || q->n == 0) {
         return 0;
     }
     // Optional: without it a tall call runs the fused kernel.
+    if (q4_1_wants_rows_umma(q)) {
+        return q->a_f16 != 0 ? 0 : q4_1_rows_scratch_bytes(q);
+    }
     const bool wanted = q->force_engine == 5 || (q->force_engine == 0 && q->m >= two_pass_min_rows(q));
     return wanted ? q4_1_two_pass_scratch_bytes(*q) : 0;
 }
@@ -761,6 +791,11 @@ int nnb200_q4_1_engine(const nnb200_q4_1_args* q)
             return q4_1_gemv_dsq_supported(*q) ? 6 : -1;
         }
         return -1;
+    }
+    if (q4_1_wants_rows_umma(q) &&
+        (q->a_f16 != 0 || (q->workspace != nullptr && q->workspace_bytes >= q4_1_rows_scratch_bytes(q) &&
+                           (reinterpret_cast<uintptr_t>(q->workspace) & 15u) == 0))) {
+        return 7;
     }
     // 1 = fused tensor-core GEMM (tcgen05), 3 = GEMV on CUDA cores, 4 = GEMV with warp-level MMA
     // after per-weight dequantisation, 5 = two-pass GEMM (expand to f16 scratch, dense tcgen05
@@ -820,6 +855,18 @@ int nnb200_linear_q4_1(const nnb200_q4_1_args* q, void* stream_v)
     case -1: return NNB200_UNSUPPORTED;   // packed weights in a shape no engine takes them in
     case 1: return launch_q4_1_gemm_umma(*q, *dev, stream);
     case 5: return launch_q4_1_two_pass(*q, *dev, stream);
+    case 7: {
+        Q4RowsCall call{q, q->a, q->lda, false};
+        if (q->a_f16 == 0) {
+            const int st = launch_split_f32_to_f16(static_cast<const float*>(q->a), q->lda, q->m, q->k, q->k, q->workspace,
+                                                   *dev, stream);
+            if (st != NNB200_OK) {
+                return st;
+            }
+            call = Q4RowsCall{q, q->workspace, q->k, true};
+        }
+        return launch_q4_1_rows_umma(call, *dev, stream);
+    }
     case 4: return launch_q4_1_gemv_mma(*q, *dev, stream);
     case 6: return launch_q4_1_gemv_dsq(*q, *dev, stream);
     default: return launch_q4_1_gemv(*q, *dev, stream);

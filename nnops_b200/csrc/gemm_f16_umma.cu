@@ -36,6 +36,7 @@
 #include "ptx.cuh"
 #include "ptx_pair.cuh"
 #include "q4_1_common.cuh"
+#include "q4_1_rows_umma.cuh"
 
 namespace nnb200 {
 
@@ -809,6 +810,17 @@ bool q4_1_two_pass_supported(const nnb200_q4_1_args& q)
            q.workspace_bytes >= q4_1_two_pass_scratch_bytes(q);
 }
 
+int launch_split_f32_to_f16(const float* a, int64_t lda, int64_t m, int64_t k, int64_t kp, void* out, const DeviceInfo& dev,
+                            cudaStream_t stream)
+{
+    const int64_t want = (m * kp + 255) / 256;
+    const int64_t cap = static_cast<int64_t>(dev.sm_count) * 16;
+    split_f32_to_f16_kernel<<<static_cast<unsigned>(want < cap ? want : cap), 256, 0, stream>>>(
+        a, lda, static_cast<int>(m), static_cast<int>(k), static_cast<int>(kp), static_cast<__half*>(out));
+    note_launch();
+    return cuda_status(cudaGetLastError());
+}
+
 int launch_q4_1_two_pass(const nnb200_q4_1_args& q, const DeviceInfo& dev, cudaStream_t stream)
 {
     FpEpilogue ep;
@@ -848,14 +860,9 @@ int launch_q4_1_two_pass(const nnb200_q4_1_args& q, const DeviceInfo& dev, cudaS
     } else {
         const int kp = static_cast<int>((q.k + 63) / 64 * 64);
         __half* a16 = reinterpret_cast<__half*>(static_cast<uint8_t*>(q.workspace) + weights_scratch_bytes(q));
-        const int64_t total = q.m * kp;
-        const int64_t want = (total + 255) / 256;
-        const int64_t cap = static_cast<int64_t>(dev.sm_count) * 16;
-        split_f32_to_f16_kernel<<<static_cast<unsigned>(want < cap ? want : cap), 256, 0, stream>>>(
-            static_cast<const float*>(q.a), q.lda, static_cast<int>(q.m), static_cast<int>(q.k), kp, a16);
-        note_launch();
-        if (cudaGetLastError() != cudaSuccess) {
-            return NNB200_INTERNAL;
+        const int st = launch_split_f32_to_f16(static_cast<const float*>(q.a), q.lda, q.m, q.k, kp, a16, dev, stream);
+        if (st != NNB200_OK) {
+            return st;
         }
         op.a = a16;
         op.lda = 2 * static_cast<int64_t>(kp);

@@ -262,7 +262,8 @@ def linear_q4_1(a: torch.Tensor, w_blocks: torch.Tensor, k: int, *, out_dtype: t
 def q4_1_engine(a: torch.Tensor, w_blocks: torch.Tensor, k: int, *, out_dtype: torch.dtype = torch.float32,
                 engine: str = "auto") -> int:
     """Engine code nnb200_linear_q4_1 would pick (1 fused GEMM, 3 GEMV on CUDA cores, 4 GEMV with warp
-    MMA, 5 two-pass GEMM) when given the scratch it asks for."""
+    MMA, 5 two-pass GEMM, 6 GEMV with deferred scaling, 7 weights in tensor memory) when given the
+    scratch it asks for."""
     n_out = w_blocks.n if isinstance(w_blocks, PackedQ41) else w_blocks.shape[0]
     out = torch.empty((a.shape[0], n_out), dtype=out_dtype, device=a.device)
     args = q4_1_args(a, w_blocks, out, k, engine=engine)

@@ -1,0 +1,72 @@
+"""Q4_1 weights as the 128-row operand in tensor memory, a few to 128 activation rows, against the oracle."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from nnops_b200 import ops, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(device, m, n, k, a_dtype, out_dtype, **kw):
+    rng = np.random.default_rng(m * 7 + n + k)
+    wb = synth.q4_1_weights(rng, n, k)
+    a = rng.standard_normal((m, k)).astype(a_dtype)
+    want = oracle.q4_1_matmul(a.astype(np.float32), wb, k, out_dtype="f32", w_round_f16=True).astype(np.float64)
+    ta, tw = torch.from_numpy(a).to(device), torch.from_numpy(wb).to(device)
+    got = [ops.linear_q4_1(ta, tw, k, out_dtype=out_dtype, engine="rows", **kw).cpu().numpy().astype(np.float64) for _ in range(2)]
+    assert np.array_equal(got[0], got[1])   # a fixed order of additions
+    # Weights rounded to f16 on both sides and exact products: what is left is the order of f32 sums
+    # (sqrt(K) roundings of 2^-24 of the running sum, K up to 8320), the remainder of an f32
+    # activation's two f16 parts (2^-22) and the f16 result's own rounding (2^-11).
+    rms = float(np.sqrt(np.mean(want ** 2)))
+    tol = 2e-5 * (rms + np.abs(want)) + (2.0 ** -11 * np.abs(want) + 2.0 ** -25 if out_dtype == torch.float16 else 0.0)
+    assert (np.abs(got[0] - want) <= tol).all(), float((np.abs(got[0] - want) - tol).max())
+
+
+@pytest.mark.parametrize("shape", [
+    # m, n, k: K of half a unit, clusters that share K (few channels), whole waves, several tiles a CTA
+    (2, 128, 128), (16, 1, 256), (9, 130, 384), (5, 1000, 2048), (17, 4096, 1152), (33, 129, 8320), (16, 9500, 640),
+    (64, 14336, 512), (65, 1000, 384), (128, 300, 4096), (100, 19000, 256), (3, 45000, 128), (7, 40000, 1152)])
+@pytest.mark.parametrize("out_dtype", [torch.float16, torch.float32])
+def test_rows_f16(cuda_device, nnb200_lib, shape, out_dtype):
+    _check(cuda_device, *shape, np.float16, out_dtype)
+
+
+@pytest.mark.parametrize("shape", [(1, 300, 256), (2, 1000, 2048), (8, 9500, 640), (9, 4096, 1152), (33, 130, 384), (64, 260, 4096),
+                                   (50, 19000, 256)])
+@pytest.mark.parametrize("out_dtype", [torch.float16, torch.float32])
+def test_rows_f32(cuda_device, nnb200_lib, shape, out_dtype):
+    _check(cuda_device, *shape, np.float32, out_dtype)
+
+
+@pytest.mark.parametrize("n", [1000, 9500])
+@pytest.mark.parametrize("act", ["none", "silu", "gelu"])
+def test_rows_epilogue(cuda_device, nnb200_lib, n, act):
+    """alpha, bias, clip and activation, with and without a split of K: the same engine's plain product, finished in f64."""
+    rng = np.random.default_rng(n)
+    m, k = 18, 768
+    wb = torch.from_numpy(synth.q4_1_weights(rng, n, k)).to(cuda_device)
+    a = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float16)).to(cuda_device)
+    bias = rng.standard_normal(n).astype(np.float32)
+    plain = ops.linear_q4_1(a, wb, k, out_dtype=torch.float32, engine="rows").double().cpu()
+    x = (plain * 0.5 + torch.from_numpy(bias).double()).clamp(-1.5, 2.0)
+    want = {"none": lambda v: v, "silu": torch.nn.functional.silu,
+            "gelu": lambda v: torch.nn.functional.gelu(v, approximate="tanh")}[act](x).numpy()
+    got = ops.linear_q4_1(a, wb, k, out_dtype=torch.float32, engine="rows", alpha=0.5, bias=bias, min_clip=-1.5, max_clip=2.0,
+                          activation=act).cpu().numpy()
+    assert np.abs(got - want).max() <= 2e-6 * 4
+
+
+def test_rows_pitched_and_chosen_by_itself(cuda_device, nnb200_lib):
+    """Pitched activations and outputs; the automatic choice from two rows up."""
+    rng = np.random.default_rng(1)
+    m, n, k = 20, 700, 512
+    wb = torch.from_numpy(synth.q4_1_weights(rng, n, k)).to(cuda_device)
+    a = torch.from_numpy(rng.standard_normal((m, k + 40)).astype(np.float16)).to(cuda_device)[:, 8:8 + k]
+    assert ops.q4_1_engine(a, wb, k, out_dtype=torch.float16) == 7
+    out = torch.full((m, n + 24), 7.0, dtype=torch.float16, device=cuda_device)
+    ops.linear_q4_1(a, wb, k, out=out[:, 8:8 + n])
+    assert torch.equal(out[:, 8:8 + n], ops.linear_q4_1(a.contiguous(), wb, k, engine="rows"))
+    assert (out[:, :8] == 7).all() and (out[:, 8 + n:] == 7).all()
