@@ -6,6 +6,7 @@ fallback for any call here.
 from __future__ import annotations
 
 import ctypes as C
+import struct
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -113,6 +114,26 @@ class Conv2dI8Args(C.Structure):
         ("zp_w_nonzero", C.c_int32), ("out_scale", C.c_float), ("out_zp", C.c_int32),
         ("workspace", C.c_void_p), ("workspace_bytes", C.c_size_t),
     ]
+
+
+_FORMATS = {C.c_void_p: "P", C.c_int64: "q", C.c_int32: "i", C.c_float: "f", C.c_size_t: "N"}
+_packers: dict = {}
+
+
+def block(cls, *values):
+    """An argument block from its leading fields' values in order (0 for a null pointer), the rest zero.
+
+    One packing call: assigning fifty ctypes fields one by one costs more than enqueueing the call."""
+    pack = _packers.get((cls, len(values)))
+    if pack is None:
+        fmt = "".join(_FORMATS[t] for _, t in cls._fields_[:len(values)])
+        pack = _packers[(cls, len(values))] = struct.Struct(f"@{fmt}").pack_into
+    args = cls()
+    try:
+        pack(args, 0, *values)
+    except (struct.error, OverflowError):   # a number outside its field: ctypes' own conversion
+        args = cls(*values)
+    return args
 
 
 SYMBOLS = [

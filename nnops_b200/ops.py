@@ -13,8 +13,26 @@ from . import capi
 _OUT_TORCH = {"s32": torch.int32, "s8": torch.int8, "u8": torch.uint8, "f32": torch.float32, "f16": torch.float16}
 
 
+def _call(fn, args, device: torch.device, what: str) -> None:
+    """Enqueue one library call on ``device``'s current stream."""
+    if torch.cuda.current_device() == device.index:
+        status = fn(C.byref(args), torch.cuda.current_stream().cuda_stream)
+    else:
+        with torch.cuda.device(device):
+            status = fn(C.byref(args), torch.cuda.current_stream().cuda_stream)
+    if status != capi.OK:
+        capi.check(status, what)
+
+
 def _stream_ptr(device: torch.device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
+
+
+def _on_device(v, dtype: torch.dtype, device: torch.device) -> torch.Tensor:
+    """``v`` as a contiguous tensor of that type on that device; itself when it is one already."""
+    if isinstance(v, torch.Tensor) and v.dtype is dtype and v.device == device and v.is_contiguous():
+        return v
+    return torch.as_tensor(v).to(device=device, dtype=dtype).contiguous()
 
 
 def _dev_array(v, dtype: torch.dtype, device: torch.device, count: int | None):
@@ -23,7 +41,9 @@ def _dev_array(v, dtype: torch.dtype, device: torch.device, count: int | None):
         return None, None
     if isinstance(v, (int, float)):
         return None, v
-    t = torch.as_tensor(v, dtype=dtype).to(device).contiguous()
+    if not isinstance(v, torch.Tensor):
+        v = torch.as_tensor(v, dtype=dtype)
+    t = _on_device(v, dtype, device)
     if count is not None and t.numel() != count:
         raise ValueError(f"expected {count} quantization entries, got {t.numel()}")
     return t, None
@@ -39,14 +59,10 @@ def gemm_i8_args(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, out_kin
     Tensors created for quantization arrays are appended to ``keep`` so they outlive the call."""
     keep = keep if keep is not None else []
     dev = a.device
-    batched = a.dim() == 3 or w.dim() == 3
-    a3 = a if a.dim() == 3 else a.unsqueeze(0)
-    w3 = w if w.dim() == 3 else w.unsqueeze(0)
-    o3 = out if out.dim() == 3 else out.unsqueeze(0)
-    batch = max(a3.shape[0], w3.shape[0]) if batched else 1
-    m, k = a3.shape[1], a3.shape[2]
-    n = w3.shape[1]
-    if w3.shape[2] != k:
+    a_batch, w_batch, o_batch = (t.shape[0] if t.dim() == 3 else 1 for t in (a, w, out))
+    m, k = a.shape[-2:]
+    n = w.shape[-2]
+    if w.shape[-1] != k:
         raise ValueError("K mismatch")
     sa, sa0 = _dev_array(scale_a, torch.float32, dev, m)
     sw, sw0 = _dev_array(scale_w, torch.float32, dev, n)
@@ -54,36 +70,27 @@ def gemm_i8_args(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, out_kin
     zw, zw0 = _dev_array(zp_w, torch.int32, dev, n)
     keep.extend(t for t in (sa, sw, za, zw) if t is not None)
     if bias is not None:
-        bdt = torch.int32 if out_kind in ("s32", "s8", "u8") else _OUT_TORCH[out_kind]
-        bias = torch.as_tensor(bias).to(device=dev, dtype=bdt).contiguous()
+        bias = _on_device(bias, torch.int32 if out_kind in ("s32", "s8", "u8") else _OUT_TORCH[out_kind], dev)
         keep.append(bias)
 
-    def stride_or_one(t, dim, size):
-        return t.stride(dim) if size > 1 else (1 if dim == 2 else t.stride(dim))
-
-    args = capi.GemmI8Args(
-        a=a3.data_ptr(), w=w3.data_ptr(), out=o3.data_ptr(), m=m, n=n, k=k,
-        a_stride_m=a3.stride(1), a_stride_k=stride_or_one(a3, 2, k),
-        w_stride_n=w3.stride(1), w_stride_k=stride_or_one(w3, 2, k),
-        ldc=o3.stride(1), batch=batch,
-        a_batch_stride=a3.stride(0) if a3.shape[0] > 1 else 0,
-        w_batch_stride=w3.stride(0) if w3.shape[0] > 1 else 0,
-        out_batch_stride=o3.stride(0) if o3.shape[0] > 1 else 0,
-        a_unsigned=int(a.dtype == torch.uint8), out_kind=capi.OUT_KINDS[out_kind],
-        bias=bias.data_ptr() if bias is not None else None,
-        relu=int(bool(relu)), activation=capi.ACTIVATIONS[activation],
-        act_alpha=act_alpha, act_beta=act_beta, min_clip=min_clip, max_clip=max_clip,
-        scale_a=sa.data_ptr() if sa is not None else None,
-        scale_w=sw.data_ptr() if sw is not None else None,
-        zp_a=za.data_ptr() if za is not None else None,
-        zp_w=zw.data_ptr() if zw is not None else None,
-        scale_a_scalar=1.0 if sa0 is None else float(sa0), scale_w_scalar=1.0 if sw0 is None else float(sw0),
-        zp_a_scalar=0 if za0 is None else int(za0), zp_w_scalar=0 if zw0 is None else int(zw0),
-        zp_a_nonzero=int(za is not None and bool((za != 0).any().item())),
-        zp_w_nonzero=int(zw is not None and bool((zw != 0).any().item())),
-        out_scale=float(out_scale), out_zp=int(out_zp),
-        workspace=None, workspace_bytes=0, force_engine=capi.ENGINES[engine],
-        r_w=r_w.data_ptr() if r_w is not None else None)
+    # Whether an ARRAY of zero points holds anything but zeros is not looked at: that would wait for
+    # the device on every call, and only to save the row sums.
+    args = capi.block(
+        capi.GemmI8Args, a.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k,
+        a.stride(-2), a.stride(-1) if k > 1 else 1, w.stride(-2), w.stride(-1) if k > 1 else 1, out.stride(-2),
+        max(a_batch, w_batch), a.stride(0) if a_batch > 1 else 0, w.stride(0) if w_batch > 1 else 0,
+        out.stride(0) if o_batch > 1 else 0,
+        int(a.dtype == torch.uint8), capi.OUT_KINDS[out_kind], bias.data_ptr() if bias is not None else 0,
+        int(bool(relu)), capi.ACTIVATIONS[activation], act_alpha, act_beta, min_clip, max_clip,
+        sa.data_ptr() if sa is not None else 0, sw.data_ptr() if sw is not None else 0,
+        za.data_ptr() if za is not None else 0, zw.data_ptr() if zw is not None else 0,
+        1.0 if sa0 is None else float(sa0), 1.0 if sw0 is None else float(sw0),
+        0 if za0 is None else int(za0), 0 if zw0 is None else int(zw0), int(za is not None), int(zw is not None),
+        float(out_scale), int(out_zp))
+    if engine != "auto":
+        args.force_engine = capi.ENGINES[engine]
+    if r_w is not None:
+        args.r_w = r_w.data_ptr()
     # min_workspace: only what the call cannot do without (no scratch for sharing K among SMs).
     size_fn = capi.lib().nnb200_gemm_i8_min_workspace_bytes if min_workspace else capi.lib().nnb200_gemm_i8_workspace_bytes
     need = size_fn(C.byref(args))
@@ -108,8 +115,7 @@ def gemm_i8(a: torch.Tensor, w: torch.Tensor, *, out_kind: str = "s32", out: tor
         out = torch.empty(shape, dtype=_OUT_TORCH[out_kind], device=a.device)
     keep: list = []
     args = gemm_i8_args(a, w, out, out_kind=out_kind, keep=keep, **kw)
-    with torch.cuda.device(a.device):
-        capi.check(capi.lib().nnb200_gemm_i8(C.byref(args), _stream_ptr(a.device)), "nnb200_gemm_i8")
+    _call(capi.lib().nnb200_gemm_i8, args, a.device, "nnb200_gemm_i8")
     return out
 
 
@@ -203,35 +209,25 @@ def q4_1_args(a: torch.Tensor, w_blocks, out: torch.Tensor, k: int, *, bias=None
               overlap_previous: bool = False, keep: list | None = None) -> capi.Q41Args:
     """``w_blocks``: raw rows (uint8 [N, ceil(K/32)*20]) or a PackedQ41."""
     keep = keep if keep is not None else []
-    if isinstance(w_blocks, PackedQ41):
-        pk = w_blocks
+    packed = isinstance(w_blocks, PackedQ41)
+    if packed:
         if a.stride(1) != 1 or out.stride(1) != 1:
             raise ValueError("activations and output must be row-major")
-        if bias is not None:
-            bias = torch.as_tensor(bias).to(device=a.device, dtype=out.dtype).contiguous()
-            keep.append(bias)
-        return capi.Q41Args(
-            a=a.data_ptr(), w_blocks=pk.qs_ptr, out=out.data_ptr(), m=a.shape[0], n=pk.n, k=k, lda=a.stride(0),
-            ldw_blocks=pk.qs_pitch, ldc=out.stride(0), a_f16=int(a.dtype == torch.float16),
-            out_f16=int(out.dtype == torch.float16), bias=bias.data_ptr() if bias is not None else None,
-            activation=capi.ACTIVATIONS[activation], act_alpha=act_alpha, act_beta=act_beta, min_clip=min_clip,
-            max_clip=max_clip, alpha=alpha, workspace=None, workspace_bytes=0, force_engine=capi.Q4_ENGINES[engine],
-            flags=capi.Q4_FLAG_OVERLAP_PREVIOUS if overlap_previous else 0, w_dm=pk.dm_ptr, ld_dm=pk.dm_pitch)
-    if w_blocks.dtype != torch.uint8 or w_blocks.dim() != 2 or w_blocks.stride(1) != 1 or w_blocks.stride(0) % 20:
-        raise ValueError("w_blocks must be a uint8 [N, row_bytes] tensor whose row pitch is a multiple of 20")
-    if a.stride(1) != 1 or out.stride(1) != 1:
-        raise ValueError("activations and output must be row-major")
+        w_ptr, n, ldw, dm_ptr, ld_dm = w_blocks.qs_ptr, w_blocks.n, w_blocks.qs_pitch, w_blocks.dm_ptr, w_blocks.dm_pitch
+    else:
+        if w_blocks.dtype != torch.uint8 or w_blocks.dim() != 2 or w_blocks.stride(1) != 1 or w_blocks.stride(0) % 20:
+            raise ValueError("w_blocks must be a uint8 [N, row_bytes] tensor whose row pitch is a multiple of 20")
+        if a.stride(1) != 1 or out.stride(1) != 1:
+            raise ValueError("activations and output must be row-major")
+        w_ptr, n, ldw, dm_ptr, ld_dm = w_blocks.data_ptr(), w_blocks.shape[0], w_blocks.stride(0) // 20, 0, 0
     if bias is not None:
-        bias = torch.as_tensor(bias).to(device=a.device, dtype=out.dtype).contiguous()
+        bias = _on_device(bias, out.dtype, a.device)
         keep.append(bias)
-    return capi.Q41Args(
-        a=a.data_ptr(), w_blocks=w_blocks.data_ptr(), out=out.data_ptr(),
-        m=a.shape[0], n=w_blocks.shape[0], k=k, lda=a.stride(0), ldw_blocks=w_blocks.stride(0) // 20,
-        ldc=out.stride(0), a_f16=int(a.dtype == torch.float16), out_f16=int(out.dtype == torch.float16),
-        bias=bias.data_ptr() if bias is not None else None, activation=capi.ACTIVATIONS[activation],
-        act_alpha=act_alpha, act_beta=act_beta, min_clip=min_clip, max_clip=max_clip, alpha=alpha,
-        workspace=None, workspace_bytes=0, force_engine=capi.Q4_ENGINES[engine],
-        flags=capi.Q4_FLAG_OVERLAP_PREVIOUS if overlap_previous else 0)
+    return capi.block(
+        capi.Q41Args, a.data_ptr(), w_ptr, out.data_ptr(), a.shape[0], n, k, a.stride(0), ldw, out.stride(0),
+        int(a.dtype == torch.float16), int(out.dtype == torch.float16), bias.data_ptr() if bias is not None else 0,
+        capi.ACTIVATIONS[activation], act_alpha, act_beta, min_clip, max_clip, alpha, 0, 0, capi.Q4_ENGINES[engine],
+        capi.Q4_FLAG_OVERLAP_PREVIOUS if overlap_previous else 0, dm_ptr, ld_dm)
 
 
 def linear_q4_1(a: torch.Tensor, w_blocks: torch.Tensor, k: int, *, out_dtype: torch.dtype | None = None,
@@ -246,7 +242,8 @@ def linear_q4_1(a: torch.Tensor, w_blocks: torch.Tensor, k: int, *, out_dtype: t
         out = torch.empty((a.shape[0], n_out), dtype=out_dtype or a.dtype, device=a.device)
     keep: list = []
     args = q4_1_args(a, w_blocks, out, k, keep=keep, **kw)
-    need = capi.lib().nnb200_q4_1_workspace_bytes(C.byref(args))
+    lib = capi.lib()
+    need = lib.nnb200_q4_1_workspace_bytes(C.byref(args))
     if need > 0:
         # Scratch for the expanded weights of the two-pass form; torch's allocator is
         # stream-ordered, so letting it go after the call is safe.
@@ -254,8 +251,7 @@ def linear_q4_1(a: torch.Tensor, w_blocks: torch.Tensor, k: int, *, out_dtype: t
         keep.append(scratch)
         args.workspace = scratch.data_ptr()
         args.workspace_bytes = need
-    with torch.cuda.device(a.device):
-        capi.check(capi.lib().nnb200_linear_q4_1(C.byref(args), _stream_ptr(a.device)), "nnb200_linear_q4_1")
+    _call(lib.nnb200_linear_q4_1, args, a.device, "nnb200_linear_q4_1")
     return out
 
 
@@ -298,8 +294,9 @@ def _quant_view(shape, axis: int, param_count: int) -> tuple[int, int, int]:
 
 
 def _quant_params(scale, zero_point, device):
-    scale = torch.as_tensor(scale, dtype=torch.float32).reshape(-1).to(device).contiguous()
-    zero_point = torch.as_tensor(zero_point).reshape(-1).to(device).contiguous()
+    scale = _on_device(torch.as_tensor(scale, dtype=torch.float32), torch.float32, device).reshape(-1)
+    zero_point = torch.as_tensor(zero_point)
+    zero_point = _on_device(zero_point, zero_point.dtype, device).reshape(-1)
     if zero_point.dtype not in (torch.int8, torch.uint8) or zero_point.numel() != scale.numel():
         raise ValueError("zero_point must be int8/uint8 with one entry per scale")
     return scale, zero_point
@@ -315,12 +312,10 @@ def quantize_linear(x: torch.Tensor, scale, zero_point, *, axis: int = -1, out_d
     outer, rows, inner = _quant_view(x.shape, axis, scale.numel())
     if rows != scale.numel():
         raise ValueError("scale count does not match the tensor and axis")
-    args = capi.QuantLinearArgs(x=x.data_ptr(), y=y.data_ptr(), outer=outer, rows=rows, inner=inner,
-                                scale=scale.data_ptr(), zero_point=zero_point.data_ptr(),
-                                zp_unsigned=int(zero_point.dtype == torch.uint8),
-                                float_f16=int(x.dtype == torch.float16), int_unsigned=int(y.dtype == torch.uint8))
-    with torch.cuda.device(x.device):
-        capi.check(capi.lib().nnb200_quantize_linear(C.byref(args), _stream_ptr(x.device)), "nnb200_quantize_linear")
+    args = capi.block(capi.QuantLinearArgs, x.data_ptr(), y.data_ptr(), outer, rows, inner, scale.data_ptr(),
+                      zero_point.data_ptr(), int(zero_point.dtype == torch.uint8), int(x.dtype == torch.float16),
+                      int(y.dtype == torch.uint8))
+    _call(capi.lib().nnb200_quantize_linear, args, x.device, "nnb200_quantize_linear")
     return y
 
 
@@ -334,13 +329,10 @@ def dequantize_linear(x: torch.Tensor, scale, zero_point, *, axis: int = -1, out
     outer, rows, inner = _quant_view(x.shape, axis, scale.numel())
     if rows != scale.numel():
         raise ValueError("scale count does not match the tensor and axis")
-    args = capi.QuantLinearArgs(x=x.data_ptr(), y=y.data_ptr(), outer=outer, rows=rows, inner=inner,
-                                scale=scale.data_ptr(), zero_point=zero_point.data_ptr(),
-                                zp_unsigned=int(zero_point.dtype == torch.uint8),
-                                float_f16=int(y.dtype == torch.float16), int_unsigned=int(x.dtype == torch.uint8))
-    with torch.cuda.device(x.device):
-        capi.check(capi.lib().nnb200_dequantize_linear(C.byref(args), _stream_ptr(x.device)),
-                   "nnb200_dequantize_linear")
+    args = capi.block(capi.QuantLinearArgs, x.data_ptr(), y.data_ptr(), outer, rows, inner, scale.data_ptr(),
+                      zero_point.data_ptr(), int(zero_point.dtype == torch.uint8), int(y.dtype == torch.float16),
+                      int(x.dtype == torch.uint8))
+    _call(capi.lib().nnb200_dequantize_linear, args, x.device, "nnb200_dequantize_linear")
     return y
 
 
@@ -354,18 +346,24 @@ def linear_fp_act(a: torch.Tensor, w: torch.Tensor, *, scale_a, zp_a=0, act_dtyp
     m, k = a.shape
     per_token = not (isinstance(scale_a, (int, float)) and isinstance(zp_a, int))
     count = m if per_token else 1
-    scale = torch.as_tensor(scale_a, dtype=torch.float32).reshape(-1).to(a.device).expand(count).contiguous()
-    zp = torch.as_tensor(zp_a, dtype=torch.int32).reshape(-1).to(a.device).expand(count).contiguous()
-    aq = torch.empty((m, k), dtype=act_dtype, device=a.device)
+    dev = a.device
+
+    def spread(v, dtype):
+        """One entry per row (or one): scalars are filled in on the device, nothing waits for a copy."""
+        if isinstance(v, (int, float)):
+            return torch.full((count,), v, dtype=dtype, device=dev)
+        return _on_device(torch.as_tensor(v, dtype=dtype).reshape(-1).to(dev).expand(count), dtype, dev)
+
+    scale, zp = spread(scale_a, torch.float32), spread(zp_a, torch.int32)
+    aq = torch.empty((m, k), dtype=act_dtype, device=dev)
     outer, rows, inner = (1, m, k) if per_token else (1, 1, m * k)
-    args = capi.QuantLinearArgs(x=a.data_ptr(), y=aq.data_ptr(), outer=outer, rows=rows, inner=inner,
-                                scale=scale.data_ptr(), zero_point=zp.data_ptr(), zp_unsigned=capi.ZP_S32,
-                                float_f16=int(a.dtype == torch.float16), int_unsigned=int(act_dtype == torch.uint8))
-    with torch.cuda.device(a.device):
-        capi.check(capi.lib().nnb200_quantize_linear(C.byref(args), _stream_ptr(a.device)), "nnb200_quantize_linear")
+    args = capi.block(capi.QuantLinearArgs, a.data_ptr(), aq.data_ptr(), outer, rows, inner, scale.data_ptr(), zp.data_ptr(),
+                      capi.ZP_S32, int(a.dtype == torch.float16), int(act_dtype == torch.uint8))
+    _call(capi.lib().nnb200_quantize_linear, args, dev, "nnb200_quantize_linear")
     out_kind = "f32" if a.dtype == torch.float32 else "f16"
+    # A scalar zero point stays one: an array would ask for the weight's row sums even if it holds zeros.
     return gemm_i8(aq, w, out_kind=out_kind, scale_a=scale if per_token else float(scale_a),
-                   zp_a=zp if per_token else int(zp_a), **kw)
+                   zp_a=int(zp_a) if isinstance(zp_a, int) else zp, **kw)
 
 
 class PackedConvI8:
@@ -417,24 +415,16 @@ def conv2d_i8(x: torch.Tensor, w, *, stride=(1, 1), dilation=(1, 1), padding=(0,
     sw, sw0 = _dev_array(scale_w, torch.float32, dev, oc)
     zw, zw0 = _dev_array(zp_w, torch.int32, dev, oc)
     if bias is not None:
-        bdt = torch.int32 if out_kind in ("s8", "u8") else _OUT_TORCH[out_kind]
-        bias = torch.as_tensor(bias).to(device=dev, dtype=bdt).contiguous()
-    args = capi.Conv2dI8Args(
-        input=x.data_ptr(), weight=w.blob.data_ptr() if packed else w.data_ptr(), out=out.data_ptr(),
-        batch=n, ih=ih, iw=iw, ic=ic, oh=oh, ow=ow, oc=oc, kh=kh, kw=kw, stride_h=stride[0], stride_w=stride[1],
-        dil_h=dilation[0], dil_w=dilation[1], pad_h=padding[0], pad_w=padding[1], groups=groups,
-        in_stride_n=x.stride(0), in_stride_h=x.stride(1), in_stride_w=x.stride(2), in_stride_c=x.stride(3),
-        w_stride_kh=0 if packed else w.stride(0), w_stride_kw=0 if packed else w.stride(1),
-        w_stride_ic=0 if packed else w.stride(2), w_stride_oc=0 if packed else w.stride(3),
-        out_stride_n=out.stride(0), out_stride_h=out.stride(1), out_stride_w=out.stride(2),
-        weight_packed=int(packed), a_unsigned=int(x.dtype == torch.uint8), out_kind=capi.OUT_KINDS[out_kind],
-        bias=bias.data_ptr() if bias is not None else None, relu=int(bool(relu)),
-        activation=capi.ACTIVATIONS[activation], act_alpha=act_alpha, act_beta=act_beta, min_clip=min_clip,
-        max_clip=max_clip, scale_w=sw.data_ptr() if sw is not None else None,
-        zp_w=zw.data_ptr() if zw is not None else None, scale_x=float(scale_x),
-        scale_w_scalar=1.0 if sw0 is None else float(sw0), zp_x=int(zp_x), zp_w_scalar=0 if zw0 is None else int(zw0),
-        zp_w_nonzero=int(zw is not None and bool((zw != 0).any().item())), out_scale=float(out_scale),
-        out_zp=int(out_zp), workspace=None, workspace_bytes=0)
+        bias = _on_device(bias, torch.int32 if out_kind in ("s8", "u8") else _OUT_TORCH[out_kind], dev)
+    args = capi.block(
+        capi.Conv2dI8Args, x.data_ptr(), w.blob.data_ptr() if packed else w.data_ptr(), out.data_ptr(),
+        n, ih, iw, ic, oh, ow, oc, kh, kw, *stride, *dilation, *padding, groups, *x.stride(),
+        *((0, 0, 0, 0) if packed else w.stride()), *out.stride()[:3],
+        int(packed), int(x.dtype == torch.uint8), capi.OUT_KINDS[out_kind],
+        bias.data_ptr() if bias is not None else 0, int(bool(relu)), capi.ACTIVATIONS[activation],
+        act_alpha, act_beta, min_clip, max_clip, sw.data_ptr() if sw is not None else 0,
+        zw.data_ptr() if zw is not None else 0, float(scale_x), 1.0 if sw0 is None else float(sw0), int(zp_x),
+        0 if zw0 is None else int(zw0), int(zw is not None and bool((zw != 0).any().item())), float(out_scale), int(out_zp))
     need = capi.lib().nnb200_conv2d_i8_workspace_bytes(C.byref(args))
     if need:
         if workspace is None or workspace.numel() < need:
@@ -442,6 +432,5 @@ def conv2d_i8(x: torch.Tensor, w, *, stride=(1, 1), dilation=(1, 1), padding=(0,
         keep.append(workspace)
         args.workspace = workspace.data_ptr()
         args.workspace_bytes = workspace.numel()
-    with torch.cuda.device(dev):
-        capi.check(capi.lib().nnb200_conv2d_i8(C.byref(args), _stream_ptr(dev)), "nnb200_conv2d_i8")
+    _call(capi.lib().nnb200_conv2d_i8, args, dev, "nnb200_conv2d_i8")
     return out
