@@ -19,6 +19,11 @@
 // accumulators, bounded waits) except that each accumulator has its own four epilogue warps;
 // same epilogue arithmetic (epilogue.cuh): results are bit-identical to every other int8 engine.
 //
+// Tiles need not be 128 channels high: without shared K a layer of several waves of tiles is cut into
+// equal ones (N = 28672 on 148 SMs: 296 tiles of 97 channels instead of 224 of 128), so that every SM
+// streams the same bytes; the rows of the MMA past a tile's channels hold whatever the ring held
+// before, and nobody reads their accumulators.
+//
 // Work split.  The unit of work is one 128-byte K block of one tile; tile t owns units
 // [t * num_kb, (t + 1) * num_kb).  Every CTA takes one contiguous range of units:
 //   * whole tiles only (CTA c gets tiles [c T / G, (c + 1) T / G)) when no scratch is given;
@@ -209,7 +214,7 @@ __global__ void __launch_bounds__(kNumThreads, 1)
 gemm_i8_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
                       const I8Epilogue ep, const int m_total, const int n_total, const int k_total,
                       const uint32_t idesc, int32_t* error_word, unsigned long long* split_counters,
-                      int32_t* split_slots, const unsigned long long split_tag)
+                      int32_t* split_slots, const unsigned long long split_tag, const int tile_rows)
 {
     using Cfg = SkinnyConfig<MP>;
     constexpr int kStages = Cfg::kStages;
@@ -226,8 +231,9 @@ gemm_i8_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5;
+    const int role = __shfl_sync(0xFFFFFFFFu, warp, 0);   // the same, warp-uniform to the compiler too
     const int lane = threadIdx.x & 31;
-    const int num_tiles = (n_total + kBlockN - 1) / kBlockN;
+    const int num_tiles = (n_total + tile_rows - 1) / tile_rows;
     const int num_kb = (k_total + kBlockKBytes - 1) / kBlockKBytes;
     const bool split = split_counters != nullptr;
     const int grid = static_cast<int>(gridDim.x);
@@ -268,7 +274,7 @@ gemm_i8_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (warp == 0) {
+    if (role == 0) {
         // ---------------- TMA producer ----------------
         if (lane == 0) {
             int stage = 0;
@@ -287,8 +293,8 @@ gemm_i8_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                     }
                     uint8_t* w_dst = stage_base + stage * Cfg::kStageBytes;
                     uint8_t* a_dst = w_dst + Cfg::kWTileBytes;
-                    mbar_expect_tx(&full_bar[stage], Cfg::kStageBytes);
-                    tma_load_2d(w_dst, &map_w, &full_bar[stage], kb * kBlockKBytes, tile * kBlockN);
+                    mbar_expect_tx(&full_bar[stage], static_cast<uint32_t>(tile_rows * kBlockKBytes + Cfg::kATileBytes));
+                    tma_load_2d(w_dst, &map_w, &full_bar[stage], kb * kBlockKBytes, tile * tile_rows);
                     tma_load_2d(a_dst, &map_a, &full_bar[stage], kb * kBlockKBytes, 0);
                     armed |= 1u << stage;
                     armed_phase = (armed_phase & ~(1u << stage)) | (phase << stage);
@@ -314,47 +320,55 @@ gemm_i8_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             }
         }
         __syncwarp();
-    } else if (warp == 1) {
+    } else if (role == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            int stage = 0;
-            uint32_t phase = 0;
-            int local_seg = 0;
-            bool ok = true;
-            for (; ok && local_seg < num_segments; ++local_seg) {
-                const Segment seg = segments.at(local_seg);
-                const int acc = local_seg & 1;
-                const uint32_t acc_phase = (local_seg >> 1) & 1u;
-                if (!mbar_wait(&acc_empty_bar[acc], acc_phase ^ 1u, abort_flag)) {
+        // The whole warp walks the loop and one elected lane issues: tensor-memory addresses and
+        // descriptors are then warp-uniform to the compiler, which is how the MMA takes its operands
+        // (N = 11008, K = 4096, 24 / 64 rows: 16.7 / 19.5 -> 16.1 / 19.2 us).
+        const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, tmem_base, 0);
+        int stage = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int local_seg = 0; ok && local_seg < num_segments; ++local_seg) {
+            const Segment seg = segments.at(local_seg);
+            const int acc = local_seg & 1;
+            const uint32_t acc_phase = (local_seg >> 1) & 1u;
+            if (!mbar_wait_warp(&acc_empty_bar[acc], acc_phase ^ 1u, abort_flag)) {
+                if (lane == 0) {
                     atomicCAS(error_word, 0, kErrAccumWait);
+                }
+                break;
+            }
+            tc_fence_after_sync();
+            const uint32_t d_tmem = tmem + static_cast<uint32_t>(acc * MP);
+            for (int kb = seg.kb0; kb < seg.kb1; ++kb) {
+                if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag)) {
+                    if (lane == 0) {
+                        atomicCAS(error_word, 0, kErrMmaWait);
+                    }
+                    ok = false;
                     break;
                 }
                 tc_fence_after_sync();
-                const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * MP);
-                for (int kb = seg.kb0; kb < seg.kb1; ++kb) {
-                    if (!mbar_wait(&full_bar[stage], phase, abort_flag)) {
-                        atomicCAS(error_word, 0, kErrMmaWait);
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after_sync();
-                    const uint32_t w_addr = smem_u32(stage_base + stage * Cfg::kStageBytes);
-                    const uint32_t a_addr = w_addr + Cfg::kWTileBytes;
-                    const uint64_t w_desc = umma_desc_sw128_kmajor(w_addr);  // the MMA's 128-row operand
-                    const uint64_t a_desc = umma_desc_sw128_kmajor(a_addr);  // its N operand: MP activation rows
+                const uint32_t w_addr = smem_u32(stage_base + stage * Cfg::kStageBytes);
+                const uint32_t a_addr = w_addr + Cfg::kWTileBytes;
+                const uint64_t w_desc = umma_desc_sw128_kmajor(w_addr);  // the MMA's 128-row operand
+                const uint64_t a_desc = umma_desc_sw128_kmajor(a_addr);  // its N operand: MP activation rows
+                if (elect_one()) {
 #pragma unroll
                     for (int ks = 0; ks < kBlockKBytes / kUmmaK; ++ks) {
                         umma_i8(d_tmem, w_desc + static_cast<uint64_t>(ks * 2), a_desc + static_cast<uint64_t>(ks * 2),
                                 idesc, (kb > seg.kb0 || ks > 0) ? 1u : 0u);
                     }
                     umma_commit(&empty_bar[stage]);
-                    if (++stage == kStages) {
-                        stage = 0;
-                        phase ^= 1u;
+                    if (kb == seg.kb1 - 1) {
+                        umma_commit(&acc_full_bar[acc]);
                     }
                 }
-                if (ok) {
-                    umma_commit(&acc_full_bar[acc]);
+                __syncwarp();
+                if (++stage == kStages) {
+                    stage = 0;
+                    phase ^= 1u;
                 }
             }
         }
@@ -376,8 +390,8 @@ gemm_i8_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             const int acc = local_seg & 1;
             const uint32_t acc_phase = (local_seg >> 1) & 1u;
             const bool partial = seg.kb0 != 0 || seg.kb1 != num_kb;  // only under the equal-share split
-            const int64_t n = static_cast<int64_t>(tile) * kBlockN + ch;
-            const bool n_ok = n < n_total;
+            const int64_t n = static_cast<int64_t>(tile) * tile_rows + ch;
+            const bool n_ok = ch < tile_rows && n < n_total;
             // This channel's terms, in registers for the whole tile.
             const int32_t zpw = (n_ok && ep.zp_w != nullptr) ? ep.zp_w[n] : ep.zp_w_scalar;
             const int32_t rw = (n_ok && ep.compensate && ep.r_w != nullptr) ? ep.r_w[n] : 0;
@@ -569,14 +583,24 @@ int launch_skinny_variant(const I8Problem& p, const I8Epilogue& ep, const Device
         return NNB200_INTERNAL;
     }
     const int m = static_cast<int>(p.m), n = static_cast<int>(p.n), k = static_cast<int>(p.k);
+    // Whole tiles over several waves: as many waves as 128-channel tiles need, cut into equal tiles (24
+    // rows, 128-channel tiles / equal ones: N = 28672, K = 8192 51.8 / 45.4 us, N = 19456, K = 4096 28.1 / 24.8).
+    // A single wave keeps 128 channels: more CTAs load the activations more often, which eats what the
+    // even weight stream gives (N = 11008, K = 4096: 24 rows 16.7 / 16.4, 64 rows 19.5 / 20.1, 128 rows
+    // 24.7 / 26.6).  Shared K evens the SMs out itself, and its scratch is laid out for 128.
+    int tile_rows = kBlockN;
+    const int waves = ((n + kBlockN - 1) / kBlockN + dev.sm_count - 1) / dev.sm_count;
+    if (split_scratch == nullptr && waves > 1) {
+        tile_rows = (n + waves * dev.sm_count - 1) / (waves * dev.sm_count);
+    }
     CUtensorMap map_w, map_a;
     if (!make_tma_2d(&map_w, p.w, 1, static_cast<uint64_t>(k), static_cast<uint64_t>(n),
-                     static_cast<uint64_t>(p.w_stride_n), kBlockKBytes, kBlockN) ||
+                     static_cast<uint64_t>(p.w_stride_n), kBlockKBytes, static_cast<uint32_t>(tile_rows)) ||
         !make_tma_2d(&map_a, p.a, 1, static_cast<uint64_t>(k), static_cast<uint64_t>(m),
                      static_cast<uint64_t>(p.a_stride_m), kBlockKBytes, MP)) {
         return NNB200_INTERNAL;
     }
-    const int num_tiles = (n + kBlockN - 1) / kBlockN;
+    const int num_tiles = (n + tile_rows - 1) / tile_rows;
     int grid = num_tiles < dev.sm_count ? num_tiles : dev.sm_count;
     unsigned long long* counters = nullptr;
     int32_t* slots = nullptr;
@@ -591,7 +615,7 @@ int launch_skinny_variant(const I8Problem& p, const I8Epilogue& ep, const Device
     // 128-row operand = weights (s8), N operand = activations (s8 or u8).
     const uint32_t idesc = umma_idesc(2, 1, p.a_unsigned ? 0u : 1u, kBlockN, MP);
     kernel<<<grid, kNumThreads, Cfg::kSmemBytes, stream>>>(map_w, map_a, ep, m, n, k, idesc, dev.error_word, counters,
-                                                             slots, tag);
+                                                             slots, tag, tile_rows);
     note_launch();
     return cuda_status(cudaGetLastError());
 }
