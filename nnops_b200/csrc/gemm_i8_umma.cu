@@ -489,7 +489,7 @@ template <int BN, int KIND, int PEERS>
 int launch_variant(const CUtensorMap& map_a, const CUtensorMap& map_w, const I8Epilogue& ep, int m, int n, int k,
                    uint32_t idesc, int vec_ok, const DeviceInfo& dev, cudaStream_t stream)
 {
-    using Cfg = TileConfig<BN, PEERS>;
+    using Cfg = TileConfig<BN, PEERS, KIND>;
     auto kernel = gemm_i8_umma_kernel<BN, KIND, PEERS>;
     constexpr int kSmem = Cfg::kSmemBytes;
     PeerMaps maps;
@@ -521,7 +521,7 @@ int launch_variant(const CUtensorMap& map_a, const CUtensorMap& map_w, const I8E
     if (knob(NNB200_KNOB_GROUP_M) > 0) {
         group_m = knob(NNB200_KNOB_GROUP_M);
     }
-    kernel<<<grid, num_threads(PEERS), kSmem, stream>>>(map_a, map_w, maps, ep, m, n, k, idesc, vec_ok, group_m,
+    kernel<<<grid, tile_threads(KIND, PEERS), kSmem, stream>>>(map_a, map_w, maps, ep, m, n, k, idesc, vec_ok, group_m,
                                                  k_rotation_step(n), dev.error_word, ConvTile{});
     note_launch();
     return cuda_status(cudaGetLastError());
@@ -584,7 +584,7 @@ int launch_conv_variant(const CUtensorMap& map_a, const CUtensorMap& map_w, cons
                         int k, uint32_t idesc, int vec_ok, const ConvTile& conv, const DeviceInfo& dev,
                         cudaStream_t stream)
 {
-    using Cfg = TileConfig<BN, 0>;
+    using Cfg = TileConfig<BN, 0, KIND>;
     auto kernel = gemm_i8_umma_kernel<BN, KIND, 0, true>;
     static std::once_flag once[kMaxDevices];
     static cudaError_t attr_err[kMaxDevices];
@@ -600,7 +600,7 @@ int launch_conv_variant(const CUtensorMap& map_a, const CUtensorMap& map_w, cons
     const int grid = num_tiles < dev.sm_count ? num_tiles : dev.sm_count;
     int group_m = static_cast<int>((40ll << 20) / (static_cast<int64_t>(kBlockM) * (k > 0 ? k : 1)));
     group_m = group_m < 4 ? 4 : group_m;
-    kernel<<<grid, num_threads(0), Cfg::kSmemBytes, stream>>>(map_a, map_w, maps, ep, m_tiles * kBlockM, n, k, idesc, vec_ok,
+    kernel<<<grid, tile_threads(KIND, 0), Cfg::kSmemBytes, stream>>>(map_a, map_w, maps, ep, m_tiles * kBlockM, n, k, idesc, vec_ok,
                                                             group_m, k_rotation_step(n), dev.error_word, conv);
     note_launch();
     return cuda_status(cudaGetLastError());

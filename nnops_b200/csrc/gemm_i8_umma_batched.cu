@@ -20,7 +20,7 @@ template <int BN, int KIND>
 int launch_batched_variant(const CUtensorMap& map_a, const CUtensorMap& map_w, const I8Epilogue& ep, int m, int n, int k,
                            uint32_t idesc, int vec_ok, const BatchTile& batch, const DeviceInfo& dev, cudaStream_t stream)
 {
-    using Cfg = TileConfig<BN, 0>;
+    using Cfg = TileConfig<BN, 0, KIND>;
     auto kernel = gemm_i8_umma_kernel<BN, KIND, 0, false, true>;
     static std::once_flag once[kMaxDevices];
     static cudaError_t attr_err[kMaxDevices];
@@ -35,7 +35,7 @@ int launch_batched_variant(const CUtensorMap& map_a, const CUtensorMap& map_w, c
     const int num_m = (m + kBlockM - 1) / kBlockM;
     const int64_t num_tiles = static_cast<int64_t>(batch.count) * num_m * ((n + BN - 1) / BN);
     const int grid = num_tiles < dev.sm_count ? static_cast<int>(num_tiles) : dev.sm_count;
-    kernel<<<grid, num_threads(0), Cfg::kSmemBytes, stream>>>(map_a, map_w, maps, ep, m, n, k, idesc, vec_ok, num_m, 0,
+    kernel<<<grid, tile_threads(KIND, 0), Cfg::kSmemBytes, stream>>>(map_a, map_w, maps, ep, m, n, k, idesc, vec_ok, num_m, 0,
                                                             dev.error_word, batch);
     note_launch();
     return cuda_status(cudaGetLastError());

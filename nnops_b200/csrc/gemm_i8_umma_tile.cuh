@@ -17,14 +17,27 @@ namespace {
 constexpr int kBlockM = 128;
 constexpr int kBlockKBytes = 128;  // one 128-byte swizzle row of K per stage
 constexpr int kUmmaK = 32;         // K per tcgen05.mma for 8-bit operands
-// TMA warp, MMA warp, then the epilogue warps: eight (two per TMEM lane quarter, each draining
-// half of the tile's columns) in the plain kernels, four in the sharded form, whose staging
-// tiles are per warp.  One warp per scheduler issues an instruction every ~4 cycles on the
-// epilogue's dependent chains; with four warps a 128 x 256 tile took ~17k cycles to drain, which
-// hid behind the main loop only from K = 4096 up.
+// TMA warp, MMA warp, then the epilogue warps.  The sharded form has four, whose staging tiles are per
+// warp; elsewhere there are two per TMEM lane quarter, each draining half of the tile's columns: one
+// warp per scheduler issues an instruction every ~4 cycles on the epilogue's dependent chains, and
+// with four warps a 128 x 256 tile took ~17k cycles to drain, which hid behind the main loop only
+// from K = 4096 up.
 constexpr int kMaxThreads = 320;
 __host__ __device__ constexpr int epilogue_warps(int peers) { return peers ? 4 : 8; }
 __host__ __device__ constexpr int num_threads(int peers) { return (2 + epilogue_warps(peers)) * 32; }
+// The single-CTA kernel's 8-bit destinations have sixteen.  Up to 256 columns they form two groups, each
+// with an accumulator of its own, that take the tiles in turn: of the ~6600 cycles eight warps needed
+// for a 128 x 256 tile, ~2300 passed between two tiles (column terms, row terms, barriers) with nothing
+// to issue, and the drain itself kept the schedulers less than two thirds busy.  A wider tile, the only
+// one of its CTA, is drained by four warps per lane quarter.  100352 x 1024 x 256 77.5 -> 63.6 us,
+// 32768 x 4096 x 256 97.2 -> 78.8, 8192 x 4096 x 1024 33.8 -> 31.3, 512 x 11008 x 4096 (320 wide) 24.6 -> 24.0.
+// The floating destinations hold twice the values per chunk in registers and keep eight.
+__host__ __device__ constexpr bool sixteen_warps(int kind, int peers)
+{
+    return peers == 0 && (kind == NNB200_OUT_S8 || kind == NNB200_OUT_U8);
+}
+__host__ __device__ constexpr int tile_epilogue_warps(int kind, int peers) { return sixteen_warps(kind, peers) ? 16 : epilogue_warps(peers); }
+__host__ __device__ constexpr int tile_threads(int kind, int peers) { return (2 + tile_epilogue_warps(kind, peers)) * 32; }
 // Columns drained by the first of the two warps of a lane quarter (whole 32-column chunks).
 __host__ __device__ constexpr int first_half_cols(int bn, int peers) { return peers ? bn : ((bn / 32 + 1) / 2) * 32; }
 
@@ -139,8 +152,11 @@ __device__ __forceinline__ void conv_border_fix(const ConvTile& conv, uint32_t (
     }
 }
 
-template <int BN, int PEERS = 0>
+template <int BN, int PEERS = 0, int KIND = NNB200_OUT_S32>
 struct TileConfig {
+    static constexpr int kEpilogueWarps = tile_epilogue_warps(KIND, PEERS);
+    static constexpr int kGroups = (kEpilogueWarps == 16 && BN <= 256) ? 2 : 1;   // groups that take the tiles in turn
+    static constexpr int kColParts = kEpilogueWarps / 4 / kGroups;                 // warps per lane quarter and group
     // Tiles wider than 256 columns (single-wave form, see launch_gemm_i8_umma) are issued as two
     // MMAs of BN / 2 columns over one A tile and keep ONE accumulator: a CTA owns exactly one tile.
     static constexpr int kNSplit = BN > 256 ? 2 : 1;
@@ -155,8 +171,8 @@ struct TileConfig {
     // Two accumulators BN columns apart (one when BN > 256); a power of two of at least that.
     static constexpr int kTmemCols = BN > 128 ? 512 : 2 * BN;
     // Per epilogue warp {scale, bias, r_w, zp_w} of the columns it drains, 4 B each.
-    static constexpr int kHalf0 = first_half_cols(BN, PEERS);
-    static constexpr int kColParamBytes = epilogue_warps(PEERS) * 4 * kHalf0 * 4;
+    static constexpr int kPartCols = (BN / 32 + kColParts - 1) / kColParts * 32;   // the last part may be narrower
+    static constexpr int kColParamBytes = kEpilogueWarps * 4 * kPartCols * 4;
     static constexpr int kBarrierBytes = (2 * kStages + 4) * 8 + 16;
     // Sharded form (PEERS = 2): two staging tiles of 32 rows x 128 B per epilogue warp, one being
     // filled while the other is being stored.  With few peers (PEERS = 1, used up to three) the
@@ -169,6 +185,7 @@ struct TileConfig {
     static constexpr int kPeerStageBytes = PEERS ? 4 * kStageTiles * 32 * kStageGroupCols : 0;
     static constexpr int kSmemBytes =
         1024 /*alignment slack*/ + kStages * kStageBytes + kPeerStageBytes + kColParamBytes + kBarrierBytes;
+    static_assert(kSmemBytes <= 227 * 1024, "shared memory");
 };
 
 // A batch of equal problems in one launch (BATCH kernels).  Steps are 0 where the operand is shared.
@@ -585,7 +602,7 @@ __device__ __forceinline__ void epilogue_chunk(const I8Epilogue& e, const I8RowT
 // BATCH: one launch for a batch of equal problems (BatchTile in the last parameter); the persistent
 // tile walk runs through all of them and the operands are read through maps with a batch axis.
 template <int BN, int KIND, int PEERS, bool CONV = false, bool BATCH = false>
-__global__ void __launch_bounds__(kMaxThreads, 1)
+__global__ void __launch_bounds__(tile_threads(KIND, PEERS), 1)
 gemm_i8_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                     const __grid_constant__ PeerMaps peer_maps, const I8Epilogue ep_all, const int m_total,
                     const int n_total, const int k_total, const uint32_t idesc, const int vec_ok, const int group_m, const int k_rot,
@@ -593,7 +610,7 @@ gemm_i8_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 {
     static_assert(!CONV || PEERS == 0, "the convolution form has no sharded epilogue");
     static_assert(!BATCH || (!CONV && PEERS == 0), "the batched form is a plain product");
-    using Cfg = TileConfig<BN, PEERS>;
+    using Cfg = TileConfig<BN, PEERS, KIND>;
     constexpr int kStages = Cfg::kStages;
     // Narrow tiles: the whole warp walks the MMA loop and one elected lane issues.  Tensor-memory
     // addresses and descriptors are then warp-uniform to the compiler, which is how the MMA takes its
@@ -645,7 +662,7 @@ gemm_i8_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(&acc_full_bar[a], 1);
-            mbar_init(&acc_empty_bar[a], epilogue_warps(PEERS));
+            mbar_init(&acc_empty_bar[a], Cfg::kEpilogueWarps / Cfg::kGroups);
         }
         *abort_flag = 0;
         mbar_init_fence();
@@ -850,18 +867,19 @@ gemm_i8_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                                ep_all.zp_a == nullptr && ep_all.r_a == nullptr;
         // The next tile's column terms are loaded into registers before this tile is drained,
         // so their latency is not paid between tiles (up to four per lane and term).
-        constexpr int kTermIters = (Cfg::kHalf0 + 31) / 32;
-        constexpr bool kPrefetch = !PEERS && kTermIters <= 4;
+        constexpr int kTermIters = (Cfg::kPartCols + 31) / 32;
+        constexpr bool kPrefetch = !PEERS && kTermIters <= 4 && Cfg::kEpilogueWarps < 16;
         ColTerms next_terms[kPrefetch ? kTermIters : 1];
-        // Two warps per lane quarter: the first drains columns [0, kHalf0), the second the rest.
-        constexpr int kHalf0 = Cfg::kHalf0;
-        const int half = PEERS ? 0 : ((warp - 2) >> 2);
-        const int col0 = half * kHalf0;
-        const int ncols = half ? BN - kHalf0 : kHalf0;
-        float* cs = reinterpret_cast<float*>(col_params + (warp - 2) * 4 * kHalf0);
-        int32_t* cb = reinterpret_cast<int32_t*>(cs) + kHalf0;
-        int32_t* cr = cb + kHalf0;
-        int32_t* cz = cr + kHalf0;
+        // The warps of a lane quarter share out the tile's columns.
+        constexpr int kPartCols = Cfg::kPartCols;
+        const int part = ((warp - 2) >> 2) % Cfg::kColParts;
+        const int group = ((warp - 2) >> 2) / Cfg::kColParts;
+        const int col0 = part * kPartCols;
+        const int ncols = min(kPartCols, BN - col0);
+        float* cs = reinterpret_cast<float*>(col_params + (warp - 2) * 4 * kPartCols);
+        int32_t* cb = reinterpret_cast<int32_t*>(cs) + kPartCols;
+        int32_t* cr = cb + kPartCols;
+        int32_t* cz = cr + kPartCols;
         int stage_turn = 0;  // sharded form: which of the warp's two staging tiles is next
         (void)stage_turn;
         // The epilogue block of one problem of the batch: its output and its operands' sums.
@@ -880,6 +898,9 @@ gemm_i8_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         };
         int local_tile = 0;
         for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++local_tile) {
+            if (Cfg::kGroups > 1 && (local_tile & 1) != group) {
+                continue;
+            }
             const TileCoord tc = coord_of(tile);
             const int acc = Cfg::kNSplit > 1 ? 0 : (local_tile & 1);
             const uint32_t acc_phase = Cfg::kNSplit > 1 ? (local_tile & 1u) : ((local_tile >> 1) & 1u);
@@ -1064,23 +1085,34 @@ gemm_i8_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     epilogue_chunk<KIND>(ep, rt, v, m, row_ok, n0, n_total, cs + c * 32, cb + c * 32, cr + c * 32,
                                          cz + c * 32, vec_ok, fold_scale, fold_comp);
                 };
-                uint32_t va[32], vb[32];
-                if (nch > 0) {
-                    tmem_ld_32x32(t_row, va);
-                }
+                if constexpr (Cfg::kEpilogueWarps == 16) {
+                    // Enough warps to cover a load's latency; one register set keeps them resident.
+                    uint32_t v[32];
 #pragma unroll 1
-                for (int c = 0; c < nch; c += 2) {
-                    tmem_ld_wait();
-                    if (c + 1 < nch) {
-                        tmem_ld_32x32(t_row + static_cast<uint32_t>((c + 1) * 32), vb);
-                    }
-                    finish(c, va);
-                    if (c + 1 < nch) {
+                    for (int c = 0; c < nch; ++c) {
+                        tmem_ld_32x32(t_row + static_cast<uint32_t>(c * 32), v);
                         tmem_ld_wait();
-                        if (c + 2 < nch) {
-                            tmem_ld_32x32(t_row + static_cast<uint32_t>((c + 2) * 32), va);
+                        finish(c, v);
+                    }
+                } else {
+                    uint32_t va[32], vb[32];
+                    if (nch > 0) {
+                        tmem_ld_32x32(t_row, va);
+                    }
+#pragma unroll 1
+                    for (int c = 0; c < nch; c += 2) {
+                        tmem_ld_wait();
+                        if (c + 1 < nch) {
+                            tmem_ld_32x32(t_row + static_cast<uint32_t>((c + 1) * 32), vb);
                         }
-                        finish(c + 1, vb);
+                        finish(c, va);
+                        if (c + 1 < nch) {
+                            tmem_ld_wait();
+                            if (c + 2 < nch) {
+                                tmem_ld_32x32(t_row + static_cast<uint32_t>((c + 2) * 32), va);
+                            }
+                            finish(c + 1, vb);
+                        }
                     }
                 }
             }
