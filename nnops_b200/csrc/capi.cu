@@ -750,15 +750,18 @@ static constexpr int64_t kRowsUmmaMaxRows = 128;
 static bool q4_1_wants_rows_umma(const nnb200_q4_1_args* q)
 {
     const int64_t b_rows = q->a_f16 != 0 ? q->m : 2 * q->m;
-    const bool few = q->m <= (q->a_f16 != 0 ? 8 : 2) && static_cast<double>(q->n) * q->k <= static_cast<double>(1 << 25);
-    const bool chosen = q->force_engine == 0 && q->m >= 2 && b_rows <= kRowsUmmaMaxRows && !few;
+    const bool few = q->m <= (q->a_f16 != 0 ? 8 : 2) && static_cast<double>(q->n) * q->k <= static_cast<double>(1 << 25) &&
+                     q4_1_gemv_mma_supported(*q);   // without it the GEMV runs on CUDA cores
+    // A K that 128 does not divide is padded to it; below 256 the other forms are as short.
+    const bool k_ok = q->k % 128 == 0 || q->k >= 256;
+    const bool chosen = q->force_engine == 0 && q->m >= 2 && b_rows <= kRowsUmmaMaxRows && !few && k_ok;
     return (chosen || q->force_engine == 7) && q4_1_rows_umma_supported(*q);
 }
 
 // Scratch for f32 activations as pairs of f16 rows.
 static size_t q4_1_rows_scratch_bytes(const nnb200_q4_1_args* q)
 {
-    return static_cast<size_t>(q->m) * static_cast<size_t>(q->k) * 4;
+    return static_cast<size_t>(q->m) * static_cast<size_t>(q4_1_rows_split_pitch(q->k)) * 4;
 }
 
 size_t nnb200_q4_1_workspace_bytes(const nnb200_q4_1_args* q)
@@ -858,12 +861,13 @@ int nnb200_linear_q4_1(const nnb200_q4_1_args* q, void* stream_v)
     case 7: {
         Q4RowsCall call{q, q->a, q->lda, false};
         if (q->a_f16 == 0) {
-            const int st = launch_split_f32_to_f16(static_cast<const float*>(q->a), q->lda, q->m, q->k, q->k, q->workspace,
+            const int64_t pitch = q4_1_rows_split_pitch(q->k);
+            const int st = launch_split_f32_to_f16(static_cast<const float*>(q->a), q->lda, q->m, q->k, pitch, q->workspace,
                                                    *dev, stream);
             if (st != NNB200_OK) {
                 return st;
             }
-            call = Q4RowsCall{q, q->workspace, q->k, true};
+            call = Q4RowsCall{q, q->workspace, pitch, true};
         }
         return launch_q4_1_rows_umma(call, *dev, stream);
     }

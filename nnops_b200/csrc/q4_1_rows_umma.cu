@@ -33,6 +33,7 @@
 
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "internal.cuh"
 #include "ptx.cuh"
@@ -59,8 +60,6 @@ template <int BLOCKS>
 struct RowsConfig {
     static constexpr int kUnitK = BLOCKS * kQ4BlockElems;
     static constexpr int kUnitBytes = BLOCKS * kQ4BlockBytes;     // 160 or 80 bytes of a row
-    static constexpr int kPieces = kUnitBytes / 16;
-    static constexpr int kRowsAtOnce = 32 / kPieces;              // rows one warp-wide copy covers
     static constexpr int kWarpUnitBytes = 32 * kUnitBytes;
     static constexpr int kDepth = BLOCKS == 8 ? 2 : 4;            // units of raw rows on their way per warp
     static constexpr int kRawBytes = kWarps * kDepth * kWarpUnitBytes;   // 122 880 either way
@@ -125,6 +124,18 @@ __device__ __forceinline__ float ld_shared_cluster_f32(uint32_t cluster_addr)
     return v;
 }
 
+// Asynchronous copy of N bytes, those past `src_bytes` as zeros.
+template <int N>
+__device__ __forceinline__ void cp_async(void* smem_dst, const void* gmem_src, uint32_t src_bytes)
+{
+    if constexpr (N == 16) {
+        cp_async_16(smem_dst, gmem_src, src_bytes);
+    } else {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(smem_u32(smem_dst)), "l"(gmem_src), "n"(N), "r"(src_bytes)
+                     : "memory");
+    }
+}
+
 // One block of a row, {d | m, four words of nibbles} -> its 32 weights as 16 f16 pairs in k order.
 // A word's bytes carry k = 4wi .. 4wi+3 in their low and 16 + the same in their high nibbles:
 // byte | 0x6400 = 1024 + q, (byte & 0xF0) | 0x5400 = 64 + q; the bias goes out exactly and d * q + m
@@ -158,7 +169,9 @@ __device__ __forceinline__ void decode_block(const uint32_t (&b)[5], uint32_t (&
 // thread some hundred cycles with its wait, so there are few: with a pair per 64 k (and barriers of
 // their own for the activations) a call at 16 x 14336 x 4096 took 34.6 us, with one per 128 k 18.6, as
 // here 16.0.  (Two issuing warps with an accumulator each: 17.8.)
-template <bool OUT_F16, int BLOCKS>
+//
+// PIECE: bytes of one copy, the most (16, 8 or 4) that the weight rows' alignment allows.
+template <bool OUT_F16, int BLOCKS, int PIECE>
 __global__ void __launch_bounds__(kThreads, 1)
 q4_1_rows_umma_kernel(const __grid_constant__ CUtensorMap map_a, const uint8_t* __restrict__ w,
                       const int64_t w_pitch_bytes, void* __restrict__ out, const int64_t ldc, const int m_total,
@@ -184,13 +197,16 @@ q4_1_rows_umma_kernel(const __grid_constant__ CUtensorMap map_a, const uint8_t* 
     const int cluster = static_cast<int>(blockIdx.x) / split;
     const int clusters = static_cast<int>(gridDim.x) / split;
     const int num_tiles = (n_total + tile_rows - 1) / tile_rows;
-    // This CTA's units; the row's last unit of 256 k may hold 128.
-    const int units_total = (k_total + kUnitK - 1) / kUnitK;
+    // This CTA's units; the row's last unit of 256 k may hold 128.  K is padded to a multiple of 128:
+    // blocks past a row's end are zeros in shared memory, activations past K zeros from TMA.
+    const int k_pad = (k_total + 127) / 128 * 128;
+    const int row_bytes = (k_total + kQ4BlockElems - 1) / kQ4BlockElems * kQ4BlockBytes;
+    const int units_total = (k_pad + kUnitK - 1) / kUnitK;
     const int u0 = units_total * rank / split;
     const int units = units_total * (rank + 1) / split - u0;
     const int slab_bytes = nb * 128;               // 64 k of the activations
     const int stage_bytes = nb * kUnitK * 2;
-    const auto slabs_of = [&](int u) { return min(kUnitK, k_total - (u0 + u) * kUnitK) / kSlotK; };   // 4 or 2
+    const auto slabs_of = [&](int u) { return min(kUnitK, k_pad - (u0 + u) * kUnitK) / kSlotK; };   // 4 or 2
 
     if (threadIdx.x == 0) {
         for (int g = 0; g < kGroups; ++g) {
@@ -212,8 +228,11 @@ q4_1_rows_umma_kernel(const __grid_constant__ CUtensorMap map_a, const uint8_t* 
     const int group = warp >> 2;
     const int quarter = warp & 3;
     uint8_t* my_raw = raw + warp * (Cfg::kDepth * Cfg::kWarpUnitBytes);
-    const int copy_row = lane / Cfg::kPieces;
-    const int copy_piece = lane - copy_row * Cfg::kPieces;
+    // The pieces of a unit's row, over the lanes: several rows at once, or several lanes' worth of one.
+    constexpr int kPieces = Cfg::kUnitBytes / PIECE;
+    constexpr int kRowsAtOnce = kPieces <= 32 ? 32 / kPieces : 1;
+    const int copy_row = kPieces <= 32 ? lane / kPieces : 0;
+    const int copy_piece = lane - copy_row * kPieces;
     int next_tile = cluster, next_u = group, next_buf = 0;   // of the next unit to copy
     const auto issue_unit = [&]() {
         while (next_u >= units) {
@@ -223,17 +242,25 @@ q4_1_rows_umma_kernel(const __grid_constant__ CUtensorMap map_a, const uint8_t* 
         if (next_tile < num_tiles) {
             const int row0 = next_tile * tile_rows + quarter * 32;
             const int rows = min(min(32, tile_rows - quarter * 32), n_total - row0);
-            const uint8_t* src = w + (row0 + copy_row) * w_pitch_bytes + static_cast<int64_t>(u0 + next_u) * Cfg::kUnitBytes + copy_piece * 16;
-            uint8_t* dst = my_raw + next_buf * Cfg::kWarpUnitBytes + copy_row * Cfg::kUnitBytes + copy_piece * 16;
-            // The second half of a unit cut short by the row's end is not there to read.
-            const bool live = copy_row < Cfg::kRowsAtOnce && copy_piece * 16 < slabs_of(next_u) * (2 * kQ4BlockBytes);
-            const int64_t step = Cfg::kRowsAtOnce * w_pitch_bytes;
+            const int64_t step = kRowsAtOnce * w_pitch_bytes;
 #pragma unroll
-            for (int i = 0; i * Cfg::kRowsAtOnce < 32; ++i) {
-                if (live && copy_row + i * Cfg::kRowsAtOnce < rows) {
-                    cp_async_16(dst + i * (Cfg::kRowsAtOnce * Cfg::kUnitBytes), src, 16);
+            for (int p = copy_piece; p < kPieces; p += 32) {
+                const int at = (u0 + next_u) * Cfg::kUnitBytes + p * PIECE;   // within the row
+                const int bytes = max(0, min(PIECE, row_bytes - at));         // the rest of the piece becomes zeros
+                const uint8_t* src = w + (row0 + copy_row) * w_pitch_bytes + (bytes > 0 ? at : 0);
+                uint8_t* dst = my_raw + next_buf * Cfg::kWarpUnitBytes + copy_row * Cfg::kUnitBytes + p * PIECE;
+                // A unit of half the k ends before the pieces do.
+                const bool live = copy_row < kRowsAtOnce && p * PIECE < slabs_of(next_u) * (2 * kQ4BlockBytes);
+#pragma unroll
+                for (int i = 0; i * kRowsAtOnce < 32; ++i) {
+                    if (live && copy_row + i * kRowsAtOnce < rows) {
+                        cp_async<PIECE>(dst + i * (kRowsAtOnce * Cfg::kUnitBytes), src, static_cast<uint32_t>(bytes));
+                    }
+                    src += step;
                 }
-                src += step;
+                if (kPieces <= 32) {
+                    break;
+                }
             }
         }
         cp_async_commit();   // one group a call, empty or not: the waits count groups
@@ -549,12 +576,12 @@ q4_1_rows_umma_kernel(const __grid_constant__ CUtensorMap map_a, const uint8_t* 
     }
 }
 
-template <bool OUT_F16, int BLOCKS>
+template <bool OUT_F16, int BLOCKS, int PIECE>
 int launch_variant(const CUtensorMap& map_a, const Q4RowsCall& c, int nb, int tile_rows, int split, int ctas,
                    const FpEpilogue& ep, const DeviceInfo& dev, cudaStream_t stream)
 {
     using Cfg = RowsConfig<BLOCKS>;
-    auto kernel = q4_1_rows_umma_kernel<OUT_F16, BLOCKS>;
+    auto kernel = q4_1_rows_umma_kernel<OUT_F16, BLOCKS, PIECE>;
     static std::once_flag once[kMaxDevices];
     static cudaError_t attr_err[kMaxDevices];
     std::call_once(once[dev.device], [&] {
@@ -587,12 +614,12 @@ int launch_variant(const CUtensorMap& map_a, const Q4RowsCall& c, int nb, int ti
 
 bool q4_1_rows_umma_supported(const nnb200_q4_1_args& q)
 {
-    // Weight rows movable in 16-byte pieces (whole groups of four blocks), activations addressable
-    // by TMA.  f32 activations come as a scratch copy that always is.
+    // Raw weight rows (4-byte aligned by the format), activations addressable by TMA; f32
+    // activations come as a scratch copy that always is.
     const int64_t b_rows = q.a_f16 != 0 ? q.m : 2 * q.m;
     const bool a_ok = q.a_f16 == 0 || ((reinterpret_cast<uintptr_t>(q.a) & 15u) == 0 && (q.lda % 8) == 0);
-    return a_ok && q.m >= 1 && b_rows <= kAccCols && q.n >= 1 && q.n <= INT32_MAX / 2 && q.k >= 128 && q.k <= INT32_MAX / 2 &&
-           (q.k % 128) == 0 && q.w_dm == nullptr && (reinterpret_cast<uintptr_t>(q.w_blocks) & 15u) == 0 && (q.ldw_blocks % 4) == 0;
+    return a_ok && q.m >= 1 && b_rows <= kAccCols && q.n >= 1 && q.n <= INT32_MAX / 2 && q.k >= 1 && q.k <= INT32_MAX / 2 &&
+           q.w_dm == nullptr && (reinterpret_cast<uintptr_t>(q.w_blocks) & 3u) == 0;
 }
 
 int launch_q4_1_rows_umma(const Q4RowsCall& c, const DeviceInfo& dev, cudaStream_t stream)
@@ -612,7 +639,7 @@ int launch_q4_1_rows_umma(const Q4RowsCall& c, const DeviceInfo& dev, cudaStream
     const int n = static_cast<int>(q.n);
     const bool wide = nb > RowsConfig<8>::kMaxRows;   // units of 128 k instead of 256
     const int unit_k = wide ? RowsConfig<4>::kUnitK : RowsConfig<8>::kUnitK;
-    const int units = static_cast<int>((q.k + unit_k - 1) / unit_k);
+    const int units = static_cast<int>(((q.k + 127) / 128 * 128 + unit_k - 1) / unit_k);
     // Every SM gets the same share of the channels: with at least half as many 128-channel tiles as
     // SMs, whole waves of equal, narrower tiles (a lane without a channel costs nothing that is
     // scarce: the weight stream is); below that, clusters that share K.
@@ -635,12 +662,20 @@ int launch_q4_1_rows_umma(const Q4RowsCall& c, const DeviceInfo& dev, cudaStream
                      static_cast<uint64_t>(c.lda) * 2, kSlotK, static_cast<uint32_t>(nb))) {
         return NNB200_INTERNAL;
     }
-    if (wide) {
-        return q.out_f16 ? launch_variant<true, 4>(map_a, c, nb, tile_rows, split, ctas, ep, dev, stream)
-                         : launch_variant<false, 4>(map_a, c, nb, tile_rows, split, ctas, ep, dev, stream);
+    const uint64_t row_bits = reinterpret_cast<uintptr_t>(q.w_blocks) | static_cast<uint64_t>(q.ldw_blocks * kQ4BlockBytes);
+    const auto launch = [&](auto piece) {
+        constexpr int P = decltype(piece)::value;
+        if (wide) {
+            return q.out_f16 ? launch_variant<true, 4, P>(map_a, c, nb, tile_rows, split, ctas, ep, dev, stream)
+                             : launch_variant<false, 4, P>(map_a, c, nb, tile_rows, split, ctas, ep, dev, stream);
+        }
+        return q.out_f16 ? launch_variant<true, 8, P>(map_a, c, nb, tile_rows, split, ctas, ep, dev, stream)
+                         : launch_variant<false, 8, P>(map_a, c, nb, tile_rows, split, ctas, ep, dev, stream);
+    };
+    if ((row_bits & 15u) == 0) {
+        return launch(std::integral_constant<int, 16>{});
     }
-    return q.out_f16 ? launch_variant<true, 8>(map_a, c, nb, tile_rows, split, ctas, ep, dev, stream)
-                     : launch_variant<false, 8>(map_a, c, nb, tile_rows, split, ctas, ep, dev, stream);
+    return (row_bits & 7u) == 0 ? launch(std::integral_constant<int, 8>{}) : launch(std::integral_constant<int, 4>{});
 }
 
 }  // namespace nnb200

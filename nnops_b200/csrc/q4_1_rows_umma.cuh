@@ -12,6 +12,8 @@ struct Q4RowsCall {
     bool hi_lo;
 };
 
+// Halves between the (hi, lo) rows of f32 activations: 16-byte rows.
+inline int64_t q4_1_rows_split_pitch(int64_t k) { return (k + 7) / 8 * 8; }
 bool q4_1_rows_umma_supported(const nnb200_q4_1_args& q);
 // [m][k] f32 rows -> rows of 2 kp halves, the f16 parts followed by the f16 remainders (zeros past k);
 // with kp == k that is 2 m rows of k halves, part and remainder in turn.

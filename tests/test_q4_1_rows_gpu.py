@@ -28,14 +28,16 @@ def _check(device, m, n, k, a_dtype, out_dtype, **kw):
 @pytest.mark.parametrize("shape", [
     # m, n, k: K of half a unit, clusters that share K (few channels), whole waves, several tiles a CTA
     (2, 128, 128), (16, 1, 256), (9, 130, 384), (5, 1000, 2048), (17, 4096, 1152), (33, 129, 8320), (16, 9500, 640),
-    (64, 14336, 512), (65, 1000, 384), (128, 300, 4096), (100, 19000, 256), (3, 45000, 128), (7, 40000, 1152)])
+    (64, 14336, 512), (65, 1000, 384), (128, 300, 4096), (100, 19000, 256), (3, 45000, 128), (7, 40000, 1152),
+    # rows of 8- and 4-byte pitch, K padded to 128 (and within a block)
+    (16, 3000, 1088), (82, 500, 8992), (11, 128, 4128), (20, 19000, 288), (128, 700, 352), (5, 260, 1000), (70, 300, 40)])
 @pytest.mark.parametrize("out_dtype", [torch.float16, torch.float32])
 def test_rows_f16(cuda_device, nnb200_lib, shape, out_dtype):
     _check(cuda_device, *shape, np.float16, out_dtype)
 
 
 @pytest.mark.parametrize("shape", [(1, 300, 256), (2, 1000, 2048), (8, 9500, 640), (9, 4096, 1152), (33, 130, 384), (64, 260, 4096),
-                                   (50, 19000, 256)])
+                                   (50, 19000, 256), (13, 700, 1056), (40, 192, 1100), (64, 300, 68)])
 @pytest.mark.parametrize("out_dtype", [torch.float16, torch.float32])
 def test_rows_f32(cuda_device, nnb200_lib, shape, out_dtype):
     _check(cuda_device, *shape, np.float32, out_dtype)
