@@ -55,3 +55,24 @@ def test_relu_zero_point_and_signs(cuda_device, nnb200_lib, knobs, relu, out_zp,
 @pytest.mark.parametrize("per_token", [False, True])
 def test_many_tiles_per_cta(cuda_device, nnb200_lib, knobs, zero_points, per_token):
     _check(cuda_device, 9000, 2070, 96, per_token=per_token, zero_points=zero_points, knobs=knobs)
+
+
+@pytest.mark.parametrize("n", [64, 68, 72, 94, 97, 99, 1000, 1001, 1002])
+@pytest.mark.parametrize("out_kind", ["s8", "f16"])
+def test_rows_of_any_pitch(cuda_device, nnb200_lib, n, out_kind):
+    """Destination rows at every byte (half) offset, whole and cut chunks; nothing beside them is written."""
+    rng = np.random.default_rng(n)
+    m, k = 200, 144
+    a = rng.integers(-127, 128, (m, k), dtype=np.int8)
+    w = rng.integers(-127, 128, (n, k), dtype=np.int8)
+    kw = dict(out_kind=out_kind, out_scale=900.0) if out_kind == "s8" else dict(out_kind=out_kind, scale_a=0.02, scale_w=0.01)
+    want = oracle.gemm_i8(a, w, **kw)
+    dtype = torch.int8 if out_kind == "s8" else torch.float16
+    for lead, pitch in [(0, n), (1, n + 3), (3, n + 7)]:
+        flat = torch.full((m * pitch + lead,), 77, dtype=dtype, device=cuda_device)
+        out = flat[lead:].as_strided((m, n), (pitch, 1))
+        ops.gemm_i8(torch.from_numpy(a).to(cuda_device), torch.from_numpy(w).to(cuda_device), out=out, engine="umma", **kw)
+        assert np.array_equal(out.cpu().numpy(), want)
+        rest = flat.clone()
+        rest[lead:].as_strided((m, n), (pitch, 1)).fill_(77)
+        assert (rest == 77).all()
