@@ -636,10 +636,11 @@ int launch_skinny_mp(const I8Problem& p, const I8Epilogue& ep, const DeviceInfo&
 
 }  // namespace
 
-// Same operand rules as the square tensor-core engine, at most 128 activation rows.
+// The square tensor-core engine's operands with k contiguous in both (its tensor maps know no other
+// pose: a [K, N] weight runs on the square engine), at most 128 activation rows.
 bool skinny_i8_supported(const I8Problem& p)
 {
-    return p.m >= 1 && p.m <= 128 && umma_i8_supported(p);
+    return p.m >= 1 && p.m <= 128 && p.a_stride_k == 1 && p.w_stride_k == 1 && umma_i8_supported(p);
 }
 
 // Scratch for the equal-share split of K over all SMs, or 0 when it would not pay.  Publishing a

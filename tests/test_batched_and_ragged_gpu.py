@@ -91,3 +91,13 @@ def test_operands_off_the_tma_rule(cuda_device, nnb200_lib, case, zero_points):
 @pytest.mark.parametrize("m", [1, 7, 17])
 def test_few_rows_off_the_tma_rule(cuda_device, nnb200_lib, m):
     _check(cuda_device, 1, m, 9001, 1500 if m > 7 else 15001, zero_points=True, seed=m)
+
+
+@pytest.mark.parametrize("shape", [(1, 512, 1024), (16, 12800, 256), (24, 10000, 128), (8, 513, 1024), (5, 1001, 1000), (24, 10001, 200)])
+@pytest.mark.parametrize("pose", ["nn", "tn"])
+def test_few_rows_with_k_by_n_weights(cuda_device, nnb200_lib, shape, pose):
+    """Few rows whose operands are not k-contiguous, as they lie and through aligned copies."""
+    m, n, k = shape
+    if pose[0] == "t" and n % 16 == 0:
+        m = (m + 15) // 16 * 16
+    _check(cuda_device, 1, m, n, k, pose=pose, zero_points=True, seed=n)
