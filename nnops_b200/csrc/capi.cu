@@ -747,62 +747,32 @@ static int64_t two_pass_min_rows(const nnb200_q4_1_args* q)
 // layer is small, where this form's set-up and the exchange between the CTAs of a cluster weigh most.
 static constexpr int64_t kRowsUmmaMaxRows = 128;
 
-static bool q4_1_wants_rows_umma(const nnb200_q4_1_args* q)
+// `other`: the engine the call would run on without this form.  The CUDA-core GEMV (3) holds weights and
+// activations in f32; here a weight is rounded to f16 and an f32 activation becomes two f16 parts, as on every
+// tensor-core form.  So the calls that would run there stay there, slower as it is (8 f16 rows of
+// 11008 x 4000: 207 us against 28), and only those that are computed from f16 weights anyway come here.
+static bool q4_1_wants_rows_umma(const nnb200_q4_1_args* q, int other)
 {
     const int64_t b_rows = q->a_f16 != 0 ? q->m : 2 * q->m;
-    const bool few = q->m <= (q->a_f16 != 0 ? 8 : 2) && static_cast<double>(q->n) * q->k <= static_cast<double>(1 << 25) &&
-                     q4_1_gemv_mma_supported(*q);   // without it the GEMV runs on CUDA cores
+    const bool few = q->m <= (q->a_f16 != 0 ? 8 : 2) && static_cast<double>(q->n) * q->k <= static_cast<double>(1 << 25);
     // A K that 128 does not divide is padded to it; below 256 the other forms are as short.
     const bool k_ok = q->k % 128 == 0 || q->k >= 256;
-    const bool chosen = q->force_engine == 0 && q->m >= 2 && b_rows <= kRowsUmmaMaxRows && !few && k_ok;
+    const bool chosen = q->force_engine == 0 && other != 3 && q->m >= 2 && b_rows <= kRowsUmmaMaxRows && !few && k_ok;
     return (chosen || q->force_engine == 7) && q4_1_rows_umma_supported(*q);
 }
 
 // Scratch for f32 activations as pairs of f16 rows.
 static size_t q4_1_rows_scratch_bytes(const nnb200_q4_1_args* q)
 {
-    return static_cast<size_t>(q->m) * static_cast<size_t>(q4_1_rows_split_pitch(q->k)) * 4;
+    return q->a_f16 != 0 ? 0 : static_cast<size_t>(q->m) * static_cast<size_t>(q4_1_rows_split_pitch(q->k)) * 4;
 }
 
-size_t nnb200_q4_1_workspace_bytes(const nnb200_q4_1_args* q)
+// Engine for raw blocks other than weights in tensor memory.
+// 1 = fused tensor-core GEMM (tcgen05), 3 = GEMV on CUDA cores, 4 = GEMV with warp-level MMA
+// after per-weight dequantisation, 5 = two-pass GEMM (expand to f16 scratch, dense tcgen05
+// GEMM), 6 = GEMV with warp-level MMA on raw nibbles and deferred scaling.
+static int q4_1_other_engine(const nnb200_q4_1_args* q)
 {
-    if (!valid_q4_args(q) || q->m == 0 || q->n == 0) {
-        return 0;
-    }
-    // Optional: without it a tall call runs the fused kernel.
-    if (q4_1_wants_rows_umma(q)) {
-        return q->a_f16 != 0 ? 0 : q4_1_rows_scratch_bytes(q);
-    }
-    const bool wanted = q->force_engine == 5 || (q->force_engine == 0 && q->m >= two_pass_min_rows(q));
-    return wanted ? q4_1_two_pass_scratch_bytes(*q) : 0;
-}
-
-int nnb200_q4_1_engine(const nnb200_q4_1_args* q)
-{
-    if (!valid_q4_args(q)) {
-        return -1;
-    }
-    if (q->w_dm != nullptr) {
-        // Packed weights (separate nibble and (d, m) planes): the two-pass GEMM for tall calls that
-        // bring its scratch, else the deferred-scaling GEMV; -1 when neither can take the call.
-        if (q->force_engine == 0 || q->force_engine == 5) {
-            if (q->m >= two_pass_min_rows(q) && q4_1_two_pass_supported(*q)) {
-                return 5;
-            }
-        }
-        if (q->force_engine == 0 || q->force_engine == 2 || q->force_engine == 6) {
-            return q4_1_gemv_dsq_supported(*q) ? 6 : -1;
-        }
-        return -1;
-    }
-    if (q4_1_wants_rows_umma(q) &&
-        (q->a_f16 != 0 || (q->workspace != nullptr && q->workspace_bytes >= q4_1_rows_scratch_bytes(q) &&
-                           (reinterpret_cast<uintptr_t>(q->workspace) & 15u) == 0))) {
-        return 7;
-    }
-    // 1 = fused tensor-core GEMM (tcgen05), 3 = GEMV on CUDA cores, 4 = GEMV with warp-level MMA
-    // after per-weight dequantisation, 5 = two-pass GEMM (expand to f16 scratch, dense tcgen05
-    // GEMM), 6 = GEMV with warp-level MMA on raw nibbles and deferred scaling.
     int gemv = 3;
     if (q->force_engine != 3) {
         // Deferred scaling pays one fix-up per (channel, block, activation column), so it wins where
@@ -833,6 +803,55 @@ int nnb200_q4_1_engine(const nnb200_q4_1_args* q)
         return 5;
     }
     return (q->m > 8 && gemm_ok) ? 1 : gemv;
+}
+
+int nnb200_q4_1_engine(const nnb200_q4_1_args* q)
+{
+    if (!valid_q4_args(q)) {
+        return -1;
+    }
+    if (q->w_dm != nullptr) {
+        // Packed weights (separate nibble and (d, m) planes): the two-pass GEMM for tall calls that
+        // bring its scratch, else the deferred-scaling GEMV; -1 when neither can take the call.
+        if (q->force_engine == 0 || q->force_engine == 5) {
+            if (q->m >= two_pass_min_rows(q) && q4_1_two_pass_supported(*q)) {
+                return 5;
+            }
+        }
+        if (q->force_engine == 0 || q->force_engine == 2 || q->force_engine == 6) {
+            return q4_1_gemv_dsq_supported(*q) ? 6 : -1;
+        }
+        return -1;
+    }
+    const int other = q4_1_other_engine(q);
+    if (q4_1_wants_rows_umma(q, other) &&
+        (q->a_f16 != 0 || (q->workspace != nullptr && q->workspace_bytes >= q4_1_rows_scratch_bytes(q) &&
+                           (reinterpret_cast<uintptr_t>(q->workspace) & 15u) == 0))) {
+        return 7;
+    }
+    return other;
+}
+
+size_t nnb200_q4_1_workspace_bytes(const nnb200_q4_1_args* q)
+{
+    if (!valid_q4_args(q) || q->m == 0 || q->n == 0) {
+        return 0;
+    }
+    // Optional: without it a tall call runs the fused kernel.
+    const bool tall = q->force_engine == 5 || (q->force_engine == 0 && q->m >= two_pass_min_rows(q));
+    const size_t two_pass = tall ? q4_1_two_pass_scratch_bytes(*q) : 0;
+    // The least scratch with which the call runs with the weights in tensor memory.  (f32 rows whose GEMV
+    // would be the one on CUDA cores come there by way of the two-pass form, so with its scratch only.)
+    const size_t rows = q4_1_rows_scratch_bytes(q);
+    for (const size_t bytes : {rows, two_pass}) {
+        nnb200_q4_1_args given = *q;
+        given.workspace = bytes > 0 ? plan_scratch_stand_in() : nullptr;
+        given.workspace_bytes = bytes;
+        if (nnb200_q4_1_engine(&given) == 7) {
+            return bytes;
+        }
+    }
+    return two_pass;
 }
 
 int nnb200_linear_q4_1(const nnb200_q4_1_args* q, void* stream_v)

@@ -26,3 +26,31 @@ def test_few_rows_engine_takes_k_contiguous_operands_only(nnb200_lib, shape, pos
     from nnops_b200 import capi
     a = _i8(nnb200_lib, *shape, pose)
     assert capi.ENGINE_NAMES[nnb200_lib.nnb200_gemm_i8_engine(C.byref(a))] == "umma"
+
+
+def _q4(m, n, k, f16, *, ldw=None, force=0, workspace=None):
+    from nnops_b200 import capi
+    blocks = (k + 31) // 32
+    return capi.Q41Args(a=BASE, w_blocks=BASE + (1 << 32), out=BASE + (2 << 32), m=m, n=n, k=k, lda=(k + 7) // 8 * 8,
+                        ldw_blocks=ldw or blocks, ldc=n, a_f16=int(f16), out_f16=0, alpha=1.0, force_engine=force,
+                        workspace=BASE + (3 << 32) if workspace else None, workspace_bytes=workspace or 0)
+
+
+@pytest.mark.parametrize("k,ldw", [(1000, None), (352, None), (4128, None), (8992, None), (1024, 33)])
+def test_q4_1_calls_held_in_f32_stay_on_the_engine_that_does(nnb200_lib, k, ldw):
+    """K off the 128 rule, or rows off the 16-byte rule: few rows run on the CUDA-core GEMV, whose weights and
+    activations are f32, whatever scratch there is."""
+    engine = lambda q: nnb200_lib.nnb200_q4_1_engine(C.byref(q))
+    for n in (64, 11008, 40000):
+        for m, f16 in [(2, True), (8, True), (2, False), (16, False)]:
+            assert nnb200_lib.nnb200_q4_1_workspace_bytes(C.byref(_q4(m, n, k, f16, ldw=ldw))) == 0
+            assert engine(_q4(m, n, k, f16, ldw=ldw, workspace=1 << 33)) == 3, (m, n, f16)
+        # Where the other engine rounds the weights to f16 too, the weights go to tensor memory ...
+        assert engine(_q4(9, n, k, True, ldw=ldw)) == 7
+        need = nnb200_lib.nnb200_q4_1_workspace_bytes(C.byref(_q4(17, n, k, False, ldw=ldw)))
+        assert engine(_q4(17, n, k, False, ldw=ldw, workspace=need)) == 7
+        # ... for 17 and more f32 rows only with the scratch that brings them off the CUDA cores.
+        assert engine(_q4(17, n, k, False, ldw=ldw, workspace=need - 1)) == 3
+    for m, f16 in [(16, True), (128, True), (5, False), (64, False)]:
+        q = _q4(m, 4096, 4096, f16)
+        assert engine(_q4(m, 4096, 4096, f16, workspace=nnb200_lib.nnb200_q4_1_workspace_bytes(C.byref(q)))) == 7

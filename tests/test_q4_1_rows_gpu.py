@@ -72,3 +72,27 @@ def test_rows_pitched_and_chosen_by_itself(cuda_device, nnb200_lib):
     ops.linear_q4_1(a, wb, k, out=out[:, 8:8 + n])
     assert torch.equal(out[:, 8:8 + n], ops.linear_q4_1(a.contiguous(), wb, k, engine="rows"))
     assert (out[:, :8] == 7).all() and (out[:, 8 + n:] == 7).all()
+
+
+@pytest.mark.parametrize("shape,dtype,magnitude", [
+    ((2, 300, 1000), np.float32, 1e-6), ((8, 129, 352), np.float32, 1e5), ((13, 200, 4128), np.float32, 1e-6),
+    ((16, 64, 1004), np.float32, 1e5), ((5, 260, 1000), np.float32, 1.0),
+    ((2, 260, 1000), np.float16, 1.0), ((8, 130, 4128), np.float16, 1.0)])
+def test_few_rows_off_the_128_rule_are_computed_in_f32(cuda_device, nnb200_lib, shape, dtype, magnitude):
+    """The automatic choice against unrounded weights, over magnitudes that two f16 parts could not hold."""
+    m, n, k = shape
+    rng = np.random.default_rng(k)
+    wb = synth.q4_1_weights(rng, n, k)
+    a = (rng.standard_normal((m, k)) * magnitude).astype(dtype)
+    blocks = wb.reshape(n, -1, 20)
+    d, low = (blocks[:, :, i:i + 2].copy().view(np.float16).astype(np.float64) for i in (0, 2))
+    nibbles = np.concatenate([blocks[:, :, 4:] & 15, blocks[:, :, 4:] >> 4], axis=2).astype(np.float64)
+    w = (d * nibbles + low).reshape(n, -1)[:, :k]
+    got = ops.linear_q4_1(torch.from_numpy(a).to(cuda_device), torch.from_numpy(wb).to(cuda_device), k,
+                          out_dtype=torch.float32).cpu().numpy()
+    # f32 throughout: a rounding of the weight, a lane's chain of fused multiply-adds (32 to a block, every
+    # 32nd block its own), five additions over the lanes: that many times 2^-24 of the sum of magnitudes.
+    # (Weights rounded to f16 are off by up to 2^-11 of a term: 50 times as much.)
+    chain = 32 * -(-((k + 31) // 32) // 32) + 6
+    x = a.astype(np.float64)
+    assert (np.abs(got - x @ w.T) <= chain * 2.0 ** -24 * (np.abs(x) @ np.abs(w).T)).all()
