@@ -1,0 +1,19 @@
+"""What the Python front end refuses before it calls the library; no GPU, the blocks are never run."""
+import pytest
+import torch
+
+from nnops_b200 import ops
+
+
+def _args(a, w, out, **kw):
+    return ops.gemm_i8_args(torch.zeros(a, dtype=torch.int8), torch.zeros(w, dtype=torch.int8), torch.zeros(out, dtype=torch.int32),
+                            out_kind="s32", **kw)
+
+
+@pytest.mark.parametrize("a,w,out", [((2, 3, 16, 64), (32, 64), (16, 32)), ((16, 64), (2, 3, 32, 64), (16, 32)),
+                                     ((16, 64), (32, 64), (1, 2, 16, 32)), ((64,), (32, 64), (1, 32)), ((16, 64), (64,), (16, 1))])
+def test_only_matrices_and_batches_of_them(nnb200_lib, a, w, out):
+    with pytest.raises(ValueError):
+        _args(a, w, out)
+    assert _args((16, 64), (32, 64), (16, 32)).batch == 1
+    assert _args((3, 16, 64), (32, 64), (3, 16, 32)).batch == 3
