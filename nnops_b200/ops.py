@@ -62,6 +62,8 @@ def gemm_i8_args(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, out_kin
     if not (a.dim() in (2, 3) and w.dim() in (2, 3) and out.dim() in (2, 3)):
         raise ValueError("a, w and out must be matrices or batches of matrices")
     a_batch, w_batch, o_batch = (t.shape[0] if t.dim() == 3 else 1 for t in (a, w, out))
+    if 1 != a_batch != w_batch != 1:
+        raise ValueError("batch mismatch")
     m, k = a.shape[-2:]
     n = w.shape[-2]
     if w.shape[-1] != k:

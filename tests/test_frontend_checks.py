@@ -17,3 +17,11 @@ def test_only_matrices_and_batches_of_them(nnb200_lib, a, w, out):
         _args(a, w, out)
     assert _args((16, 64), (32, 64), (16, 32)).batch == 1
     assert _args((3, 16, 64), (32, 64), (3, 16, 32)).batch == 3
+
+
+def test_batches_agree_or_are_one(nnb200_lib):
+    """The kernels would walk the shorter batch past its end."""
+    for a, w in [(2, 3), (3, 2)]:
+        with pytest.raises(ValueError):
+            _args((a, 16, 64), (w, 32, 64), (3, 16, 32))
+    assert _args((1, 16, 64), (3, 32, 64), (3, 16, 32)).a_batch_stride == 0
