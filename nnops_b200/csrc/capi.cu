@@ -402,17 +402,49 @@ struct I8AlignPlan {
     nnb200_gemm_i8_args aligned;     // the call over the copies
 };
 
-// From this many multiply-adds on the copies pay: a copy launch and a tensor-core launch against one of
-// the generic engine take 7.6 / 11.2 us at 2^20.8, 8.4 / 28.5 at 2^25.4, 14.0 / 80.4 at 2^26, 41.8 / 1477 at
-// 2^33 (CUDA-graph timings); a problem of 2^19 is a single short wave of generic tiles.
-static constexpr int64_t kRealignMinMacs = int64_t{1} << 19;
+// Whether the copies pay.  The generic engine needs a step per 32 of K and 32 x 32 outputs, about 1.7 us
+// each as long as the device holds all tiles at once and 4.7 ns a tile beyond that, after 3 us; the
+// copies and the engine behind them 7 to 9 us where that is the square engine with few tiles, 11 to 15
+// where the rows are so few, or the channels so many, that another one is picked.  CUDA-graph timings,
+// us, generic / copies:
+//   M x N       K = 17        33            65           100          129          200          500
+//   16 x 1000                 5.7 / 12.8    7.2 / 13.1   9.8 / 12.6   11.4 / 13.1  16.1 / 12.8  35.0 / 13.4
+//   64 x 1000   5.3 / 7.8     7.0 / 7.9     8.6 / 8.1    11.7 / 7.8   13.3 / 8.2   19.0 / 8.0   41.3 / 8.5
+//   1024 x 1000 11.0 / 9.2    16.4 / 10.1   22.5 / 9.8   28.3 / 9.2   33.8 / 9.8   46.9 / 9.3   101 / 9.7
+//   64 x 10000  8.6 / 26.1    12.5 / 26.6   17.2 / 26.8  21.5 / 25.2  25.5 / 26.5  34.5 / 25.2  75.0 / 25.4
+//   256 x 10000 22.3 / 17.2   34.6 / 17.6   48.0 / 17.9  60.8 / 16.4  73.7 / 17.6  102 / 16.4   222 / 16.6
+//   2 x 100000  17.6 / 57.4   32.0 / 58.4   47.2 / 58.2  63.6 / 49.2  76.9 / 59.1  107 / 47.4   241 / 53.9
+// So: always from six steps up; from four with more than 16 rows where the square engine follows; from
+// three where the tiles fill the device many times; below that with both rows and channels enough for
+// that.  Operands that are not k-contiguous are copied as K long rows, too few of them to fill the
+// device while K is this short.  In a batch the generic engine is launched once a product, the copies
+// and the square engine once (64 x 33 x 33 x 33: 397 / 9.3, 8 x 200 x 200 x 50: 51.9 / 9.2).
+static bool i8_copies_pay(const nnb200_gemm_i8_args* a)
+{
+    const double macs = static_cast<double>(a->m) * a->n * a->k * a->batch;
+    if (macs < static_cast<double>(1 << 19)) {
+        return false;   // a single short wave of generic tiles
+    }
+    if (a->k > 160 || (a->batch >= 4 && a->m + a->n <= 2048)) {
+        return true;
+    }
+    if (a->a_stride_k != 1 || a->w_stride_k != 1) {
+        return false;
+    }
+    const DeviceInfo* dev = current_device_info();
+    const int64_t sms = dev != nullptr ? dev->sm_count : 148;
+    const bool square_follows = a->m > 64 || (a->m > 16 && a->n <= 64 * sms);
+    const int64_t tiles = ((a->m + 31) / 32) * ((a->n + 31) / 32);
+    return (a->k > 96 && square_follows) || (a->k > 64 && tiles * ((a->k + 31) / 32) >= 12000) ||
+           (a->m >= 128 && a->n >= 128 && static_cast<double>(a->m) * a->n >= static_cast<double>(1 << 19));
+}
 
 static I8AlignPlan i8_align_plan(const nnb200_gemm_i8_args* a, uint8_t* scratch)
 {
     I8AlignPlan plan;
     std::memset(&plan, 0, sizeof(plan));
     if (a->force_engine != NNB200_ENGINE_AUTO || sharded_out(a) || a->m > INT32_MAX || a->n > INT32_MAX ||
-        a->k > INT32_MAX || static_cast<double>(a->m) * a->n * a->k * a->batch < static_cast<double>(kRealignMinMacs)) {
+        a->k > INT32_MAX || !i8_copies_pay(a)) {
         return plan;
     }
     for (int64_t b = 0; b < (a->batch < 2 ? 1 : 2); ++b) {
@@ -726,8 +758,8 @@ static bool valid_q4_args(const nnb200_q4_1_args* q)
 // decoding them inside the GEMM (measured on config 4's weights: equal at 128 rows, 64 us
 // against 100 us at 256).
 static constexpr int64_t kTwoPassMinRows = 256;
-// f32 activations have no fused tensor-core form (their only other route walks the weights once
-// per 8 rows): the two-pass form, with the activations split into [hi | lo] f16, serves them from here up.
+// f32 activations have no fused tensor-core form (above 64 rows their only other route walks the weights
+// once per 8 rows): the two-pass form, with the activations split into [hi | lo] f16, serves them from here up.
 static constexpr int64_t kTwoPassMinRowsF32 = 17;
 
 static int64_t two_pass_min_rows(const nnb200_q4_1_args* q)

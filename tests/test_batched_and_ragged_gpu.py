@@ -101,3 +101,16 @@ def test_few_rows_with_k_by_n_weights(cuda_device, nnb200_lib, shape, pose):
     if pose[0] == "t" and n % 16 == 0:
         m = (m + 15) // 16 * 16
     _check(cuda_device, 1, m, n, k, pose=pose, zero_points=True, seed=n)
+
+
+@pytest.mark.parametrize("case", [
+    # m, n, k, pose: rows of one turn and more a warp, few long rows a block each, both with and without sums
+    (300, 300, 2100, "nt"), (300, 300, 9001, "nt"), (2, 1100, 2049, "nt"), (33, 5001, 260, "nn"), (40, 9999, 300, "tn"),
+    # K too short for the copies to pay: the generic engine
+    (2, 9000, 33, "nt"), (64, 1001, 64, "nn"), (16, 1000, 129, "nt")])
+@pytest.mark.parametrize("zero_points", [False, True])
+def test_copies_of_few_long_rows_and_short_k(cuda_device, nnb200_lib, case, zero_points):
+    m, n, k, pose = case
+    copied = k > 160
+    _check(cuda_device, 1, m, n, k, pose=pose, zero_points=zero_points, seed=m + k, out_kind="s32",
+           launches=None if zero_points else (2 if copied else 1))

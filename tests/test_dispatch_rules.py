@@ -54,3 +54,19 @@ def test_q4_1_calls_held_in_f32_stay_on_the_engine_that_does(nnb200_lib, k, ldw)
     for m, f16 in [(16, True), (128, True), (5, False), (64, False)]:
         q = _q4(m, 4096, 4096, f16)
         assert engine(_q4(m, 4096, 4096, f16, workspace=nnb200_lib.nnb200_q4_1_workspace_bytes(C.byref(q)))) == 7
+
+
+@pytest.mark.parametrize("call,pays", [
+    # Time falls from six generic steps of K up, from four with more than 16 rows, and with outputs enough.
+    ((1, 28672, 8191), True), ((16, 1000, 257), True), ((16, 1000, 129), False), ((33, 1000, 129), True), ((64, 10001, 129), False),
+    ((1, 100000, 33), False), ((2, 100000, 17), False), ((64, 100000, 65), True), ((1024, 1000, 17), True), ((64, 1000, 65), False),
+    ((3, 100, 300), False)])
+def test_copies_into_aligned_rows_only_where_they_pay(nnb200_lib, call, pays):
+    """The scratch asked for beyond the least is the copies' (K is off the 16-byte rule in every case)."""
+    m, n, k = call
+    a = _i8(nnb200_lib, m, n, k)
+    a.a_stride_m = a.w_stride_n = k
+    copies = nnb200_lib.nnb200_gemm_i8_workspace_bytes(C.byref(a)) - nnb200_lib.nnb200_gemm_i8_min_workspace_bytes(C.byref(a))
+    up = lambda v, to: -(-v // to) * to
+    want = sum(up(rows * up(k, 16), 256) for rows in (m, n)) if pays else 0
+    assert copies >= want and (copies == 0) == (want == 0)
