@@ -547,7 +547,21 @@ static bool i8_batched_call(const nnb200_gemm_i8_args* a, const DeviceInfo& dev,
     // Products whose outputs overlap keep the order of one launch after another.
     const bool apart = (a->out_batch_stride >= (a->m - 1) * a->ldc + a->n) ||
                        (a->out_batch_stride >= a->n && a->out_batch_stride * (a->batch - 1) + a->n <= a->ldc);
-    return apart && umma_i8_batched_supported(problem_of(a, 0), *b, dev);
+    if (!apart || !umma_i8_batched_supported(problem_of(a, 0), *b, dev)) {
+        return false;
+    }
+    // Few rows alone run on the streaming engine, which spreads one product's channels 16 to a CTA and its K
+    // over the warps; a tile here walks all of K.  Until the launches add up that is the slower way.
+    // The estimates, in 10 ns, are fits to CUDA-graph timings of 15 layers at 1 to 16 rows (us, alone /
+    // batched: 2 x 1 x 2048 x 3968 7.1 / 12.6, 4 x 8 x 512 x 15360 26.9 / 35.1, 6 x 4 x 64 x 65536 98.8 / 134;
+    // 8 x 1 x 2048 x 3968 31.5 / 15.0, 2 x 8 x 16384 x 448 15.2 / 9.2, 8 x 8 x 4032 x 2048 33.1 / 12.3).
+    if (a->force_engine == NNB200_ENGINE_AUTO && pick_i8_engine(a, problem_of(a, 0)) == NNB200_ENGINE_DECODE) {
+        const double kb = static_cast<double>((a->k + 127) / 128);
+        const double one = 230.0 + 0.01 * static_cast<double>(a->n) + 20.0 * static_cast<double>(a->m < 4 ? a->m : 4) +
+                           (a->m <= 8 ? 2.4 : 5.2) * kb;
+        return one * static_cast<double>(a->batch) > 550.0 + 28.0 * kb;
+    }
+    return true;
 }
 
 // One call's kernels.  `reserved`: bytes of the workspace between the sums and the optional

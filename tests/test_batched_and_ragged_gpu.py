@@ -114,3 +114,10 @@ def test_copies_of_few_long_rows_and_short_k(cuda_device, nnb200_lib, case, zero
     copied = k > 160
     _check(cuda_device, 1, m, n, k, pose=pose, zero_points=zero_points, seed=m + k, out_kind="s32",
            launches=None if zero_points else (2 if copied else 1))
+
+
+@pytest.mark.parametrize("batch,m,n,k,launches", [(2, 1, 512, 4096, 2), (3, 8, 256, 4096, 3), (2, 16, 1024, 1024, 2), (6, 4, 64, 16384, 6),
+                                                  (8, 8, 512, 1024, 1), (2, 17, 512, 4096, 1), (16, 1, 64, 16384, 1)])
+def test_few_rows_in_a_small_batch(cuda_device, nnb200_lib, batch, m, n, k, launches):
+    """A launch of the streaming engine each until one launch of the tile kernel is shorter."""
+    _check(cuda_device, batch, m, n, k, launches=launches, seed=k)
