@@ -800,9 +800,33 @@ static constexpr int64_t kRowsUmmaMaxRows = 128;
 static bool q4_1_wants_rows_umma(const nnb200_q4_1_args* q, int other)
 {
     const int64_t b_rows = q->a_f16 != 0 ? q->m : 2 * q->m;
-    const bool few = q->m <= (q->a_f16 != 0 ? 8 : 2) && static_cast<double>(q->n) * q->k <= static_cast<double>(1 << 25);
-    // A K that 128 does not divide is padded to it; below 256 the other forms are as short.
-    const bool k_ok = q->k % 128 == 0 || q->k >= 256;
+    // The GEMV serves up to 8 f16 or 4 f32 rows in one pass of the weights.
+    const double weights = static_cast<double>(q->n) * q->k;
+    const bool few = (q->m <= (q->a_f16 != 0 ? 8 : 2) && weights <= static_cast<double>(1 << 25)) ||
+                     (q->a_f16 == 0 && q->m <= 4 && q->n <= 4096 && q->k <= 2048 && weights <= static_cast<double>(1 << 22));
+    // The forms with the activations as the 128-row operand cost about 5 us and 1 for each 100 of K; this one
+    // costs its set-up and what a row costs to write out, more where the CTAs of a cluster add up their parts
+    // first (layers of up to 74 tiles on 148 SMs, K beyond one unit).  A K that 128 does not divide comes in
+    // smaller copies and is padded to it.  us, the best other form / this one:
+    //   f16, N = 4096    K = 256      384         512         768         288         544
+    //   33 rows          8.1 / 5.8    9.4 / 8.0   11.0 / 8.1  13.7 / 8.0  9.3 / 9.9   12.2 / 10.0
+    //   64 rows          8.1 / 6.5    9.3 / 9.7   11.0 / 9.8  13.7 / 9.5  9.2 / 11.5  11.9 / 11.4
+    //   128 rows         8.4 / 13.1   10.0 / 12.1 11.3 / 11.3 14.0 / 11.7 9.2 / 12.7  12.2 / 12.3
+    //   N = 9472, 128    9.2 / 13.3   10.5 / 13.8 12.1 / 13.9 14.8 / 14.8 10.1 / 14.3 12.7 / 15.4
+    //   N = 14336, 128   9.0 / 8.6    10.4 / 9.4  11.9 / 10.1 14.8 / 11.5 9.8 / 10.4  12.7 / 12.1
+    //   f32, N = 2048, 64 10.4 / 11.5 11.6 / 11.2 12.9 / 10.8 15.6 / 10.5 11.2 / 11.7 13.9 / 11.0
+    const DeviceInfo* dev = current_device_info();
+    const bool shared = (q->n + 127) / 128 * 2 <= (dev != nullptr ? dev->sm_count : 148);
+    const int64_t pad = q->k % 128 == 0 ? 0 : 192;
+    bool k_ok = pad == 0 || q->k >= 256;
+    if (q->a_f16 == 0) {
+        k_ok = k_ok && (q->n > 4096 || q->k >= 5 * q->m);
+    } else if (!shared) {
+        k_ok = k_ok && (pad == 0 || q->k > 3 * q->m + pad);
+    } else {
+        const int64_t per_row = q->m <= 64 ? 7 : (q->n <= 4096 ? 4 : 6);
+        k_ok = (pad == 0 && q->m <= 64 && q->k <= 256) || q->k >= per_row * q->m + pad;
+    }
     const bool chosen = q->force_engine == 0 && other != 3 && q->m >= 2 && b_rows <= kRowsUmmaMaxRows && !few && k_ok;
     return (chosen || q->force_engine == 7) && q4_1_rows_umma_supported(*q);
 }

@@ -576,32 +576,51 @@ q4_1_rows_umma_kernel(const __grid_constant__ CUtensorMap map_a, const uint8_t* 
     }
 }
 
+// `split`: the most CTAs that may share a tile.
 template <bool OUT_F16, int BLOCKS, int PIECE>
-int launch_variant(const CUtensorMap& map_a, const Q4RowsCall& c, int nb, int tile_rows, int split, int ctas,
+int launch_variant(const CUtensorMap& map_a, const Q4RowsCall& c, int nb, int tile_rows, int split, int tiles,
                    const FpEpilogue& ep, const DeviceInfo& dev, cudaStream_t stream)
 {
     using Cfg = RowsConfig<BLOCKS>;
     auto kernel = q4_1_rows_umma_kernel<OUT_F16, BLOCKS, PIECE>;
     static std::once_flag once[kMaxDevices];
     static cudaError_t attr_err[kMaxDevices];
-    std::call_once(once[dev.device], [&] {
-        attr_err[dev.device] = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
-    });
-    if (attr_err[dev.device] != cudaSuccess) {
-        return NNB200_INTERNAL;
-    }
+    static int resident[kMaxDevices][kMaxSplit + 1];   // clusters of that many CTAs the device holds at once
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(ctas));
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = Cfg::kSmemBytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = static_cast<unsigned>(split);
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    std::call_once(once[dev.device], [&] {
+        attr_err[dev.device] = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+        for (int s = 2; s <= kMaxSplit && attr_err[dev.device] == cudaSuccess; ++s) {
+            attr[0].val.clusterDim.x = static_cast<unsigned>(s);
+            cfg.gridDim = dim3(static_cast<unsigned>(dev.sm_count / s * s));
+            int count = 0;
+            if (cudaOccupancyMaxActiveClusters(&count, kernel, &cfg) == cudaSuccess) {
+                resident[dev.device][s] = count;
+            } else {
+                (void)cudaGetLastError();   // no clusters of that many: the launch takes a smaller one
+            }
+        }
+    });
+    if (attr_err[dev.device] != cudaSuccess) {
+        return NNB200_INTERNAL;
+    }
+    // Clusters live within a group of SMs, so fewer of them fit than the SMs would hold: sixteen of eight do
+    // not, and a second turn for the last ones costs more than all (2048 channels, K = 4096: 4 f32 rows 14.3 ->
+    // 9.6 us; K = 1024: 128 f16 rows 17.5 -> 10.5).
+    while (split > 1 && resident[dev.device][split] < tiles) {
+        --split;
+    }
+    const int ctas = split > 1 ? tiles * split : (tiles < dev.sm_count ? tiles : dev.sm_count);
+    attr[0].val.clusterDim.x = static_cast<unsigned>(split);
+    cfg.gridDim = dim3(static_cast<unsigned>(ctas));
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, map_a, static_cast<const uint8_t*>(c.q->w_blocks),
                                              c.q->ldw_blocks * kQ4BlockBytes, c.q->out, c.q->ldc, static_cast<int>(c.q->m),
                                              c.hi_lo ? 1 : 0, nb, static_cast<int>(c.q->n), static_cast<int>(c.q->k), tile_rows,
@@ -655,7 +674,6 @@ int launch_q4_1_rows_umma(const Q4RowsCall& c, const DeviceInfo& dev, cudaStream
     int tile_rows = (n + tiles - 1) / tiles;
     tile_rows = tile_rows > kTileRows ? kTileRows : tile_rows;
     tiles = (n + tile_rows - 1) / tile_rows;
-    const int ctas = split > 1 ? tiles * split : (tiles < dev.sm_count ? tiles : dev.sm_count);
 
     CUtensorMap map_a;
     if (!make_tma_2d(&map_a, c.a, 2, static_cast<uint64_t>(q.k), static_cast<uint64_t>(b_rows),
@@ -666,11 +684,11 @@ int launch_q4_1_rows_umma(const Q4RowsCall& c, const DeviceInfo& dev, cudaStream
     const auto launch = [&](auto piece) {
         constexpr int P = decltype(piece)::value;
         if (wide) {
-            return q.out_f16 ? launch_variant<true, 4, P>(map_a, c, nb, tile_rows, split, ctas, ep, dev, stream)
-                             : launch_variant<false, 4, P>(map_a, c, nb, tile_rows, split, ctas, ep, dev, stream);
+            return q.out_f16 ? launch_variant<true, 4, P>(map_a, c, nb, tile_rows, split, tiles, ep, dev, stream)
+                             : launch_variant<false, 4, P>(map_a, c, nb, tile_rows, split, tiles, ep, dev, stream);
         }
-        return q.out_f16 ? launch_variant<true, 8, P>(map_a, c, nb, tile_rows, split, ctas, ep, dev, stream)
-                         : launch_variant<false, 8, P>(map_a, c, nb, tile_rows, split, ctas, ep, dev, stream);
+        return q.out_f16 ? launch_variant<true, 8, P>(map_a, c, nb, tile_rows, split, tiles, ep, dev, stream)
+                         : launch_variant<false, 8, P>(map_a, c, nb, tile_rows, split, tiles, ep, dev, stream);
     };
     if ((row_bits & 15u) == 0) {
         return launch(std::integral_constant<int, 16>{});

@@ -70,3 +70,17 @@ def test_copies_into_aligned_rows_only_where_they_pay(nnb200_lib, call, pays):
     up = lambda v, to: -(-v // to) * to
     want = sum(up(rows * up(k, 16), 256) for rows in (m, n)) if pays else 0
     assert copies >= want and (copies == 0) == (want == 0)
+
+
+@pytest.mark.parametrize("m,n,k,f16,engine", [
+    # parts of a cluster to add up: K beyond one unit has to pay for it
+    (33, 4096, 384, True, 7), (64, 4096, 256, True, 7), (64, 4096, 384, True, 1), (64, 4096, 512, True, 7), (65, 4096, 256, True, 1),
+    (128, 4096, 384, True, 1), (128, 4096, 512, True, 7), (128, 9472, 640, True, 1), (128, 9472, 768, True, 7),
+    (33, 4096, 288, True, 1), (64, 4096, 672, True, 7), (9, 4096, 128, True, 7),
+    # a tile a CTA
+    (128, 14336, 256, True, 7), (64, 14336, 288, True, 1), (64, 28672, 416, True, 7),
+    (3, 1024, 1024, False, 4), (4, 4096, 1024, False, 4), (5, 1024, 1024, False, 7), (3, 4096, 4096, False, 7), (3, 14336, 256, False, 7),
+    (64, 2048, 256, False, 5), (64, 2048, 384, False, 7), (64, 14336, 256, False, 7)])
+def test_q4_1_weights_in_tensor_memory_where_k_is_long_enough(nnb200_lib, m, n, k, f16, engine):
+    need = nnb200_lib.nnb200_q4_1_workspace_bytes(C.byref(_q4(m, n, k, f16)))
+    assert nnb200_lib.nnb200_q4_1_engine(C.byref(_q4(m, n, k, f16, workspace=need))) == engine
