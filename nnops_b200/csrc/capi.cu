@@ -827,7 +827,8 @@ static bool q4_1_wants_rows_umma(const nnb200_q4_1_args* q, int other)
         const int64_t per_row = q->m <= 64 ? 7 : (q->n <= 4096 ? 4 : 6);
         k_ok = (pad == 0 && q->m <= 64 && q->k <= 256) || q->k >= per_row * q->m + pad;
     }
-    const bool chosen = q->force_engine == 0 && other != 3 && q->m >= 2 && b_rows <= kRowsUmmaMaxRows && !few && k_ok;
+    // Deferred scaling for more than one row is what knob Q4_GEMV = 2 asks for.
+    const bool chosen = q->force_engine == 0 && other != 3 && other != 6 && q->m >= 2 && b_rows <= kRowsUmmaMaxRows && !few && k_ok;
     return (chosen || q->force_engine == 7) && q4_1_rows_umma_supported(*q);
 }
 

@@ -20,6 +20,9 @@
 //     memory and the MMAs of different units overlap.
 //   * Few channels: `split` CTAs (a cluster) share a tile's K and add up their accumulators
 //     through distributed shared memory in a fixed order -- the result does not depend on timing.
+//   * Launched with programmatic stream serialization when the caller allows it
+//     (NNB200_Q4_FLAG_OVERLAP_PREVIOUS): barriers, tensor memory and the first units' weights are set up
+//     before griddepcontrol.wait, activations (by TMA, never through L1) read and outputs written after it.
 //   * f32 activations are given as two f16 rows each, high part and remainder; the epilogue adds the
 //     two accumulator columns (see split_f32_to_f16_kernel).
 //
@@ -276,6 +279,10 @@ q4_1_rows_umma_kernel(const __grid_constant__ CUtensorMap map_a, const uint8_t* 
         tmem_alloc(tmem_slot, kTmemCols);
         tmem_relinquish();
     }
+    // Let the next kernel in the stream begin its own prologue; then nothing but weights is touched before
+    // the previous one has completed.  No-ops for a launch without the programmatic-serialization attribute.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -590,10 +597,12 @@ int launch_variant(const CUtensorMap& map_a, const Q4RowsCall& c, int nb, int ti
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = Cfg::kSmemBytes;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     std::call_once(once[dev.device], [&] {
@@ -621,6 +630,7 @@ int launch_variant(const CUtensorMap& map_a, const Q4RowsCall& c, int nb, int ti
     const int ctas = split > 1 ? tiles * split : (tiles < dev.sm_count ? tiles : dev.sm_count);
     attr[0].val.clusterDim.x = static_cast<unsigned>(split);
     cfg.gridDim = dim3(static_cast<unsigned>(ctas));
+    cfg.numAttrs = (c.q->flags & NNB200_Q4_FLAG_OVERLAP_PREVIOUS) != 0 ? 2 : 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, map_a, static_cast<const uint8_t*>(c.q->w_blocks),
                                              c.q->ldw_blocks * kQ4BlockBytes, c.q->out, c.q->ldc, static_cast<int>(c.q->m),
                                              c.hi_lo ? 1 : 0, nb, static_cast<int>(c.q->n), static_cast<int>(c.q->k), tile_rows,

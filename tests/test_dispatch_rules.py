@@ -84,3 +84,12 @@ def test_copies_into_aligned_rows_only_where_they_pay(nnb200_lib, call, pays):
 def test_q4_1_weights_in_tensor_memory_where_k_is_long_enough(nnb200_lib, m, n, k, f16, engine):
     need = nnb200_lib.nnb200_q4_1_workspace_bytes(C.byref(_q4(m, n, k, f16)))
     assert nnb200_lib.nnb200_q4_1_engine(C.byref(_q4(m, n, k, f16, workspace=need))) == engine
+
+
+def test_q4_gemv_knob_comes_before_the_weights_in_tensor_memory(nnb200_lib, knobs):
+    engine = lambda m, f16: nnb200_lib.nnb200_q4_1_engine(C.byref(_q4(m, 28672, 4096, f16, workspace=1 << 33)))
+    assert (engine(4, True), engine(4, False), engine(1, True)) == (7, 7, 6)
+    knobs("q4_gemv", 2)
+    assert (engine(4, True), engine(4, False), engine(1, True)) == (6, 6, 6)
+    knobs("q4_gemv", 1)
+    assert (engine(4, True), engine(4, False), engine(1, True)) == (7, 7, 4)

@@ -96,3 +96,26 @@ def test_few_rows_off_the_128_rule_are_computed_in_f32(cuda_device, nnb200_lib, 
     chain = 32 * -(-((k + 31) // 32) // 32) + 6
     x = a.astype(np.float64)
     assert (np.abs(got - x @ w.T) <= chain * 2.0 ** -24 * (np.abs(x) @ np.abs(w).T)).all()
+
+
+@pytest.mark.parametrize("n", [1024, 9600])   # clusters that share K; a tile a CTA
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_overlap_with_the_preceding_kernel(cuda_device, nnb200_lib, n, dtype):
+    """Each call reads what the one before wrote, and what a kernel without the attribute wrote."""
+    rng = np.random.default_rng(n)
+    wb = torch.from_numpy(synth.q4_1_weights(rng, n, n)).to(cuda_device)
+    x0 = torch.from_numpy(rng.standard_normal((16, n))).to(device=cuda_device, dtype=dtype)
+
+    def chain(overlap):
+        x, seen = x0 * 1.0, []
+        for step in range(6):
+            x = ops.linear_q4_1(x, wb, n, alpha=0.02, out_dtype=dtype, engine="rows", overlap_previous=overlap)
+            if step == 2:
+                x = x * 1.5
+            seen.append(x)
+        return torch.stack(seen)
+
+    want = chain(False)
+    assert torch.isfinite(want).all() and want.abs().max() > 0
+    for _ in range(5):
+        assert torch.equal(chain(True), want)
