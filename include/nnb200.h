@@ -63,6 +63,8 @@ extern "C" {
 #define NNB200_ENGINE_DECODE 4  /* M <= 16, K % 64 == 0: streaming loads + warp MMA        */
 #define NNB200_ENGINE_SKINNY 5  /* M <= 128: tcgen05 with the weights as the 128-row operand */
 
+#define NNB200_ZP_NOT_KNOWN 2   /* zp_a_nonzero / zp_w_nonzero: the caller has not looked */
+
 /*
  * One int8 matmul call: out[b][m][n] = epilogue( sum_k A[b][m][k] * W[b][n][k] ).
  * Replaces the parameter block the reference launcher takes
@@ -118,7 +120,9 @@ typedef struct nnb200_gemm_i8_args {
     float scale_a_scalar, scale_w_scalar;
     int32_t zp_a_scalar, zp_w_scalar;
     int32_t zp_a_nonzero; /* caller's promise about the ARRAYS: 0 = every zp_a[] entry is 0 */
-    int32_t zp_w_nonzero; /* (lets the backend skip the R_a / R_w sweeps); scalars are checked here */
+    int32_t zp_w_nonzero; /* (lets the backend skip the R_a / R_w sweeps); scalars are checked here.
+                             NNB200_ZP_NOT_KNOWN: the sweeps look at the entries on the device first
+                             and read no operand when all are 0. */
     float out_scale;
     int32_t out_zp;
     void* workspace;

@@ -70,6 +70,7 @@ class Q41Args(C.Structure):
 
 
 Q4_FLAG_OVERLAP_PREVIOUS = 1
+ZP_NOT_KNOWN = 2   # whether an array of zero points holds anything but zeros: looked at on the device
 
 # Every symbol include/nnb200.h declares: (name, restype, argtypes).
 ZP_S8, ZP_U8, ZP_S32 = 0, 1, 2   # nnb200_quant_linear_args.zp_unsigned: storage type of the zero points

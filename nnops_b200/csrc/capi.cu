@@ -669,8 +669,12 @@ static int run_gemm_i8(const nnb200_gemm_i8_args* a, const DeviceInfo* dev, cuda
                 const bool sa = sweep_a && !(shared_a && e > b);
                 const bool sw = sweep_w && !(shared_w && e > b);
                 if (sa || sw) {
-                    const int st = launch_i8_sums(problem_of(a, e), sa ? r_a + (e - b) * (slot / 4) : nullptr,
-                                                  sw ? r_w + (e - b) * (slot / 4) : nullptr, stream);
+                    I8Sums sums;
+                    sums.r_a = sa ? r_a + (e - b) * (slot / 4) : nullptr;
+                    sums.r_w = sw ? r_w + (e - b) * (slot / 4) : nullptr;
+                    sums.look_w = a->zp_w_scalar == 0 && a->zp_w_nonzero == NNB200_ZP_NOT_KNOWN ? a->zp_w : nullptr;
+                    sums.look_a = a->zp_a_scalar == 0 && a->zp_a_nonzero == NNB200_ZP_NOT_KNOWN ? a->zp_a : nullptr;
+                    const int st = launch_i8_sums(problem_of(a, e), sums, *dev, stream);
                     if (st != NNB200_OK) {
                         return st;
                     }

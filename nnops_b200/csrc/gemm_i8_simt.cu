@@ -83,42 +83,67 @@ __global__ void __launch_bounds__(256) gemm_i8_generic_kernel(const I8Problem p,
     }
 }
 
-// One block per row of a [rows, k] int8 matrix with arbitrary strides.
+// Whether any of the `count` zero points differs from zero; the same answer for the whole block.
+__device__ __forceinline__ bool any_zero_point(const int32_t* zp, int64_t count)
+{
+    constexpr int kEach = 16;   // in flight at once: one round trip for 2048 of them
+    for (int64_t base = 0; base < count; base += kEach * 128) {
+        int32_t any = 0;
+#pragma unroll
+        for (int j = 0; j < kEach; ++j) {
+            const int64_t i = base + j * 128 + threadIdx.x;
+            any |= i < count ? zp[i] : 0;
+        }
+        if (__syncthreads_or(any) != 0) {
+            return true;
+        }
+    }
+    return false;
+}
+
+// The sum of each row of a [rows, k] int8 matrix with arbitrary strides, a block to a row.  `look`: the
+// zero points that the sums will be multiplied with, when the caller does not know whether any is
+// non-zero; if none is, the matrix is not read and the sums stay as they are.
 template <bool UNSIGNED>
 __global__ void __launch_bounds__(128) i8_sums_kernel(const uint8_t* x, int64_t rows, int64_t k, int64_t stride_row,
-                                                      int64_t stride_k, int32_t* out)
+                                                      int64_t stride_k, int32_t* out, const int32_t* look, int64_t look_count)
 {
-    const int64_t r = blockIdx.x;
-    const uint8_t* row = x + r * stride_row;
-    int32_t s = 0;
-    if (stride_k == 1 && (reinterpret_cast<uintptr_t>(row) & 3u) == 0) {
-        const int64_t k4 = k / 4;
-        const uint32_t* row4 = reinterpret_cast<const uint32_t*>(row);
-        for (int64_t i = threadIdx.x; i < k4; i += blockDim.x) {
-            const uint32_t v = row4[i];
-            s = UNSIGNED ? __dp4a(v, 0x01010101u, static_cast<uint32_t>(s))
-                         : __dp4a(static_cast<int32_t>(v), 0x01010101, s);
-        }
-        for (int64_t i = k4 * 4 + threadIdx.x; i < k; i += blockDim.x) {
-            s += UNSIGNED ? static_cast<int32_t>(row[i]) : static_cast<int32_t>(static_cast<int8_t>(row[i]));
-        }
-    } else {
-        for (int64_t i = threadIdx.x; i < k; i += blockDim.x) {
-            const uint8_t v = row[i * stride_k];
-            s += UNSIGNED ? static_cast<int32_t>(v) : static_cast<int32_t>(static_cast<int8_t>(v));
-        }
+    if (look != nullptr && !any_zero_point(look, look_count)) {
+        return;
     }
     __shared__ int32_t part[4];
+    for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
+        const uint8_t* row = x + r * stride_row;
+        int32_t s = 0;
+        if (stride_k == 1 && (reinterpret_cast<uintptr_t>(row) & 3u) == 0) {
+            const int64_t k4 = k / 4;
+            const uint32_t* row4 = reinterpret_cast<const uint32_t*>(row);
+            for (int64_t i = threadIdx.x; i < k4; i += blockDim.x) {
+                const uint32_t v = row4[i];
+                s = UNSIGNED ? __dp4a(v, 0x01010101u, static_cast<uint32_t>(s))
+                             : __dp4a(static_cast<int32_t>(v), 0x01010101, s);
+            }
+            for (int64_t i = k4 * 4 + threadIdx.x; i < k; i += blockDim.x) {
+                s += UNSIGNED ? static_cast<int32_t>(row[i]) : static_cast<int32_t>(static_cast<int8_t>(row[i]));
+            }
+        } else {
+            for (int64_t i = threadIdx.x; i < k; i += blockDim.x) {
+                const uint8_t v = row[i * stride_k];
+                s += UNSIGNED ? static_cast<int32_t>(v) : static_cast<int32_t>(static_cast<int8_t>(v));
+            }
+        }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        part[threadIdx.x >> 5] = s;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        out[r] = part[0] + part[1] + part[2] + part[3];
+        for (int o = 16; o > 0; o >>= 1) {
+            s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+        }
+        if ((threadIdx.x & 31) == 0) {
+            part[threadIdx.x >> 5] = s;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            out[r] = part[0] + part[1] + part[2] + part[3];
+        }
+        __syncthreads();
     }
 }
 
@@ -254,22 +279,30 @@ int launch_gemm_i8_narrow(const I8Problem& p, const I8Epilogue& ep, const Device
     return cuda_status(cudaGetLastError());
 }
 
-int launch_i8_sums(const I8Problem& p, int32_t* r_a, int32_t* r_w, cudaStream_t stream)
+int launch_i8_sums(const I8Problem& p, const I8Sums& sums, const DeviceInfo& dev, cudaStream_t stream)
 {
     // Either destination may be null: that sweep is skipped.
     const uint8_t* a = static_cast<const uint8_t*>(p.a);
     const uint8_t* w = static_cast<const uint8_t*>(p.w);
-    if (r_a != nullptr) {
+    // A block looks at the zero points once, so with them there are only as many blocks as the device holds.
+    const auto grid = [&](int64_t rows, const int32_t* look) {
+        const int64_t most = static_cast<int64_t>(dev.sm_count) * 16;
+        return static_cast<unsigned>(look != nullptr && rows > most ? most : rows);
+    };
+    if (sums.r_a != nullptr) {
         if (p.a_unsigned) {
-            i8_sums_kernel<true><<<static_cast<unsigned>(p.m), 128, 0, stream>>>(a, p.m, p.k, p.a_stride_m, p.a_stride_k, r_a);
+            i8_sums_kernel<true><<<grid(p.m, sums.look_w), 128, 0, stream>>>(a, p.m, p.k, p.a_stride_m, p.a_stride_k, sums.r_a,
+                                                                             sums.look_w, p.n);
         } else {
-            i8_sums_kernel<false><<<static_cast<unsigned>(p.m), 128, 0, stream>>>(a, p.m, p.k, p.a_stride_m, p.a_stride_k, r_a);
+            i8_sums_kernel<false><<<grid(p.m, sums.look_w), 128, 0, stream>>>(a, p.m, p.k, p.a_stride_m, p.a_stride_k, sums.r_a,
+                                                                              sums.look_w, p.n);
         }
     }
-    if (r_w != nullptr) {
-        i8_sums_kernel<false><<<static_cast<unsigned>(p.n), 128, 0, stream>>>(w, p.n, p.k, p.w_stride_n, p.w_stride_k, r_w);
+    if (sums.r_w != nullptr) {
+        i8_sums_kernel<false><<<grid(p.n, sums.look_a), 128, 0, stream>>>(w, p.n, p.k, p.w_stride_n, p.w_stride_k, sums.r_w,
+                                                                          sums.look_a, p.m);
     }
-    note_launch((r_a != nullptr ? 1 : 0) + (r_w != nullptr ? 1 : 0));
+    note_launch((sums.r_a != nullptr ? 1 : 0) + (sums.r_w != nullptr ? 1 : 0));
     return cuda_status(cudaGetLastError());
 }
 

@@ -163,7 +163,15 @@ bool skinny_i8_supported(const I8Problem& p);
 
 // R_a[m] = sum_k A[m][k] and R_w[n] = sum_k W[n][k] into int32 scratch; r_w == nullptr skips the
 // sweep over W (the caller has the sums already).
-int launch_i8_sums(const I8Problem& p, int32_t* r_a, int32_t* r_w, cudaStream_t stream);
+// Row sums of the operands, null = not wanted.  look_w / look_a: the zero points that r_a / r_w will be
+// multiplied with, if only the device knows whether any of them is non-zero (else null).
+struct I8Sums {
+    int32_t* r_a;
+    int32_t* r_w;
+    const int32_t* look_w;   // [n]
+    const int32_t* look_a;   // [m]
+};
+int launch_i8_sums(const I8Problem& p, const I8Sums& sums, const DeviceInfo& dev, cudaStream_t stream);
 
 int launch_q4_1_gemv(const nnb200_q4_1_args& a, const DeviceInfo& dev, cudaStream_t stream);
 int launch_q4_1_gemv_mma(const nnb200_q4_1_args& a, const DeviceInfo& dev, cudaStream_t stream);

@@ -77,8 +77,8 @@ def gemm_i8_args(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, out_kin
         bias = _on_device(bias, torch.int32 if out_kind in ("s32", "s8", "u8") else _OUT_TORCH[out_kind], dev)
         keep.append(bias)
 
-    # Whether an ARRAY of zero points holds anything but zeros is not looked at: that would wait for
-    # the device on every call, and only to save the row sums.
+    # Whether an ARRAY of zero points holds anything but zeros is left for the device to see: looking here
+    # would wait for it on every call.
     args = capi.block(
         capi.GemmI8Args, a.data_ptr(), w.data_ptr(), out.data_ptr(), m, n, k,
         a.stride(-2), a.stride(-1) if k > 1 else 1, w.stride(-2), w.stride(-1) if k > 1 else 1, out.stride(-2),
@@ -89,8 +89,8 @@ def gemm_i8_args(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, out_kin
         sa.data_ptr() if sa is not None else 0, sw.data_ptr() if sw is not None else 0,
         za.data_ptr() if za is not None else 0, zw.data_ptr() if zw is not None else 0,
         1.0 if sa0 is None else float(sa0), 1.0 if sw0 is None else float(sw0),
-        0 if za0 is None else int(za0), 0 if zw0 is None else int(zw0), int(za is not None), int(zw is not None),
-        float(out_scale), int(out_zp))
+        0 if za0 is None else int(za0), 0 if zw0 is None else int(zw0),
+        capi.ZP_NOT_KNOWN if za is not None else 0, capi.ZP_NOT_KNOWN if zw is not None else 0, float(out_scale), int(out_zp))
     if engine != "auto":
         args.force_engine = capi.ENGINES[engine]
     if r_w is not None:
