@@ -127,6 +127,12 @@ def build_tests(force=False) -> list[Path]:
         _run([CXX, *COMMON, "-o", out, shard_src, f"-L{LIB_DIR}", "-lnnb200", *cuda, "-lrt", "-pthread",
               *_rpath(LIB_DIR, CUDA_HOME / "lib64")])
     outs.append(out)
+    # The backend's way round a failed allocation; the program fakes the library calls that need a GPU.
+    scratch_src = ROOT / "tests" / "cpp" / "test_scratch.cpp"
+    out = BIN_DIR / "test_scratch"
+    if force or _stale(out, [scratch_src, host_lib]):
+        _run([CXX, *COMMON, "-o", out, scratch_src, f"-L{LIB_DIR}", "-lnnb200_host", "-lnnb200", *_rpath(LIB_DIR)])
+    outs.append(out)
     bench_src = ROOT / "tests" / "cpp" / "bench_linear_op.cpp"
     out = BIN_DIR / "bench_linear_op_standalone"
     if force or _stale(out, [bench_src, host_lib]):

@@ -195,15 +195,20 @@ Status run_i8(const I8Call& c, const ComputeContext& ctx)
     if (qa.zero_point != 0 || qw.zero_point != 0 || qa.zero_point_data != nullptr || qw.zero_point_data != nullptr) {
         st.reserve_raw(((m_bytes + 255) & ~size_t(255)) + ((n_bytes + 255) & ~size_t(255)));
     }
-    // Optional scratch with which the few-row engine shares K evenly among the SMs.  The library
-    // sizes it from shapes and pointers alone (zero points do not enter), so the block as filled
-    // so far is enough to ask.
+    // Optional scratch: with it the few-row engine shares K evenly among the SMs, and operands off the
+    // 16-byte rule are copied into aligned rows.  The library sizes it from shapes and pointers alone
+    // (zero points do not enter), so the block as filled so far is enough to ask.
     g.a = a.ptr<void>();
     g.w = w.ptr<void>();
     g.out = out.ptr<void>();
-    st.reserve_raw(nnb200_gemm_i8_workspace_bytes(&g) - nnb200_gemm_i8_min_workspace_bytes(&g));
+    size_t optional = nnb200_gemm_i8_workspace_bytes(&g) - nnb200_gemm_i8_min_workspace_bytes(&g);
+    st.reserve_raw(optional);
     if (const int e = st.allocate(); e != NNB200_OK) {
-        return to_status(e);
+        // The copies can be as large as the weight; the call runs without, only slower.
+        if (optional == 0 || st.allocate_without(optional) != NNB200_OK) {
+            return to_status(e);
+        }
+        optional = 0;
     }
     DeviceArray sa, za, sw, zw;
     for (const int e : {st.place(qa.scale_data, m_bytes, false, sa), st.place(qa.zero_point_data, m_bytes, true, za)}) {
@@ -239,7 +244,7 @@ Status run_i8(const I8Call& c, const ComputeContext& ctx)
     g.w = w.ptr<void>();
     g.out = out.ptr<void>();
     // Zero-point scratch is sized from the argument block; reserve it now that the block is final.
-    const size_t need = nnb200_gemm_i8_workspace_bytes(&g);
+    const size_t need = optional > 0 ? nnb200_gemm_i8_workspace_bytes(&g) : nnb200_gemm_i8_min_workspace_bytes(&g);
     if (need > 0) {
         g.workspace = st.take_raw(need);
         g.workspace_bytes = need;

@@ -63,6 +63,12 @@ public:
     }
     void reserve_raw(size_t bytes) { total_ += (bytes + 255) & ~size_t(255); }
     int allocate() { return total_ == 0 ? NNB200_OK : nnb200_scratch_alloc_async(&base_, total_, stream_); }
+    /// The same without `bytes` that reserve_raw was asked for, after allocate() has failed.
+    int allocate_without(size_t bytes)
+    {
+        total_ -= (bytes + 255) & ~size_t(255);
+        return allocate();
+    }
 
     /// Device address of `host` (copied if it is host memory); int32 arrays report whether any
     /// entry is non-zero so the backend can skip the zero-point sweeps.

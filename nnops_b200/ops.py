@@ -95,13 +95,22 @@ def gemm_i8_args(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, out_kin
         args.force_engine = capi.ENGINES[engine]
     if r_w is not None:
         args.r_w = r_w.data_ptr()
-    # min_workspace: only what the call cannot do without (no scratch for sharing K among SMs).
-    size_fn = capi.lib().nnb200_gemm_i8_min_workspace_bytes if min_workspace else capi.lib().nnb200_gemm_i8_workspace_bytes
-    need = size_fn(C.byref(args))
-    if need:
-        if workspace is None:
+    # min_workspace: only what the call cannot do without (no scratch for sharing K among SMs, no aligned copies).
+    lib = capi.lib()
+    need = (lib.nnb200_gemm_i8_min_workspace_bytes if min_workspace else lib.nnb200_gemm_i8_workspace_bytes)(C.byref(args))
+    if need and workspace is None:
+        try:
             workspace = torch.empty(need, dtype=torch.uint8, device=dev)
+        except torch.OutOfMemoryError:
+            # What exceeds the least only buys speed (a copy of the weight off the 16-byte rule, say).
+            least = lib.nnb200_gemm_i8_min_workspace_bytes(C.byref(args))
+            if least == need:
+                raise
+            need = least
+            workspace = torch.empty(need, dtype=torch.uint8, device=dev) if need else None
+        if workspace is not None:
             keep.append(workspace)
+    if need:
         args.workspace = workspace.data_ptr()
         args.workspace_bytes = workspace.numel()
     return args

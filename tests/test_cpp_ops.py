@@ -26,6 +26,14 @@ def test_host_side_builds(nnb200_lib):
         assert r.returncode == 77, r.stdout + r.stderr
 
 
+def test_linear_runs_with_less_scratch_when_memory_is_short(nnb200_lib):
+    """Against fakes of the allocation and the GEMM entry: no GPU needed."""
+    from nnops_b200.host import build as host_build
+    host_build.build_tests()
+    r = subprocess.run([str(BIN / "test_scratch")], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("name", ["test_ops_standalone", "test_ops_dropin"])
 def test_cpp_operator_tests(cuda_device, name):

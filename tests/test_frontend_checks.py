@@ -25,3 +25,28 @@ def test_batches_agree_or_are_one(nnb200_lib):
         with pytest.raises(ValueError):
             _args((a, 16, 64), (w, 32, 64), (3, 16, 32))
     assert _args((1, 16, 64), (3, 32, 64), (3, 16, 32)).a_batch_stride == 0
+
+
+@pytest.mark.parametrize("zp_a", [0, 7])
+def test_scratch_beyond_the_least_may_fail_to_be_had(nnb200_lib, monkeypatch, zp_a):
+    """A weight off the 16-byte rule asks for scratch of its own size; without it the call has what it needs."""
+    empty = torch.empty
+
+    def short_of_memory(n, *args, **kw):
+        if n > limit:
+            raise torch.OutOfMemoryError("out of memory")
+        return empty(n, *args, **kw)
+
+    limit = 1 << 40
+    monkeypatch.setattr(torch, "empty", short_of_memory)
+    keep = []
+    full = _args((3, 2049), (5000, 2049), (3, 5000), zp_a=zp_a, keep=keep)
+    assert full.workspace_bytes > 5000 * 2049
+    limit = 1 << 20
+    least = _args((3, 2049), (5000, 2049), (3, 5000), zp_a=zp_a, keep=keep)
+    need = nnb200_lib.nnb200_gemm_i8_min_workspace_bytes(least)
+    assert least.workspace_bytes == need and bool(least.workspace) == (need > 0) == (zp_a != 0)
+    limit = 0
+    if zp_a:
+        with pytest.raises(torch.OutOfMemoryError):
+            _args((3, 2049), (5000, 2049), (3, 5000), zp_a=zp_a, keep=keep)
