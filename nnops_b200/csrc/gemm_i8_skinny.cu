@@ -585,6 +585,7 @@ int launch_skinny_variant(const I8Problem& p, const I8Epilogue& ep, const Device
     const int m = static_cast<int>(p.m), n = static_cast<int>(p.n), k = static_cast<int>(p.k);
     // Whole tiles over several waves: as many waves as 128-channel tiles need, cut into equal tiles (24
     // rows, 128-channel tiles / equal ones: N = 28672, K = 8192 51.8 / 45.4 us, N = 19456, K = 4096 28.1 / 24.8).
+    // A caller that brings the scratch for shared K gets that on the first of the two: 45.7.
     // A single wave keeps 128 channels: more CTAs load the activations more often, which eats what the
     // even weight stream gives (N = 11008, K = 4096: 24 rows 16.7 / 16.4, 64 rows 19.5 / 20.1, 128 rows
     // 24.7 / 26.6).  Shared K evens the SMs out itself, and its scratch is laid out for 128.
@@ -650,7 +651,15 @@ bool skinny_i8_supported(const I8Problem& p)
 // has to stream.  Measured, 24 rows, whole tiles -> shared K (us):
 //   one wave of tiles:  N=4096,K=28672 70.1 -> 31.6;  N=4096,K=14336 38.5 -> 22.2;  N=8192,K=8192
 //   25.3 -> 22.2;  N=14336,K=8192 28.1 -> 29.5;  N=11008,K=4096 16.5 -> 18.3;
-//   two waves, the second half empty:  N=28672,K=8192 52.0 -> 47.6 (48 rows 54.9 -> 51.8).
+// With several waves the alternative is equal tiles, which already give every SM the same bytes; what they
+// lose is a step a K block and wave, whether or not the tile is full.  Shared K / equal tiles, 24 and 64
+// rows (us), by waves of 128-channel tiles:
+//   1.03  N=19456,K=8192 34.5 / 42.2, 39.8 / 46.5       1.16  N=22016,K=8192 37.8 / 42.5, 42.9 / 47.2
+//   1.30  N=24576,K=8192 40.3 / 42.8, 45.7 / 47.4       1.51  N=28672,K=8192 45.7 / 44.4, 51.5 / 49.3
+//   1.51  N=28672,K=4096 26.9 / 26.0, 34.0 / 30.6       1.51  N=28672,K=16384 80.4 / 80.7, 87.1 / 87.8
+//   1.69  N=32000,K=8192 51.6 / 47.9, 58.5 / 53.4       2.27  N=43008,K=8192 63.4 / 62.5, 70.5 / 68.7
+// (The line for several waves was drawn against 128-channel tiles, 52.0 -> 47.6 at N=28672,K=8192.  Against
+// equal ones it would lie nearer 7/10 full: from there to 9/10 shared K is 0 to 10 % the slower form.)
 // Hence: with one wave, share when the busiest CTA sheds at least 30 K blocks, plus 0.7 per row
 // above 12; with several waves, when the last one is less than 9/10 full, a share is at least 48
 // K blocks and there are at most 64 rows.
