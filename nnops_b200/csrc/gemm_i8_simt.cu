@@ -10,6 +10,8 @@
 //   * sums     -- R_a[m] = sum_k A[m][k], R_w[n] = sum_k W[n][k] for zero-point compensation
 //                 (replaces i8_row_sums_kernel / i8_col_sums_kernel, matmul_i8_common.cuh:270-350).
 
+#include <type_traits>
+
 #include "internal.cuh"
 
 namespace nnb200 {
@@ -101,49 +103,90 @@ __device__ __forceinline__ bool any_zero_point(const int32_t* zp, int64_t count)
     return false;
 }
 
-// The sum of each row of a [rows, k] int8 matrix with arbitrary strides, a block to a row.  `look`: the
-// zero points that the sums will be multiplied with, when the caller does not know whether any is
-// non-zero; if none is, the matrix is not read and the sums stay as they are.
+// One block per row of a [rows, k] int8 matrix with arbitrary strides.
 template <bool UNSIGNED>
 __global__ void __launch_bounds__(128) i8_sums_kernel(const uint8_t* x, int64_t rows, int64_t k, int64_t stride_row,
-                                                      int64_t stride_k, int32_t* out, const int32_t* look, int64_t look_count)
+                                                      int64_t stride_k, int32_t* out)
 {
-    if (look != nullptr && !any_zero_point(look, look_count)) {
-        return;
+    const int64_t r = blockIdx.x;
+    const uint8_t* row = x + r * stride_row;
+    int32_t s = 0;
+    if (stride_k == 1 && (reinterpret_cast<uintptr_t>(row) & 3u) == 0) {
+        const int64_t k4 = k / 4;
+        const uint32_t* row4 = reinterpret_cast<const uint32_t*>(row);
+        for (int64_t i = threadIdx.x; i < k4; i += blockDim.x) {
+            const uint32_t v = row4[i];
+            s = UNSIGNED ? __dp4a(v, 0x01010101u, static_cast<uint32_t>(s))
+                         : __dp4a(static_cast<int32_t>(v), 0x01010101, s);
+        }
+        for (int64_t i = k4 * 4 + threadIdx.x; i < k; i += blockDim.x) {
+            s += UNSIGNED ? static_cast<int32_t>(row[i]) : static_cast<int32_t>(static_cast<int8_t>(row[i]));
+        }
+    } else {
+        for (int64_t i = threadIdx.x; i < k; i += blockDim.x) {
+            const uint8_t v = row[i * stride_k];
+            s += UNSIGNED ? static_cast<int32_t>(v) : static_cast<int32_t>(static_cast<int8_t>(v));
+        }
     }
     __shared__ int32_t part[4];
-    for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        part[threadIdx.x >> 5] = s;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        out[r] = part[0] + part[1] + part[2] + part[3];
+    }
+}
+
+template <bool UNSIGNED>
+__device__ __forceinline__ int32_t add_bytes(uint32_t v, int32_t s)
+{
+    return UNSIGNED ? static_cast<int32_t>(__dp4a(v, 0x01010101u, static_cast<uint32_t>(s)))
+                    : __dp4a(static_cast<int32_t>(v), 0x01010101, s);
+}
+
+// The same where the caller does not know whether any of the zero points that the sums will be multiplied
+// with differs from zero: if none does, the matrix is not read and the sums stay as they are.  Rows of
+// contiguous bytes, 16-byte aligned.  A block
+// looks once, so there are no more of them than the device holds, and its warps take rows in turn, no
+// barrier between them (28672 x 8192: a warp to a row 37 us, a block to a row in turn 59, the kernel
+// above 34; 11008 x 4096 5 us, the kernel above 10).
+template <bool UNSIGNED>
+__global__ void __launch_bounds__(128) i8_sums_look_kernel(const uint8_t* x, int64_t rows, int64_t k, int64_t stride_row,
+                                                           int32_t* out, const int32_t* look, int64_t look_count)
+{
+    if (!any_zero_point(look, look_count)) {
+        return;
+    }
+    const int lane = threadIdx.x & 31;
+    for (int64_t r = static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5); r < rows; r += static_cast<int64_t>(gridDim.x) * 4) {
         const uint8_t* row = x + r * stride_row;
         int32_t s = 0;
-        if (stride_k == 1 && (reinterpret_cast<uintptr_t>(row) & 3u) == 0) {
-            const int64_t k4 = k / 4;
-            const uint32_t* row4 = reinterpret_cast<const uint32_t*>(row);
-            for (int64_t i = threadIdx.x; i < k4; i += blockDim.x) {
-                const uint32_t v = row4[i];
-                s = UNSIGNED ? __dp4a(v, 0x01010101u, static_cast<uint32_t>(s))
-                             : __dp4a(static_cast<int32_t>(v), 0x01010101, s);
-            }
-            for (int64_t i = k4 * 4 + threadIdx.x; i < k; i += blockDim.x) {
-                s += UNSIGNED ? static_cast<int32_t>(row[i]) : static_cast<int32_t>(static_cast<int8_t>(row[i]));
-            }
-        } else {
-            for (int64_t i = threadIdx.x; i < k; i += blockDim.x) {
-                const uint8_t v = row[i * stride_k];
-                s += UNSIGNED ? static_cast<int32_t>(v) : static_cast<int32_t>(static_cast<int8_t>(v));
-            }
+        const int64_t k16 = k / 16;
+        const uint4* row16 = reinterpret_cast<const uint4*>(row);
+#pragma unroll 8
+        for (int64_t i = lane; i < k16; i += 32) {
+            const uint4 v = row16[i];
+            s = add_bytes<UNSIGNED>(v.x, s);
+            s = add_bytes<UNSIGNED>(v.y, s);
+            s = add_bytes<UNSIGNED>(v.z, s);
+            s = add_bytes<UNSIGNED>(v.w, s);
+        }
+        for (int64_t i = k16 * 16 + lane; i < k; i += 32) {
+            const uint8_t v = row[i];
+            s += UNSIGNED ? static_cast<int32_t>(v) : static_cast<int32_t>(static_cast<int8_t>(v));
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
         }
-        if ((threadIdx.x & 31) == 0) {
-            part[threadIdx.x >> 5] = s;
+        if (lane == 0) {
+            out[r] = s;
         }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            out[r] = part[0] + part[1] + part[2] + part[3];
-        }
-        __syncthreads();
     }
 }
 
@@ -284,27 +327,29 @@ int launch_i8_sums(const I8Problem& p, const I8Sums& sums, const DeviceInfo& dev
     // Either destination may be null: that sweep is skipped.
     const uint8_t* a = static_cast<const uint8_t*>(p.a);
     const uint8_t* w = static_cast<const uint8_t*>(p.w);
-    // A block looks at the zero points once, so with them there are only as many blocks as the device holds;
-    // where the looks together would read more than a quarter of the operand, none is taken (24 x 28672 x
-    // 8192: one look at 28672 zero points a block 9 us, sweeping the 24 rows 2.5).
-    const int64_t most = static_cast<int64_t>(dev.sm_count) * 16;
-    const auto sweep = [&](auto kernel, const uint8_t* x, int64_t rows, int64_t stride_row, int64_t stride_k, int32_t* out,
+    // A look is taken where all blocks' looks together read at most a quarter of the operand (24 x 28672 x
+    // 8192: one look at 28672 zero points a block 9 us, sweeping the 24 rows 2.5), and where rows are wide loads.
+    const int64_t resident = static_cast<int64_t>(dev.sm_count) * 16;
+    const auto sweep = [&](auto is_unsigned, const uint8_t* x, int64_t rows, int64_t stride_row, int64_t stride_k, int32_t* out,
                            const int32_t* look, int64_t look_count) {
-        int64_t blocks = rows;
-        if (look != nullptr) {
-            const int64_t resident = rows < most ? rows : most;
-            const bool cheap = static_cast<double>(rows) * p.k >= 4.0 * sizeof(int32_t) * resident * look_count;
-            look = cheap ? look : nullptr;
-            blocks = cheap ? resident : rows;
+        constexpr bool U = decltype(is_unsigned)::value;
+        const int64_t blocks = (rows + 3) / 4 < resident ? (rows + 3) / 4 : resident;
+        const bool wide = stride_k == 1 && ((reinterpret_cast<uintptr_t>(x) | static_cast<uint64_t>(stride_row)) & 15u) == 0;
+        if (look != nullptr && wide && static_cast<double>(rows) * p.k >= 4.0 * sizeof(int32_t) * blocks * look_count) {
+            i8_sums_look_kernel<U><<<static_cast<unsigned>(blocks), 128, 0, stream>>>(x, rows, p.k, stride_row, out, look, look_count);
+        } else {
+            i8_sums_kernel<U><<<static_cast<unsigned>(rows), 128, 0, stream>>>(x, rows, p.k, stride_row, stride_k, out);
         }
-        kernel<<<static_cast<unsigned>(blocks), 128, 0, stream>>>(x, rows, p.k, stride_row, stride_k, out, look, look_count);
     };
     if (sums.r_a != nullptr) {
-        sweep(p.a_unsigned ? i8_sums_kernel<true> : i8_sums_kernel<false>, a, p.m, p.a_stride_m, p.a_stride_k, sums.r_a,
-              sums.look_w, p.n);
+        if (p.a_unsigned) {
+            sweep(std::true_type{}, a, p.m, p.a_stride_m, p.a_stride_k, sums.r_a, sums.look_w, p.n);
+        } else {
+            sweep(std::false_type{}, a, p.m, p.a_stride_m, p.a_stride_k, sums.r_a, sums.look_w, p.n);
+        }
     }
     if (sums.r_w != nullptr) {
-        sweep(i8_sums_kernel<false>, w, p.n, p.w_stride_n, p.w_stride_k, sums.r_w, sums.look_a, p.m);
+        sweep(std::false_type{}, w, p.n, p.w_stride_n, p.w_stride_k, sums.r_w, sums.look_a, p.m);
     }
     note_launch((sums.r_a != nullptr ? 1 : 0) + (sums.r_w != nullptr ? 1 : 0));
     return cuda_status(cudaGetLastError());

@@ -59,9 +59,12 @@ def gemm_i8_args(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, out_kin
     Tensors created for quantization arrays are appended to ``keep`` so they outlive the call."""
     keep = keep if keep is not None else []
     dev = a.device
-    if not (a.dim() in (2, 3) and w.dim() in (2, 3) and out.dim() in (2, 3)):
+    ad, wd, od = a.dim(), w.dim(), out.dim()
+    if not (1 < ad < 4 and 1 < wd < 4 and 1 < od < 4):
         raise ValueError("a, w and out must be matrices or batches of matrices")
-    a_batch, w_batch, o_batch = (t.shape[0] if t.dim() == 3 else 1 for t in (a, w, out))
+    a_batch = a.shape[0] if ad == 3 else 1
+    w_batch = w.shape[0] if wd == 3 else 1
+    o_batch = out.shape[0] if od == 3 else 1
     if 1 != a_batch != w_batch != 1:
         raise ValueError("batch mismatch")
     m, k = a.shape[-2:]

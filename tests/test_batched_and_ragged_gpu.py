@@ -19,7 +19,7 @@ def _store(x: np.ndarray, transposed: bool, device, offset: int = 0):
 
 
 def _check(device, batch, m, n, k, *, pose="nt", out_kind="s8", shared_a=False, shared_w=False, unsigned=False, zero_points=False,
-           offset=0, launches=None, seed=0):
+           offset=0, launches=None, seed=0, min_workspace=False):
     rng = np.random.default_rng(seed)
     a = rng.integers(0, 256, ((1 if shared_a else batch), m, k)).astype(np.uint8) if unsigned else \
         rng.integers(-127, 128, ((1 if shared_a else batch), m, k), dtype=np.int8)
@@ -36,7 +36,7 @@ def _check(device, batch, m, n, k, *, pose="nt", out_kind="s8", shared_a=False, 
     if batch > 1:
         ta, tw = (ta[0] if shared_a else ta), (tw[0] if shared_w else tw)
     before = capi.lib().nnb200_launch_count()
-    got = ops.gemm_i8(ta, tw, out_kind=out_kind, **kw).cpu().numpy()
+    got = ops.gemm_i8(ta, tw, out_kind=out_kind, min_workspace=min_workspace, **kw).cpu().numpy()
     if launches is not None:
         assert capi.lib().nnb200_launch_count() - before == launches
     if batch == 1:
@@ -121,3 +121,12 @@ def test_copies_of_few_long_rows_and_short_k(cuda_device, nnb200_lib, case, zero
 def test_few_rows_in_a_small_batch(cuda_device, nnb200_lib, batch, m, n, k, launches):
     """A launch of the streaming engine each until one launch of the tile kernel is shorter."""
     _check(cuda_device, batch, m, n, k, launches=launches, seed=k)
+
+
+@pytest.mark.parametrize("case", [(2049, 0, "nt", 1), (2050, 1, "nn", 1), (700, 0, "nt", 3)])
+@pytest.mark.parametrize("zero_points", [False, True])
+def test_operands_off_the_tma_rule_with_the_least_scratch(cuda_device, nnb200_lib, case, zero_points):
+    """No room for copies: the generic engine, a launch a product."""
+    k, offset, pose, batch = case
+    _check(cuda_device, batch, 65, 301, k, pose=pose, offset=offset, zero_points=zero_points, min_workspace=True, seed=k,
+           launches=None if zero_points else batch)

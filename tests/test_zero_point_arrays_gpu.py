@@ -9,7 +9,7 @@ from nnops_b200 import ops
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("shape", [(1, 300, 512), (5, 4000, 200), (40, 130, 1024), (3000, 33, 2064), (60, 5000, 1024), (2100, 260, 128)])
+@pytest.mark.parametrize("shape", [(1, 300, 512), (7, 9001, 528), (5, 4000, 200), (40, 130, 1024), (3000, 33, 2064), (60, 5000, 1024), (2100, 260, 128)])
 @pytest.mark.parametrize("live_a", [None, "first", "last"])
 @pytest.mark.parametrize("live_w", [None, "last"])
 @pytest.mark.parametrize("out_kind", ["s8", "f32"])
@@ -33,9 +33,9 @@ def test_zero_arrays_read_no_operand(cuda_device, nnb200_lib, shape, live_a, liv
         return   # copied into aligned rows, and the sums ride along
     # The workspace starts with the sums of A's rows (wanted by zero points of W), then those of W's; a sweep
     # that is shorter than its blocks' looks at the array goes ahead without.
-    blocks = 16 * torch.cuda.get_device_properties(cuda_device).multi_processor_count
+    most = 16 * torch.cuda.get_device_properties(cuda_device).multi_processor_count
     at_w = (m + 63) // 64 * 64
     for start, x, count, live in ((0, a, n, live_w), (at_w, w, m, live_a)):
         sums = workspace[start:start + len(x)].cpu().numpy()
-        looks = x.size >= 16 * min(len(x), blocks) * count
+        looks = x.size >= 16 * min(-(-len(x) // 4), most) * count
         assert (sums == untouched).all() if looks and not live else np.array_equal(sums, x.sum(axis=1, dtype=np.int32))
