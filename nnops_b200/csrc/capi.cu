@@ -819,15 +819,18 @@ static bool q4_1_wants_rows_umma(const nnb200_q4_1_args* q, int other)
     //   N = 9472, 128    9.2 / 13.3   10.5 / 13.8 12.1 / 13.9 14.8 / 14.8 10.1 / 14.3 12.7 / 15.4
     //   N = 14336, 128   9.0 / 8.6    10.4 / 9.4  11.9 / 10.1 14.8 / 11.5 9.8 / 10.4  12.7 / 12.1
     //   f32, N = 2048, 64 10.4 / 11.5 11.6 / 11.2 12.9 / 10.8 15.6 / 10.5 11.2 / 11.7 13.9 / 11.0
+    // An activation beyond Relu costs the others 40 us, their epilogues' unrolled code fetched cold, and this
+    // one next to nothing: 43 rows of 226 x 320 with silu 50 / 9.2.
+    const bool plain = q->activation == NNB200_ACT_NONE || q->activation == NNB200_ACT_RELU;
     const DeviceInfo* dev = current_device_info();
     const bool shared = (q->n + 127) / 128 * 2 <= (dev != nullptr ? dev->sm_count : 148);
     const int64_t pad = q->k % 128 == 0 ? 0 : 192;
     bool k_ok = pad == 0 || q->k >= 256;
-    if (q->a_f16 == 0) {
+    if (plain && q->a_f16 == 0) {
         k_ok = k_ok && (q->n > 4096 || q->k >= 5 * q->m);
-    } else if (!shared) {
+    } else if (plain && !shared) {
         k_ok = k_ok && (pad == 0 || q->k > 3 * q->m + pad);
-    } else {
+    } else if (plain) {
         const int64_t per_row = q->m <= 64 ? 7 : (q->n <= 4096 ? 4 : 6);
         k_ok = (pad == 0 && q->m <= 64 && q->k <= 256) || q->k >= per_row * q->m + pad;
     }

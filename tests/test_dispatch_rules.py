@@ -83,7 +83,10 @@ def test_copies_into_aligned_rows_only_where_they_pay(nnb200_lib, call, pays):
     (64, 2048, 256, False, 5), (64, 2048, 384, False, 7), (64, 14336, 256, False, 7)])
 def test_q4_1_weights_in_tensor_memory_where_k_is_long_enough(nnb200_lib, m, n, k, f16, engine):
     need = nnb200_lib.nnb200_q4_1_workspace_bytes(C.byref(_q4(m, n, k, f16)))
-    assert nnb200_lib.nnb200_q4_1_engine(C.byref(_q4(m, n, k, f16, workspace=need))) == engine
+    q = _q4(m, n, k, f16, workspace=need or 1 << 33)
+    assert nnb200_lib.nnb200_q4_1_engine(C.byref(q)) == engine
+    q.activation = 3   # the other GEMMs' epilogues fetch it cold
+    assert nnb200_lib.nnb200_q4_1_engine(C.byref(q)) == (7 if engine in (1, 5) else engine)
 
 
 def test_q4_gemv_knob_comes_before_the_weights_in_tensor_memory(nnb200_lib, knobs):
