@@ -121,8 +121,8 @@ typedef struct nnb200_gemm_i8_args {
     int32_t zp_a_scalar, zp_w_scalar;
     int32_t zp_a_nonzero; /* caller's promise about the ARRAYS: 0 = every zp_a[] entry is 0 */
     int32_t zp_w_nonzero; /* (lets the backend skip the R_a / R_w sweeps); scalars are checked here.
-                             NNB200_ZP_NOT_KNOWN: the sweeps look at the entries on the device first
-                             and read no operand when all are 0. */
+                             NNB200_ZP_NOT_KNOWN: a sweep that is long enough looks at the entries
+                             on the device first and reads no operand when all are 0. */
     float out_scale;
     int32_t out_zp;
     void* workspace;
@@ -359,9 +359,15 @@ typedef struct nnb200_q4_1_args {
 /* Optional device scratch (16-byte aligned).  Non-zero for tall problems (f16 activations: m >= 256;
  * f32 activations: m >= 17): given that many bytes, the call expands the weights to f16 once into
  * the scratch (and splits f32 activations into [hi | lo] f16 halves there) and runs a dense
- * tensor-core GEMM over them; without it (NULL or too small) the same call runs the fused kernel
- * (f16) or the GEMV engine tile by tile (f32).  The scratch is dead when the call's work has
- * completed on the stream. */
+ * tensor-core GEMM over them; and for 2 to 64 rows of f32 activations on engine 7, which splits them
+ * there.  Without it (NULL or too small) the same call runs the fused kernel (f16) or the GEMV
+ * engine tile by tile (f32).  The scratch is dead when the call's work has completed on the stream.
+ *
+ * Precision: engines 1, 4, 5 and 7 round every weight to f16 once and take f32 activations as the sum
+ * of two f16 values, which holds them to 2^-22 of their size from about 1e-5 up, with fewer bits
+ * below that, and as NaN beyond f16's range; engine 6 takes such activations in the same way.  Engine 3
+ * holds weights and activations in f32; the automatic choice gives it up to 8 rows (f32: up to 16) of
+ * layers whose k is not a multiple of 128 or whose weight rows are not 16-byte aligned. */
 NNB200_API size_t nnb200_q4_1_workspace_bytes(const nnb200_q4_1_args* args);
 NNB200_API int nnb200_linear_q4_1(const nnb200_q4_1_args* args, void* stream);
 NNB200_API int nnb200_q4_1_engine(const nnb200_q4_1_args* args);

@@ -9,8 +9,9 @@
 //     TMA, 128-byte swizzle, out-of-range rows/columns zero-filled by the hardware;
 //   * warp 1 issues tcgen05.mma kind::i8 (M128 x N=BN x K32) into one of two TMEM
 //     accumulators and frees ring slots with tcgen05.commit;
-//   * warps 2-5 drain the other accumulator with tcgen05.ld and apply the fused epilogue
-//     (zero-point compensation, int32 bias, Relu, requantisation / dequantisation) in
+//   * the other warps -- sixteen for 8-bit destinations, eight for the rest, four in the sharded
+//     form (see sixteen_warps) -- drain the other accumulator with tcgen05.ld and apply the fused
+//     epilogue (zero-point compensation, int32 bias, Relu, requantisation / dequantisation) in
 //     registers, so the epilogue of tile i overlaps the main loop of tile i+1.
 //
 // Sharded form (template flag PEERS): the epilogue of an 8-bit destination stages 32 rows x 128

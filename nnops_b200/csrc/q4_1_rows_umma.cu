@@ -26,9 +26,10 @@
 //   * f32 activations are given as two f16 rows each, high part and remainder; the epilogue adds the
 //     two accumulator columns (see split_f32_to_f16_kernel).
 //
-// What bounds it: the tensor pipe.  A = 128 x 16 f16 from tensor memory takes 35 clocks an MMA
-// whatever the rows (16 of them use an eighth of the multiplies), 256 MMAs a CTA at K = 4096, and each
-// commit drains the pipe; decoding takes about 1400 clocks a warp and unit, three groups at a time.
+// What bounds it: instruction issue.  16 rows of 28672 x 8192 issue 4.5 warp instructions for 32 weights
+// (decoding, stores to tensor memory, copies, polls), 64 % of the issue slots of the active cycles, the
+// integer pipe 52 %; the tensor pipe is busy 9 %, DRAM 34 % of peak.  What the MMAs cost is latency: 35 clocks
+// each to issue (A = 128 x 16 from tensor memory, whatever the rows) and some hundred to drain for a commit.
 // 16 rows of 14336 x 4096 take 16.0 us (50.5 before; the weights' HBM time is 5.7), 28672 x 8192 46.8
 // (186), 4096 x 4096 9.0 (49.3).
 //
