@@ -691,7 +691,15 @@ static int run_gemm_i8(const nnb200_gemm_i8_args* a, const DeviceInfo* dev, cuda
         if (batched) {
             return launch_gemm_i8_umma_batched(p, batch, ep, *dev, stream);
         }
-        switch (a->batch == 1 ? engine0 : pick_i8_engine(a, p)) {
+        int engine = a->batch == 1 ? engine0 : pick_i8_engine(a, p);
+        // The few-row engine with K shared in clusters takes part of what the rows and channels alone give to
+        // two others; nnb200_gemm_i8_engine keeps naming those.
+        if (a->force_engine == NNB200_ENGINE_AUTO && !sharded_out(a) &&
+            (engine == NNB200_ENGINE_UMMA || engine == NNB200_ENGINE_DECODE) &&
+            skinny_i8_preferred(p, engine == NNB200_ENGINE_DECODE, *dev)) {
+            engine = NNB200_ENGINE_SKINNY;
+        }
+        switch (engine) {
         case NNB200_ENGINE_UMMA: st = launch_gemm_i8_umma(p, ep, *dev, stream); break;
         case NNB200_ENGINE_NARROW: st = launch_gemm_i8_narrow(p, ep, *dev, stream); break;
         case NNB200_ENGINE_DECODE: st = launch_gemm_i8_decode(p, ep, *dev, stream); break;

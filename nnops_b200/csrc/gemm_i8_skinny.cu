@@ -1,4 +1,4 @@
-// int8 GEMM for a handful of activation rows (17 <= M <= 128: batched decode, short prefills).
+// int8 GEMM for a handful of activation rows (9 <= M <= 128: batched decode, short prefills).
 //
 // With so few rows the whole cost is streaming W once, and the square-tile engine
 // (gemm_i8_umma.cu) is a poor fit: it pads the activations to a 128-row MMA operand, re-reads
@@ -19,6 +19,12 @@
 // accumulators, bounded waits) except that each accumulator has its own four epilogue warps;
 // same epilogue arithmetic (epilogue.cuh): results are bit-identical to every other int8 engine.
 //
+// What bounds it: the weight stream once several hundred KB a CTA are on their way (28672 x 8192, 24 rows:
+// 41.7 us = 0.89 of measured HBM); below that the start -- 0.6 us to the first load, 2 us to the first weights
+// with every SM asking at once -- and the tail.  A K block of 128 bytes takes the issuing warps 200 to 250 cycles
+// (525 while their waits branched, see mbar_wait_converged): 24 rows of 11008 x 4096 15.6 -> 10.8 us, 64 rows
+// 18.8 -> 11.7, 128 rows 24.8 -> 14.0.
+//
 // Tiles need not be 128 channels high: without shared K a layer of several waves of tiles is cut into
 // equal ones (N = 28672 on 148 SMs: 296 tiles of 97 channels instead of 224 of 128), so that every SM
 // streams the same bytes; the rows of the MMA past a tile's channels hold whatever the ring held
@@ -26,7 +32,10 @@
 //
 // Work split.  The unit of work is one 128-byte K block of one tile; tile t owns units
 // [t * num_kb, (t + 1) * num_kb).  Every CTA takes one contiguous range of units:
-//   * whole tiles only (CTA c gets tiles [c T / G, (c + 1) T / G)) when no scratch is given;
+//   * with so few tiles that two or more CTAs a tile find an SM each: clusters of up to eight CTAs share a
+//     tile's K; their sums meet through distributed shared memory, each CTA finishing its share of the
+//     rows (4096 x 4096, 24 rows: 15.3 us with whole tiles, 17.4 on the square engine -> 6.9);
+//   * whole tiles only (CTA c gets an equal run of them) when no scratch is given;
 //   * an equal share of ALL units (CTA c gets [c U / G, (c + 1) U / G)) when the caller gave
 //     scratch: a range then starts and ends in the middle of tiles, so that every SM streams
 //     the same number of weight bytes whatever N / 128 is (224 tiles on 148 SMs would otherwise
@@ -41,9 +50,11 @@
 #include <chrono>
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
 
 #include "internal.cuh"
 #include "ptx.cuh"
+#include "ptx_pair.cuh"
 
 namespace nnb200 {
 
@@ -57,6 +68,7 @@ constexpr int kUmmaK = 32;
 // partial sums, each a chain of L2 round trips) of consecutive pieces run side by side.
 constexpr int kNumThreads = 320;
 constexpr int kEpilogueThreads = 128;  // per group
+constexpr int kMaxParts = 8;           // CTAs of a cluster that share a tile's K
 
 template <int MP>
 struct SkinnyConfig {
@@ -65,18 +77,20 @@ struct SkinnyConfig {
     static constexpr int kStageBytes = kWTileBytes + kATileBytes;
     static constexpr int kStages = (192 * 1024) / kStageBytes > 10 ? 10 : (192 * 1024) / kStageBytes;
     static constexpr int kTmemCols = 2 * MP < 32 ? 32 : 2 * MP;  // two accumulators of MP columns
-    static constexpr int kRowTermBytes = 128 * 16;                // I8RowTerms of up to 128 activation rows
+    static constexpr int kRowTerms = 136;                         // I8RowTerms of up to 128 activation rows, groups of rows read past the last
+    static constexpr int kRowTermBytes = kRowTerms * 16;
     static constexpr int kBarrierBytes = (2 * kStages + 4) * 8 + 16;
     static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kRowTermBytes + kBarrierBytes;
 };
 
-// First unit of CTA c's range (c = G gives the end of the last range).
-__device__ __forceinline__ int64_t range_begin(int c, int grid, int num_tiles, int num_kb, bool split)
+// First unit of CTA c's range (c = G gives the end of the last range).  The launcher keeps the number of
+// units below 2^31.
+__device__ __forceinline__ int range_begin(int c, int grid, int num_tiles, int num_kb)
 {
-    if (split) {
-        return static_cast<int64_t>(c) * (static_cast<int64_t>(num_tiles) * num_kb) / grid;
-    }
-    return (static_cast<int64_t>(c) * num_tiles / grid) * num_kb;
+    // floor(c * total / grid) without a 64-bit division (some hundred cycles each at the kernel's start).
+    const int total = num_tiles * num_kb;
+    const int q = total / grid, r = total - q * grid;
+    return c * q + static_cast<int>(static_cast<unsigned>(c) * static_cast<unsigned>(r) / static_cast<unsigned>(grid));
 }
 
 // The CTA whose range contains unit u under the equal-share split.
@@ -101,14 +115,14 @@ struct Segment {
 // finishes (tail), then the whole tiles.  Parts go first so that they are published early and
 // the exchange with the neighbours hides behind the whole tiles that follow.
 struct SegmentList {
-    int64_t head0, head1, tail0, tail1;
+    int head0, head1, tail0, tail1;
     int tile0, tile1;
     int num_kb;
 
-    __device__ __forceinline__ SegmentList(int64_t u_begin, int64_t u_end, int nkb) : num_kb(nkb)
+    __device__ __forceinline__ SegmentList(int u_begin, int u_end, int nkb) : num_kb(nkb)
     {
-        const int64_t first_full = (u_begin + nkb - 1) / nkb * nkb;
-        const int64_t last_full_end = u_end / nkb * nkb;
+        const int first_full = (u_begin + nkb - 1) / nkb * nkb;
+        const int last_full_end = u_end / nkb * nkb;
         head0 = u_begin;
         head1 = first_full < u_end ? first_full : u_end;
         if (last_full_end >= first_full && last_full_end < u_end) {
@@ -117,8 +131,18 @@ struct SegmentList {
         } else {
             tail0 = tail1 = 0;
         }
-        tile0 = static_cast<int>(first_full / nkb);
-        tile1 = last_full_end > first_full ? static_cast<int>(last_full_end / nkb) : tile0;
+        tile0 = first_full / nkb;
+        tile1 = last_full_end > first_full ? last_full_end / nkb : tile0;
+    }
+    // Whole tiles [t0, t1); no division at the kernel's start.
+    struct Whole {
+        int t0, t1;
+    };
+    __device__ __forceinline__ SegmentList(Whole w, int nkb) : num_kb(nkb)
+    {
+        head0 = head1 = tail0 = tail1 = 0;
+        tile0 = w.t0;
+        tile1 = w.t1;
     }
     __device__ __forceinline__ int count() const
     {
@@ -129,18 +153,18 @@ struct SegmentList {
         Segment s;
         if (head1 > head0) {
             if (i == 0) {
-                s.tile = static_cast<int>(head0 / num_kb);
-                s.kb0 = static_cast<int>(head0 - static_cast<int64_t>(s.tile) * num_kb);
-                s.kb1 = s.kb0 + static_cast<int>(head1 - head0);
+                s.tile = head0 / num_kb;
+                s.kb0 = head0 - s.tile * num_kb;
+                s.kb1 = s.kb0 + (head1 - head0);
                 return s;
             }
             --i;
         }
         if (tail1 > tail0) {
             if (i == 0) {
-                s.tile = static_cast<int>(tail0 / num_kb);
+                s.tile = tail0 / num_kb;
                 s.kb0 = 0;
-                s.kb1 = static_cast<int>(tail1 - tail0);
+                s.kb1 = tail1 - tail0;
                 return s;
             }
             --i;
@@ -148,6 +172,15 @@ struct SegmentList {
         s.tile = tile0 + i;
         s.kb0 = 0;
         s.kb1 = num_kb;
+        return s;
+    }
+    // For loops that issue MMAs or copies: warp-uniform to the compiler as well.
+    __device__ __forceinline__ Segment uniform_at(int i) const
+    {
+        Segment s = at(i);
+        s.tile = warp_uniform(s.tile);
+        s.kb0 = warp_uniform(s.kb0);
+        s.kb1 = warp_uniform(s.kb1);
         return s;
     }
 };
@@ -209,12 +242,136 @@ __device__ __forceinline__ void collect_parts(int32_t (&sum)[32], const int32_t*
     }
 }
 
+// One channel's epilogue terms, held by the thread that finishes its sums.
+struct ChannelTerms {
+    int32_t zpw, rw, bias_i;
+    float s_w, bias_f;
+};
+
+template <int KIND>
+__device__ __forceinline__ ChannelTerms channel_terms(const I8Epilogue& ep, int64_t n, bool n_ok)
+{
+    ChannelTerms c;
+    c.zpw = (n_ok && ep.zp_w != nullptr) ? ep.zp_w[n] : ep.zp_w_scalar;
+    c.rw = (n_ok && ep.compensate && ep.r_w != nullptr) ? ep.r_w[n] : 0;
+    c.s_w = (n_ok && ep.scale_w != nullptr) ? ep.scale_w[n] : ep.scale_w_scalar;
+    c.bias_i = 0;
+    c.bias_f = 0.0f;
+    if (n_ok && ep.bias != nullptr) {
+        if constexpr (KIND <= NNB200_OUT_U8) {
+            c.bias_i = static_cast<const int32_t*>(ep.bias)[n];
+        } else if constexpr (KIND == NNB200_OUT_F32) {
+            c.bias_f = static_cast<const float*>(ep.bias)[n];
+        } else {
+            c.bias_f = __half2float(static_cast<const __half*>(ep.bias)[n]);
+        }
+    }
+    return c;
+}
+
+// Epilogue and store of one channel's sums for activation rows [m0, m0 + ROWS), clipped at m_end.  A few rows
+// at a time in a loop, with every switch taken once per group and none per element: one element after
+// the other, each behind its own branches, cost 200 cycles a row (64 rows into f16: 27.0 us a call of
+// which 13 were this), and the 32 unrolled copies were mostly fetched cold.
+template <int KIND, int ROWS>
+__device__ __forceinline__ void finish_rows(const I8Epilogue& ep, const I8RowTerms* row_terms, const uint32_t (&acc)[ROWS],
+                                            int m0, int m_end, int64_t n, bool n_ok, const ChannelTerms& ct)
+{
+    I8RowTerms t[ROWS];
+    int32_t v[ROWS];
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) {
+        t[j] = row_terms[m0 + j];   // the table has entries past the last row
+        v[j] = static_cast<int32_t>(acc[j]);
+    }
+    if (ep.compensate) {
+#pragma unroll
+        for (int j = 0; j < ROWS; ++j) {
+            v[j] = i8_compensate(v[j], t[j].zpa, ct.zpw, t[j].ra, ct.rw, ep.k);
+        }
+    }
+    const int64_t idx = static_cast<int64_t>(m0) * ep.ldc + n;
+    if constexpr (KIND <= NNB200_OUT_U8) {
+        const int32_t relu_lo = ep.relu ? 0 : INT32_MIN;
+        const float zpf = static_cast<float>(ep.out_zp);
+        const float lo = (KIND == NNB200_OUT_S8 ? -128.0f : 0.0f) - zpf;
+        const float hi = (KIND == NNB200_OUT_S8 ? 127.0f : 255.0f) - zpf;
+#pragma unroll
+        for (int j = 0; j < ROWS; ++j) {
+            v[j] = max(static_cast<int32_t>(static_cast<uint32_t>(v[j]) + static_cast<uint32_t>(ct.bias_i)), relu_lo);
+            if constexpr (KIND != NNB200_OUT_S32) {
+                v[j] = i8_requant(v[j], __fmul_rn(t[j].row_k, ct.s_w), lo, hi, ep.out_zp);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < ROWS; ++j) {
+            if (m0 + j < m_end && n_ok) {
+                if constexpr (KIND == NNB200_OUT_S32) {
+                    static_cast<int32_t*>(ep.out)[idx + j * ep.ldc] = v[j];
+                } else {
+                    static_cast<uint8_t*>(ep.out)[idx + j * ep.ldc] = static_cast<uint8_t>(v[j]);
+                }
+            }
+        }
+    } else {
+        float f[ROWS];
+#pragma unroll
+        for (int j = 0; j < ROWS; ++j) {
+            f[j] = __fmul_rn(__int2float_rn(v[j]), __fmul_rn(t[j].s_a, ct.s_w));
+            const float fb = __fadd_rn(f[j], ct.bias_f);
+            f[j] = ct.bias_f != 0.0f ? fb : f[j];   // a zero bias is not added (-0 stays -0)
+            f[j] = fminf(fmaxf(f[j], ep.min_clip), ep.max_clip);
+        }
+        const auto activate = [&](auto act) {
+#pragma unroll
+            for (int j = 0; j < ROWS; ++j) {
+                f[j] = act_apply(decltype(act)::value, ep.act_alpha, ep.act_beta, f[j]);
+            }
+        };
+        switch (ep.activation) {
+        case NNB200_ACT_RELU: activate(std::integral_constant<int, NNB200_ACT_RELU>{}); break;
+        case NNB200_ACT_RELU6: activate(std::integral_constant<int, NNB200_ACT_RELU6>{}); break;
+        case NNB200_ACT_LEAKY_RELU: activate(std::integral_constant<int, NNB200_ACT_LEAKY_RELU>{}); break;
+        case NNB200_ACT_SIGMOID: activate(std::integral_constant<int, NNB200_ACT_SIGMOID>{}); break;
+        case NNB200_ACT_TANH: activate(std::integral_constant<int, NNB200_ACT_TANH>{}); break;
+        case NNB200_ACT_GELU: activate(std::integral_constant<int, NNB200_ACT_GELU>{}); break;
+        case NNB200_ACT_SILU: activate(std::integral_constant<int, NNB200_ACT_SILU>{}); break;
+        case NNB200_ACT_HARD_SWISH: activate(std::integral_constant<int, NNB200_ACT_HARD_SWISH>{}); break;
+        case NNB200_ACT_ELU: activate(std::integral_constant<int, NNB200_ACT_ELU>{}); break;
+        default: break;
+        }
+#pragma unroll
+        for (int j = 0; j < ROWS; ++j) {
+            if (m0 + j < m_end && n_ok) {
+                if constexpr (KIND == NNB200_OUT_F32) {
+                    static_cast<float*>(ep.out)[idx + j * ep.ldc] = f[j];
+                } else {
+                    static_cast<__half*>(ep.out)[idx + j * ep.ldc] = __float2half_rn(f[j]);
+                }
+            }
+        }
+    }
+}
+
+__device__ __forceinline__ uint32_t ld_shared_cluster_u32(uint32_t cluster_addr)
+{
+    uint32_t v;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(cluster_addr) : "memory");
+    return v;
+}
+
+// How whole tiles are dealt to CTAs, or with parts > 1 the K blocks of a tile to the CTAs of a cluster: per_cta
+// each, one more for the first `longer`.
+struct Shares {
+    int parts, per_cta, longer;
+};
+
 template <int MP, int KIND>
 __global__ void __launch_bounds__(kNumThreads, 1)
 gemm_i8_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
                       const I8Epilogue ep, const int m_total, const int n_total, const int k_total,
                       const uint32_t idesc, int32_t* error_word, unsigned long long* split_counters,
-                      int32_t* split_slots, const unsigned long long split_tag, const int tile_rows)
+                      int32_t* split_slots, const unsigned long long split_tag, const int tile_rows, const int num_tiles, const Shares shares)
 {
     using Cfg = SkinnyConfig<MP>;
     constexpr int kStages = Cfg::kStages;
@@ -233,180 +390,237 @@ gemm_i8_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     const int warp = threadIdx.x >> 5;
     const int role = __shfl_sync(0xFFFFFFFFu, warp, 0);   // the same, warp-uniform to the compiler too
     const int lane = threadIdx.x & 31;
-    const int num_tiles = (n_total + tile_rows - 1) / tile_rows;
     const int num_kb = (k_total + kBlockKBytes - 1) / kBlockKBytes;
     const bool split = split_counters != nullptr;
     const int grid = static_cast<int>(gridDim.x);
-    const int64_t u_begin = range_begin(static_cast<int>(blockIdx.x), grid, num_tiles, num_kb, split);
-    const int64_t u_end = range_begin(static_cast<int>(blockIdx.x) + 1, grid, num_tiles, num_kb, split);
-    const SegmentList segments(u_begin, u_end, num_kb);
-    const int num_segments = segments.count();
+    const int cta = static_cast<int>(blockIdx.x);
+    // shares.parts > 1: a cluster of that many CTAs works one tile, each on its share of the K blocks.
+    const int parts = shares.parts;
+    const int rank = parts > 1 ? static_cast<int>(cluster_cta_rank()) : 0;
+    const int cluster = parts > 1 ? static_cast<int>(cluster_id()) : 0;
+    const SegmentList segments =
+        split ? SegmentList(range_begin(cta, grid, num_tiles, num_kb), range_begin(cta + 1, grid, num_tiles, num_kb), num_kb)
+              : SegmentList(SegmentList::Whole{cta * shares.per_cta + min(cta, shares.longer),
+                                               (cta + 1) * shares.per_cta + min(cta + 1, shares.longer)}, num_kb);
+    const int num_segments = parts > 1 ? 1 : warp_uniform(segments.count());
+    const auto segment_at = [&](int i) {
+        if (parts > 1) {
+            return Segment{cluster, rank * shares.per_cta + min(rank, shares.longer),
+                           (rank + 1) * shares.per_cta + min(rank + 1, shares.longer)};
+        }
+        return segments.uniform_at(i);
+    };
 
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < kStages; ++s) {
-            mbar_init(&full_bar[s], 1);
-            mbar_init(&empty_bar[s], 1);
+    // ---------------- TMA producer (warp 0) ----------------
+    // Like the MMA warp below: the whole warp walks the loop, one elected lane issues, and no branch
+    // depends on what a wait returned.  Its loads need no barrier but the ring's, which it sets up itself, and
+    // start before the CTA has met.
+    uint32_t spent = 0;   // probes of this role's waits
+    int stage = 0;
+    uint32_t phase = 0;
+    if (role == 0) {
+        if (lane == 0) {
+            for (int s = 0; s < kStages; ++s) {
+                mbar_init(&full_bar[s], 1);
+                mbar_init(&empty_bar[s], 1);
+            }
+            for (int a = 0; a < 2; ++a) {
+                mbar_init(&acc_full_bar[a], 1);
+                mbar_init(&acc_empty_bar[a], kEpilogueThreads / 32);
+            }
+            *abort_flag = 0;
+            mbar_init_fence();
         }
-        for (int a = 0; a < 2; ++a) {
-            mbar_init(&acc_full_bar[a], 1);
-            mbar_init(&acc_empty_bar[a], kEpilogueThreads / 32);
-        }
-        *abort_flag = 0;
-        mbar_init_fence();
-    }
-    if (warp == 0 && lane == 0) {
-        tma_prefetch_desc(&map_w);
-        tma_prefetch_desc(&map_a);
-    }
-    if (warp == 1) {
+        __syncwarp();
+        named_barrier_arrive(1, kNumThreads);   // the others meet below; this warp needs nothing of theirs
+    } else if (warp == 1) {
         tmem_alloc(tmem_slot, Cfg::kTmemCols);
         tmem_relinquish();
     }
     // Per-row epilogue terms of every activation row, once per CTA (the rows are the same for all tiles).
-    if (warp >= 2) {
+    else {
         const int t = threadIdx.x - 64;
-        if (t < m_total) {
-            row_terms[t] = i8_row_terms(ep, t);
+        if (t < Cfg::kRowTerms) {
+            row_terms[t] = i8_row_terms(ep, t < m_total ? t : 0);
         }
     }
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
+    if (role != 0) {
+        tc_fence_before_sync();
+        named_barrier_sync(1, kNumThreads);
+        tc_fence_after_sync();
+    }
     const uint32_t tmem_base = *tmem_slot;
 
     if (role == 0) {
-        // ---------------- TMA producer ----------------
-        if (lane == 0) {
-            int stage = 0;
-            uint32_t phase = 0;
-            uint32_t armed = 0;
-            uint32_t armed_phase = 0;
-            bool ok = true;
-            for (int si = 0; ok && si < num_segments; ++si) {
-                const Segment seg = segments.at(si);
-                const int tile = seg.tile;
-                for (int kb = seg.kb0; kb < seg.kb1; ++kb) {
-                    if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag)) {
-                        atomicCAS(error_word, 0, kErrProducerWait);
-                        ok = false;
-                        break;
-                    }
-                    uint8_t* w_dst = stage_base + stage * Cfg::kStageBytes;
-                    uint8_t* a_dst = w_dst + Cfg::kWTileBytes;
-                    mbar_expect_tx(&full_bar[stage], static_cast<uint32_t>(tile_rows * kBlockKBytes + Cfg::kATileBytes));
-                    tma_load_2d(w_dst, &map_w, &full_bar[stage], kb * kBlockKBytes, tile * tile_rows);
-                    tma_load_2d(a_dst, &map_a, &full_bar[stage], kb * kBlockKBytes, 0);
-                    armed |= 1u << stage;
-                    armed_phase = (armed_phase & ~(1u << stage)) | (phase << stage);
-                    if (++stage == kStages) {
-                        stage = 0;
-                        phase ^= 1u;
-                    }
-                }
-            }
-            if (!ok) {
-                // Copies already issued still land in shared memory: wait (bounded) for the armed slots.
-                const long long t0 = clock64();
-                for (int s = 0; s < kStages; ++s) {
-                    if ((armed >> s) & 1u) {
-                        while (!mbar_try_wait(&full_bar[s], (armed_phase >> s) & 1u)) {
-                            if (clock64() - t0 > kWaitLimitCycles) {
-                                atomicCAS(error_word, 0, kErrDrainWait);
-                                break;
-                            }
-                        }
-                    }
-                }
-            }
-        }
-        __syncwarp();
-    } else if (role == 1) {
-        // ---------------- MMA issuer ----------------
-        // The whole warp walks the loop and one elected lane issues: tensor-memory addresses and
-        // descriptors are then warp-uniform to the compiler, which is how the MMA takes its operands
-        // (N = 11008, K = 4096, 24 / 64 rows: 16.7 / 19.5 -> 16.1 / 19.2 us).
-        const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, tmem_base, 0);
-        int stage = 0;
-        uint32_t phase = 0;
-        bool ok = true;
-        for (int local_seg = 0; ok && local_seg < num_segments; ++local_seg) {
-            const Segment seg = segments.at(local_seg);
-            const int acc = local_seg & 1;
-            const uint32_t acc_phase = (local_seg >> 1) & 1u;
-            if (!mbar_wait_warp(&acc_empty_bar[acc], acc_phase ^ 1u, abort_flag)) {
-                if (lane == 0) {
-                    atomicCAS(error_word, 0, kErrAccumWait);
-                }
-                break;
-            }
-            tc_fence_after_sync();
-            const uint32_t d_tmem = tmem + static_cast<uint32_t>(acc * MP);
+        uint32_t issued = 0;
+        for (int si = 0; si < num_segments; ++si) {
+            const Segment seg = segment_at(si);
+            const int row = seg.tile * tile_rows;
             for (int kb = seg.kb0; kb < seg.kb1; ++kb) {
-                if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag)) {
-                    if (lane == 0) {
-                        atomicCAS(error_word, 0, kErrMmaWait);
-                    }
-                    ok = false;
-                    break;
-                }
-                tc_fence_after_sync();
-                const uint32_t w_addr = smem_u32(stage_base + stage * Cfg::kStageBytes);
-                const uint32_t a_addr = w_addr + Cfg::kWTileBytes;
-                const uint64_t w_desc = umma_desc_sw128_kmajor(w_addr);  // the MMA's 128-row operand
-                const uint64_t a_desc = umma_desc_sw128_kmajor(a_addr);  // its N operand: MP activation rows
-                if (elect_one()) {
-#pragma unroll
-                    for (int ks = 0; ks < kBlockKBytes / kUmmaK; ++ks) {
-                        umma_i8(d_tmem, w_desc + static_cast<uint64_t>(ks * 2), a_desc + static_cast<uint64_t>(ks * 2),
-                                idesc, (kb > seg.kb0 || ks > 0) ? 1u : 0u);
-                    }
-                    umma_commit(&empty_bar[stage]);
-                    if (kb == seg.kb1 - 1) {
-                        umma_commit(&acc_full_bar[acc]);
-                    }
+                mbar_wait_converged(&empty_bar[stage], phase ^ 1u, abort_flag, spent);
+                if (elect_one() && !wait_failed(spent)) {
+                    uint8_t* w_dst = stage_base + stage * Cfg::kStageBytes;
+                    mbar_expect_tx(&full_bar[stage], static_cast<uint32_t>(tile_rows * kBlockKBytes + Cfg::kATileBytes));
+                    tma_load_2d(w_dst, &map_w, &full_bar[stage], kb * kBlockKBytes, row);
+                    tma_load_2d(w_dst + Cfg::kWTileBytes, &map_a, &full_bar[stage], kb * kBlockKBytes, 0);
                 }
                 __syncwarp();
+                issued += wait_failed(spent) ? 0u : 1u;
                 if (++stage == kStages) {
                     stage = 0;
                     phase ^= 1u;
                 }
             }
         }
+        if (wait_failed(spent) && lane == 0) {
+            atomicCAS(error_word, 0, kErrProducerWait);
+            if (!drain_ring(full_bar, kStages, issued)) {
+                atomicCAS(error_word, 0, kErrDrainWait);
+            }
+        }
         __syncwarp();
+        if (parts > 1) {
+            cluster_sync_all();
+            cluster_sync_all_relaxed();
+        }
+    } else if (role == 1) {
+        // ---------------- MMA issuer ----------------
+        // The whole warp walks the loop and one elected lane issues: tensor-memory addresses and
+        // descriptors are then warp-uniform to the compiler, which is how the MMA takes its operands.
+        // The waits keep it so (see mbar_wait_converged): a K block of four MMAs takes 160 to 256 cycles
+        // of tensor pipe, and the loop took 525 cycles a block while its waits branched.
+        const uint32_t tmem = warp_uniform(tmem_base);
+        // The ring's descriptors advance by addition; the activations' tile lies behind the weights'.
+        const uint64_t first_desc = umma_desc_sw128_kmajor(smem_u32(stage_base));
+        uint64_t w_desc = first_desc;   // the MMA's 128-row operand
+        for (int local_seg = 0; local_seg < num_segments; ++local_seg) {
+            const Segment seg = segment_at(local_seg);
+            const int acc = local_seg & 1;
+            const uint32_t acc_phase = (local_seg >> 1) & 1u;
+            mbar_wait_converged(&acc_empty_bar[acc], acc_phase ^ 1u, abort_flag, spent);
+            tc_fence_after_sync();
+            const uint32_t d_tmem = tmem + static_cast<uint32_t>(acc * MP);
+            uint32_t accumulate = 0;
+            for (int kb = seg.kb0; kb < seg.kb1; ++kb) {
+                mbar_wait_converged(&full_bar[stage], phase, abort_flag, spent);
+                tc_fence_after_sync();
+                const uint64_t a_desc = w_desc + Cfg::kWTileBytes / 16;  // its N operand: MP activation rows
+                if (elect_one()) {
+#pragma unroll
+                    for (int ks = 0; ks < kBlockKBytes / kUmmaK; ++ks) {
+                        umma_i8(d_tmem, w_desc + static_cast<uint64_t>(ks * 2), a_desc + static_cast<uint64_t>(ks * 2),
+                                idesc, ks > 0 ? 1u : accumulate);
+                    }
+                    umma_commit(&empty_bar[stage]);
+                }
+                __syncwarp();
+                accumulate = 1;
+                w_desc += Cfg::kStageBytes / 16;
+                if (++stage == kStages) {
+                    stage = 0;
+                    phase ^= 1u;
+                    w_desc = first_desc;
+                }
+            }
+            if (elect_one()) {
+                umma_commit(&acc_full_bar[acc]);
+            }
+            __syncwarp();
+        }
+        if (wait_failed(spent)) {
+            if (lane == 0) {
+                atomicCAS(error_word, 0, kErrMmaWait);
+            }
+            umma_settle_after_failure();
+        }
+        __syncwarp();
+        if (parts > 1) {
+            cluster_sync_all();
+            cluster_sync_all_relaxed();
+        }
     } else {
         // ---------------- epilogue warps: one channel per thread ----------------
         const int quarter = warp & 3;
-        const float zpf = static_cast<float>(ep.out_zp);
-        const float lo = (KIND == NNB200_OUT_S8 ? -128.0f : 0.0f) - zpf;
-        const float hi = (KIND == NNB200_OUT_S8 ? 127.0f : 255.0f) - zpf;
         const int ch = quarter * 32 + lane;  // this thread's channel within the tile
         const int64_t total_units = static_cast<int64_t>(num_tiles) * num_kb;
         const size_t slot_elems = static_cast<size_t>(kBlockN) * static_cast<size_t>(m_total);
         const int group = (warp - 2) >> 2;
-        int local_seg = group;
-        for (; local_seg < num_segments; local_seg += 2) {
-            const Segment seg = segments.at(local_seg);
+        if (parts > 1) {
+            // Each CTA of the cluster finishes its share of the tile's rows, four at a time per warp, from
+            // everybody's sums.  The first pass stores nothing: it brings the instructions in while the weights
+            // stream (cold, they took longer than the work itself).
+            const int64_t n = static_cast<int64_t>(cluster) * tile_rows + ch;
+            const bool n_ok = ch < tile_rows && n < n_total;
+            const ChannelTerms ct = channel_terms<KIND>(ep, n, n_ok);
+            uint32_t* mine = reinterpret_cast<uint32_t*>(stage_base) + ch;
+            int row = 0, row_end = 1, store_end = 0, part = rank, part_step = 0;   // first pass: its own sums only, the others' CTAs may not have begun
+#pragma unroll 1
+            for (int pass = 0; pass < 2; ++pass) {
+                if (pass == 1) {
+                    part_step = 1;
+                    if (mbar_wait_warp(&acc_full_bar[0], 0, abort_flag)) {
+                        tc_fence_after_sync();
+                        const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+                        // This CTA's sums, [row][channel], where the ring was: all its loads have been consumed.
+#pragma unroll 1
+                        for (int r = group * 8; r < m_total; r += 16) {
+                            uint32_t v[8];
+                            tmem_ld_32x8(t_row + static_cast<uint32_t>(r), v);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) {
+                                mine[(r + j) * kBlockN] = v[j];
+                            }
+                        }
+                    } else if (lane == 0) {
+                        atomicCAS(error_word, 0, kErrEpilogueWait);
+                    }
+                    __syncwarp();
+                    cluster_sync_all();
+                    row = rank * m_total / parts + group * 4;
+                    store_end = row_end = (rank + 1) * m_total / parts;
+                    part = 0;
+                }
+#pragma unroll 1
+                for (int r = row; r < row_end; r += 8) {
+                    // All loads before any sum: one round trip to the other SMs.
+                    uint32_t theirs[kMaxParts][4];
+#pragma unroll
+                    for (int p = 0; p < kMaxParts; ++p) {
+                        if (p < parts) {
+                            const uint32_t from = map_to_cta(smem_u32(mine), static_cast<uint32_t>(part + p * part_step));
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                theirs[p][j] = ld_shared_cluster_u32(from + static_cast<uint32_t>((r + j) * kBlockN) * 4);
+                            }
+                        }
+                    }
+                    uint32_t v[4] = {0, 0, 0, 0};
+#pragma unroll
+                    for (int p = 0; p < kMaxParts; ++p) {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            v[j] += p < parts ? theirs[p][j] : 0u;
+                        }
+                    }
+                    finish_rows<KIND, 4>(ep, row_terms, v, r, store_end, n, n_ok, ct);
+                }
+            }
+            __syncwarp();
+            cluster_sync_all_relaxed();   // nobody leaves while its sums may still be read
+        }
+        // A CTA that holds one piece has both groups work on it, eight rows in turn.
+        const bool shared = num_segments == 1 && !split;
+        for (int local_seg = shared ? 0 : group; parts == 1 && local_seg < num_segments; local_seg += 2) {
+            const Segment seg = segment_at(local_seg);
             const int tile = seg.tile;
             const int acc = local_seg & 1;
             const uint32_t acc_phase = (local_seg >> 1) & 1u;
-            const bool partial = seg.kb0 != 0 || seg.kb1 != num_kb;  // only under the equal-share split
+            const bool partial = split && (seg.kb0 != 0 || seg.kb1 != num_kb);
             const int64_t n = static_cast<int64_t>(tile) * tile_rows + ch;
             const bool n_ok = ch < tile_rows && n < n_total;
             // This channel's terms, in registers for the whole tile.
-            const int32_t zpw = (n_ok && ep.zp_w != nullptr) ? ep.zp_w[n] : ep.zp_w_scalar;
-            const int32_t rw = (n_ok && ep.compensate && ep.r_w != nullptr) ? ep.r_w[n] : 0;
-            const float s_w = (n_ok && ep.scale_w != nullptr) ? ep.scale_w[n] : ep.scale_w_scalar;
-            int32_t bias_i = 0;
-            float bias_f = 0.0f;
-            if (n_ok && ep.bias != nullptr) {
-                if constexpr (KIND <= NNB200_OUT_U8) {
-                    bias_i = static_cast<const int32_t*>(ep.bias)[n];
-                } else if constexpr (KIND == NNB200_OUT_F32) {
-                    bias_f = static_cast<const float*>(ep.bias)[n];
-                } else {
-                    bias_f = __half2float(static_cast<const __half*>(ep.bias)[n]);
-                }
-            }
+            const ChannelTerms ct = channel_terms<KIND>(ep, n, n_ok);
 
             // Part of a tile.  While this piece's MMAs are still running, look whether everybody else
             // has published already; if so this warp will finish the tile and fetches the others'
@@ -432,13 +646,48 @@ gemm_i8_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 }
             }
 
+            const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
+                                   static_cast<uint32_t>(acc * MP);
+            if (!partial) {
+                // A whole tile.  The first of the CTA's starts with a pass that stores nothing: it brings the
+                // instructions in while the weights stream (cold, they took longer than the work itself).
+                bool ok = true;
+#pragma unroll 1
+                for (int pass = local_seg < 2 ? 0 : 1; pass < 2; ++pass) {
+                    int row = 0, row_end = 1;
+                    if (pass == 1) {
+                        ok = mbar_wait_warp(&acc_full_bar[acc], acc_phase, abort_flag);
+                        if (!ok) {
+                            break;
+                        }
+                        tc_fence_after_sync();
+                        row = shared ? group * 8 : 0;
+                        row_end = m_total;
+                    }
+#pragma unroll 1
+                    for (int r = row; r < row_end; r += shared ? 16 : 8) {
+                        uint32_t v[8];
+                        tmem_ld_32x8(t_row + static_cast<uint32_t>(r), v);
+                        tmem_ld_wait();
+                        finish_rows<KIND, 8>(ep, row_terms, v, r, pass == 1 ? row_end : 0, n, n_ok, ct);
+                    }
+                }
+                if (!ok) {
+                    atomicCAS(error_word, 0, kErrEpilogueWait);
+                    break;
+                }
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(&acc_empty_bar[acc]);
+                }
+                continue;
+            }
             if (!mbar_wait_warp(&acc_full_bar[acc], acc_phase, abort_flag)) {
                 atomicCAS(error_word, 0, kErrEpilogueWait);
                 break;
             }
             tc_fence_after_sync();
-            const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
-                                   static_cast<uint32_t>(acc * MP);
             // Otherwise: publish this warp's 32 channels, count in, and carry on only if every other
             // part of the tile has been published by then.
             bool finish = true;
@@ -498,42 +747,21 @@ gemm_i8_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 if (c * 32 >= m_total || !finish) {
                     break;  // uniform
                 }
-                uint32_t v[32];
-                tmem_ld_32x32(t_row + static_cast<uint32_t>(c * 32), v);
-                tmem_ld_wait();
-                if (partial) {
-                    if (!(early && c == 0)) {
-                        collect_parts(early_sum, split_slots, slot_elems, ch, first_cta, last_cta,
-                                      static_cast<int>(blockIdx.x), c * 32, m_total);
-                    }
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        v[j] += static_cast<uint32_t>(early_sum[j]);
-                    }
+                if (!(early && c == 0)) {
+                    collect_parts(early_sum, split_slots, slot_elems, ch, first_cta, last_cta,
+                                  static_cast<int>(blockIdx.x), c * 32, m_total);
                 }
 #pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    const int m = c * 32 + j;
-                    if (m < m_total && n_ok) {
-                        const I8RowTerms t = row_terms[m];
-                        const int64_t idx = static_cast<int64_t>(m) * ep.ldc + n;
-                        const int32_t raw = static_cast<int32_t>(v[j]);
-                        if constexpr (KIND == NNB200_OUT_S32) {
-                            static_cast<int32_t*>(ep.out)[idx] = i8_int_value(ep, t, raw, zpw, rw, bias_i);
-                        } else if constexpr (KIND == NNB200_OUT_S8) {
-                            const int32_t val = i8_int_value(ep, t, raw, zpw, rw, bias_i);
-                            static_cast<int8_t*>(ep.out)[idx] =
-                                static_cast<int8_t>(i8_requant(val, __fmul_rn(t.row_k, s_w), lo, hi, ep.out_zp));
-                        } else if constexpr (KIND == NNB200_OUT_U8) {
-                            const int32_t val = i8_int_value(ep, t, raw, zpw, rw, bias_i);
-                            static_cast<uint8_t*>(ep.out)[idx] =
-                                static_cast<uint8_t>(i8_requant(val, __fmul_rn(t.row_k, s_w), lo, hi, ep.out_zp));
-                        } else if constexpr (KIND == NNB200_OUT_F32) {
-                            static_cast<float*>(ep.out)[idx] = i8_fp_value(ep, t, raw, zpw, rw, s_w, bias_f);
-                        } else {
-                            static_cast<__half*>(ep.out)[idx] =
-                                __float2half_rn(i8_fp_value(ep, t, raw, zpw, rw, s_w, bias_f));
-                        }
+                for (int r = 0; r < 32; r += 8) {
+                    uint32_t v[8];
+                    tmem_ld_32x8(t_row + static_cast<uint32_t>(c * 32 + r), v);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        v[j] += static_cast<uint32_t>(early_sum[r + j]);
+                    }
+                    if (c * 32 + r < m_total) {
+                        finish_rows<KIND, 8>(ep, row_terms, v, c * 32 + r, m_total, n, n_ok, ct);
                     }
                 }
             }
@@ -547,6 +775,7 @@ gemm_i8_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
 
     // ---------------- teardown ----------------
     tc_fence_before_sync();
+    __syncwarp();
     __syncthreads();
     if (warp == 1) {
         tc_fence_after_sync();
@@ -568,6 +797,17 @@ unsigned long long next_split_tag()
     return t;
 }
 
+// CTAs that share a tile's K, by way of their cluster: as many as leave every tile's cluster an SM per CTA.
+int cluster_parts(const I8Problem& p, const DeviceInfo& dev)
+{
+    const int64_t tiles = (p.n + kBlockN - 1) / kBlockN;
+    const int64_t num_kb = (p.k + kBlockKBytes - 1) / kBlockKBytes;
+    int64_t parts = dev.sm_count / tiles;
+    parts = parts > kMaxParts ? kMaxParts : parts;
+    parts = parts > num_kb / 4 ? num_kb / 4 : parts;
+    return parts > 1 ? static_cast<int>(parts) : 1;
+}
+
 template <int MP, int KIND>
 int launch_skinny_variant(const I8Problem& p, const I8Epilogue& ep, const DeviceInfo& dev, void* split_scratch,
                           cudaStream_t stream)
@@ -576,8 +816,29 @@ int launch_skinny_variant(const I8Problem& p, const I8Epilogue& ep, const Device
     auto kernel = gemm_i8_skinny_kernel<MP, KIND>;
     static std::once_flag once[kMaxDevices];
     static cudaError_t attr_err[kMaxDevices];
+    static int resident[kMaxDevices][kMaxParts + 1];   // clusters of that many CTAs the device holds at once
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(kNumThreads);
+    cfg.dynamicSmemBytes = Cfg::kSmemBytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
     std::call_once(once[dev.device], [&] {
         attr_err[dev.device] = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+        cfg.numAttrs = 1;
+        for (int c = 2; c <= kMaxParts && attr_err[dev.device] == cudaSuccess; ++c) {
+            attr.val.clusterDim.x = static_cast<unsigned>(c);
+            cfg.gridDim = dim3(static_cast<unsigned>(dev.sm_count / c * c));
+            int count = 0;
+            if (cudaOccupancyMaxActiveClusters(&count, kernel, &cfg) == cudaSuccess) {
+                resident[dev.device][c] = count;
+            } else {
+                (void)cudaGetLastError();   // no clusters of that many: the launch takes a smaller one
+            }
+        }
     });
     if (attr_err[dev.device] != cudaSuccess) {
         return NNB200_INTERNAL;
@@ -587,9 +848,13 @@ int launch_skinny_variant(const I8Problem& p, const I8Epilogue& ep, const Device
     // rows, 128-channel tiles / equal ones: N = 28672, K = 8192 51.8 / 45.4 us, N = 19456, K = 4096 28.1 / 24.8).
     // A caller that brings the scratch for shared K gets that on the first of the two: 45.7.
     // A single wave keeps 128 channels: more CTAs load the activations more often, which eats what the
-    // even weight stream gives (N = 11008, K = 4096: 24 rows 16.7 / 16.4, 64 rows 19.5 / 20.1, 128 rows
-    // 24.7 / 26.6).  Shared K evens the SMs out itself, and its scratch is laid out for 128.
+    // even weight stream gives (64 and 128 rows lost 3 and 8 % at N = 11008, K = 4096, 24 rows won 2).  Shared
+    // K evens the SMs out itself, and its scratch is laid out for 128.
     int tile_rows = kBlockN;
+    int parts = split_scratch != nullptr && knob(NNB200_KNOB_I8_SHARE_K) == 2 ? 1 : cluster_parts(p, dev);
+    while (parts > 1 && resident[dev.device][parts] < (n + kBlockN - 1) / kBlockN) {
+        --parts;
+    }
     const int waves = ((n + kBlockN - 1) / kBlockN + dev.sm_count - 1) / dev.sm_count;
     if (split_scratch == nullptr && waves > 1) {
         tile_rows = (n + waves * dev.sm_count - 1) / (waves * dev.sm_count);
@@ -606,7 +871,9 @@ int launch_skinny_variant(const I8Problem& p, const I8Epilogue& ep, const Device
     unsigned long long* counters = nullptr;
     int32_t* slots = nullptr;
     unsigned long long tag = 0;
-    if (split_scratch != nullptr) {
+    if (parts > 1) {
+        grid = num_tiles * parts;
+    } else if (split_scratch != nullptr) {
         // Equal shares of all K blocks over every SM.
         grid = dev.sm_count;
         counters = static_cast<unsigned long long*>(split_scratch);
@@ -615,10 +882,17 @@ int launch_skinny_variant(const I8Problem& p, const I8Epilogue& ep, const Device
     }
     // 128-row operand = weights (s8), N operand = activations (s8 or u8).
     const uint32_t idesc = umma_idesc(2, 1, p.a_unsigned ? 0u : 1u, kBlockN, MP);
-    kernel<<<grid, kNumThreads, Cfg::kSmemBytes, stream>>>(map_w, map_a, ep, m, n, k, idesc, dev.error_word, counters,
-                                                             slots, tag, tile_rows);
+    cfg.gridDim = dim3(static_cast<unsigned>(grid));
+    attr.val.clusterDim.x = static_cast<unsigned>(parts);
+    cfg.numAttrs = parts > 1 ? 1 : 0;
+    Shares shares{parts, 0, 0};
+    const int dealt = parts > 1 ? (k + kBlockKBytes - 1) / kBlockKBytes : num_tiles, hands = parts > 1 ? parts : grid;
+    shares.per_cta = dealt / hands;
+    shares.longer = dealt % hands;
+    const cudaError_t launched = cudaLaunchKernelEx(&cfg, kernel, map_w, map_a, ep, m, n, k, idesc, dev.error_word, counters, slots,
+                                                    tag, tile_rows, num_tiles, shares);
     note_launch();
-    return cuda_status(cudaGetLastError());
+    return cuda_status(launched);
 }
 
 template <int MP>
@@ -641,7 +915,36 @@ int launch_skinny_mp(const I8Problem& p, const I8Epilogue& ep, const DeviceInfo&
 // pose: a [K, N] weight runs on the square engine), at most 128 activation rows.
 bool skinny_i8_supported(const I8Problem& p)
 {
-    return p.m >= 1 && p.m <= 128 && p.a_stride_k == 1 && p.w_stride_k == 1 && umma_i8_supported(p);
+    return p.m >= 1 && p.m <= 128 && p.a_stride_k == 1 && p.w_stride_k == 1 && umma_i8_supported(p) &&
+           (p.n / kBlockN + 1) * (p.k / kBlockKBytes + 1) < (int64_t{1} << 29);   // units are counted in 32 bits
+}
+
+// Whether a call that the square engine or the streaming engine (up to 16 rows) would get by its number of
+// rows and channels is better off here, on clusters that share K.  CUDA-graph timings, weights beyond L2,
+// here / square engine, us:
+//   rows   N = 1024                                4096                                8192
+//     32   K = 512 4.2 / 4.5, 4096 5.1 / 8.6       512 4.4 / 5.1, 4096 7.2 / 9.6       4096 9.8 / 10.5, 8192 14.4 / 16.8
+//     64   512 4.9 / 4.6, 2048 5.4 / 6.2           512 5.0 / 4.8, 4096 8.1 / 9.5       2048 8.4 / 7.8, 8192 15.4 / 16.7
+//    128   2048 6.7 / 6.4, 4096 7.2 / 8.8          2048 8.1 / 7.3, 4096 9.5 / 9.9      4096 13.2 / 10.6
+// and here / streaming engine at 16 rows:
+//          2048 4.2 / 3.8, 4096 4.9 / 5.6          2048 5.5 / 5.1, 4096 6.9 / 7.7      512 4.1 / 5.8, 4096 9.4 / 14.4
+//   N = 64: K = 4096 4.9 / 4.7, 8192 5.1 / 6.3.
+bool skinny_i8_preferred(const I8Problem& p, bool over_streaming, const DeviceInfo& dev)
+{
+    if (!skinny_i8_supported(p) || p.m < 9) {
+        return false;
+    }
+    const int64_t tiles = (p.n + kBlockN - 1) / kBlockN;
+    if (over_streaming) {
+        return tiles * 3 > dev.sm_count || p.k >= 8192 || (p.n >= 1024 && p.k >= 4096);
+    }
+    if (p.m <= 32) {
+        return true;
+    }
+    if (p.m <= 64) {
+        return tiles * 3 <= dev.sm_count ? p.k >= 2048 : p.k >= 8192;
+    }
+    return tiles * 4 <= dev.sm_count && p.k >= 4096;
 }
 
 // Scratch for the equal-share split of K over all SMs, or 0 when it would not pay.  Publishing a
@@ -663,7 +966,9 @@ bool skinny_i8_supported(const I8Problem& p)
 // Hence: with one wave, share when the busiest CTA sheds at least 30 K blocks, plus 0.7 per row
 // above 12; with several waves, when the last one is less than 9/10 full, a share is at least 48
 // K blocks and there are at most 64 rows.
-// Knob I8_SHARE_K = 0 turns the split off; 2 offers it from 8 K blocks per SM (measurement, tests).
+// A caller that brings the scratch where clusters share K gets those all the same (4096 x 14336, 24 rows: 21.3 us
+// on the scratch, 13.3 in clusters; the offer stays, engines are named by it).
+// Knob I8_SHARE_K = 0 turns this split off; 2 offers it from 8 K blocks per SM and prefers it (measurement, tests).
 size_t skinny_i8_split_bytes(const I8Problem& p, const DeviceInfo& dev)
 {
     if (!skinny_i8_supported(p)) {

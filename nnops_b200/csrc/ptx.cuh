@@ -41,6 +41,10 @@ __device__ __forceinline__ bool elect_one()
     return pred != 0;
 }
 
+// A value that is the same in every lane of a converged warp, known as such to the compiler.
+__device__ __forceinline__ int warp_uniform(int v) { return __shfl_sync(0xFFFFFFFFu, v, 0); }
+__device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __shfl_sync(0xFFFFFFFFu, v, 0); }
+
 // ---- mbarrier ---------------------------------------------------------------------------
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count)
@@ -142,6 +146,69 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
     }
     ok = __shfl_sync(0xFFFFFFFFu, ok, 0);
     return ok != 0;
+}
+
+// Wait of a whole warp that stays warp-uniform to the compiler: every lane polls, and nothing branches on
+// the outcome.  `spent` counts the probes of the wait under way (each suspends the warp for up to ~4 us)
+// and stays at the limit once a wait has run out or another role has aborted; later waits of the same
+// role then fall through at once, so a loop that goes on regardless still ends, in the time its own
+// instructions take.  The loops that issue tcgen05.mma are built on this: after a branch on a polled
+// value the compiler no longer knows the warp converged and hands the MMA its tensor-memory address and
+// descriptors register by register, and a suspend-time hint costs a hundred cycles on a barrier that is
+// ready.  Loop of one wait and four M128 x N32 x K32 MMAs (160 cycles of tensor pipe): 443 cycles with
+// mbar_wait_warp, 500 with one thread and mbar_wait, 185 with this; N128 (256 cycles): 467 / 500 / 262.
+constexpr uint32_t kWaitProbes = 500000;   // 2 s of suspended probes
+
+__device__ __forceinline__ void mbar_wait_converged(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t& spent)
+{
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        ".reg .u32 f;\n\t"
+        "WAIT_LOOP:\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "@p bra WAIT_DONE;\n\t"
+        "ld.volatile.shared.u32 f, [%3];\n\t"
+        "mad.lo.u32 %0, f, %4, %0;\n\t"
+        "add.u32 %0, %0, 1;\n\t"
+        "setp.lt.u32 q, %0, %4;\n\t"
+        "@!q st.volatile.shared.u32 [%3], 1;\n\t"
+        "@q bra WAIT_LOOP;\n\t"
+        "WAIT_DONE:\n\t"
+        "setp.lt.u32 q, %0, %4;\n\t"
+        "selp.u32 %0, 0, %4, q;\n\t"
+        "}"
+        : "+&r"(spent)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(smem_u32(const_cast<const int*>(abort_flag))), "r"(kWaitProbes)
+        : "memory");
+}
+
+__device__ __forceinline__ bool wait_failed(uint32_t spent) { return spent >= kWaitProbes; }
+
+// After a failed wait: the MMAs already issued are left the time to finish (a full queue is a few
+// microseconds) before the CTA gives its tensor memory back.
+__device__ __forceinline__ void umma_settle_after_failure()
+{
+    const long long t0 = clock64();
+    while (clock64() - t0 < 1'000'000) {
+    }
+}
+
+// After the producer's wait failed: `issued` stages have been loaded in turn into `stages` slots, and what is in
+// flight still lands in shared memory; wait (bounded) for the last load of every slot.  False if one
+// did not land.
+__device__ __forceinline__ bool drain_ring(uint64_t* full_bar, int stages, uint32_t issued)
+{
+    const long long t0 = clock64();
+    const uint32_t first = issued > static_cast<uint32_t>(stages) ? issued - static_cast<uint32_t>(stages) : 0u;
+    for (uint32_t i = first; i < issued; ++i) {
+        while (!mbar_try_wait(&full_bar[i % static_cast<uint32_t>(stages)], (i / static_cast<uint32_t>(stages)) & 1u)) {
+            if (clock64() - t0 > kWaitLimitCycles) {
+                return false;
+            }
+        }
+    }
+    return true;
 }
 
 // ---- TMA --------------------------------------------------------------------------------
@@ -360,6 +427,15 @@ __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&v)[32])
         : "memory");
 }
 
+// The same, 8 columns.
+__device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&v)[8])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+
 __device__ __forceinline__ void tmem_ld_wait()
 {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -381,6 +457,12 @@ __device__ __forceinline__ void multimem_st_16(void* mc_addr, uint4 v)
     asm volatile("multimem.st.relaxed.sys.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(mc_addr), "f"(__uint_as_float(v.x)),
                  "f"(__uint_as_float(v.y)), "f"(__uint_as_float(v.z)), "f"(__uint_as_float(v.w))
                  : "memory");
+}
+
+// The arrival of a warp that does not wait itself.
+__device__ __forceinline__ void named_barrier_arrive(uint32_t id, uint32_t nthreads)
+{
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
 // Named barrier over a subset of the CTA's warps.

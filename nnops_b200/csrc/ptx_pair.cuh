@@ -16,6 +16,13 @@ __device__ __forceinline__ uint32_t cluster_cta_rank()
     return r;
 }
 
+__device__ __forceinline__ uint32_t cluster_id()
+{
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%clusterid.x;" : "=r"(r));
+    return r;
+}
+
 // Address of the same shared-memory location in CTA `rank` of this cluster (shared::cluster window).
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank)
 {
@@ -29,6 +36,14 @@ __device__ __forceinline__ void cluster_sync_all()
 {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// The same without ordering memory: for "I have read what was yours", after the values read have been used.
+// The releasing form waits for the caller's global stores to be acknowledged first, about a microsecond.
+__device__ __forceinline__ void cluster_sync_all_relaxed()
+{
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
 }
 
 // Arrive on an mbarrier that may live in the other CTA (address from map_to_cta).
@@ -91,6 +106,32 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
             }
         }
     }
+}
+
+// mbar_wait_converged with the cluster-scope probe.
+__device__ __forceinline__ void mbar_wait_converged_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                                            uint32_t& spent)
+{
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        ".reg .u32 f;\n\t"
+        "WAIT_LOOP:\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "@p bra WAIT_DONE;\n\t"
+        "ld.volatile.shared.u32 f, [%3];\n\t"
+        "mad.lo.u32 %0, f, %4, %0;\n\t"
+        "add.u32 %0, %0, 1;\n\t"
+        "setp.lt.u32 q, %0, %4;\n\t"
+        "@!q st.volatile.shared.u32 [%3], 1;\n\t"
+        "@q bra WAIT_LOOP;\n\t"
+        "WAIT_DONE:\n\t"
+        "setp.lt.u32 q, %0, %4;\n\t"
+        "selp.u32 %0, 0, %4, q;\n\t"
+        "}"
+        : "+&r"(spent)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(smem_u32(const_cast<const int*>(abort_flag))), "r"(kWaitProbes)
+        : "memory");
 }
 
 // 2-D tiled load into THIS CTA's shared memory whose byte count is reported to the mbarrier at
