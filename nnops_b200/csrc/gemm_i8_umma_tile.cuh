@@ -659,13 +659,6 @@ gemm_i8_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     static_assert(!BATCH || (!CONV && PEERS == 0), "the batched form is a plain product");
     using Cfg = TileConfig<BN, PEERS, KIND>;
     constexpr int kStages = Cfg::kStages;
-    // Narrow tiles: the whole warp walks the MMA loop and one elected lane issues.  Tensor-memory
-    // addresses and descriptors are then warp-uniform to the compiler, which is how the MMA takes its
-    // operands, and an MMA of 64 columns no longer waits for its own issue (64 x 4096 x 4096 14.0 -> 12.9
-    // us, 200 x 4096 x 4096 14.6 -> 13.5).  A 256-column MMA takes longer than either way of issuing it,
-    // and the kernels for wide tiles measured 3-9 % slower in this form.
-    constexpr bool kWarpIssue = BN <= 128;
-
     extern __shared__ uint8_t smem_raw[];
     // The swizzled tiles must start on a 1024-byte boundary.
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -681,7 +674,7 @@ gemm_i8_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5;
-    const int role = kWarpIssue ? __shfl_sync(0xFFFFFFFFu, warp, 0) : warp;   // the same, warp-uniform to the compiler too
+    const int role = warp_uniform(warp);   // the same, warp-uniform to the compiler too
     const int lane = threadIdx.x & 31;
     // Operand poses ride in bits 4-5 of vec_ok: bit 4 = A stored [K][M], bit 5 = W stored [K][N]
     // (MN-major operands: the tensor maps, the descriptors and the K step change, nothing else).
@@ -702,77 +695,90 @@ gemm_i8_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const auto batch_of = [&](int tile) { return BATCH ? static_cast<int>(by_elem.div(static_cast<uint32_t>(tile))) : 0; };
     const auto coord_of = [&](int tile) { return walk(BATCH ? tile - batch_of(tile) * elem_tiles : tile); };
 
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < kStages; ++s) {
-            mbar_init(&full_bar[s], 1);
-            mbar_init(&empty_bar[s], 1);
+    // The producer warp sets the barriers up and starts to load at once: it needs nothing of the others, who
+    // meet at a barrier of their own.
+    constexpr uint32_t kThreads = tile_threads(KIND, PEERS);
+    uint32_t spent = 0;   // probes of this role's waits
+    int stage = 0;
+    uint32_t phase = 0;
+    if (role == 0) {
+        if (lane == 0) {
+            for (int s = 0; s < kStages; ++s) {
+                mbar_init(&full_bar[s], 1);
+                mbar_init(&empty_bar[s], 1);
+            }
+            for (int a = 0; a < 2; ++a) {
+                mbar_init(&acc_full_bar[a], 1);
+                mbar_init(&acc_empty_bar[a], Cfg::kEpilogueWarps / Cfg::kGroups);
+            }
+            *abort_flag = 0;
+            mbar_init_fence();
         }
-        for (int a = 0; a < 2; ++a) {
-            mbar_init(&acc_full_bar[a], 1);
-            mbar_init(&acc_empty_bar[a], Cfg::kEpilogueWarps / Cfg::kGroups);
+        __syncwarp();
+        named_barrier_arrive(1, kThreads);
+    } else {
+        if (role == 1) {
+            if (lane == 0) {
+                tma_prefetch_desc(&map_a);
+                tma_prefetch_desc(&map_w);
+            }
+            __syncwarp();
+            tmem_alloc(tmem_slot, Cfg::kTmemCols);
+            tmem_relinquish();
         }
-        *abort_flag = 0;
-        mbar_init_fence();
+        tc_fence_before_sync();
+        named_barrier_sync(1, kThreads);
+        tc_fence_after_sync();
     }
-    if (warp == 0 && lane == 0) {
-        tma_prefetch_desc(&map_a);
-        tma_prefetch_desc(&map_w);
-    }
-    if (warp == 1) {
-        tmem_alloc(tmem_slot, Cfg::kTmemCols);
-        tmem_relinquish();
-    }
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = *tmem_slot;   // not the producer's
 
     if (role == 0) {
         // ---------------- TMA producer ----------------
-        if (lane == 0) {
-            int stage = 0;
-            uint32_t phase = 0;
-            uint32_t armed = 0;        // bit s: slot s has been armed at least once
-            uint32_t armed_phase = 0;  // bit s: parity of the phase slot s was last armed in
-            bool ok = true;
-            for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
-                const TileCoord tc = coord_of(tile);
-                const int bat = batch_of(tile);
-                (void)bat;
-                const int rot = k_rotation(tile, k_rot, num_kb);
-                for (int step = 0; step < num_kb; ++step) {
-                    const int kb = step + rot < num_kb ? step + rot : step + rot - num_kb;
-                    if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag)) {
-                        atomicCAS(error_word, 0, kErrProducerWait);
-                        ok = false;
-                        break;
-                    }
+        // The whole warp walks the loop, one elected lane issues, and no branch depends on what a wait
+        // returned (see mbar_wait_converged); the same in the MMA warp.
+        uint32_t issued = 0;
+        for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+            const TileCoord at = coord_of(tile);
+            const int m_blk = warp_uniform(at.m_blk), n_blk = warp_uniform(at.n_blk);
+            const int bat = warp_uniform(batch_of(tile));
+            (void)bat;
+            const int rot = warp_uniform(k_rotation(tile, k_rot, num_kb));
+            int patch_w = 0, patch_h = 0, patch_img = 0, tap_a = 0, tap_b = 0, tap_c = 0;   // CONV
+            (void)patch_w; (void)patch_h; (void)patch_img; (void)tap_a; (void)tap_b; (void)tap_c;
+            if constexpr (CONV) {
+                const ConvPatch pt = conv_patch(conv, m_blk);
+                patch_w = warp_uniform((pt.tw << conv.bw_log2) * conv.sw - conv.pw);
+                patch_h = warp_uniform(pt.th * conv.bh * conv.sh - conv.ph);
+                patch_img = warp_uniform(pt.img);
+                const int tap = rot / conv.kb_per_tap;
+                tap_c = warp_uniform(rot - tap * conv.kb_per_tap);
+                tap_a = warp_uniform(tap / conv.kw);
+                tap_b = warp_uniform(tap - tap_a * conv.kw);
+            }
+            int kb = rot;
+            for (int step = 0; step < num_kb; ++step) {
+                mbar_wait_converged(&empty_bar[stage], phase ^ 1u, abort_flag, spent);
+                if (elect_one() && !wait_failed(spent)) {
                     uint8_t* a_dst = stage_base + stage * Cfg::kStageBytes;
                     uint8_t* b_dst = a_dst + Cfg::kATileBytes;
                     mbar_expect_tx(&full_bar[stage], Cfg::kStageBytes);
                     if constexpr (CONV) {
                         // Patch (image, th, tw) shifted by the k-block's tap; 128 channels of it.
-                        const ConvPatch pt = conv_patch(conv, tc.m_blk);
-                        const int tap = kb / conv.kb_per_tap;
-                        const int c0 = (kb - tap * conv.kb_per_tap) * kBlockKBytes;
-                        const int ta = tap / conv.kw;
-                        const int tb = tap - ta * conv.kw;
-                        tma_load_4d(a_dst, &map_a, &full_bar[stage], conv.c_base + c0,
-                                    (pt.tw << conv.bw_log2) * conv.sw - conv.pw + tb * conv.dw,
-                                    pt.th * conv.bh * conv.sh - conv.ph + ta * conv.dh, pt.img);
+                        tma_load_4d(a_dst, &map_a, &full_bar[stage], conv.c_base + tap_c * kBlockKBytes,
+                                    patch_w + tap_b * conv.dw, patch_h + tap_a * conv.dh, patch_img);
                     } else if constexpr (BATCH) {
                         // Either pose through a map {contiguous index, the other, batch, 1}.
                         const int az = bat * conv.a_step;
                         if (pose & 1) {
-                            tma_load_4d(a_dst, &map_a, &full_bar[stage], tc.m_blk * kBlockM, kb * kBlockKBytes, az, 0);
+                            tma_load_4d(a_dst, &map_a, &full_bar[stage], m_blk * kBlockM, kb * kBlockKBytes, az, 0);
                         } else {
-                            tma_load_4d(a_dst, &map_a, &full_bar[stage], kb * kBlockKBytes, tc.m_blk * kBlockM, az, 0);
+                            tma_load_4d(a_dst, &map_a, &full_bar[stage], kb * kBlockKBytes, m_blk * kBlockM, az, 0);
                         }
                     } else if (pose & 1) {
                         // A stored [K][M]: the box is 128 k-rows of 128 m-bytes.
-                        tma_load_2d(a_dst, &map_a, &full_bar[stage], tc.m_blk * kBlockM, kb * kBlockKBytes);
+                        tma_load_2d(a_dst, &map_a, &full_bar[stage], m_blk * kBlockM, kb * kBlockKBytes);
                     } else {
-                        tma_load_2d(a_dst, &map_a, &full_bar[stage], kb * kBlockKBytes, tc.m_blk * kBlockM);
+                        tma_load_2d(a_dst, &map_a, &full_bar[stage], kb * kBlockKBytes, m_blk * kBlockM);
                     }
                     if constexpr (BATCH) {
                         const int wz = bat * conv.w_step;
@@ -780,124 +786,115 @@ gemm_i8_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 #pragma unroll
                             for (int blk = 0; blk < BN / 128; ++blk) {
                                 tma_load_4d(b_dst + blk * (128 * kBlockKBytes), &map_w, &full_bar[stage],
-                                            tc.n_blk * BN + blk * 128, kb * kBlockKBytes, wz, 0);
+                                            n_blk * BN + blk * 128, kb * kBlockKBytes, wz, 0);
                             }
                         } else {
-                            tma_load_4d(b_dst, &map_w, &full_bar[stage], kb * kBlockKBytes, tc.n_blk * BN, wz, 0);
+                            tma_load_4d(b_dst, &map_w, &full_bar[stage], kb * kBlockKBytes, n_blk * BN, wz, 0);
                         }
                     } else if (pose & 2) {
                         // W stored [K][N]: one box of 128 k-rows x 128 n-bytes per 128 columns of the tile.
 #pragma unroll
                         for (int blk = 0; blk < BN / 128; ++blk) {
                             tma_load_2d(b_dst + blk * (128 * kBlockKBytes), &map_w, &full_bar[stage],
-                                        tc.n_blk * BN + blk * 128, kb * kBlockKBytes);
+                                        n_blk * BN + blk * 128, kb * kBlockKBytes);
                         }
                     } else {
 #pragma unroll
                         for (int h = 0; h < Cfg::kNSplit; ++h) {  // TMA boxes hold at most 256 rows
                             tma_load_2d(b_dst + h * Cfg::kMmaN * kBlockKBytes, &map_w, &full_bar[stage], kb * kBlockKBytes,
-                                        tc.n_blk * BN + h * Cfg::kMmaN);
+                                        n_blk * BN + h * Cfg::kMmaN);
                         }
                     }
-                    armed |= 1u << stage;
-                    armed_phase = (armed_phase & ~(1u << stage)) | (phase << stage);
-                    if (++stage == kStages) {
-                        stage = 0;
-                        phase ^= 1u;
-                    }
                 }
-            }
-            if (!ok) {
-                // Copies already issued still land in shared memory: wait (bounded) for the
-                // armed slots so the CTA does not exit underneath them.
-                const long long t0 = clock64();
-                for (int s = 0; s < kStages; ++s) {
-                    if ((armed >> s) & 1u) {
-                        // The full barrier of the phase this slot was last armed in completes
-                        // when its bytes have landed.
-                        while (!mbar_try_wait(&full_bar[s], (armed_phase >> s) & 1u)) {
-                            if (clock64() - t0 > kWaitLimitCycles) {
-                                atomicCAS(error_word, 0, kErrDrainWait);
-                                break;
+                __syncwarp();
+                issued += wait_failed(spent) ? 0u : 1u;
+                if (++stage == kStages) {
+                    stage = 0;
+                    phase ^= 1u;
+                }
+                if constexpr (CONV) {
+                    if (++tap_c == conv.kb_per_tap) {
+                        tap_c = 0;
+                        if (++tap_b == conv.kw) {
+                            tap_b = 0;
+                            if (++tap_a == conv.kh) {
+                                tap_a = 0;
                             }
                         }
                     }
                 }
+                if (++kb == num_kb) {
+                    kb = 0;
+                }
+            }
+        }
+        if (wait_failed(spent) && lane == 0) {
+            atomicCAS(error_word, 0, kErrProducerWait);
+            // Copies already issued still land in shared memory: the CTA must not exit underneath them.
+            if (!drain_ring(full_bar, kStages, issued)) {
+                atomicCAS(error_word, 0, kErrDrainWait);
             }
         }
         __syncwarp();
     } else if (role == 1) {
         // ---------------- MMA issuer ----------------
-        if (kWarpIssue || lane == 0) {
-            const auto wait = [&](uint64_t* bar, uint32_t parity) {
-                return kWarpIssue ? mbar_wait_warp(bar, parity, abort_flag) : mbar_wait(bar, parity, abort_flag);
-            };
-            const uint32_t tmem = kWarpIssue ? __shfl_sync(0xFFFFFFFFu, tmem_base, 0) : tmem_base;
-            int stage = 0;
-            uint32_t phase = 0;
-            int local_tile = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x, ++local_tile) {
-                const int acc = Cfg::kNSplit > 1 ? 0 : (local_tile & 1);
-                const uint32_t acc_phase = Cfg::kNSplit > 1 ? (local_tile & 1u) : ((local_tile >> 1) & 1u);
-                if (!wait(&acc_empty_bar[acc], acc_phase ^ 1u)) {
-                    if (lane == 0) {
-                        atomicCAS(error_word, 0, kErrAccumWait);
-                    }
-                    break;
-                }
+        const uint32_t tmem = warp_uniform(tmem_base);
+        // K-major tiles step 32 bytes along their 128-byte rows per MMA (+2 in the descriptor's 16-byte
+        // units); MN-major tiles step 32 k-rows of 128 bytes (+256).  The ring's descriptors advance by addition.
+        const uint32_t ring = smem_u32(stage_base);
+        const uint64_t a_first = (pose & 1) ? umma_desc_sw128_mnmajor(ring, 128 * kBlockKBytes) : umma_desc_sw128_kmajor(ring);
+        const uint64_t b_first = (pose & 2) ? umma_desc_sw128_mnmajor(ring + Cfg::kATileBytes, 128 * kBlockKBytes)
+                                            : umma_desc_sw128_kmajor(ring + Cfg::kATileBytes);
+        const uint64_t a_step = (pose & 1) ? 256u : 2u;
+        const uint64_t b_step = (pose & 2) ? 256u : 2u;
+        uint64_t a_desc = a_first, b_desc = b_first;
+        int local_tile = 0;
+        for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++local_tile) {
+            const int acc = Cfg::kNSplit > 1 ? 0 : (local_tile & 1);
+            const uint32_t acc_phase = Cfg::kNSplit > 1 ? (local_tile & 1u) : ((local_tile >> 1) & 1u);
+            mbar_wait_converged(&acc_empty_bar[acc], acc_phase ^ 1u, abort_flag, spent);
+            tc_fence_after_sync();
+            const uint32_t d_tmem = tmem + static_cast<uint32_t>(acc * BN);
+            uint32_t accumulate = 0;
+            for (int kb = 0; kb < num_kb; ++kb) {
+                mbar_wait_converged(&full_bar[stage], phase, abort_flag, spent);
                 tc_fence_after_sync();
-                const uint32_t d_tmem = tmem + static_cast<uint32_t>(acc * BN);
-                for (int kb = 0; kb < num_kb; ++kb) {
-                    if (!wait(&full_bar[stage], phase)) {
-                        if (lane == 0) {
-                            atomicCAS(error_word, 0, kErrMmaWait);
-                        }
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after_sync();
-                    const uint32_t a_addr = smem_u32(stage_base + stage * Cfg::kStageBytes);
-                    const uint32_t b_addr = a_addr + Cfg::kATileBytes;
-                    // K-major tiles step 32 bytes along their 128-byte rows per MMA (+2 in the
-                    // descriptor's 16-byte units); MN-major tiles step 32 k-rows of 128 bytes (+256).
-                    const uint64_t a_desc = (pose & 1) ? umma_desc_sw128_mnmajor(a_addr, 128 * kBlockKBytes)
-                                                       : umma_desc_sw128_kmajor(a_addr);
-                    const uint64_t b_desc = (pose & 2) ? umma_desc_sw128_mnmajor(b_addr, 128 * kBlockKBytes)
-                                                       : umma_desc_sw128_kmajor(b_addr);
-                    const uint64_t a_step = (pose & 1) ? 256u : 2u;
-                    const uint64_t b_step = (pose & 2) ? 256u : 2u;
-                    if (!kWarpIssue || elect_one()) {
+                if (elect_one()) {
 #pragma unroll
-                        for (int ks = 0; ks < kBlockKBytes / kUmmaK; ++ks) {
+                    for (int ks = 0; ks < kBlockKBytes / kUmmaK; ++ks) {
 #pragma unroll
-                            for (int h = 0; h < Cfg::kNSplit; ++h) {
-                                // Second half of a wide tile: kMmaN rows further down the W tile (16-byte
-                                // descriptor units), kMmaN columns further along the accumulator.
-                                umma_i8(d_tmem + static_cast<uint32_t>(h * Cfg::kMmaN),
-                                        a_desc + static_cast<uint64_t>(ks) * a_step,
-                                        b_desc + static_cast<uint64_t>(ks) * b_step +
-                                            static_cast<uint64_t>(h * (Cfg::kMmaN * kBlockKBytes / 16)),
-                                        idesc, (kb > 0 || ks > 0) ? 1u : 0u);
-                            }
-                        }
-                        umma_commit(&empty_bar[stage]);  // slot is free once these MMAs have read it
-                        if (kWarpIssue && kb == num_kb - 1) {
-                            umma_commit(&acc_full_bar[acc]);  // accumulator complete
+                        for (int h = 0; h < Cfg::kNSplit; ++h) {
+                            // Second half of a wide tile: kMmaN rows further down the W tile (16-byte
+                            // descriptor units), kMmaN columns further along the accumulator.
+                            umma_i8(d_tmem + static_cast<uint32_t>(h * Cfg::kMmaN), a_desc + static_cast<uint64_t>(ks) * a_step,
+                                    b_desc + static_cast<uint64_t>(ks) * b_step +
+                                        static_cast<uint64_t>(h * (Cfg::kMmaN * kBlockKBytes / 16)),
+                                    idesc, ks > 0 ? 1u : accumulate);
                         }
                     }
-                    if (kWarpIssue) {
-                        __syncwarp();
-                    }
-                    if (++stage == kStages) {
-                        stage = 0;
-                        phase ^= 1u;
-                    }
+                    umma_commit(&empty_bar[stage]);  // slot is free once these MMAs have read it
                 }
-                if (!kWarpIssue && ok) {
-                    umma_commit(&acc_full_bar[acc]);
+                __syncwarp();
+                accumulate = 1;
+                a_desc += Cfg::kStageBytes / 16;
+                b_desc += Cfg::kStageBytes / 16;
+                if (++stage == kStages) {
+                    stage = 0;
+                    phase ^= 1u;
+                    a_desc = a_first;
+                    b_desc = b_first;
                 }
             }
+            if (elect_one()) {
+                umma_commit(&acc_full_bar[acc]);  // accumulator complete
+            }
+            __syncwarp();
+        }
+        if (wait_failed(spent)) {
+            if (lane == 0) {
+                atomicCAS(error_word, 0, kErrMmaWait);
+            }
+            umma_settle_after_failure();
         }
         __syncwarp();
     } else {
