@@ -100,6 +100,7 @@ gemm_i8_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5;
+    const int role = warp_uniform(warp);   // the same, warp-uniform to the compiler too
     const int lane = threadIdx.x & 31;
     const uint32_t rank = cluster_cta_rank();  // 0 = pair leader
     const int pair = static_cast<int>(blockIdx.x >> 1);
@@ -135,44 +136,49 @@ gemm_i8_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (warp == 0) {
+    // In both issuing roles the whole warp walks the loop, one elected lane issues, and no branch depends on
+    // what a wait returned (see mbar_wait_converged).
+    uint32_t spent = 0;   // probes of this role's waits
+    int stage = 0;
+    uint32_t phase = 0;
+    if (role == 0) {
         // ---------------- TMA producer (each CTA loads its own halves) ----------------
-        if (lane == 0) {
-            int stage = 0;
-            uint32_t phase = 0;
-            bool ok = true;
-            for (int tile = pair; ok && tile < num_tiles; tile += num_pairs) {
-                const TileCoord tc = walk(tile);
-                const int m0 = tc.m_blk * kPairM + static_cast<int>(rank) * kBlockM;
-                const int n0 = tc.n_blk * BN + static_cast<int>(rank) * (BN / 2);
-                const int rot = k_rotation(tile, k_rot, num_kb);
-                for (int kb = 0; kb < num_kb; kb += SUB) {
-                    if (!mbar_wait_cluster(&empty_bar[stage], phase ^ 1u, abort_flag)) {
-                        atomicCAS(error_word, 0, kErrProducerWait);
-                        ok = false;
-                        break;
-                    }
-                    const int nsub = (num_kb - kb) < SUB ? (num_kb - kb) : SUB;
-                    if (rank == 0) {
-                        mbar_expect_tx(&full_bar[stage], 2 * nsub * Cfg::kStageBytes);
-                    }
-                    const uint32_t leader_full = map_to_cta(smem_u32(&full_bar[stage]), 0);
+        for (int tile = pair; tile < num_tiles; tile += num_pairs) {
+            const TileCoord tc = walk(tile);
+            const int m0 = warp_uniform(tc.m_blk * kPairM + static_cast<int>(rank) * kBlockM);
+            const int n0 = warp_uniform(tc.n_blk * BN + static_cast<int>(rank) * (BN / 2));
+            const int rot = warp_uniform(k_rotation(tile, k_rot, num_kb));
+            int patch_w = 0, patch_h = 0, patch_img = 0, tap_a = 0, tap_b = 0, tap_c = 0;   // CONV
+            (void)patch_w; (void)patch_h; (void)patch_img; (void)tap_a; (void)tap_b; (void)tap_c;
+            if constexpr (CONV) {
+                // This CTA's patch of the pair (2 * m_blk + rank), shifted by the k-block's tap.
+                const ConvPatch pt = conv_patch(conv, 2 * tc.m_blk + static_cast<int>(rank));
+                patch_w = warp_uniform((pt.tw << conv.bw_log2) * conv.sw - conv.pw);
+                patch_h = warp_uniform(pt.th * conv.bh * conv.sh - conv.ph);
+                patch_img = warp_uniform(pt.img);
+                const int tap = rot / conv.kb_per_tap;
+                tap_c = warp_uniform(rot - tap * conv.kb_per_tap);
+                tap_a = warp_uniform(tap / conv.kw);
+                tap_b = warp_uniform(tap - tap_a * conv.kw);
+            }
+            int kx = rot;
+            for (int kb = 0; kb < num_kb; kb += SUB) {
+                mbar_wait_converged_cluster(&empty_bar[stage], phase ^ 1u, abort_flag, spent);
+                const int nsub = (num_kb - kb) < SUB ? (num_kb - kb) : SUB;
+                const uint32_t leader_full = map_to_cta(smem_u32(&full_bar[stage]), 0);
+                const bool issue = elect_one() && !wait_failed(spent);
+                if (issue && rank == 0) {
+                    mbar_expect_tx(&full_bar[stage], 2 * nsub * Cfg::kStageBytes);
+                }
 #pragma unroll
-                    for (int j = 0; j < SUB; ++j) {
-                        if (j < nsub) {
-                            uint8_t* a_dst = stage_base + stage * kSlotBytes + j * Cfg::kStageBytes;
-                            uint8_t* b_dst = a_dst + Cfg::kATileBytes;
-                            const int kx = kb + j + rot < num_kb ? kb + j + rot : kb + j + rot - num_kb;
+                for (int j = 0; j < SUB; ++j) {
+                    if (j < nsub) {
+                        uint8_t* a_dst = stage_base + stage * kSlotBytes + j * Cfg::kStageBytes;
+                        uint8_t* b_dst = a_dst + Cfg::kATileBytes;
+                        if (issue) {
                             if constexpr (CONV) {
-                                // This CTA's patch of the pair (2 * m_blk + rank), shifted by the k-block's tap.
-                                const ConvPatch pt = conv_patch(conv, 2 * tc.m_blk + static_cast<int>(rank));
-                                const int tap = kx / conv.kb_per_tap;
-                                const int c0 = (kx - tap * conv.kb_per_tap) * kBlockKBytes;
-                                const int ta = tap / conv.kw;
-                                const int tb = tap - ta * conv.kw;
-                                tma_load_4d_pair(a_dst, &map_a, leader_full, conv.c_base + c0,
-                                                 (pt.tw << conv.bw_log2) * conv.sw - conv.pw + tb * conv.dw,
-                                                 pt.th * conv.bh * conv.sh - conv.ph + ta * conv.dh, pt.img);
+                                tma_load_4d_pair(a_dst, &map_a, leader_full, conv.c_base + tap_c * kBlockKBytes,
+                                                 patch_w + tap_b * conv.dw, patch_h + tap_a * conv.dh, patch_img);
                             } else if constexpr ((POSE & 1) != 0) {
                                 // A stored [K][M]: 128 k-rows of this CTA's 128 m-bytes.
                                 tma_load_2d_pair(a_dst, &map_a, leader_full, m0, kx * kBlockKBytes);
@@ -186,57 +192,66 @@ gemm_i8_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                                 tma_load_2d_pair(b_dst, &map_w, leader_full, kx * kBlockKBytes, n0);
                             }
                         }
+                        __syncwarp();
+                        if constexpr (CONV) {
+                            if (++tap_c == conv.kb_per_tap) {
+                                tap_c = 0;
+                                if (++tap_b == conv.kw) {
+                                    tap_b = 0;
+                                    if (++tap_a == conv.kh) {
+                                        tap_a = 0;
+                                    }
+                                }
+                            }
+                        }
+                        if (++kx == num_kb) {
+                            kx = 0;
+                        }
                     }
-                    if (++stage == kStages) {
-                        stage = 0;
-                        phase ^= 1u;
-                    }
+                }
+                if (++stage == kStages) {
+                    stage = 0;
+                    phase ^= 1u;
                 }
             }
         }
+        if (wait_failed(spent) && lane == 0) {
+            atomicCAS(error_word, 0, kErrProducerWait);
+        }
         __syncwarp();
-    } else if (warp == 1) {
+    } else if (role == 1) {
         // ---------------- MMA issuer (pair leader only) ----------------
-        if (lane == 0 && rank == 0) {
-            int stage = 0;
-            uint32_t phase = 0;
-            int local_tile = 0;
-            bool ok = true;
-            for (int tile = pair; ok && tile < num_tiles; tile += num_pairs, ++local_tile) {
-                const int acc = local_tile & 1;
-                const uint32_t acc_phase = (local_tile >> 1) & 1u;
-                if (!mbar_wait_cluster(&acc_empty_bar[acc], acc_phase ^ 1u, abort_flag)) {
-                    atomicCAS(error_word, 0, kErrAccumWait);
-                    break;
-                }
+        const uint32_t tmem = warp_uniform(tmem_base);
+        // MN-major tiles (POSE bits): 32 k-rows of 128 bytes per K step instead of 32 bytes along the row, as in
+        // the single-CTA kernel.  The ring's descriptors advance by addition.
+        const uint32_t ring = smem_u32(stage_base);
+        const uint64_t a_first = (POSE & 1) ? umma_desc_sw128_mnmajor(ring, 128 * kBlockKBytes) : umma_desc_sw128_kmajor(ring);
+        const uint64_t b_first = (POSE & 2) ? umma_desc_sw128_mnmajor(ring + Cfg::kATileBytes, 128 * kBlockKBytes)
+                                            : umma_desc_sw128_kmajor(ring + Cfg::kATileBytes);
+        constexpr uint64_t a_step = (POSE & 1) ? 256u : 2u;
+        constexpr uint64_t b_step = (POSE & 2) ? 256u : 2u;
+        uint64_t a_desc = a_first, b_desc = b_first;
+        int local_tile = 0;
+        for (int tile = pair; rank == 0 && tile < num_tiles; tile += num_pairs, ++local_tile) {
+            const int acc = local_tile & 1;
+            const uint32_t acc_phase = (local_tile >> 1) & 1u;
+            mbar_wait_converged_cluster(&acc_empty_bar[acc], acc_phase ^ 1u, abort_flag, spent);
+            tc_fence_after_sync();
+            const uint32_t d_tmem = tmem + static_cast<uint32_t>(acc * 256);
+            uint32_t accumulate = 0;
+            for (int kb = 0; kb < num_kb; kb += SUB) {
+                mbar_wait_converged_cluster(&full_bar[stage], phase, abort_flag, spent);
                 tc_fence_after_sync();
-                const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * 256);
-                for (int kb = 0; kb < num_kb; kb += SUB) {
-                    if (!mbar_wait_cluster(&full_bar[stage], phase, abort_flag)) {
-                        atomicCAS(error_word, 0, kErrMmaWait);
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after_sync();
-                    const int nsub = (num_kb - kb) < SUB ? (num_kb - kb) : SUB;
+                const int nsub = (num_kb - kb) < SUB ? (num_kb - kb) : SUB;
+                if (elect_one()) {
 #pragma unroll
                     for (int j = 0; j < SUB; ++j) {
                         if (j < nsub) {
-                            const uint32_t a_addr = smem_u32(stage_base + stage * kSlotBytes + j * Cfg::kStageBytes);
-                            const uint32_t b_addr = a_addr + Cfg::kATileBytes;
-                            // MN-major tiles (POSE bits): 32 k-rows of 128 bytes per K step instead of 32 bytes
-                            // along the row, as in the single-CTA kernel.
-                            const uint64_t a_desc = (POSE & 1) ? umma_desc_sw128_mnmajor(a_addr, 128 * kBlockKBytes)
-                                                               : umma_desc_sw128_kmajor(a_addr);
-                            const uint64_t b_desc = (POSE & 2) ? umma_desc_sw128_mnmajor(b_addr, 128 * kBlockKBytes)
-                                                               : umma_desc_sw128_kmajor(b_addr);
-                            constexpr uint64_t a_step = (POSE & 1) ? 256u : 2u;
-                            constexpr uint64_t b_step = (POSE & 2) ? 256u : 2u;
 #pragma unroll
                             for (int ks = 0; ks < kBlockKBytes / kUmmaK; ++ks) {
-                                umma_i8_pair(d_tmem, a_desc + static_cast<uint64_t>(ks) * a_step,
-                                             b_desc + static_cast<uint64_t>(ks) * b_step, idesc,
-                                             (kb > 0 || j > 0 || ks > 0) ? 1u : 0u);
+                                umma_i8_pair(d_tmem, a_desc + static_cast<uint64_t>(j * (Cfg::kStageBytes / 16)) + static_cast<uint64_t>(ks) * a_step,
+                                             b_desc + static_cast<uint64_t>(j * (Cfg::kStageBytes / 16)) + static_cast<uint64_t>(ks) * b_step,
+                                             idesc, (j > 0 || ks > 0) ? 1u : accumulate);
                             }
                         }
                     }
@@ -248,21 +263,34 @@ gemm_i8_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                         umma_commit_pair(map_to_cta(e, 0));
                         umma_commit_pair(map_to_cta(e, 1));
                     }
-                    if (++stage == kStages) {
-                        stage = 0;
-                        phase ^= 1u;
-                    }
                 }
-                if (ok) {
-                    if constexpr (MC) {
-                        umma_commit_pair_mask(&acc_full_bar[acc], 3);
-                    } else {
-                        const uint32_t f = smem_u32(&acc_full_bar[acc]);
-                        umma_commit_pair(map_to_cta(f, 0));
-                        umma_commit_pair(map_to_cta(f, 1));
-                    }
+                __syncwarp();
+                accumulate = 1;
+                a_desc += kSlotBytes / 16;
+                b_desc += kSlotBytes / 16;
+                if (++stage == kStages) {
+                    stage = 0;
+                    phase ^= 1u;
+                    a_desc = a_first;
+                    b_desc = b_first;
                 }
             }
+            if (elect_one()) {
+                if constexpr (MC) {
+                    umma_commit_pair_mask(&acc_full_bar[acc], 3);
+                } else {
+                    const uint32_t f = smem_u32(&acc_full_bar[acc]);
+                    umma_commit_pair(map_to_cta(f, 0));
+                    umma_commit_pair(map_to_cta(f, 1));
+                }
+            }
+            __syncwarp();
+        }
+        if (wait_failed(spent)) {
+            if (lane == 0) {
+                atomicCAS(error_word, 0, kErrMmaWait);
+            }
+            umma_settle_after_failure();
         }
         __syncwarp();
     } else {
