@@ -253,129 +253,130 @@ gemm_f16_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5;
+    const int role = warp_uniform(warp);   // the same, warp-uniform to the compiler too
     const int lane = threadIdx.x & 31;
     const int num_m = (m_total + kBlockM - 1) / kBlockM;
     const int num_n = (n_total + BN - 1) / BN;
     const int num_tiles = num_m * num_n;
     const int num_kb = (k_total + kBlockK - 1) / kBlockK;
 
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < kStages; ++s) {
-            mbar_init(&full_bar[s], 1);
-            mbar_init(&empty_bar[s], 1);
-        }
-        for (int a = 0; a < 2; ++a) {
-            mbar_init(&acc_full_bar[a], 1);
-            mbar_init(&acc_empty_bar[a], kEpilogueThreads / 32);
-        }
-        *abort_flag = 0;
-        mbar_init_fence();
-    }
-    if (warp == 0 && lane == 0) {
-        tma_prefetch_desc(&map_a);
-        tma_prefetch_desc(&map_w);
-    }
-    if (warp == 1) {
-        tmem_alloc(tmem_slot, Cfg::kTmemCols);
-        tmem_relinquish();
-    }
-    tc_fence_before_sync();
-    __syncthreads();
-    tc_fence_after_sync();
-    const uint32_t tmem_base = *tmem_slot;
-
-    if (warp == 0) {
-        // ---------------- TMA producer ----------------
+    // The producer warp sets the barriers up and starts to load at once; the others meet at a barrier of
+    // their own.  In both issuing roles the whole warp walks the loop, one elected lane issues, and no
+    // branch depends on what a wait returned (see mbar_wait_converged).
+    uint32_t spent = 0;   // probes of this role's waits
+    int stage = 0;
+    uint32_t phase = 0;
+    if (role == 0) {
         if (lane == 0) {
-            int stage = 0;
-            uint32_t phase = 0;
-            uint32_t armed = 0;        // bit s: slot s has been armed at least once
-            uint32_t armed_phase = 0;  // bit s: parity of the phase slot s was last armed in
-            bool ok = true;
-            for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
-                const TileCoord tc = tile_coord(tile, num_m, num_n, group_m);
-                for (int kb = 0; kb < num_kb; ++kb) {
-                    if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag)) {
-                        atomicCAS(error_word, 0, kErrProducerWait);
-                        ok = false;
-                        break;
-                    }
+            for (int s = 0; s < kStages; ++s) {
+                mbar_init(&full_bar[s], 1);
+                mbar_init(&empty_bar[s], 1);
+            }
+            for (int a = 0; a < 2; ++a) {
+                mbar_init(&acc_full_bar[a], 1);
+                mbar_init(&acc_empty_bar[a], kEpilogueThreads / 32);
+            }
+            *abort_flag = 0;
+            mbar_init_fence();
+        }
+        __syncwarp();
+        named_barrier_arrive(1, kNumThreads);
+    } else {
+        if (role == 1) {
+            if (lane == 0) {
+                tma_prefetch_desc(&map_a);
+                tma_prefetch_desc(&map_w);
+            }
+            __syncwarp();
+            tmem_alloc(tmem_slot, Cfg::kTmemCols);
+            tmem_relinquish();
+        }
+        tc_fence_before_sync();
+        named_barrier_sync(1, kNumThreads);
+        tc_fence_after_sync();
+    }
+    const uint32_t tmem_base = *tmem_slot;   // not the producer's
+
+    if (role == 0) {
+        // ---------------- TMA producer ----------------
+        uint32_t issued = 0;
+        for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+            const TileCoord tc = tile_coord(tile, num_m, num_n, group_m);
+            const int m0 = warp_uniform(tc.m_blk * kBlockM), n0 = warp_uniform(tc.n_blk * BN);
+            // With split activations ([hi | lo] along K) the weights repeat every w_wrap_k, a multiple of the k-block.
+            int wk = 0;
+            for (int kb = 0; kb < num_kb; ++kb) {
+                mbar_wait_converged(&empty_bar[stage], phase ^ 1u, abort_flag, spent);
+                if (elect_one() && !wait_failed(spent)) {
                     uint8_t* a_dst = stage_base + stage * Cfg::kStageBytes;
-                    uint8_t* b_dst = a_dst + Cfg::kATileBytes;
                     mbar_expect_tx(&full_bar[stage], Cfg::kStageBytes);
                     // x coordinates are in elements: kb * 64 halves = a multiple of 128 bytes.
-                    // With split activations ([hi | lo] along K) the weights repeat every w_wrap_k.
-                    const int wk = w_wrap_k > 0 ? (kb * kBlockK) % w_wrap_k : kb * kBlockK;
-                    tma_load_2d(a_dst, &map_a, &full_bar[stage], kb * kBlockK, tc.m_blk * kBlockM);
-                    tma_load_2d(b_dst, &map_w, &full_bar[stage], wk, tc.n_blk * BN);
-                    armed |= 1u << stage;
-                    armed_phase = (armed_phase & ~(1u << stage)) | (phase << stage);
-                    if (++stage == kStages) {
-                        stage = 0;
-                        phase ^= 1u;
-                    }
+                    tma_load_2d(a_dst, &map_a, &full_bar[stage], kb * kBlockK, m0);
+                    tma_load_2d(a_dst + Cfg::kATileBytes, &map_w, &full_bar[stage], wk, n0);
+                }
+                __syncwarp();
+                issued += wait_failed(spent) ? 0u : 1u;
+                wk += kBlockK;
+                wk = wk == w_wrap_k ? 0 : wk;
+                if (++stage == kStages) {
+                    stage = 0;
+                    phase ^= 1u;
                 }
             }
-            if (!ok) {
-                // Copies already issued still land in shared memory: wait (bounded) for the armed
-                // slots so the CTA does not exit underneath them.
-                const long long t0 = clock64();
-                for (int s = 0; s < kStages; ++s) {
-                    if ((armed >> s) & 1u) {
-                        while (!mbar_try_wait(&full_bar[s], (armed_phase >> s) & 1u)) {
-                            if (clock64() - t0 > kWaitLimitCycles) {
-                                atomicCAS(error_word, 0, kErrDrainWait);
-                                break;
-                            }
-                        }
-                    }
-                }
+        }
+        if (wait_failed(spent) && lane == 0) {
+            atomicCAS(error_word, 0, kErrProducerWait);
+            // Copies already issued still land in shared memory: the CTA must not exit underneath them.
+            if (!drain_ring(full_bar, kStages, issued)) {
+                atomicCAS(error_word, 0, kErrDrainWait);
             }
         }
         __syncwarp();
-    } else if (warp == 1) {
+    } else if (role == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            int stage = 0;
-            uint32_t phase = 0;
-            int local_tile = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x, ++local_tile) {
-                const int acc = local_tile & 1;
-                const uint32_t acc_phase = (local_tile >> 1) & 1u;
-                if (!mbar_wait(&acc_empty_bar[acc], acc_phase ^ 1u, abort_flag)) {
-                    atomicCAS(error_word, 0, kErrAccumWait);
-                    break;
-                }
+        const uint32_t tmem = warp_uniform(tmem_base);
+        const uint64_t first_desc = umma_desc_sw128_kmajor(smem_u32(stage_base));
+        uint64_t a_desc = first_desc;
+        int local_tile = 0;
+        for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++local_tile) {
+            const int acc = local_tile & 1;
+            const uint32_t acc_phase = (local_tile >> 1) & 1u;
+            mbar_wait_converged(&acc_empty_bar[acc], acc_phase ^ 1u, abort_flag, spent);
+            tc_fence_after_sync();
+            const uint32_t d_tmem = tmem + static_cast<uint32_t>(acc * 256);
+            uint32_t accumulate = 0;
+            for (int kb = 0; kb < num_kb; ++kb) {
+                mbar_wait_converged(&full_bar[stage], phase, abort_flag, spent);
                 tc_fence_after_sync();
-                const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * 256);
-                for (int kb = 0; kb < num_kb; ++kb) {
-                    if (!mbar_wait(&full_bar[stage], phase, abort_flag)) {
-                        atomicCAS(error_word, 0, kErrMmaWait);
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after_sync();
-                    const uint32_t a_addr = smem_u32(stage_base + stage * Cfg::kStageBytes);
-                    const uint32_t b_addr = a_addr + Cfg::kATileBytes;
-                    const uint64_t a_desc = umma_desc_sw128_kmajor(a_addr);
-                    const uint64_t b_desc = umma_desc_sw128_kmajor(b_addr);
+                const uint64_t b_desc = a_desc + Cfg::kATileBytes / 16;
+                if (elect_one()) {
 #pragma unroll
                     for (int ks = 0; ks < kBlockKBytes / kUmmaKBytes; ++ks) {
                         // +32 bytes of K per step = +2 in the descriptor's 16-byte address units.
                         umma_f16(d_tmem, a_desc + static_cast<uint64_t>(ks * 2), b_desc + static_cast<uint64_t>(ks * 2),
-                                 idesc, (kb > 0 || ks > 0) ? 1u : 0u);
+                                 idesc, ks > 0 ? 1u : accumulate);
                     }
                     umma_commit(&empty_bar[stage]);
-                    if (++stage == kStages) {
-                        stage = 0;
-                        phase ^= 1u;
-                    }
                 }
-                if (ok) {
-                    umma_commit(&acc_full_bar[acc]);
+                __syncwarp();
+                accumulate = 1;
+                a_desc += Cfg::kStageBytes / 16;
+                if (++stage == kStages) {
+                    stage = 0;
+                    phase ^= 1u;
+                    a_desc = first_desc;
                 }
             }
+            if (elect_one()) {
+                umma_commit(&acc_full_bar[acc]);
+            }
+            __syncwarp();
+        }
+        if (wait_failed(spent)) {
+            if (lane == 0) {
+                atomicCAS(error_word, 0, kErrMmaWait);
+            }
+            umma_settle_after_failure();
         }
         __syncwarp();
     } else {
@@ -467,6 +468,7 @@ gemm_f16_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5;
+    const int role = warp_uniform(warp);   // the same, warp-uniform to the compiler too
     const int lane = threadIdx.x & 31;
     const uint32_t rank = cluster_cta_rank();  // 0 = pair leader
     const int pair = static_cast<int>(blockIdx.x >> 1);
@@ -501,82 +503,76 @@ gemm_f16_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (warp == 0) {
+    // Both issuing roles as in the single-CTA kernel: whole warp, one elected lane, waits nothing branches on.
+    uint32_t spent = 0;   // probes of this role's waits
+    int stage = 0;
+    uint32_t phase = 0;
+    if (role == 0) {
         // ---------------- TMA producer (each CTA loads its own halves) ----------------
-        if (lane == 0) {
-            int stage = 0;
-            uint32_t phase = 0;
-            bool ok = true;
-            for (int tile = pair; ok && tile < num_tiles; tile += num_pairs) {
-                const TileCoord tc = tile_coord(tile, num_m, num_n, group_m);
-                const int m0 = tc.m_blk * kPairM + static_cast<int>(rank) * kBlockM;
-                const int n0 = tc.n_blk * BN + static_cast<int>(rank) * (BN / 2);
-                for (int kb = 0; kb < num_kb; kb += SUB) {
-                    if (!mbar_wait_cluster(&empty_bar[stage], phase ^ 1u, abort_flag)) {
-                        atomicCAS(error_word, 0, kErrProducerWait);
-                        ok = false;
-                        break;
-                    }
-                    const int nsub = (num_kb - kb) < SUB ? (num_kb - kb) : SUB;
-                    if (rank == 0) {
-                        mbar_expect_tx(&full_bar[stage], 2 * nsub * Cfg::kStageBytes);
-                    }
-                    const uint32_t leader_full = map_to_cta(smem_u32(&full_bar[stage]), 0);
+        for (int tile = pair; tile < num_tiles; tile += num_pairs) {
+            const TileCoord tc = tile_coord(tile, num_m, num_n, group_m);
+            const int m0 = warp_uniform(tc.m_blk * kPairM + static_cast<int>(rank) * kBlockM);
+            const int n0 = warp_uniform(tc.n_blk * BN + static_cast<int>(rank) * (BN / 2));
+            int wk = 0;   // repeats every w_wrap_k, a multiple of the k-block
+            for (int kb = 0; kb < num_kb; kb += SUB) {
+                mbar_wait_converged_cluster(&empty_bar[stage], phase ^ 1u, abort_flag, spent);
+                const int nsub = (num_kb - kb) < SUB ? (num_kb - kb) : SUB;
+                const uint32_t leader_full = map_to_cta(smem_u32(&full_bar[stage]), 0);
+                const bool issue = elect_one() && !wait_failed(spent);
+                if (issue && rank == 0) {
+                    mbar_expect_tx(&full_bar[stage], 2 * nsub * Cfg::kStageBytes);
+                }
 #pragma unroll
-                    for (int j = 0; j < SUB; ++j) {
-                        if (j < nsub) {
+                for (int j = 0; j < SUB; ++j) {
+                    if (j < nsub) {
+                        if (issue) {
                             uint8_t* a_dst = stage_base + stage * kSlotBytes + j * Cfg::kStageBytes;
-                            uint8_t* b_dst = a_dst + Cfg::kATileBytes;
-                            const int k0 = (kb + j) * kBlockK;
-                            const int wk = w_wrap_k > 0 ? k0 % w_wrap_k : k0;
-                            tma_load_2d_pair(a_dst, &map_a, leader_full, k0, m0);
-                            tma_load_2d_pair(b_dst, &map_w, leader_full, wk, n0);
+                            tma_load_2d_pair(a_dst, &map_a, leader_full, (kb + j) * kBlockK, m0);
+                            tma_load_2d_pair(a_dst + Cfg::kATileBytes, &map_w, leader_full, wk, n0);
                         }
+                        __syncwarp();
+                        wk += kBlockK;
+                        wk = wk == w_wrap_k ? 0 : wk;
                     }
-                    if (++stage == kStages) {
-                        stage = 0;
-                        phase ^= 1u;
-                    }
+                }
+                if (++stage == kStages) {
+                    stage = 0;
+                    phase ^= 1u;
                 }
             }
         }
+        if (wait_failed(spent) && lane == 0) {
+            atomicCAS(error_word, 0, kErrProducerWait);
+        }
         __syncwarp();
-    } else if (warp == 1) {
+    } else if (role == 1) {
         // ---------------- MMA issuer (pair leader only) ----------------
-        if (lane == 0 && rank == 0) {
-            int stage = 0;
-            uint32_t phase = 0;
-            int local_tile = 0;
-            bool ok = true;
-            for (int tile = pair; ok && tile < num_tiles; tile += num_pairs, ++local_tile) {
-                const int acc = local_tile & 1;
-                const uint32_t acc_phase = (local_tile >> 1) & 1u;
-                if (!mbar_wait_cluster(&acc_empty_bar[acc], acc_phase ^ 1u, abort_flag)) {
-                    atomicCAS(error_word, 0, kErrAccumWait);
-                    break;
-                }
+        const uint32_t tmem = warp_uniform(tmem_base);
+        const uint64_t first_desc = umma_desc_sw128_kmajor(smem_u32(stage_base));
+        uint64_t slot_desc = first_desc;
+        int local_tile = 0;
+        for (int tile = pair; rank == 0 && tile < num_tiles; tile += num_pairs, ++local_tile) {
+            const int acc = local_tile & 1;
+            const uint32_t acc_phase = (local_tile >> 1) & 1u;
+            mbar_wait_converged_cluster(&acc_empty_bar[acc], acc_phase ^ 1u, abort_flag, spent);
+            tc_fence_after_sync();
+            const uint32_t d_tmem = tmem + static_cast<uint32_t>(acc * 256);
+            uint32_t accumulate = 0;
+            for (int kb = 0; kb < num_kb; kb += SUB) {
+                mbar_wait_converged_cluster(&full_bar[stage], phase, abort_flag, spent);
                 tc_fence_after_sync();
-                const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * 256);
-                for (int kb = 0; kb < num_kb; kb += SUB) {
-                    if (!mbar_wait_cluster(&full_bar[stage], phase, abort_flag)) {
-                        atomicCAS(error_word, 0, kErrMmaWait);
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after_sync();
-                    const int nsub = (num_kb - kb) < SUB ? (num_kb - kb) : SUB;
+                const int nsub = (num_kb - kb) < SUB ? (num_kb - kb) : SUB;
+                if (elect_one()) {
 #pragma unroll
                     for (int j = 0; j < SUB; ++j) {
                         if (j < nsub) {
-                            const uint32_t a_addr = smem_u32(stage_base + stage * kSlotBytes + j * Cfg::kStageBytes);
-                            const uint32_t b_addr = a_addr + Cfg::kATileBytes;
-                            const uint64_t a_desc = umma_desc_sw128_kmajor(a_addr);
-                            const uint64_t b_desc = umma_desc_sw128_kmajor(b_addr);
+                            const uint64_t a_desc = slot_desc + static_cast<uint64_t>(j * (Cfg::kStageBytes / 16));
+                            const uint64_t b_desc = a_desc + Cfg::kATileBytes / 16;
 #pragma unroll
                             for (int ks = 0; ks < kBlockKBytes / kUmmaKBytes; ++ks) {
                                 umma_f16_pair(d_tmem, a_desc + static_cast<uint64_t>(ks * 2),
                                               b_desc + static_cast<uint64_t>(ks * 2), idesc,
-                                              (kb > 0 || j > 0 || ks > 0) ? 1u : 0u);
+                                              (j > 0 || ks > 0) ? 1u : accumulate);
                             }
                         }
                     }
@@ -588,21 +584,32 @@ gemm_f16_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
                         umma_commit_pair(map_to_cta(e, 0));
                         umma_commit_pair(map_to_cta(e, 1));
                     }
-                    if (++stage == kStages) {
-                        stage = 0;
-                        phase ^= 1u;
-                    }
                 }
-                if (ok) {
-                    if constexpr (MC) {
-                        umma_commit_pair_mask(&acc_full_bar[acc], 3);
-                    } else {
-                        const uint32_t f = smem_u32(&acc_full_bar[acc]);
-                        umma_commit_pair(map_to_cta(f, 0));
-                        umma_commit_pair(map_to_cta(f, 1));
-                    }
+                __syncwarp();
+                accumulate = 1;
+                slot_desc += kSlotBytes / 16;
+                if (++stage == kStages) {
+                    stage = 0;
+                    phase ^= 1u;
+                    slot_desc = first_desc;
                 }
             }
+            if (elect_one()) {
+                if constexpr (MC) {
+                    umma_commit_pair_mask(&acc_full_bar[acc], 3);
+                } else {
+                    const uint32_t f = smem_u32(&acc_full_bar[acc]);
+                    umma_commit_pair(map_to_cta(f, 0));
+                    umma_commit_pair(map_to_cta(f, 1));
+                }
+            }
+            __syncwarp();
+        }
+        if (wait_failed(spent)) {
+            if (lane == 0) {
+                atomicCAS(error_word, 0, kErrMmaWait);
+            }
+            umma_settle_after_failure();
         }
         __syncwarp();
     } else {

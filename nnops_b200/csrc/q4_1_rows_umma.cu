@@ -335,33 +335,26 @@ q4_1_rows_umma_kernel(const __grid_constant__ CUtensorMap map_a, const uint8_t* 
         // ---------------- MMA issuer ----------------
         // The whole warp walks the loop and one elected lane issues: addresses and descriptors are then
         // warp-uniform to the compiler, which is how the MMA takes its operands.  From a loop run by one
-        // lane an MMA took 93 clocks to issue, 35 this way (the call 23.6 us, then 17.8).
-        const uint32_t d_tmem = __shfl_sync(0xFFFFFFFFu, tmem_base, 0);
+        // lane an MMA took 93 clocks to issue, 35 this way (the call 23.6 us, then 17.8).  The waits keep
+        // it so (see mbar_wait_converged).
+        const uint32_t d_tmem = warp_uniform(tmem_base);
         const uint64_t ring_desc = umma_desc_sw128_kmajor(smem_u32(ring));
         const uint64_t slab_step = static_cast<uint64_t>(slab_bytes >> 4);
+        const int my_units = warp_uniform(units);
+        uint32_t spent = 0;
         int stage = 0;
         uint32_t phase = 0, acc_phase = 1;
-        bool ok = true;
-        for (int tile = cluster; ok && tile < num_tiles; tile += clusters) {
-            if (!mbar_wait_warp(acc_empty, acc_phase, abort_flag)) {
-                if (lane == 0) {
-                    atomicCAS(error_word, 0, kErrAccumWait);
-                }
-                break;
-            }
+        for (int tile = warp_uniform(cluster); tile < num_tiles; tile += warp_uniform(clusters)) {
+            mbar_wait_converged(acc_empty, acc_phase, abort_flag, spent);
+            tc_fence_after_sync();
             acc_phase ^= 1u;
-            for (int u = 0; u < units; ++u) {
-                if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag)) {
-                    if (lane == 0) {
-                        atomicCAS(error_word, 0, kErrMmaWait);
-                    }
-                    ok = false;
-                    break;
-                }
+            uint32_t accumulate = 0;
+            for (int u = 0; u < my_units; ++u) {
+                mbar_wait_converged(&full_bar[stage], phase, abort_flag, spent);
                 tc_fence_after_sync();
                 const uint64_t b_desc = ring_desc + static_cast<uint64_t>((stage * stage_bytes) >> 4);
                 const uint32_t a_tmem = d_tmem + static_cast<uint32_t>(kAccCols + stage * Cfg::kUnitCols);
-                const int slabs = slabs_of(u);
+                const int slabs = warp_uniform(slabs_of(u));
                 if (elect_one()) {
 #pragma unroll
                     for (int i = 0; i < kUnitK / kSlotK; ++i) {
@@ -370,22 +363,31 @@ q4_1_rows_umma_kernel(const __grid_constant__ CUtensorMap map_a, const uint8_t* 
                             for (int ks = 0; ks < kSlotK / 16; ++ks) {
                                 umma_f16_ts(d_tmem, a_tmem + i * (kSlotK / 2) + ks * 8,
                                             b_desc + i * slab_step + static_cast<uint64_t>(ks * 2), idesc,
-                                            (u > 0 || i > 0 || ks > 0) ? 1u : 0u);
+                                            (i > 0 || ks > 0) ? 1u : accumulate);
                             }
                         }
                     }
                     umma_commit(&empty_bar[stage]);
-                    if (u == units - 1) {
-                        umma_commit(acc_full);
-                    }
                 }
                 __syncwarp();
+                accumulate = 1;
                 if (++stage == kGroups) {
                     stage = 0;
                     phase ^= 1u;
                 }
             }
+            if (elect_one()) {
+                umma_commit(acc_full);
+            }
+            __syncwarp();
         }
+        if (wait_failed(spent)) {
+            if (lane == 0) {
+                atomicCAS(error_word, 0, kErrMmaWait);
+            }
+            umma_settle_after_failure();
+        }
+        __syncwarp();
     } else {
         // ---------------- decoding warps, then the epilogue of each tile ----------------
         const uint32_t lane_bits = static_cast<uint32_t>(quarter * 32) << 16;
