@@ -444,13 +444,15 @@ NNB200_API int nnb200_q4_1_packed_view(const void* blob, int64_t n, int64_t k, n
 #define NNB200_ZP_S8 0
 #define NNB200_ZP_U8 1
 #define NNB200_ZP_S32 2 /* the int32 zero points of a view's QuantParams (fp-activation route) */
+#define NNB200_ZP_HOST 3      /* zero_point: ONE int32 in HOST memory for all rows, read before the call returns */
+#define NNB200_PARAMS_HOST 4  /* that, and scale: one float in host memory (rows == 1) */
 
 typedef struct nnb200_quant_linear_args {
     const void* x;
     void* y;
     int64_t outer, rows, inner;
     const float* scale;     /* [rows] */
-    const void* zero_point; /* [rows], s8 or u8 */
+    const void* zero_point; /* [rows], s8, u8 or s32 */
     int32_t zp_unsigned;    /* NNB200_ZP_*: storage type of zero_point */
     int32_t float_f16;      /* floating side (x of quantize, y of dequantize) is f16, else f32 */
     int32_t int_unsigned;   /* integer side (y of quantize, x of dequantize) is u8, else s8 */

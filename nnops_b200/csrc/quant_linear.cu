@@ -78,16 +78,27 @@ struct QuantView {
     const float* scale;
     const void* zero_point;
     int32_t zp_unsigned;
+    int32_t zp_value;      // NNB200_ZP_HOST / NNB200_PARAMS_HOST
+    float scale_value;     // NNB200_PARAMS_HOST
 };
 
-// zp_unsigned carries NNB200_ZP_*: s8, u8 or int32 storage of the zero points.
+// zp_unsigned carries NNB200_ZP_*: s8, u8 or int32 storage of the zero points, or one value that came with the
+// call (a fill kernel for the array and its launch are then not needed).
 __device__ __forceinline__ float load_zp(const QuantView& v, int64_t r)
 {
+    if (v.zp_unsigned >= NNB200_ZP_HOST) {
+        return static_cast<float>(v.zp_value);
+    }
     if (v.zp_unsigned == NNB200_ZP_S32) {
         return static_cast<float>(static_cast<const int32_t*>(v.zero_point)[r]);
     }
     return v.zp_unsigned == NNB200_ZP_U8 ? static_cast<float>(static_cast<const uint8_t*>(v.zero_point)[r])
                                          : static_cast<float>(static_cast<const int8_t*>(v.zero_point)[r]);
+}
+
+__device__ __forceinline__ float load_scale(const QuantView& v, int64_t r)
+{
+    return v.zp_unsigned == NNB200_PARAMS_HOST ? v.scale_value : v.scale[r];
 }
 
 // fma, round-half-even with saturation to the 8-bit range in one conversion; the x86
@@ -177,7 +188,7 @@ quantize_vec_kernel(const QuantView v, const IDX groups, const FastDiv per_row, 
             if (gidx < groups) {
                 int64_t r, i0;
                 locate<IDX, VEC>(v, per_row, by_rows, gidx, r, i0);
-                const float inv = __frcp_rn(v.scale[r]);  // correctly rounded: identical to 1.0f / scale
+                const float inv = __frcp_rn(load_scale(v, r));  // correctly rounded: identical to 1.0f / scale
                 const float zp = load_zp(v, r);
                 if constexpr (X_F16) {
                     const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&raw[u].x));
@@ -214,7 +225,7 @@ __global__ void __launch_bounds__(kThreads) quantize_cols_kernel(const QuantView
     float inv[VEC], zp[VEC];
 #pragma unroll
     for (int j = 0; j < VEC; ++j) {
-        inv[j] = __frcp_rn(v.scale[g * VEC + j]);
+        inv[j] = __frcp_rn(load_scale(v, g * VEC + j));
         zp[j] = load_zp(v, g * VEC + j);
     }
     const int64_t stride = static_cast<int64_t>(gridDim.y) * blockDim.y;
@@ -273,7 +284,7 @@ __global__ void __launch_bounds__(kThreads) dequantize_cols_kernel(const QuantVi
     float s[VEC], zp[VEC];
 #pragma unroll
     for (int j = 0; j < VEC; ++j) {
-        s[j] = v.scale[g * VEC + j];
+        s[j] = load_scale(v, g * VEC + j);
         zp[j] = load_zp(v, g * VEC + j);
     }
     const int64_t stride = static_cast<int64_t>(gridDim.y) * blockDim.y;
@@ -342,7 +353,7 @@ dequantize_vec_kernel(const QuantView v, const IDX groups, const FastDiv per_row
             if (gidx < groups) {
                 int64_t r, i0;
                 locate<IDX, VEC>(v, per_row, by_rows, gidx, r, i0);
-                const float s = v.scale[r];
+                const float s = load_scale(v, r);
                 const float zp = load_zp(v, r);
                 const float neg_zs = __fmul_rn(-zp, s);
                 const bool tail = i0 >= body;  // body is a multiple of 16, i0 of VEC: the whole group agrees
@@ -379,7 +390,7 @@ __global__ void __launch_bounds__(kThreads) quantize_scalar_kernel(const QuantVi
         const int64_t row = e / v.inner;
         const int64_t r = row % v.rows;
         const float x = X_F16 ? __half2float(static_cast<const __half*>(v.x)[e]) : static_cast<const float*>(v.x)[e];
-        static_cast<uint8_t*>(v.y)[e] = static_cast<uint8_t>(quant_one<OUT_U8>(x, __frcp_rn(v.scale[r]), load_zp(v, r)));
+        static_cast<uint8_t*>(v.y)[e] = static_cast<uint8_t>(quant_one<OUT_U8>(x, __frcp_rn(load_scale(v, r)), load_zp(v, r)));
     }
 }
 
@@ -392,7 +403,7 @@ __global__ void __launch_bounds__(kThreads) dequantize_scalar_kernel(const Quant
         const int64_t row = e / v.inner;
         const int64_t r = row % v.rows;
         const int64_t i = e - row * v.inner;
-        const float s = v.scale[r];
+        const float s = load_scale(v, r);
         const float zp = load_zp(v, r);
         const float f = dequant_one<IN_U8>(static_cast<const uint8_t*>(v.x)[e], 0, s, zp, __fmul_rn(-zp, s), i >= body);
         if constexpr (Y_F16) {
@@ -503,11 +514,23 @@ int run_dequantize(const QuantView& v, int64_t numel, bool aligned, const Device
     return cuda_status(cudaGetLastError());
 }
 
+QuantView view_of(const nnb200_quant_linear_args& q)
+{
+    QuantView v{q.x, q.y, q.outer, q.rows, q.inner, q.scale, q.zero_point, q.zp_unsigned, 0, 0.0f};
+    if (q.zp_unsigned >= NNB200_ZP_HOST) {
+        v.zp_value = *static_cast<const int32_t*>(q.zero_point);
+    }
+    if (q.zp_unsigned == NNB200_PARAMS_HOST) {
+        v.scale_value = *q.scale;
+    }
+    return v;
+}
+
 }  // namespace
 
 int launch_quantize_linear(const nnb200_quant_linear_args& q, const DeviceInfo& dev, cudaStream_t stream)
 {
-    const QuantView v{q.x, q.y, q.outer, q.rows, q.inner, q.scale, q.zero_point, q.zp_unsigned};
+    const QuantView v = view_of(q);
     const int64_t numel = q.outer * q.rows * q.inner;
     const bool f16 = q.float_f16 != 0;
     const bool u8 = q.int_unsigned != 0;
@@ -523,7 +546,7 @@ int launch_quantize_linear(const nnb200_quant_linear_args& q, const DeviceInfo& 
 
 int launch_dequantize_linear(const nnb200_quant_linear_args& q, const DeviceInfo& dev, cudaStream_t stream)
 {
-    const QuantView v{q.x, q.y, q.outer, q.rows, q.inner, q.scale, q.zero_point, q.zp_unsigned};
+    const QuantView v = view_of(q);
     const int64_t numel = q.outer * q.rows * q.inner;
     const bool f16 = q.float_f16 != 0;
     const bool u8 = q.int_unsigned != 0;
