@@ -2,8 +2,8 @@
 
     python -m nnops_b200.build [--force] [--verbose]
 
-Output: nnops_b200/lib/libnnb200.so (git-ignored; shipped to GPU machines as a built file).
-nvcc cross-compiles without a GPU.  -fmad=false keeps every f32 multiply and add separately
+Output: nnops_b200/lib/libnnb200.so and torch_front.so, the tensor front end's compiled half (git-ignored; shipped to
+GPU machines as built files).  nvcc cross-compiles without a GPU.  -fmad=false keeps every f32 multiply and add separately
 rounded unless a kernel asks for an fma explicitly -- the int8 requantisation must match the
 CPU arithmetic bit for bit.
 """
@@ -20,7 +20,10 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB_DIR = PKG / "lib"
 LIB = LIB_DIR / "libnnb200.so"
+FRONT = LIB_DIR / "torch_front.so"
+FRONT_SRC = PKG / "host" / "torch_front.cpp"
 NVCC = os.environ.get("NNB200_NVCC", "/usr/local/cuda/bin/nvcc")
+CXX = os.environ.get("NNB200_CXX", "g++")
 
 SOURCES = ["capi.cu", "gemm_i8_umma.cu", "gemm_i8_umma_batched.cu", "i8_realign.cu", "gemm_i8_simt.cu", "gemm_i8_decode.cu", "gemm_i8_skinny.cu", "q4_1_gemv.cu", "q4_1_gemv_mma.cu", "q4_1_gemv_dsq.cu", "q4_1_gemm_umma.cu", "q4_1_rows_umma.cu", "gemm_f16_umma.cu", "shard_gather.cu", "quant_linear.cu", "prepack.cu", "static_scratch.cu", "mma_peak.cu", "conv2d_i8.cu"]
 
@@ -50,6 +53,24 @@ def _stale(out: Path, deps: list[Path]) -> bool:
     return any(d.stat().st_mtime > t for d in deps if d.exists())
 
 
+def build_front(force: bool = False) -> Path:
+    """host/torch_front.cpp against this interpreter's torch."""
+    if force or _stale(FRONT, [FRONT_SRC, PKG.parent / "include" / "nnb200.h"]):
+        import sysconfig
+
+        import torch
+        root = Path(torch.__file__).resolve().parent
+        include = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", sysconfig.get_paths()["include"],
+                   Path(os.environ.get("CUDA_HOME", "/usr/local/cuda")) / "include"]
+        r = subprocess.run([CXX, "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden",
+                            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-isystem{i}" for i in include),
+                            str(FRONT_SRC), "-o", str(FRONT), f"-L{root / 'lib'}", f"-Wl,-rpath,{root / 'lib'}", "-ltorch_python",
+                            "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10"], capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"g++ failed on {FRONT_SRC.name}:\n{r.stdout}\n{r.stderr}")
+    return FRONT
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     LIB_DIR.mkdir(exist_ok=True)
     obj_dir = LIB_DIR / "obj"
@@ -67,8 +88,10 @@ def build(force: bool = False, verbose: bool = False) -> Path:
                 print(r.stderr)
         return obj
 
-    with ThreadPoolExecutor(max_workers=len(SOURCES)) as ex:
+    with ThreadPoolExecutor(max_workers=len(SOURCES) + 1) as ex:
+        front = ex.submit(build_front, force)
         objs = list(ex.map(compile_one, SOURCES))
+        front.result()
     if force or _stale(LIB, objs):
         r = subprocess.run([NVCC, "-shared", "-o", str(LIB), *map(str, objs)],
                            capture_output=True, text=True)

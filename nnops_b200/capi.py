@@ -6,11 +6,14 @@ fallback for any call here.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import struct
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
 LIB_PATH = PKG / "lib" / "libnnb200.so"
+FRONT_PATH = PKG / "lib" / "torch_front.so"
 
 OK, INVALID_ARGUMENT, UNSUPPORTED, NOT_INITIALIZED, OUT_OF_MEMORY, INTERNAL = range(6)
 STATUS_NAMES = ["ok", "invalid_argument", "unsupported", "not_initialized", "out_of_memory", "internal"]
@@ -74,6 +77,7 @@ ZP_NOT_KNOWN = 2   # whether an array of zero points holds anything but zeros: l
 
 # Every symbol include/nnb200.h declares: (name, restype, argtypes).
 ZP_S8, ZP_U8, ZP_S32 = 0, 1, 2   # nnb200_quant_linear_args.zp_unsigned: storage type of the zero points
+ZP_HOST, PARAMS_HOST = 3, 4      # one int32 zero point in host memory for all rows; that, and one float scale
 
 
 class I8Packed(C.Structure):
@@ -202,6 +206,16 @@ def lib() -> C.CDLL:
             fn.argtypes = args
         _lib = l
     return _lib
+
+
+def torch_front():
+    """The compiled marshalling of the tensor front end (host/torch_front.cpp).  Raises if it has not been built."""
+    if not FRONT_PATH.exists():
+        raise RuntimeError(f"{FRONT_PATH} is missing: build it with `python -m nnops_b200.build`")
+    loader = importlib.machinery.ExtensionFileLoader("torch_front", str(FRONT_PATH))
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("torch_front", loader))
+    loader.exec_module(module)
+    return module
 
 
 class Nnb200Error(RuntimeError):

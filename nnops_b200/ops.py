@@ -4,11 +4,29 @@ layer.  torch provides device memory and streams only; every computation is a li
 from __future__ import annotations
 
 import ctypes as C
+import inspect
 import math
 
 import torch
 
 from . import capi
+
+_native = None
+
+
+def _front():
+    """host/torch_front.cpp, bound to the library capi has loaded: the usual calls without the interpreter.  Each
+    of its functions answers None, with nothing done, to what is not one of those; the code below then does
+    the call, or says what is wrong with it."""
+    global _native
+    if _native is None:
+        front, lib = capi.torch_front(), capi.lib()
+        front.bind(*(C.cast(getattr(lib, name), C.c_void_p).value for name in (
+            "nnb200_gemm_i8_workspace_bytes", "nnb200_gemm_i8", "nnb200_q4_1_workspace_bytes", "nnb200_linear_q4_1",
+            "nnb200_quantize_linear", "nnb200_dequantize_linear", "nnb200_conv2d_i8_workspace_bytes", "nnb200_conv2d_i8")), capi.check)
+        _native = front
+    return _native
+
 
 _OUT_TORCH = {"s32": torch.int32, "s8": torch.int8, "u8": torch.uint8, "f32": torch.float32, "f16": torch.float16}
 
@@ -121,6 +139,9 @@ def gemm_i8_args(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, out_kin
 
 def gemm_i8(a: torch.Tensor, w: torch.Tensor, *, out_kind: str = "s32", out: torch.Tensor | None = None, **kw):
     """out = epilogue(a @ w^T) on the current CUDA stream.  Returns the output tensor."""
+    made = (_native or _front()).gemm_i8(a, w, out_kind, out, kw)
+    if made is not None:
+        return made
     if not a.is_cuda:
         raise RuntimeError("nnops_b200.gemm_i8 needs CUDA tensors; there is no CPU path")
     batched = a.dim() == 3 or w.dim() == 3
@@ -249,6 +270,12 @@ def q4_1_args(a: torch.Tensor, w_blocks, out: torch.Tensor, k: int, *, bias=None
 def linear_q4_1(a: torch.Tensor, w_blocks: torch.Tensor, k: int, *, out_dtype: torch.dtype | None = None,
                 out: torch.Tensor | None = None, **kw) -> torch.Tensor:
     """out[M,N] = a[M,K] @ dequant(w_blocks)[N,K]^T.  ``w_blocks``: uint8 [N, ceil(K/32)*20]."""
+    w = w_blocks
+    if isinstance(w, PackedQ41):
+        w = (w.qs_ptr, w.n, w.qs_pitch, w.dm_ptr, w.dm_pitch)
+    made = (_native or _front()).linear_q4_1(a, w, k, out_dtype, out, kw)
+    if made is not None:
+        return made
     if not a.is_cuda:
         raise RuntimeError("nnops_b200.linear_q4_1 needs CUDA tensors; there is no CPU path")
     if a.dtype not in (torch.float16, torch.float32):
@@ -321,6 +348,9 @@ def _quant_params(scale, zero_point, device):
 def quantize_linear(x: torch.Tensor, scale, zero_point, *, axis: int = -1, out_dtype: torch.dtype = torch.int8,
                     out: torch.Tensor | None = None) -> torch.Tensor:
     """QuantizeLinear on the GPU: f32/f16 -> s8/u8."""
+    made = (_native or _front()).quantize_linear(x, scale, zero_point, axis, out_dtype, out)
+    if made is not None:
+        return made
     if x.dtype not in (torch.float32, torch.float16) or not x.is_contiguous():
         raise ValueError("x must be a contiguous f32/f16 tensor")
     scale, zero_point = _quant_params(scale, zero_point, x.device)
@@ -338,6 +368,9 @@ def quantize_linear(x: torch.Tensor, scale, zero_point, *, axis: int = -1, out_d
 def dequantize_linear(x: torch.Tensor, scale, zero_point, *, axis: int = -1, out_dtype: torch.dtype = torch.float32,
                       out: torch.Tensor | None = None) -> torch.Tensor:
     """DequantizeLinear on the GPU: s8/u8 -> f32/f16."""
+    made = (_native or _front()).dequantize_linear(x, scale, zero_point, axis, out_dtype, out)
+    if made is not None:
+        return made
     if x.dtype not in (torch.int8, torch.uint8) or not x.is_contiguous():
         raise ValueError("x must be a contiguous int8/uint8 tensor")
     scale, zero_point = _quant_params(scale, zero_point, x.device)
@@ -357,6 +390,9 @@ def linear_fp_act(a: torch.Tensor, w: torch.Tensor, *, scale_a, zp_a=0, act_dtyp
     the same two C-ABI calls the C++ backend glue makes for this route (quantise A with its
     per-tensor / per-token scale and int32 zero point, then the int8 matmul with the
     dequantizing epilogue).  ``scale_a`` / ``zp_a`` are scalars or per-row arrays."""
+    made = (_native or _front()).linear_fp_act(a, w, scale_a, zp_a, act_dtype, kw)
+    if made is not None:
+        return made
     if a.dim() != 2 or a.dtype not in (torch.float32, torch.float16) or not a.is_contiguous():
         raise ValueError("a must be a contiguous 2-D f32/f16 tensor")
     m, k = a.shape
@@ -409,12 +445,20 @@ def conv2d_out_hw(ih, iw, kh, kw, stride=(1, 1), dilation=(1, 1), padding=(0, 0)
     return oh, ow
 
 
-def conv2d_i8(x: torch.Tensor, w, *, stride=(1, 1), dilation=(1, 1), padding=(0, 0), groups: int = 1,
-              out_kind: str = "s8", out: torch.Tensor | None = None, bias=None, relu=False, activation="none",
-              act_alpha=0.0, act_beta=1.0, min_clip=-math.inf, max_clip=math.inf, scale_x=1.0, zp_x=0, scale_w=1.0,
-              zp_w=0, out_scale=1.0, out_zp=0, workspace: torch.Tensor | None = None) -> torch.Tensor:
+def conv2d_i8(x: torch.Tensor, w, *, out_kind: str = "s8", out: torch.Tensor | None = None, **kw) -> torch.Tensor:
     """int8 Conv2D on the current CUDA stream: x [N, IH, IW, IC] u8/s8 (NHWC, any strides), w an s8 HWIO filter
-    [KH, KW, IC/G, OC] or a PackedConvI8; returns [N, OH, OW, OC]."""
+    [KH, KW, IC/G, OC] or a PackedConvI8; returns [N, OH, OW, OC].  The other arguments: see _conv2d_i8."""
+    if isinstance(w, PackedConvI8):
+        made = (_native or _front()).conv2d_i8(x, w.blob, (w.kh, w.kw, w.icg, w.oc), out_kind, out, kw)
+        if made is not None:
+            return made
+    return _conv2d_i8(x, w, out_kind=out_kind, out=out, **kw)
+
+
+def _conv2d_i8(x: torch.Tensor, w, *, stride=(1, 1), dilation=(1, 1), padding=(0, 0), groups: int = 1,
+               out_kind: str = "s8", out: torch.Tensor | None = None, bias=None, relu=False, activation="none",
+               act_alpha=0.0, act_beta=1.0, min_clip=-math.inf, max_clip=math.inf, scale_x=1.0, zp_x=0, scale_w=1.0,
+               zp_w=0, out_scale=1.0, out_zp=0, workspace: torch.Tensor | None = None) -> torch.Tensor:
     if not x.is_cuda:
         raise RuntimeError("nnops_b200.conv2d_i8 needs CUDA tensors; there is no CPU path")
     dev = x.device
@@ -450,3 +494,6 @@ def conv2d_i8(x: torch.Tensor, w, *, stride=(1, 1), dilation=(1, 1), padding=(0,
         args.workspace_bytes = workspace.numel()
     _call(capi.lib().nnb200_conv2d_i8, args, dev, "nnb200_conv2d_i8")
     return out
+
+
+conv2d_i8.__signature__ = inspect.signature(_conv2d_i8)
