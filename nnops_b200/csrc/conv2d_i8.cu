@@ -34,6 +34,7 @@
 #include <cstring>
 
 #include "internal.cuh"
+#include "ptx.cuh"
 #include "epilogue.cuh"
 
 namespace nnb200 {
@@ -68,6 +69,7 @@ struct GatherParams {
 template <bool VEC>
 __global__ void __launch_bounds__(256) conv_gather_i8_kernel(const GatherParams p, const int rows_per_block)
 {
+    previous_kernel_done();
     extern __shared__ __align__(8) uint8_t gather_smem[];
     const int cpr = p.kp >> 4;   // pieces per row
     int64_t* row_base = reinterpret_cast<int64_t*>(gather_smem);          // [rows_per_block]
@@ -277,6 +279,7 @@ struct BorderParams {
 
 __global__ void __launch_bounds__(256) conv_border_table_kernel(const BorderParams p)
 {
+    previous_kernel_done();
     const int classes = (p.nh + 1) * (p.nw + 1);
     const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= static_cast<int64_t>(classes) * p.oc) {
@@ -636,9 +639,10 @@ int nnb200_conv2d_i8(const nnb200_conv2d_i8_args* a, void* stream_v)
                 return NNB200_INTERNAL;   // implicit_form() admits only geometries with at most eight classes
             }
             const int64_t items = static_cast<int64_t>(bp.nh + 1) * (bp.nw + 1) * g.oc;
-            conv_border_table_kernel<<<static_cast<unsigned>((items + 255) / 256), 256, 0, stream>>>(bp);
+            const cudaError_t launched = launch_overlapping(conv_border_table_kernel, dim3(static_cast<unsigned>((items + 255) / 256)),
+                                                            dim3(256), 0, stream, 1, bp);
             note_launch();
-            if (cudaGetLastError() != cudaSuccess) {
+            if (launched != cudaSuccess) {
                 return NNB200_INTERNAL;
             }
         }
@@ -728,13 +732,10 @@ int nnb200_conv2d_i8(const nnb200_conv2d_i8_args* a, void* stream_v)
         const int64_t cap = static_cast<int64_t>(dev->sm_count) * 8;
         blocks = blocks > cap ? cap : blocks;
         const size_t smem = static_cast<size_t>(rows_per_block) * 16 + static_cast<size_t>(cpr) * 16;
-        if (vec) {
-            conv_gather_i8_kernel<true><<<static_cast<unsigned>(blocks), 256, smem, stream>>>(p, rows_per_block);
-        } else {
-            conv_gather_i8_kernel<false><<<static_cast<unsigned>(blocks), 256, smem, stream>>>(p, rows_per_block);
-        }
+        const cudaError_t launched = launch_overlapping(vec ? conv_gather_i8_kernel<true> : conv_gather_i8_kernel<false>,
+                                                        dim3(static_cast<unsigned>(blocks)), dim3(256), smem, stream, 1, p, rows_per_block);
         note_launch();
-        const int st = cuda_status(cudaGetLastError());
+        const int st = cuda_status(launched);
         if (st != NNB200_OK) {
             return st;
         }

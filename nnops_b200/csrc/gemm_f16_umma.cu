@@ -92,6 +92,7 @@ __global__ void __launch_bounds__(256) q4_1_expand_f16_kernel(const uint8_t* __r
                                                               const int rows, const int nblk,
                                                               __half* __restrict__ out, const int64_t ld_out)
 {
+    previous_kernel_done();
     const int half_blocks = 2 * nblk;
     const bool planes = dm_plane != nullptr;
     const int64_t pitch = ldw_blocks * (planes ? 16 : kQ4BlockBytes);
@@ -144,6 +145,7 @@ __global__ void __launch_bounds__(256) split_f32_to_f16_kernel(const float* __re
                                                                const int m, const int k, const int kp,
                                                                __half* __restrict__ out)
 {
+    previous_kernel_done();
     const int64_t total = static_cast<int64_t>(m) * kp;
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -281,6 +283,7 @@ gemm_f16_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         }
         __syncwarp();
         named_barrier_arrive(1, kNumThreads);
+        previous_kernel_done();
     } else {
         if (role == 1) {
             if (lane == 0) {
@@ -290,6 +293,8 @@ gemm_f16_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             __syncwarp();
             tmem_alloc(tmem_slot, Cfg::kTmemCols);
             tmem_relinquish();
+        } else {
+            previous_kernel_done();
         }
         tc_fence_before_sync();
         named_barrier_sync(1, kNumThreads);
@@ -324,6 +329,7 @@ gemm_f16_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 }
             }
         }
+        let_next_kernel_start();
         if (wait_failed(spent) && lane == 0) {
             atomicCAS(error_word, 0, kErrProducerWait);
             // Copies already issued still land in shared memory: the CTA must not exit underneath them.
@@ -501,6 +507,7 @@ gemm_f16_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     tc_fence_before_sync();
     cluster_sync_all();  // both CTAs' barriers and TMEM exist before anything is signalled across
     tc_fence_after_sync();
+    previous_kernel_done();
     const uint32_t tmem_base = *tmem_slot;
 
     // Both issuing roles as in the single-CTA kernel: whole warp, one elected lane, waits nothing branches on.
@@ -541,6 +548,7 @@ gemm_f16_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
                 }
             }
         }
+        let_next_kernel_start();
         if (wait_failed(spent) && lane == 0) {
             atomicCAS(error_word, 0, kErrProducerWait);
         }
@@ -699,11 +707,10 @@ int launch_f16_variant(const nnb200_q4_1_args& q, const F16Operands& op, const F
     // Raster group: m-blocks whose band of A (128 x K halves each) stays within ~40 MB of L2.
     int group_m = static_cast<int>((40ll << 20) / (static_cast<int64_t>(kBlockM) * 2 * (k > 0 ? k : 1)));
     group_m = group_m < 4 ? 4 : group_m;
-    kernel<<<grid, kNumThreads, Cfg::kSmemBytes, stream>>>(map_a, map_w, q.out, q.ldc, m, n, k, op.w_wrap_k, ep,
-                                                           umma_idesc(1, 0, 0, kBlockM, BN), vec_ok, group_m,
-                                                           dev.error_word);
+    const cudaError_t launched = launch_overlapping(kernel, dim3(static_cast<unsigned>(grid)), dim3(kNumThreads), Cfg::kSmemBytes, stream, 1,
+                                                    map_a, map_w, q.out, q.ldc, m, n, k, op.w_wrap_k, ep, umma_idesc(1, 0, 0, kBlockM, BN), vec_ok, group_m, dev.error_word);
     note_launch();
-    return cuda_status(cudaGetLastError());
+    return cuda_status(launched);
 }
 
 
@@ -756,11 +763,10 @@ int launch_f16_pair_variant(const nnb200_q4_1_args& q, const F16Operands& op, co
                        (((reinterpret_cast<uintptr_t>(q.out) & 31u) == 0 && (out_pitch & 31u) == 0) ? 2 : 0);
     int group_m = static_cast<int>((40ll << 20) / (static_cast<int64_t>(2 * kBlockM) * 2 * (k > 0 ? k : 1)));
     group_m = group_m < 2 ? 2 : group_m;
-    kernel<<<2 * pairs, kNumThreads, Cfg::kSmemBytes, stream>>>(map_a, map_w, q.out, q.ldc, m, n, k, op.w_wrap_k, ep,
-                                                               umma_idesc(1, 0, 0, 2 * kBlockM, BN), vec_ok, group_m,
-                                                               dev.error_word);
+    const cudaError_t launched = launch_overlapping(kernel, dim3(static_cast<unsigned>(2 * pairs)), dim3(kNumThreads), Cfg::kSmemBytes, stream, 1,
+                                                    map_a, map_w, q.out, q.ldc, m, n, k, op.w_wrap_k, ep, umma_idesc(1, 0, 0, 2 * kBlockM, BN), vec_ok, group_m, dev.error_word);
     note_launch();
-    return cuda_status(cudaGetLastError());
+    return cuda_status(launched);
 }
 
 // Width of the output tile: 256 unless a narrower one saves more than 8 % of the padded work
@@ -822,10 +828,11 @@ int launch_split_f32_to_f16(const float* a, int64_t lda, int64_t m, int64_t k, i
 {
     const int64_t want = (m * kp + 255) / 256;
     const int64_t cap = static_cast<int64_t>(dev.sm_count) * 16;
-    split_f32_to_f16_kernel<<<static_cast<unsigned>(want < cap ? want : cap), 256, 0, stream>>>(
-        a, lda, static_cast<int>(m), static_cast<int>(k), static_cast<int>(kp), static_cast<__half*>(out));
+    const cudaError_t launched = launch_overlapping(split_f32_to_f16_kernel, dim3(static_cast<unsigned>(want < cap ? want : cap)), dim3(256), 0,
+                                                    stream, 1, a, lda, static_cast<int>(m), static_cast<int>(k), static_cast<int>(kp),
+                                                    static_cast<__half*>(out));
     note_launch();
-    return cuda_status(cudaGetLastError());
+    return cuda_status(launched);
 }
 
 int launch_q4_1_two_pass(const nnb200_q4_1_args& q, const DeviceInfo& dev, cudaStream_t stream)
@@ -847,11 +854,12 @@ int launch_q4_1_two_pass(const nnb200_q4_1_args& q, const DeviceInfo& dev, cudaS
         const int64_t want = (q.n + 1) / 2;
         const int64_t cap = static_cast<int64_t>(dev.sm_count) * 16;
         const unsigned grid = static_cast<unsigned>(want < cap ? want : cap);
-        q4_1_expand_f16_kernel<<<grid, 256, 0, stream>>>(static_cast<const uint8_t*>(q.w_blocks), q.ldw_blocks,
-                                                         static_cast<const uint32_t*>(q.w_dm), q.ld_dm,
-                                                         static_cast<int>(q.n), static_cast<int>(nblk), w_f16, ldw);
+        const cudaError_t launched = launch_overlapping(q4_1_expand_f16_kernel, dim3(grid), dim3(256), 0, stream, 1,
+                                                        static_cast<const uint8_t*>(q.w_blocks), q.ldw_blocks,
+                                                        static_cast<const uint32_t*>(q.w_dm), q.ld_dm, static_cast<int>(q.n),
+                                                        static_cast<int>(nblk), w_f16, ldw);
         note_launch();
-        if (cudaGetLastError() != cudaSuccess) {
+        if (launched != cudaSuccess) {
             return NNB200_INTERNAL;
         }
     }

@@ -27,6 +27,7 @@
 #include <mutex>
 
 #include "internal.cuh"
+#include "ptx.cuh"
 
 namespace nnb200 {
 
@@ -69,6 +70,7 @@ __device__ __forceinline__ void mma_m16n8k32(int32_t (&d)[4], uint32_t a0, uint3
 template <int M_TILES, bool A_UNSIGNED>
 __global__ void __launch_bounds__(kWarps * 32, 3) gemm_i8_decode_kernel(const I8Problem p, const I8Epilogue ep)
 {
+    previous_kernel_done();
     __shared__ int4 partial[kWarps][M_TILES][32];
 
     const int warp = threadIdx.x >> 5;
@@ -183,21 +185,22 @@ int launch_gemm_i8_decode(const I8Problem& p, const I8Epilogue& ep, const Device
 {
     const unsigned grid = static_cast<unsigned>((p.n + kRows - 1) / kRows);
     const int threads = kWarps * 32;
+    cudaError_t launched;
     if (p.m <= 8) {
         if (p.a_unsigned) {
-            gemm_i8_decode_kernel<1, true><<<grid, threads, 0, stream>>>(p, ep);
+            launched = launch_overlapping(gemm_i8_decode_kernel<1, true>, dim3(grid), dim3(threads), 0, stream, 1, p, ep);
         } else {
-            gemm_i8_decode_kernel<1, false><<<grid, threads, 0, stream>>>(p, ep);
+            launched = launch_overlapping(gemm_i8_decode_kernel<1, false>, dim3(grid), dim3(threads), 0, stream, 1, p, ep);
         }
     } else {
         if (p.a_unsigned) {
-            gemm_i8_decode_kernel<2, true><<<grid, threads, 0, stream>>>(p, ep);
+            launched = launch_overlapping(gemm_i8_decode_kernel<2, true>, dim3(grid), dim3(threads), 0, stream, 1, p, ep);
         } else {
-            gemm_i8_decode_kernel<2, false><<<grid, threads, 0, stream>>>(p, ep);
+            launched = launch_overlapping(gemm_i8_decode_kernel<2, false>, dim3(grid), dim3(threads), 0, stream, 1, p, ep);
         }
     }
     note_launch();
-    return cuda_status(cudaGetLastError());
+    return cuda_status(launched);
 }
 
 }  // namespace nnb200

@@ -13,6 +13,7 @@
 #include <type_traits>
 
 #include "internal.cuh"
+#include "ptx.cuh"
 
 namespace nnb200 {
 
@@ -24,6 +25,7 @@ constexpr int kTileK = 32;
 template <bool A_UNSIGNED>
 __global__ void __launch_bounds__(256) gemm_i8_generic_kernel(const I8Problem p, const I8Epilogue ep)
 {
+    previous_kernel_done();
     __shared__ int32_t a_s[kTile][kTileK + 1];
     __shared__ int32_t w_s[kTile][kTileK + 1];
 
@@ -108,6 +110,7 @@ template <bool UNSIGNED>
 __global__ void __launch_bounds__(128) i8_sums_kernel(const uint8_t* x, int64_t rows, int64_t k, int64_t stride_row,
                                                       int64_t stride_k, int32_t* out)
 {
+    previous_kernel_done();
     const int64_t r = blockIdx.x;
     const uint8_t* row = x + r * stride_row;
     int32_t s = 0;
@@ -159,6 +162,7 @@ template <bool UNSIGNED>
 __global__ void __launch_bounds__(128) i8_sums_look_kernel(const uint8_t* x, int64_t rows, int64_t k, int64_t stride_row,
                                                            int32_t* out, const int32_t* look, int64_t look_count)
 {
+    previous_kernel_done();
     if (!any_zero_point(look, look_count)) {
         return;
     }
@@ -277,13 +281,14 @@ int launch_gemm_i8_generic(const I8Problem& p, const I8Epilogue& ep, const Devic
     if (grid.y > 65535u) {
         return NNB200_UNSUPPORTED;
     }
+    cudaError_t launched;
     if (p.a_unsigned) {
-        gemm_i8_generic_kernel<true><<<grid, 256, 0, stream>>>(p, ep);
+        launched = launch_overlapping(gemm_i8_generic_kernel<true>, grid, dim3(256), 0, stream, 1, p, ep);
     } else {
-        gemm_i8_generic_kernel<false><<<grid, 256, 0, stream>>>(p, ep);
+        launched = launch_overlapping(gemm_i8_generic_kernel<false>, grid, dim3(256), 0, stream, 1, p, ep);
     }
     note_launch();
-    return cuda_status(cudaGetLastError());
+    return cuda_status(launched);
 }
 
 bool narrow_i8_supported(const I8Problem& p)
@@ -330,15 +335,18 @@ int launch_i8_sums(const I8Problem& p, const I8Sums& sums, const DeviceInfo& dev
     // A look is taken where all blocks' looks together read at most a quarter of the operand (24 x 28672 x
     // 8192: one look at 28672 zero points a block 9 us, sweeping the 24 rows 2.5), and where rows are wide loads.
     const int64_t resident = static_cast<int64_t>(dev.sm_count) * 16;
+    cudaError_t launched = cudaSuccess;
     const auto sweep = [&](auto is_unsigned, const uint8_t* x, int64_t rows, int64_t stride_row, int64_t stride_k, int32_t* out,
                            const int32_t* look, int64_t look_count) {
         constexpr bool U = decltype(is_unsigned)::value;
         const int64_t blocks = (rows + 3) / 4 < resident ? (rows + 3) / 4 : resident;
         const bool wide = stride_k == 1 && ((reinterpret_cast<uintptr_t>(x) | static_cast<uint64_t>(stride_row)) & 15u) == 0;
         if (look != nullptr && wide && static_cast<double>(rows) * p.k >= 4.0 * sizeof(int32_t) * blocks * look_count) {
-            i8_sums_look_kernel<U><<<static_cast<unsigned>(blocks), 128, 0, stream>>>(x, rows, p.k, stride_row, out, look, look_count);
+            launched = launch_overlapping(i8_sums_look_kernel<U>, dim3(static_cast<unsigned>(blocks)), dim3(128), 0, stream, 1, x, rows, p.k,
+                                          stride_row, out, look, look_count);
         } else {
-            i8_sums_kernel<U><<<static_cast<unsigned>(rows), 128, 0, stream>>>(x, rows, p.k, stride_row, stride_k, out);
+            launched = launch_overlapping(i8_sums_kernel<U>, dim3(static_cast<unsigned>(rows)), dim3(128), 0, stream, 1, x, rows, p.k,
+                                          stride_row, stride_k, out);
         }
     };
     if (sums.r_a != nullptr) {
@@ -348,11 +356,11 @@ int launch_i8_sums(const I8Problem& p, const I8Sums& sums, const DeviceInfo& dev
             sweep(std::false_type{}, a, p.m, p.a_stride_m, p.a_stride_k, sums.r_a, sums.look_w, p.n);
         }
     }
-    if (sums.r_w != nullptr) {
+    if (sums.r_w != nullptr && launched == cudaSuccess) {
         sweep(std::false_type{}, w, p.n, p.w_stride_n, p.w_stride_k, sums.r_w, sums.look_a, p.m);
     }
     note_launch((sums.r_a != nullptr ? 1 : 0) + (sums.r_w != nullptr ? 1 : 0));
-    return cuda_status(cudaGetLastError());
+    return cuda_status(launched);
 }
 
 }  // namespace nnb200

@@ -433,12 +433,14 @@ gemm_i8_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         }
         __syncwarp();
         named_barrier_arrive(1, kNumThreads);   // the others meet below; this warp needs nothing of theirs
+        previous_kernel_done();
     } else if (warp == 1) {
         tmem_alloc(tmem_slot, Cfg::kTmemCols);
         tmem_relinquish();
     }
     // Per-row epilogue terms of every activation row, once per CTA (the rows are the same for all tiles).
     else {
+        previous_kernel_done();
         const int t = threadIdx.x - 64;
         if (t < Cfg::kRowTerms) {
             row_terms[t] = i8_row_terms(ep, t < m_total ? t : 0);
@@ -472,6 +474,7 @@ gemm_i8_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 }
             }
         }
+        let_next_kernel_start();
         if (wait_failed(spent) && lane == 0) {
             atomicCAS(error_word, 0, kErrProducerWait);
             if (!drain_ring(full_bar, kStages, issued)) {
@@ -882,14 +885,11 @@ int launch_skinny_variant(const I8Problem& p, const I8Epilogue& ep, const Device
     }
     // 128-row operand = weights (s8), N operand = activations (s8 or u8).
     const uint32_t idesc = umma_idesc(2, 1, p.a_unsigned ? 0u : 1u, kBlockN, MP);
-    cfg.gridDim = dim3(static_cast<unsigned>(grid));
-    attr.val.clusterDim.x = static_cast<unsigned>(parts);
-    cfg.numAttrs = parts > 1 ? 1 : 0;
     Shares shares{parts, 0, 0};
     const int dealt = parts > 1 ? (k + kBlockKBytes - 1) / kBlockKBytes : num_tiles, hands = parts > 1 ? parts : grid;
     shares.per_cta = dealt / hands;
     shares.longer = dealt % hands;
-    const cudaError_t launched = cudaLaunchKernelEx(&cfg, kernel, map_w, map_a, ep, m, n, k, idesc, dev.error_word, counters, slots,
+    const cudaError_t launched = launch_overlapping(kernel, dim3(static_cast<unsigned>(grid)), dim3(kNumThreads), Cfg::kSmemBytes, stream, parts, map_w, map_a, ep, m, n, k, idesc, dev.error_word, counters, slots,
                                                     tag, tile_rows, num_tiles, shares);
     note_launch();
     return cuda_status(launched);

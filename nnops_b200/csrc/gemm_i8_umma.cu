@@ -134,6 +134,7 @@ gemm_i8_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     tc_fence_before_sync();
     cluster_sync_all();  // both CTAs' barriers and TMEM exist before anything is signalled across
     tc_fence_after_sync();
+    previous_kernel_done();
     const uint32_t tmem_base = *tmem_slot;
 
     // In both issuing roles the whole warp walks the loop, one elected lane issues, and no branch depends on
@@ -215,6 +216,7 @@ gemm_i8_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 }
             }
         }
+        let_next_kernel_start();
         if (wait_failed(spent) && lane == 0) {
             atomicCAS(error_word, 0, kErrProducerWait);
         }
@@ -493,11 +495,10 @@ int launch_pair_variant(const I8Problem& p, const I8Epilogue& ep, int m, int n, 
     int group_m = static_cast<int>((40ll << 20) / (static_cast<int64_t>(2 * kBlockM) * (k > 0 ? k : 1)));
     group_m = group_m < 2 ? 2 : group_m;
     constexpr uint32_t major_bits = ((POSE & 1) ? kUmmaAMajorMN : 0u) | ((POSE & 2) ? kUmmaBMajorMN : 0u);
-    kernel<<<2 * pairs, num_threads(0), Cfg::kSmemBytes, stream>>>(map_a, map_w, ep, m, n, k,
-                                                               umma_idesc(2, a_fmt, 1, 2 * kBlockM, BN) | major_bits, vec_ok, group_m,
-                                                               k_rotation_step(n), dev.error_word, ConvTile{});
+    const cudaError_t launched = launch_overlapping(kernel, dim3(static_cast<unsigned>(2 * pairs)), dim3(num_threads(0)), Cfg::kSmemBytes, stream, 1,
+                                                    map_a, map_w, ep, m, n, k, umma_idesc(2, a_fmt, 1, 2 * kBlockM, BN) | major_bits, vec_ok, group_m, k_rotation_step(n), dev.error_word, ConvTile{});
     note_launch();
-    return cuda_status(cudaGetLastError());
+    return cuda_status(launched);
 }
 
 template <int BN, int SUB = 1, bool MC = false, int POSE = 0>
@@ -550,10 +551,10 @@ int launch_variant(const CUtensorMap& map_a, const CUtensorMap& map_w, const I8E
     if (knob(NNB200_KNOB_GROUP_M) > 0) {
         group_m = knob(NNB200_KNOB_GROUP_M);
     }
-    kernel<<<grid, tile_threads(KIND, PEERS), kSmem, stream>>>(map_a, map_w, maps, ep, m, n, k, idesc, vec_ok, group_m,
-                                                 k_rotation_step(n), dev.error_word, ConvTile{});
+    const cudaError_t launched = launch_overlapping(kernel, dim3(static_cast<unsigned>(grid)), dim3(tile_threads(KIND, PEERS)), kSmem, stream, 1,
+                                                    map_a, map_w, maps, ep, m, n, k, idesc, vec_ok, group_m, k_rotation_step(n), dev.error_word, ConvTile{});
     note_launch();
-    return cuda_status(cudaGetLastError());
+    return cuda_status(launched);
 }
 
 template <int BN>
@@ -629,10 +630,10 @@ int launch_conv_variant(const CUtensorMap& map_a, const CUtensorMap& map_w, cons
     const int grid = num_tiles < dev.sm_count ? num_tiles : dev.sm_count;
     int group_m = static_cast<int>((40ll << 20) / (static_cast<int64_t>(kBlockM) * (k > 0 ? k : 1)));
     group_m = group_m < 4 ? 4 : group_m;
-    kernel<<<grid, tile_threads(KIND, 0), Cfg::kSmemBytes, stream>>>(map_a, map_w, maps, ep, m_tiles * kBlockM, n, k, idesc, vec_ok,
-                                                            group_m, k_rotation_step(n), dev.error_word, conv);
+    const cudaError_t launched = launch_overlapping(kernel, dim3(static_cast<unsigned>(grid)), dim3(tile_threads(KIND, 0)), Cfg::kSmemBytes, stream, 1,
+                                                    map_a, map_w, maps, ep, m_tiles * kBlockM, n, k, idesc, vec_ok, group_m, k_rotation_step(n), dev.error_word, conv);
     note_launch();
-    return cuda_status(cudaGetLastError());
+    return cuda_status(launched);
 }
 
 // The CTA-pair form of the same: two patches per 256 x 256 tile, each CTA loading its own patch
@@ -672,11 +673,10 @@ int launch_conv_pair_variant(const CUtensorMap& map_a, const CUtensorMap& map_w,
     const int pairs = num_tiles < max_pairs[dev.device] ? num_tiles : max_pairs[dev.device];
     int group_m = static_cast<int>((40ll << 20) / (static_cast<int64_t>(2 * kBlockM) * (k > 0 ? k : 1)));
     group_m = group_m < 2 ? 2 : group_m;
-    kernel<<<2 * pairs, num_threads(0), Cfg::kSmemBytes, stream>>>(map_a, map_w, ep, m_tiles * kBlockM, n, k,
-                                                               umma_idesc(2, a_fmt, 1, 2 * kBlockM, BN), vec_ok, group_m,
-                                                               k_rotation_step(n), dev.error_word, conv);
+    const cudaError_t launched = launch_overlapping(kernel, dim3(static_cast<unsigned>(2 * pairs)), dim3(num_threads(0)), Cfg::kSmemBytes, stream, 1,
+                                                    map_a, map_w, ep, m_tiles * kBlockM, n, k, umma_idesc(2, a_fmt, 1, 2 * kBlockM, BN), vec_ok, group_m, k_rotation_step(n), dev.error_word, conv);
     note_launch();
-    return cuda_status(cudaGetLastError());
+    return cuda_status(launched);
 }
 
 int launch_conv_pair(const CUtensorMap& map_a, const CUtensorMap& map_w, const I8Epilogue& ep, int m_tiles, int n, int k,

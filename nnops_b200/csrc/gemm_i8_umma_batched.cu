@@ -35,10 +35,10 @@ int launch_batched_variant(const CUtensorMap& map_a, const CUtensorMap& map_w, c
     const int num_m = (m + kBlockM - 1) / kBlockM;
     const int64_t num_tiles = static_cast<int64_t>(batch.count) * num_m * ((n + BN - 1) / BN);
     const int grid = num_tiles < dev.sm_count ? static_cast<int>(num_tiles) : dev.sm_count;
-    kernel<<<grid, tile_threads(KIND, 0), Cfg::kSmemBytes, stream>>>(map_a, map_w, maps, ep, m, n, k, idesc, vec_ok, num_m, 0,
-                                                            dev.error_word, batch);
+    const cudaError_t launched = launch_overlapping(kernel, dim3(static_cast<unsigned>(grid)), dim3(tile_threads(KIND, 0)), Cfg::kSmemBytes, stream, 1,
+                                                    map_a, map_w, maps, ep, m, n, k, idesc, vec_ok, num_m, 0, dev.error_word, batch);
     note_launch();
-    return cuda_status(cudaGetLastError());
+    return cuda_status(launched);
 }
 
 template <int BN>

@@ -716,6 +716,7 @@ gemm_i8_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
         __syncwarp();
         named_barrier_arrive(1, kThreads);
+        previous_kernel_done();
     } else {
         if (role == 1) {
             if (lane == 0) {
@@ -725,6 +726,8 @@ gemm_i8_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             __syncwarp();
             tmem_alloc(tmem_slot, Cfg::kTmemCols);
             tmem_relinquish();
+        } else {
+            previous_kernel_done();
         }
         tc_fence_before_sync();
         named_barrier_sync(1, kThreads);
@@ -828,6 +831,7 @@ gemm_i8_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 }
             }
         }
+        let_next_kernel_start();
         if (wait_failed(spent) && lane == 0) {
             atomicCAS(error_word, 0, kErrProducerWait);
             // Copies already issued still land in shared memory: the CTA must not exit underneath them.

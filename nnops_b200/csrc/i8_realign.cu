@@ -14,6 +14,7 @@
 // would read the operand again.  Bytes past the row's end, up to the pitch, are zeros.
 
 #include "internal.cuh"
+#include "ptx.cuh"
 #include "i8_realign.cuh"
 
 namespace nnb200 {
@@ -43,6 +44,7 @@ __device__ __forceinline__ uint32_t load_word(const uint8_t* row, int64_t at, in
 template <int TEAM>
 __global__ void __launch_bounds__(kWarps * 32) i8_realign_kernel(const I8RealignJob a, const I8RealignJob w)
 {
+    previous_kernel_done();
     constexpr int kTeams = kWarps * 32 / TEAM;
     __shared__ int32_t part[kWarps];
     const int lane = threadIdx.x % TEAM;
@@ -123,13 +125,14 @@ int launch_i8_realign(const I8RealignJob& a, const I8RealignJob& w, const Device
     const bool wide = rows <= static_cast<int64_t>(dev.sm_count) * 8 && pitch > 4 * 512;
     const int64_t blocks = wide ? rows : (rows + kWarps - 1) / kWarps;
     const unsigned grid = static_cast<unsigned>(blocks < most ? blocks : most);
+    cudaError_t launched;
     if (wide) {
-        i8_realign_kernel<kWarps * 32><<<grid, kWarps * 32, 0, stream>>>(a, w);
+        launched = launch_overlapping(i8_realign_kernel<kWarps * 32>, dim3(grid), dim3(kWarps * 32), 0, stream, 1, a, w);
     } else {
-        i8_realign_kernel<32><<<grid, kWarps * 32, 0, stream>>>(a, w);
+        launched = launch_overlapping(i8_realign_kernel<32>, dim3(grid), dim3(kWarps * 32), 0, stream, 1, a, w);
     }
     note_launch();
-    return cuda_status(cudaGetLastError());
+    return cuda_status(launched);
 }
 
 }  // namespace nnb200

@@ -211,4 +211,36 @@ inline int cuda_status(cudaError_t e)
     return e == cudaSuccess ? NNB200_OK : NNB200_INTERNAL;
 }
 
+// A launch whose blocks may become resident while the previous kernel of the stream is still running
+// (programmatic stream serialization).  EVERY block of such a kernel executes previous_kernel_done() before it
+// touches global memory, reads included: scratch and outputs may be memory the previous kernel still uses, and a
+// kernel that ended without having waited would let its successor overtake its predecessor.  What comes
+// before it -- barriers, tensor memory, descriptors -- and the launch itself cost 2 to 4 us a call otherwise.
+// A kernel lets the next one start only near its end (or, where its blocks come in several turns, by ending): the
+// blocks of at most one kernel then wait for another, and that one has all of its own running.
+template <class... P, class... A>
+inline cudaError_t launch_overlapping(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster,
+                                      A&&... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = static_cast<unsigned>(cluster);
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();   // reported by the status, not left behind
+    }
+    return e;
+}
+
 }  // namespace nnb200

@@ -41,6 +41,20 @@ __device__ __forceinline__ bool elect_one()
     return pred != 0;
 }
 
+// ---- programmatic dependent launch (see launch_overlapping) --------------------------------
+
+// Once every block has said so or ended, the next kernel's blocks may take what room there is.
+__device__ __forceinline__ void let_next_kernel_start()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Returns when the previous kernel has completed and its writes are visible; at once without the launch attribute.
+__device__ __forceinline__ void previous_kernel_done()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // A value that is the same in every lane of a converged warp, known as such to the compiler.
 __device__ __forceinline__ int warp_uniform(int v) { return __shfl_sync(0xFFFFFFFFu, v, 0); }
 __device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __shfl_sync(0xFFFFFFFFu, v, 0); }

@@ -137,6 +137,7 @@ q4_1_gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const uint8_t* 
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
+    previous_kernel_done();
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
@@ -523,11 +524,11 @@ int launch_variant(const nnb200_q4_1_args& q, const CUtensorMap& map_a, const Fp
                         ((static_cast<uint64_t>(q.ldc) * elem) & 15u) == 0)
                            ? 1
                            : 0;
-    kernel<<<grid, Cfg::kNumThreads, Cfg::kSmemBytes, stream>>>(
-        map_a, static_cast<const uint8_t*>(q.w_blocks), q.ldw_blocks, q.out, q.ldc, m, n, k, ep,
-        umma_idesc(1, 0, 0, kHalfM, kTileN), vec_ok, dev.error_word);
+    const cudaError_t launched = launch_overlapping(kernel, dim3(static_cast<unsigned>(grid)), dim3(Cfg::kNumThreads), Cfg::kSmemBytes, stream, 1,
+                                                    map_a, static_cast<const uint8_t*>(q.w_blocks), q.ldw_blocks, q.out, q.ldc, m, n, k,
+                                                    ep, umma_idesc(1, 0, 0, kHalfM, kTileN), vec_ok, dev.error_word);
     note_launch();
-    return cuda_status(cudaGetLastError());
+    return cuda_status(launched);
 }
 
 }  // namespace

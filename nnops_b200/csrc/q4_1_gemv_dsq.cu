@@ -353,7 +353,7 @@ q4_1_gemv_dsq_kernel(const uint8_t* __restrict__ w, const int64_t w_pitch_bytes,
                      const int64_t dm_pitch_bytes, const void* __restrict__ a_v,
                      const int64_t lda, void* __restrict__ out, const int64_t ldc, const int m_count,
                      const int n_total, const int k_total, const DsqLayout lay, const FpEpilogue ep,
-                     const int a_vec_ok, int32_t* error_word)
+                     const int a_vec_ok, int32_t* error_word, const int early)
 {
     constexpr int G = 8 / MP;
     constexpr int kConsumers = NC;
@@ -395,10 +395,16 @@ q4_1_gemv_dsq_kernel(const uint8_t* __restrict__ w, const int64_t w_pitch_bytes,
     }
     __syncthreads();
     // The next kernel in the stream may start its own prologue (and its weight stream) now.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (early) {
+        let_next_kernel_start();
+    }
 
     if (warp == kProducerWarp) {
-        // ---- producer: weights never depend on the preceding kernel, so no griddepcontrol.wait here ----
+        // ---- producer: where the caller says that no kernel before this one writes the weights (early), it
+        // does not wait for the preceding kernel ----
+        if (!early) {
+            previous_kernel_done();
+        }
         int slot = 0;
         uint32_t empty_parity = 1;   // a fresh barrier passes a wait on parity 1: the first round needs no wait
         bool ok = true;
@@ -451,7 +457,7 @@ q4_1_gemv_dsq_kernel(const uint8_t* __restrict__ w, const int64_t w_pitch_bytes,
     }
 
     // Activations are read and outputs written only after the preceding kernel has completed.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    previous_kernel_done();
 
     if (warp == kReducerWarp) {
         // ---- reducer: sum the consumer warps' partials per tile in a fixed order, finish, store ----
@@ -712,7 +718,7 @@ bool plan_layout(int mp, int64_t k, int consumers, bool packed, DsqLayout* out)
 }
 
 using DsqKernel = void (*)(const uint8_t*, int64_t, const uint8_t*, int64_t, const void*, int64_t, void*, int64_t, int, int,
-                           int, DsqLayout, FpEpilogue, int, int32_t*);
+                           int, DsqLayout, FpEpilogue, int, int32_t*, int);
 
 template <int MP, int NC, bool PACKED>
 DsqKernel pick_kernel(bool out_f16, bool a_f32)
@@ -835,9 +841,9 @@ int launch_q4_1_gemv_dsq(const nnb200_q4_1_args& q, const DeviceInfo& dev, cudaS
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
-        cfg.numAttrs = overlap ? 1 : 0;
+        cfg.numAttrs = 1;
         const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, w, pitch, w_dm, dm_pitch, a, q.lda, out, q.ldc, m_count, n, k, lay, ep,
-                                                 a_vec_ok, dev.error_word);
+                                                 a_vec_ok, dev.error_word, overlap ? 1 : 0);
         note_launch();
         if (e != cudaSuccess) {
             return NNB200_INTERNAL;

@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
 q4_1_gemv_mma_kernel(const uint8_t* __restrict__ w, const int64_t w_pitch_bytes, const void* __restrict__ a_v,
                      const int64_t lda, void* __restrict__ out, const int64_t ldc, const int m_count,
                      const int n_total, const int k_total, const int num_bufs, const FpEpilogue ep,
-                     const int a_vec_ok, int32_t* error_word)
+                     const int a_vec_ok, int32_t* error_word, const int early)
 {
     // [warp][buf][kSliceBufBytes]; num_bufs = min(kBufs, chunks of K).
     extern __shared__ __align__(128) uint8_t slices[];
@@ -245,15 +245,18 @@ q4_1_gemv_mma_kernel(const uint8_t* __restrict__ w, const int64_t w_pitch_bytes,
         mbar_init_fence();
     }
     __syncwarp();
-    // Weights never depend on the preceding kernel: start streaming them right away.
+    // Start streaming the weights: right away where the caller says that no kernel before this one writes them
+    // (early; the next kernel in the stream may then begin its own prologue too), else once the previous one
+    // has completed, as with activations and outputs.
+    if (early) {
+        let_next_kernel_start();
+    } else {
+        previous_kernel_done();
+    }
     for (int b = 0; b < num_bufs && b < num_chunks; ++b) {
         issue_slice(b, b);
     }
-    // Let the next kernel in the stream begin its own prologue, then wait until the previous
-    // one has completed before touching activations or outputs.  Both are no-ops for a launch
-    // without the programmatic-serialization attribute.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    previous_kernel_done();
     __syncthreads();  // abort_word initialised for every warp
 
     float acc0[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -381,9 +384,9 @@ cudaError_t launch_one(unsigned grid, bool overlap, cudaStream_t stream, const u
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = overlap ? 1 : 0;
+    cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, q4_1_gemv_mma_kernel<OUT_F16, A_F32>, w, pitch, a, lda, out, ldc, m_count, n, k,
-                              num_bufs, ep, a_vec_ok, error_word);
+                              num_bufs, ep, a_vec_ok, error_word, overlap ? 1 : 0);
 }
 
 }  // namespace

@@ -20,9 +20,9 @@
 //     memory and the MMAs of different units overlap.
 //   * Few channels: `split` CTAs (a cluster) share a tile's K and add up their accumulators
 //     through distributed shared memory in a fixed order -- the result does not depend on timing.
-//   * Launched with programmatic stream serialization when the caller allows it
-//     (NNB200_Q4_FLAG_OVERLAP_PREVIOUS): barriers, tensor memory and the first units' weights are set up
-//     before griddepcontrol.wait, activations (by TMA, never through L1) read and outputs written after it.
+//   * Launched with programmatic stream serialization: barriers and tensor memory are set up before
+//     griddepcontrol.wait, and with NNB200_Q4_FLAG_OVERLAP_PREVIOUS the first units' weights fetched;
+//     activations are read (by TMA, never through L1) and outputs written after it.
 //   * f32 activations are given as two f16 rows each, high part and remainder; the epilogue adds the
 //     two accumulator columns (see split_f32_to_f16_kernel).
 //
@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 q4_1_rows_umma_kernel(const __grid_constant__ CUtensorMap map_a, const uint8_t* __restrict__ w,
                       const int64_t w_pitch_bytes, void* __restrict__ out, const int64_t ldc, const int m_total,
                       const int hi_lo, const int nb, const int n_total, const int k_total, const int tile_rows,
-                      const int split, const FpEpilogue ep, const uint32_t idesc, int32_t* error_word)
+                      const int split, const FpEpilogue ep, const uint32_t idesc, int32_t* error_word, const int early)
 {
     using Cfg = RowsConfig<BLOCKS>;
     constexpr int kUnitK = Cfg::kUnitK;
@@ -271,7 +271,12 @@ q4_1_rows_umma_kernel(const __grid_constant__ CUtensorMap map_a, const uint8_t* 
         next_u += kGroups;
         next_buf = next_buf + 1 == Cfg::kDepth ? 0 : next_buf + 1;
     };
+    // Nothing but weights is touched before the previous kernel has completed, and those only where the
+    // caller says that no kernel before this one writes them (early).
     if (warp < kWarps) {
+        if (!early) {
+            previous_kernel_done();
+        }
 #pragma unroll 1
         for (int s = 0; s < Cfg::kDepth; ++s) {
             issue_unit();
@@ -280,10 +285,10 @@ q4_1_rows_umma_kernel(const __grid_constant__ CUtensorMap map_a, const uint8_t* 
         tmem_alloc(tmem_slot, kTmemCols);
         tmem_relinquish();
     }
-    // Let the next kernel in the stream begin its own prologue; then nothing but weights is touched before
-    // the previous one has completed.  No-ops for a launch without the programmatic-serialization attribute.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (early) {
+        let_next_kernel_start();
+    }
+    previous_kernel_done();
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -381,6 +386,7 @@ q4_1_rows_umma_kernel(const __grid_constant__ CUtensorMap map_a, const uint8_t* 
             }
             __syncwarp();
         }
+        let_next_kernel_start();
         if (wait_failed(spent)) {
             if (lane == 0) {
                 atomicCAS(error_word, 0, kErrMmaWait);
@@ -633,11 +639,12 @@ int launch_variant(const CUtensorMap& map_a, const Q4RowsCall& c, int nb, int ti
     const int ctas = split > 1 ? tiles * split : (tiles < dev.sm_count ? tiles : dev.sm_count);
     attr[0].val.clusterDim.x = static_cast<unsigned>(split);
     cfg.gridDim = dim3(static_cast<unsigned>(ctas));
-    cfg.numAttrs = (c.q->flags & NNB200_Q4_FLAG_OVERLAP_PREVIOUS) != 0 ? 2 : 1;
+    cfg.numAttrs = 2;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, map_a, static_cast<const uint8_t*>(c.q->w_blocks),
                                              c.q->ldw_blocks * kQ4BlockBytes, c.q->out, c.q->ldc, static_cast<int>(c.q->m),
                                              c.hi_lo ? 1 : 0, nb, static_cast<int>(c.q->n), static_cast<int>(c.q->k), tile_rows,
-                                             split, ep, umma_idesc(1, 0, 0, kTileRows, static_cast<uint32_t>(nb)), dev.error_word);
+                                             split, ep, umma_idesc(1, 0, 0, kTileRows, static_cast<uint32_t>(nb)), dev.error_word,
+                                             (c.q->flags & NNB200_Q4_FLAG_OVERLAP_PREVIOUS) != 0 ? 1 : 0);
     note_launch();
     return cuda_status(e);
 }

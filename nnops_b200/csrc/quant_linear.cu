@@ -34,6 +34,7 @@
 #include <type_traits>
 
 #include "internal.cuh"
+#include "ptx.cuh"
 
 namespace nnb200 {
 
@@ -171,6 +172,7 @@ template <bool X_F16, bool OUT_U8, typename IDX>
 __global__ void __launch_bounds__(kThreads)
 quantize_vec_kernel(const QuantView v, const IDX groups, const FastDiv per_row, const FastDiv by_rows)
 {
+    previous_kernel_done();
     constexpr int VEC = X_F16 ? 8 : 4;
     const IDX stride = static_cast<IDX>(gridDim.x) * kThreads;
     for (IDX base = static_cast<IDX>(blockIdx.x) * kThreads + threadIdx.x; base < groups; base += stride * kUnroll) {
@@ -216,6 +218,7 @@ quantize_vec_kernel(const QuantView v, const IDX groups, const FastDiv per_row, 
 template <bool X_F16, bool OUT_U8>
 __global__ void __launch_bounds__(kThreads) quantize_cols_kernel(const QuantView v)
 {
+    previous_kernel_done();
     constexpr int VEC = X_F16 ? 8 : 4;
     const int64_t groups = v.rows / VEC;
     const int64_t g = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -275,6 +278,7 @@ __global__ void __launch_bounds__(kThreads) quantize_cols_kernel(const QuantView
 template <bool IN_U8, bool Y_F16>
 __global__ void __launch_bounds__(kThreads) dequantize_cols_kernel(const QuantView v)
 {
+    previous_kernel_done();
     constexpr int VEC = Y_F16 ? 8 : 4;
     const int64_t groups = v.rows / VEC;
     const int64_t g = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -331,6 +335,7 @@ template <bool IN_U8, bool Y_F16, typename IDX>
 __global__ void __launch_bounds__(kThreads)
 dequantize_vec_kernel(const QuantView v, const IDX groups, const FastDiv per_row, const FastDiv by_rows)
 {
+    previous_kernel_done();
     constexpr int VEC = Y_F16 ? 8 : 4;
     const IDX stride = static_cast<IDX>(gridDim.x) * kThreads;
     const int64_t body = v.inner - v.inner % 16;
@@ -385,6 +390,7 @@ dequantize_vec_kernel(const QuantView v, const IDX groups, const FastDiv per_row
 template <bool X_F16, bool OUT_U8>
 __global__ void __launch_bounds__(kThreads) quantize_scalar_kernel(const QuantView v, const int64_t numel)
 {
+    previous_kernel_done();
     const int64_t stride = static_cast<int64_t>(gridDim.x) * kThreads;
     for (int64_t e = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x; e < numel; e += stride) {
         const int64_t row = e / v.inner;
@@ -397,6 +403,7 @@ __global__ void __launch_bounds__(kThreads) quantize_scalar_kernel(const QuantVi
 template <bool IN_U8, bool Y_F16>
 __global__ void __launch_bounds__(kThreads) dequantize_scalar_kernel(const QuantView v, const int64_t numel)
 {
+    previous_kernel_done();
     const int64_t stride = static_cast<int64_t>(gridDim.x) * kThreads;
     const int64_t body = v.inner - v.inner % 16;
     for (int64_t e = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x; e < numel; e += stride) {
@@ -466,24 +473,25 @@ int run_quantize(const QuantView& v, int64_t numel, bool aligned, const DeviceIn
     if (aligned && cols_form(v, VEC)) {
         dim3 grid, block;
         cols_shape(v, VEC, dev, grid, block);
-        quantize_cols_kernel<X_F16, OUT_U8><<<grid, block, 0, stream>>>(v);
+        const cudaError_t launched = launch_overlapping(quantize_cols_kernel<X_F16, OUT_U8>, grid, block, 0, stream, 1, v);
         note_launch();
-        return cuda_status(cudaGetLastError());
+        return cuda_status(launched);
     }
     const int64_t groups = numel / VEC;
     FastDiv per_row, by_rows;
     make_divisors(v, VEC, groups, per_row, by_rows);
+    cudaError_t launched;
     if (!vec_ok) {
-        quantize_scalar_kernel<X_F16, OUT_U8><<<grid_for(numel, dev), kThreads, 0, stream>>>(v, numel);
+        launched = launch_overlapping(quantize_scalar_kernel<X_F16, OUT_U8>, dim3(grid_for(numel, dev)), dim3(kThreads), 0, stream, 1, v, numel);
     } else if (groups <= 0x7FFFFFFF) {
-        quantize_vec_kernel<X_F16, OUT_U8, uint32_t>
-            <<<grid_for(groups, dev), kThreads, 0, stream>>>(v, static_cast<uint32_t>(groups), per_row, by_rows);
+        launched = launch_overlapping(quantize_vec_kernel<X_F16, OUT_U8, uint32_t>, dim3(grid_for(groups, dev)), dim3(kThreads), 0, stream, 1, v,
+                                      static_cast<uint32_t>(groups), per_row, by_rows);
     } else {
-        quantize_vec_kernel<X_F16, OUT_U8, uint64_t>
-            <<<grid_for(groups, dev), kThreads, 0, stream>>>(v, static_cast<uint64_t>(groups), per_row, by_rows);
+        launched = launch_overlapping(quantize_vec_kernel<X_F16, OUT_U8, uint64_t>, dim3(grid_for(groups, dev)), dim3(kThreads), 0, stream, 1, v,
+                                      static_cast<uint64_t>(groups), per_row, by_rows);
     }
     note_launch();
-    return cuda_status(cudaGetLastError());
+    return cuda_status(launched);
 }
 
 template <bool IN_U8, bool Y_F16>
@@ -494,24 +502,25 @@ int run_dequantize(const QuantView& v, int64_t numel, bool aligned, const Device
     if (aligned && cols_form(v, VEC)) {
         dim3 grid, block;
         cols_shape(v, VEC, dev, grid, block);
-        dequantize_cols_kernel<IN_U8, Y_F16><<<grid, block, 0, stream>>>(v);
+        const cudaError_t launched = launch_overlapping(dequantize_cols_kernel<IN_U8, Y_F16>, grid, block, 0, stream, 1, v);
         note_launch();
-        return cuda_status(cudaGetLastError());
+        return cuda_status(launched);
     }
     const int64_t groups = numel / VEC;
     FastDiv per_row, by_rows;
     make_divisors(v, VEC, groups, per_row, by_rows);
+    cudaError_t launched;
     if (!vec_ok) {
-        dequantize_scalar_kernel<IN_U8, Y_F16><<<grid_for(numel, dev), kThreads, 0, stream>>>(v, numel);
+        launched = launch_overlapping(dequantize_scalar_kernel<IN_U8, Y_F16>, dim3(grid_for(numel, dev)), dim3(kThreads), 0, stream, 1, v, numel);
     } else if (groups <= 0x7FFFFFFF) {
-        dequantize_vec_kernel<IN_U8, Y_F16, uint32_t>
-            <<<grid_for(groups, dev), kThreads, 0, stream>>>(v, static_cast<uint32_t>(groups), per_row, by_rows);
+        launched = launch_overlapping(dequantize_vec_kernel<IN_U8, Y_F16, uint32_t>, dim3(grid_for(groups, dev)), dim3(kThreads), 0, stream, 1, v,
+                                      static_cast<uint32_t>(groups), per_row, by_rows);
     } else {
-        dequantize_vec_kernel<IN_U8, Y_F16, uint64_t>
-            <<<grid_for(groups, dev), kThreads, 0, stream>>>(v, static_cast<uint64_t>(groups), per_row, by_rows);
+        launched = launch_overlapping(dequantize_vec_kernel<IN_U8, Y_F16, uint64_t>, dim3(grid_for(groups, dev)), dim3(kThreads), 0, stream, 1, v,
+                                      static_cast<uint64_t>(groups), per_row, by_rows);
     }
     note_launch();
-    return cuda_status(cudaGetLastError());
+    return cuda_status(launched);
 }
 
 QuantView view_of(const nnb200_quant_linear_args& q)
