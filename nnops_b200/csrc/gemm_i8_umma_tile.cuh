@@ -944,6 +944,7 @@ gemm_i8_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 return ep_all;
             }
         };
+        int staged_base = 0;
         int local_tile = 0;
         for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++local_tile) {
             if (Cfg::kGroups > 1 && (local_tile & 1) != group) {
@@ -957,11 +958,15 @@ gemm_i8_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
             // This tile's per-column terms: fetched while the previous tile was being drained
             // (kPrefetch), or now, hidden behind the tile's main loop.
+            // Tiles that follow one another in a CTA mostly share their columns: then the terms are there already, and
+            // no round trip to the L2 stands between two tiles (1x1 convolution 256 -> 1024 71.8 -> 62.8 us).
+            const bool stage_terms = BATCH || n_base != staged_base || local_tile < Cfg::kGroups;
+            staged_base = n_base;
             __syncwarp();  // previous tile's reads of the staging are done
 #pragma unroll
             for (int i = 0; i < kTermIters; ++i) {
                 const int j = lane + i * 32;
-                if (j < ncols) {
+                if (stage_terms && j < ncols) {
                     const ColTerms ct = finish_col_terms<KIND>(
                         ep, (kPrefetch && local_tile > 0) ? next_terms[kPrefetch ? i : 0] : load_col_terms<KIND>(ep, n_base + j, n_total),
                         fold_scale, folded_row_k, fold_comp);
