@@ -1,4 +1,4 @@
-// int8 GEMM for a handful of activation rows (9 <= M <= 128: batched decode, short prefills).
+// int8 GEMM for a handful of activation rows (up to 128: decode, batched decode, short prefills).
 //
 // With so few rows the whole cost is streaming W once, and the square-tile engine
 // (gemm_i8_umma.cu) is a poor fit: it pads the activations to a 128-row MMA operand, re-reads
@@ -850,16 +850,16 @@ int launch_skinny_variant(const I8Problem& p, const I8Epilogue& ep, const Device
     // Whole tiles over several waves: as many waves as 128-channel tiles need, cut into equal tiles (24
     // rows, 128-channel tiles / equal ones: N = 28672, K = 8192 51.8 / 45.4 us, N = 19456, K = 4096 28.1 / 24.8).
     // A caller that brings the scratch for shared K gets that on the first of the two: 45.7.
-    // A single wave keeps 128 channels: more CTAs load the activations more often, which eats what the
-    // even weight stream gives (64 and 128 rows lost 3 and 8 % at N = 11008, K = 4096, 24 rows won 2).  Shared
-    // K evens the SMs out itself, and its scratch is laid out for 128.
+    // A single wave of whole tiles is cut likewise up to 32 rows (N = 11008, K = 4096: 16 rows 10.7 / 9.7, 24 rows
+    // 10.3 / 10.0); with more, the activations that more CTAs load eat what the even weight stream gives (64 and
+    // 128 rows lost 3 and 8 %).  Shared K evens the SMs out itself, and its scratch is laid out for 128.
     int tile_rows = kBlockN;
     int parts = split_scratch != nullptr && knob(NNB200_KNOB_I8_SHARE_K) == 2 ? 1 : cluster_parts(p, dev);
     while (parts > 1 && resident[dev.device][parts] < (n + kBlockN - 1) / kBlockN) {
         --parts;
     }
     const int waves = ((n + kBlockN - 1) / kBlockN + dev.sm_count - 1) / dev.sm_count;
-    if (split_scratch == nullptr && waves > 1) {
+    if (split_scratch == nullptr && parts == 1 && (waves > 1 || p.m <= 32)) {
         tile_rows = (n + waves * dev.sm_count - 1) / (waves * dev.sm_count);
     }
     CUtensorMap map_w, map_a;
@@ -926,17 +926,23 @@ bool skinny_i8_supported(const I8Problem& p)
 //     32   K = 512 4.2 / 4.5, 4096 5.1 / 8.6       512 4.4 / 5.1, 4096 7.2 / 9.6       4096 9.8 / 10.5, 8192 14.4 / 16.8
 //     64   512 4.9 / 4.6, 2048 5.4 / 6.2           512 5.0 / 4.8, 4096 8.1 / 9.5       2048 8.4 / 7.8, 8192 15.4 / 16.7
 //    128   2048 6.7 / 6.4, 4096 7.2 / 8.8          2048 8.1 / 7.3, 4096 9.5 / 9.9      4096 13.2 / 10.6
-// and here / streaming engine at 16 rows:
-//          2048 4.2 / 3.8, 4096 4.9 / 5.6          2048 5.5 / 5.1, 4096 6.9 / 7.7      512 4.1 / 5.8, 4096 9.4 / 14.4
-//   N = 64: K = 4096 4.9 / 4.7, 8192 5.1 / 6.3.
+// and here / streaming engine:
+//     16   2048 3.6 / 3.4, 4096 4.1 / 5.1          2048 4.5 / 4.7, 4096 5.8 / 7.3      512 3.3 / 5.4, 2048 5.7 / 8.2
+//      4   2048 3.4 / 3.0, 4096 3.7 / 4.0          2048 4.5 / 4.3, 4096 5.8 / 5.9      512 3.5 / 5.2, 8192 12.9 / 16.8
+//      1   2048 3.4 / 2.5, 8192 4.5 / 6.4          4096 5.6 / 5.4, 16384 12.6 / 14.2   512 3.4 / 4.1, 2048 5.6 / 6.7
+//   N = 64, 8192: 16 rows 4.2 / 5.7, 4 rows 3.9 / 4.3, one 3.5 / 3.8; N = 6144, 4096: 16 rows 7.4 / 8.1, 4 rows 7.7 / 6.8;
+//   N = 28672, 8192: 16 rows 40.0 / 56.8, one 38.0 / 40.9; 28672, 1024: one 7.7 / 12.3.  The one place past 6272
+//   channels where one row is better off there: too many tiles for clusters and too few for the SMs, with a
+//   long K (N = 11008: K = 1024 4.8 / 5.9, 4096 11.3 / 10.4; N = 14336, 4096 12.3 / 13.6).
 bool skinny_i8_preferred(const I8Problem& p, bool over_streaming, const DeviceInfo& dev)
 {
-    if (!skinny_i8_supported(p) || p.m < 9) {
+    if (!skinny_i8_supported(p)) {
         return false;
     }
     const int64_t tiles = (p.n + kBlockN - 1) / kBlockN;
     if (over_streaming) {
-        return tiles * 3 > dev.sm_count || p.k >= 8192 || (p.n >= 1024 && p.k >= 4096);
+        const bool sparse = p.m == 1 && p.k > 2048 && tiles * 2 > dev.sm_count && tiles * 4 <= dev.sm_count * 3;
+        return (tiles * 3 > dev.sm_count && !sparse) || p.k >= 8192 || (p.m > 8 && p.n >= 1024 && p.k >= 4096);
     }
     if (p.m <= 32) {
         return true;

@@ -46,9 +46,10 @@ def test_clusters_share_k(cuda_device, nnb200_lib, m, shape):
 
 
 @pytest.mark.parametrize("shape", [(9, 8192, 512), (16, 1024, 4096), (16, 96, 8192), (24, 4096, 1024), (32, 64, 512), (64, 4096, 2048),
-                                   (64, 9472, 8192), (128, 2048, 4096), (128, 4736, 4096)])
+                                   (64, 9472, 8192), (128, 2048, 4096), (128, 4736, 4096),
+                                   (1, 6400, 512), (1, 64, 8192), (1, 11008, 2048), (4, 11008, 2112), (8, 19000, 512)])
 def test_calls_routed_to_clusters(cuda_device, nnb200_lib, shape):
-    """The smallest K of each row of the rule, and a call with only the minimum workspace."""
+    """The smallest K of each row of the rule, one row to a handful, and a call with only the minimum workspace."""
     m, n, k = shape
     _case(cuda_device, m, n, k, "f16", engine="auto", seed=m + k)
     a = torch.randint(-127, 128, (m, k), dtype=torch.int8, device=cuda_device)
