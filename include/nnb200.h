@@ -352,8 +352,10 @@ typedef struct nnb200_q4_1_args {
 /* The launch may begin while the preceding kernel of the stream is still finishing
  * (programmatic dependent launch): its weight fetch overlaps that kernel's tail; activations
  * are read and outputs written only after that kernel has completed.  Only set this when
- * the preceding kernel does not write w_blocks.  Honoured by the GEMV engines 4 and 6 and by
- * engine 7 (f32 rows: its own pass over the activations still starts behind that kernel). */
+ * the preceding kernel does not write w_blocks; what came before that one has completed by
+ * then, as no kernel of this library lets its successor start before its own predecessor
+ * has.  Honoured by the GEMV engines 4 and 6 and by engine 7 (f32 rows: its own pass over the
+ * activations still starts behind that kernel). */
 #define NNB200_Q4_FLAG_OVERLAP_PREVIOUS 1
 
 /* Optional device scratch (16-byte aligned).  Non-zero for tall problems (f16 activations: m >= 256;

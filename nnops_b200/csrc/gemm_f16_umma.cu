@@ -293,6 +293,7 @@ gemm_f16_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             __syncwarp();
             tmem_alloc(tmem_slot, Cfg::kTmemCols);
             tmem_relinquish();
+            named_barrier_arrive(2, 64);   // the producer, before it lets the next kernel start
         } else {
             previous_kernel_done();
         }
@@ -329,6 +330,7 @@ gemm_f16_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 }
             }
         }
+        named_barrier_sync(2, 64);   // tensor memory is allocated
         let_next_kernel_start();
         if (wait_failed(spent) && lane == 0) {
             atomicCAS(error_word, 0, kErrProducerWait);

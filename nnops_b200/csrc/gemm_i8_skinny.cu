@@ -437,6 +437,7 @@ gemm_i8_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     } else if (warp == 1) {
         tmem_alloc(tmem_slot, Cfg::kTmemCols);
         tmem_relinquish();
+        named_barrier_arrive(2, 64);   // the producer, before it lets the next kernel start
     }
     // Per-row epilogue terms of every activation row, once per CTA (the rows are the same for all tiles).
     else {
@@ -474,6 +475,7 @@ gemm_i8_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 }
             }
         }
+        named_barrier_sync(2, 64);   // tensor memory is allocated
         let_next_kernel_start();
         if (wait_failed(spent) && lane == 0) {
             atomicCAS(error_word, 0, kErrProducerWait);

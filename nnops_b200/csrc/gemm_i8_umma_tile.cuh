@@ -726,6 +726,7 @@ gemm_i8_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             __syncwarp();
             tmem_alloc(tmem_slot, Cfg::kTmemCols);
             tmem_relinquish();
+            named_barrier_arrive(2, 64);   // the producer, before it lets the next kernel start
         } else {
             previous_kernel_done();
         }
@@ -831,6 +832,7 @@ gemm_i8_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 }
             }
         }
+        named_barrier_sync(2, 64);   // tensor memory is allocated
         let_next_kernel_start();
         if (wait_failed(spent) && lane == 0) {
             atomicCAS(error_word, 0, kErrProducerWait);

@@ -216,8 +216,9 @@ inline int cuda_status(cudaError_t e)
 // touches global memory, reads included: scratch and outputs may be memory the previous kernel still uses, and a
 // kernel that ended without having waited would let its successor overtake its predecessor.  What comes
 // before it -- barriers, tensor memory, descriptors -- and the launch itself cost 2 to 4 us a call otherwise.
-// A kernel lets the next one start only near its end (or, where its blocks come in several turns, by ending): the
-// blocks of at most one kernel then wait for another, and that one has all of its own running.
+// A kernel lets the next one start only after its own wait and its block's last load (or, where its blocks come in
+// several turns, by ending), flagged Q4_1 products included: the blocks of at most one kernel then wait for
+// another, and that one has all of its own running.
 template <class... P, class... A>
 inline cudaError_t launch_overlapping(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster,
                                       A&&... args)

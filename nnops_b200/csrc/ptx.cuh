@@ -43,16 +43,19 @@ __device__ __forceinline__ bool elect_one()
 
 // ---- programmatic dependent launch (see launch_overlapping) --------------------------------
 
-// Once every block has said so or ended, the next kernel's blocks may take what room there is.
-__device__ __forceinline__ void let_next_kernel_start()
-{
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 // Returns when the previous kernel has completed and its writes are visible; at once without the launch attribute.
 __device__ __forceinline__ void previous_kernel_done()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// Once every block has said so or ended, the next kernel's blocks may take what room there is.  Never before this
+// kernel's own wait, which is therefore part of it: with kernels that let their successor in while they waited
+// themselves, a stream had three kernels in flight, two of them holding shared and tensor memory for a third.
+// Nor before the block's tensor memory is allocated, which the successor's block could otherwise take first.
+__device__ __forceinline__ void let_next_kernel_start()
+{
+    asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // A value that is the same in every lane of a converged warp, known as such to the compiler.

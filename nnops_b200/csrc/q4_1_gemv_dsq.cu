@@ -394,10 +394,6 @@ q4_1_gemv_dsq_kernel(const uint8_t* __restrict__ w, const int64_t w_pitch_bytes,
         mbar_init_fence();
     }
     __syncthreads();
-    // The next kernel in the stream may start its own prologue (and its weight stream) now.
-    if (early) {
-        let_next_kernel_start();
-    }
 
     if (warp == kProducerWarp) {
         // ---- producer: where the caller says that no kernel before this one writes the weights (early), it
@@ -439,6 +435,11 @@ q4_1_gemv_dsq_kernel(const uint8_t* __restrict__ w, const int64_t w_pitch_bytes,
                     empty_parity ^= 1u;
                 }
             }
+        }
+        // Every load is on its way: the next kernel in the stream may start its own prologue (and, where its caller
+        // allows that, its weight stream).
+        if (early) {
+            let_next_kernel_start();
         }
         // No copy may still be in flight when the CTA retires: wait (without consuming) for the
         // latest phase of every slot that was ever filled.

@@ -246,17 +246,19 @@ q4_1_gemv_mma_kernel(const uint8_t* __restrict__ w, const int64_t w_pitch_bytes,
     }
     __syncwarp();
     // Start streaming the weights: right away where the caller says that no kernel before this one writes them
-    // (early; the next kernel in the stream may then begin its own prologue too), else once the previous one
-    // has completed, as with activations and outputs.
-    if (early) {
-        let_next_kernel_start();
-    } else {
+    // (early), else once the previous one has completed, as with activations and outputs.
+    if (!early) {
         previous_kernel_done();
     }
     for (int b = 0; b < num_bufs && b < num_chunks; ++b) {
         issue_slice(b, b);
     }
     previous_kernel_done();
+    // The next kernel in the stream may begin its own prologue once every load is on its way.  The blocks come in
+    // turns on a tall layer: those of the last one have the say.
+    if (early && num_chunks <= num_bufs) {
+        let_next_kernel_start();
+    }
     __syncthreads();  // abort_word initialised for every warp
 
     float acc0[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -324,6 +326,9 @@ q4_1_gemv_mma_kernel(const uint8_t* __restrict__ w, const int64_t w_pitch_bytes,
         if (ch + num_bufs < num_chunks) {
             __syncwarp();  // every lane has finished reading this buffer
             issue_slice(ch + num_bufs, buf);
+            if (early && ch + num_bufs == num_chunks - 1) {
+                let_next_kernel_start();
+            }
         }
     }
 

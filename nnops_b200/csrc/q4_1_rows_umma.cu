@@ -285,9 +285,6 @@ q4_1_rows_umma_kernel(const __grid_constant__ CUtensorMap map_a, const uint8_t* 
         tmem_alloc(tmem_slot, kTmemCols);
         tmem_relinquish();
     }
-    if (early) {
-        let_next_kernel_start();
-    }
     previous_kernel_done();
     tc_fence_before_sync();
     __syncthreads();

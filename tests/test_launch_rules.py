@@ -1,0 +1,46 @@
+"""What every kernel that overlaps its neighbours in the stream keeps to, read from the sources: such a mistake is a
+hang or a stale read on the GPU now and then, which no run on one can be trusted to show."""
+import re
+from pathlib import Path
+
+CSRC = Path(__file__).resolve().parent.parent / "nnops_b200" / "csrc"
+
+
+def _code(path):
+    """The file without its comments."""
+    return re.sub(r"/\*.*?\*/", "", re.sub(r"//[^\n]*", "", path.read_text()), flags=re.S)
+
+
+def _sources():
+    return {p.name: _code(p) for p in sorted(CSRC.glob("*.cu*"))}
+
+
+def _body(text, at):
+    """The braced block that opens at or after ``at``."""
+    start = at = text.index("{", at)
+    depth = 0
+    while True:
+        depth += {"{": 1, "}": -1}.get(text[at], 0)
+        at += 1
+        if depth == 0:
+            return text[start:at]
+
+
+def test_no_kernel_lets_its_successor_start_before_its_own_wait():
+    """Or three kernels are in flight, two of them holding what they have while they wait."""
+    for name, text in _sources().items():
+        assert ("griddepcontrol" in text) == (name == "ptx.cuh"), name
+    ptx = _sources()["ptx.cuh"]
+    assert ptx.count("griddepcontrol.launch_dependents") == 1
+    body = _body(ptx, ptx.index("void let_next_kernel_start("))
+    assert body.index("griddepcontrol.wait;") < body.index("griddepcontrol.launch_dependents;")
+
+
+def test_tensor_memory_is_allocated_before_the_successor_may_start():
+    """A producer warp that has not met the allocating warp does so first."""
+    for name, text in _sources().items():
+        for at in (m.start() for m in re.finditer(r"named_barrier_arrive\(1, ", text)):
+            kernel_end = text.find("__global__", at)
+            kernel = text[at:kernel_end if kernel_end > 0 else len(text)]
+            assert kernel.index("tmem_alloc(") < kernel.index("named_barrier_arrive(2, 64)"), name
+            assert kernel.index("named_barrier_sync(2, 64)") < kernel.index("let_next_kernel_start()"), name
