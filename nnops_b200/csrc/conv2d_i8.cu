@@ -134,8 +134,8 @@ __global__ void __launch_bounds__(256) conv_gather_i8_kernel(const GatherParams 
                 v = make_uint4(pad4, pad4, pad4, pad4);
                 if (static_cast<uint32_t>(ih) < static_cast<uint32_t>(p.ih) &&
                     static_cast<uint32_t>(iw) < static_cast<uint32_t>(p.iw)) {
-                    v = __ldg(reinterpret_cast<const uint4*>(base + static_cast<int64_t>(ih) * p.in_h +
-                                                             static_cast<int64_t>(iw) * p.in_w + tap_c[c]));
+                    v = *reinterpret_cast<const uint4*>(base + static_cast<int64_t>(ih) * p.in_h +
+                                                        static_cast<int64_t>(iw) * p.in_w + tap_c[c]);
                 }
             } else {
                 uint32_t w[4] = {0u, 0u, 0u, 0u};

@@ -87,8 +87,8 @@ __device__ __forceinline__ TileCoord tile_coord(int tile, int num_m, int num_n, 
 // flight before it decodes either.
 // dm_plane != nullptr: the weights are packed (nnb200_q4_1_pack) -- `w` is then the nibble plane,
 // 16 bytes per block, and dm_plane the (d, m) plane with rows ld_dm entries apart.
-__global__ void __launch_bounds__(256) q4_1_expand_f16_kernel(const uint8_t* __restrict__ w, const int64_t ldw_blocks,
-                                                              const uint32_t* __restrict__ dm_plane, const int64_t ld_dm,
+__global__ void __launch_bounds__(256) q4_1_expand_f16_kernel(const uint8_t* w, const int64_t ldw_blocks,
+                                                              const uint32_t* dm_plane, const int64_t ld_dm,
                                                               const int rows, const int nblk,
                                                               __half* __restrict__ out, const int64_t ld_out)
 {
@@ -108,14 +108,14 @@ __global__ void __launch_bounds__(256) q4_1_expand_f16_kernel(const uint8_t* __r
                 if (r < rows) {
                     if (planes) {
                         const uint32_t* src = reinterpret_cast<const uint32_t*>(w + r * pitch + b * 16);
-                        dm[u] = __ldg(dm_plane + r * ld_dm + b);
-                        q0[u] = __ldg(src + 2 * h);
-                        q1[u] = __ldg(src + 1 + 2 * h);
+                        dm[u] = dm_plane[r * ld_dm + b];
+                        q0[u] = src[2 * h];
+                        q1[u] = src[1 + 2 * h];
                     } else {
                         const uint32_t* src = reinterpret_cast<const uint32_t*>(w + r * pitch + b * kQ4BlockBytes);
-                        dm[u] = __ldg(src);
-                        q0[u] = __ldg(src + 1 + 2 * h);
-                        q1[u] = __ldg(src + 2 + 2 * h);
+                        dm[u] = src[0];
+                        q0[u] = src[1 + 2 * h];
+                        q1[u] = src[2 + 2 * h];
                     }
                 }
             }
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(256) q4_1_expand_f16_kernel(const uint8_t* __r
 // GEMM over [hi | lo] (weights repeating along K) reproduces an f32-activation product to f32
 // accuracy.  Row m of `out` is [hi(0..kp) | lo(0..kp)], kp = K rounded up to 64, zeros past K.
 // Values beyond the f16 range (|a| > 65504) become infinities, as in any f16 activation pipeline.
-__global__ void __launch_bounds__(256) split_f32_to_f16_kernel(const float* __restrict__ a, const int64_t lda,
+__global__ void __launch_bounds__(256) split_f32_to_f16_kernel(const float* a, const int64_t lda,
                                                                const int m, const int k, const int kp,
                                                                __half* __restrict__ out)
 {
@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(256) split_f32_to_f16_kernel(const float* __re
         const int c = static_cast<int>(i - r * kp);
         float v = 0.0f;
         if (c < k) {
-            v = a[r * lda + c];
+            v = __ldcg(a + r * lda + c);   // the loads of several turns stay together
         }
         const __half hi = __float2half_rn(v);
         const __half lo = __float2half_rn(v - __half2float(hi));

@@ -41,7 +41,7 @@ constexpr int kUnroll = 4;   // steps whose loads are in flight together
 __device__ __forceinline__ uint4 ld_stream_16(const void* p)
 {
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                  : "l"(p));
     return v;
@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(kWarps * 32, 3) gemm_i8_decode_kernel(const I8
         for (int u = 0; u < kUnroll; ++u) {
 #pragma unroll
             for (int t = 0; t < M_TILES; ++t) {
-                const uint4 av = __ldg(reinterpret_cast<const uint4*>(a_row[t] + static_cast<int64_t>(s + u) * kChunk));
+                const uint4 av = *reinterpret_cast<const uint4*>(a_row[t] + static_cast<int64_t>(s + u) * kChunk);
                 mma_m16n8k32<A_UNSIGNED>(acc[t], lo[u].x, hi[u].x, lo[u].y, hi[u].y, av.x, av.y);
                 mma_m16n8k32<A_UNSIGNED>(acc[t], lo[u].z, hi[u].z, lo[u].w, hi[u].w, av.z, av.w);
             }
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(kWarps * 32, 3) gemm_i8_decode_kernel(const I8
         const uint4 hi = ld_stream_16(w_hi + static_cast<int64_t>(s) * kChunk);
 #pragma unroll
         for (int t = 0; t < M_TILES; ++t) {
-            const uint4 av = __ldg(reinterpret_cast<const uint4*>(a_row[t] + static_cast<int64_t>(s) * kChunk));
+            const uint4 av = *reinterpret_cast<const uint4*>(a_row[t] + static_cast<int64_t>(s) * kChunk);
             mma_m16n8k32<A_UNSIGNED>(acc[t], lo.x, hi.x, lo.y, hi.y, av.x, av.y);
             mma_m16n8k32<A_UNSIGNED>(acc[t], lo.z, hi.z, lo.w, hi.w, av.z, av.w);
         }

@@ -136,7 +136,7 @@ __device__ __forceinline__ void conv_border_fix(const ConvTile& conv, uint32_t (
     if (n0 + 32 <= n_total && (reinterpret_cast<uintptr_t>(tb) & 15u) == 0) {
 #pragma unroll
         for (int j = 0; j < 32; j += 4) {
-            const int4 t4 = __ldg(reinterpret_cast<const int4*>(tb + j));
+            const int4 t4 = *reinterpret_cast<const int4*>(tb + j);
             v[j] += static_cast<uint32_t>(conv.zp_x) * static_cast<uint32_t>(t4.x);
             v[j + 1] += static_cast<uint32_t>(conv.zp_x) * static_cast<uint32_t>(t4.y);
             v[j + 2] += static_cast<uint32_t>(conv.zp_x) * static_cast<uint32_t>(t4.z);

@@ -28,7 +28,7 @@ constexpr int kWarps = 8;
 __device__ __forceinline__ uint32_t load_word(const uint8_t* row, int64_t at, int64_t cols)
 {
     if (at >= 0 && at + 4 <= cols) {
-        return __ldg(reinterpret_cast<const uint32_t*>(row + at));
+        return *reinterpret_cast<const uint32_t*>(row + at);
     }
     uint32_t v = 0;
 #pragma unroll

@@ -214,7 +214,9 @@ inline int cuda_status(cudaError_t e)
 // A launch whose blocks may become resident while the previous kernel of the stream is still running
 // (programmatic stream serialization).  EVERY block of such a kernel executes previous_kernel_done() before it
 // touches global memory, reads included: scratch and outputs may be memory the previous kernel still uses, and a
-// kernel that ended without having waited would let its successor overtake its predecessor.  What comes
+// kernel that ended without having waited would let its successor overtake its predecessor.  And it reads with
+// coherent loads (no __ldg, no const __restrict__ that lets the compiler choose one): the non-coherent path is for
+// memory that nobody writes while the kernel is there, and the previous kernel does, before the wait.  What comes
 // before it -- barriers, tensor memory, descriptors -- and the launch itself cost 2 to 4 us a call otherwise.
 // A kernel lets the next one start only after its own wait and its block's last load (or, where its blocks come in
 // several turns, by ending), flagged Q4_1 products included: the blocks of at most one kernel then wait for

@@ -82,7 +82,7 @@ __device__ __forceinline__ TileCoord tile_coord(int tile, int num_m, int num_n)
 
 template <bool OUT_F16, bool COOP, int MH>
 __global__ void __launch_bounds__(Q4Config<COOP, MH>::kNumThreads, 1)
-q4_1_gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const uint8_t* __restrict__ w,
+q4_1_gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const uint8_t* w,
                       const int64_t ldw_blocks, void* __restrict__ out, const int64_t ldc, const int m_total,
                       const int n_total, const int k_total, const FpEpilogue ep, const uint32_t idesc,
                       const int vec_ok, int32_t* error_word)
@@ -386,7 +386,7 @@ q4_1_gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const uint8_t* 
                 const uint32_t* src = reinterpret_cast<const uint32_t*>(w + n * pitch + static_cast<int64_t>(b) * kQ4BlockBytes);
 #pragma unroll
                 for (int i = 0; i < 5; ++i) {
-                    next[i] = __ldg(src + i);
+                    next[i] = src[i];
                 }
             } else {
 #pragma unroll

@@ -349,8 +349,8 @@ __device__ __forceinline__ void dsq_group(uint32_t wlo, uint32_t whi, uint32_t d
 // plane with rows dm_pitch_bytes apart; otherwise `w` is the raw 20-byte-block stream.
 template <int MP, bool OUT_F16, bool A_F32, int NC, bool PACKED>
 __global__ void __launch_bounds__((NC + 2) * 32, NC == 8 ? 2 : 1)
-q4_1_gemv_dsq_kernel(const uint8_t* __restrict__ w, const int64_t w_pitch_bytes, const uint8_t* __restrict__ w_dm,
-                     const int64_t dm_pitch_bytes, const void* __restrict__ a_v,
+q4_1_gemv_dsq_kernel(const uint8_t* w, const int64_t w_pitch_bytes, const uint8_t* w_dm,
+                     const int64_t dm_pitch_bytes, const void* a_v,
                      const int64_t lda, void* __restrict__ out, const int64_t ldc, const int m_count,
                      const int n_total, const int k_total, const DsqLayout lay, const FpEpilogue ep,
                      const int a_vec_ok, int32_t* error_word, const int early)

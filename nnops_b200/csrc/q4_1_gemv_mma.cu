@@ -184,7 +184,7 @@ __device__ __forceinline__ void mma_block(const uint32_t* s_lo, const uint32_t* 
 // m_count..2*m_count-1 their lo parts (so m_count <= 4), summed in the final reduction.
 template <bool OUT_F16, bool A_F32>
 __global__ void __launch_bounds__(kWarps * 32, 2)
-q4_1_gemv_mma_kernel(const uint8_t* __restrict__ w, const int64_t w_pitch_bytes, const void* __restrict__ a_v,
+q4_1_gemv_mma_kernel(const uint8_t* w, const int64_t w_pitch_bytes, const void* a_v,
                      const int64_t lda, void* __restrict__ out, const int64_t ldc, const int m_count,
                      const int n_total, const int k_total, const int num_bufs, const FpEpilogue ep,
                      const int a_vec_ok, int32_t* error_word, const int early)

@@ -177,7 +177,7 @@ __device__ __forceinline__ void decode_block(const uint32_t (&b)[5], uint32_t (&
 // PIECE: bytes of one copy, the most (16, 8 or 4) that the weight rows' alignment allows.
 template <bool OUT_F16, int BLOCKS, int PIECE>
 __global__ void __launch_bounds__(kThreads, 1)
-q4_1_rows_umma_kernel(const __grid_constant__ CUtensorMap map_a, const uint8_t* __restrict__ w,
+q4_1_rows_umma_kernel(const __grid_constant__ CUtensorMap map_a, const uint8_t* w,
                       const int64_t w_pitch_bytes, void* __restrict__ out, const int64_t ldc, const int m_total,
                       const int hi_lo, const int nb, const int n_total, const int k_total, const int tile_rows,
                       const int split, const FpEpilogue ep, const uint32_t idesc, int32_t* error_word, const int early)

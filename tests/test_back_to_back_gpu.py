@@ -51,3 +51,100 @@ def test_flagged_q4_1_calls_among_others(cuda_device, nnb200_lib, m, engines, n)
 
     want = _same_with_and_without_waiting(chain)
     assert all(torch.isfinite(t.float()).all() and t.float().abs().max() > 0 for t in want)
+
+
+def _s8(rng, device, *shape):
+    return torch.from_numpy(rng.integers(-127, 128, shape, dtype=np.int8)).to(device)
+
+
+def _producers(rng, device):
+    """Every kernel that lets its successor start before its epilogue: three inputs each, and a call into ``out``."""
+    def i8(m, n, k, engine):
+        w, sw = _s8(rng, device, n, k), torch.rand(n, device=device) * 0.02 + 0.001
+        xs = [_s8(rng, device, m, k) for _ in range(3)]
+        out = torch.empty((m, n), dtype=torch.int8, device=device)
+        return xs, lambda x: ops.gemm_i8(x, w, out_kind="s8", out=out, out_scale=0.6 * k ** 0.5, scale_w=sw, engine=engine)
+
+    def q4(m, n, k, engine, dtype=torch.float16, **kw):
+        w = torch.from_numpy(synth.q4_1_weights(rng, n, k)).to(device)
+        xs = [torch.from_numpy(rng.standard_normal((m, k)).astype(np.float16)).to(device) for _ in range(3)]
+        out = torch.empty((m, n), dtype=dtype, device=device)
+        return xs, lambda x: ops.linear_q4_1(x, w, k, out=out, alpha=0.05, engine=engine, **kw)
+
+    return {"few rows, clusters": lambda: i8(16, 2048, 1024, "skinny"), "few rows, tiles": lambda: i8(16, 19456, 256, "skinny"),
+            "tile": lambda: i8(200, 2048, 512, "umma"), "pair": lambda: i8(512, 6144, 2048, "umma"),
+            "dense f16": lambda: q4(256, 2048, 512, "gemm_two_pass"), "dense f16, pair": lambda: q4(1024, 6144, 512, "gemm_two_pass"),
+            "rows": lambda: q4(16, 2048, 1024, "rows"), "rows, f32": lambda: q4(16, 2048, 1024, "rows", torch.float32),
+            "rows, flagged": lambda: q4(16, 19456, 256, "rows", overlap_previous=True)}
+
+
+def _consumers(rng, device, x):
+    """Calls that read ``x``, by kernel: as activations, as weights, as an image, as elements."""
+    m, n = x.shape
+    few = min(m, 8)
+    i32 = lambda c: torch.from_numpy(rng.integers(-9, 10, c).astype(np.int32)).to(device)
+    f32 = lambda c: torch.rand(c, device=device) * 0.02 + 0.001
+    if x.dtype == torch.int8:
+        w, a, zp_m, zp_n = _s8(rng, device, 256, n), _s8(rng, device, 8, n), i32(m), i32(256)
+        wide, scales, zeros = _s8(rng, device, 256 * 24, n), f32(m), torch.zeros(m, dtype=torch.int8, device=device)
+        image, planes = x.view(m, n // 256, 8, 32), x.view(m, n // 512, 4, 128)
+        small, large = ops.prepack_conv2d_i8(_s8(rng, device, 3, 3, 32, 48)), ops.prepack_conv2d_i8(_s8(rng, device, 3, 3, 128, 128))
+        calls = {
+            "decode": lambda: ops.gemm_i8(x[:few], w, engine="decode"), "few rows": lambda: ops.gemm_i8(x[:few], w, engine="skinny"),
+            "tile": lambda: ops.gemm_i8(x, w, engine="umma"), "generic": lambda: ops.gemm_i8(x, w[:33], engine="generic"),
+            "narrow": lambda: ops.gemm_i8(x[:few], w, engine="narrow"),
+            "sums": lambda: ops.gemm_i8(x, w, zp_a=zp_m, zp_w=zp_n), "sums, other operands": lambda: ops.gemm_i8(x, w, zp_a=5, zp_w=zp_n),
+            "realign": lambda: ops.gemm_i8(x[:, 3:-2], w[:, 3:-2], zp_w=zp_n),
+            "weights, decode": lambda: ops.gemm_i8(a, x, engine="decode"), "weights, few rows": lambda: ops.gemm_i8(a, x, engine="skinny"),
+            "weights, tile": lambda: ops.gemm_i8(w, x, engine="umma"), "weights, realign": lambda: ops.gemm_i8(a[:, 1:], x[:, 1:], zp_a=3),
+            "batch": lambda: ops.gemm_i8(x.view(4, m // 4, n), x.view(4, m // 4, n)),
+            "gather": lambda: ops.conv2d_i8(image, small, padding=(1, 1), out_kind="f32", zp_x=3),
+            "implicit": lambda: ops.conv2d_i8(planes, large, padding=(1, 1), out_kind="f32", zp_x=3),
+            "dequantize": lambda: ops.dequantize_linear(x, scales, zeros),
+        }
+        if m >= 256:
+            calls["pair"] = lambda: ops.gemm_i8(x, wide, engine="umma")
+        return calls
+    blocks = torch.from_numpy(synth.q4_1_weights(rng, 512, n)).to(device)
+    scales, zeros = f32(m), torch.zeros(m, dtype=torch.int8, device=device)
+    w8 = _s8(rng, device, 256, n)
+    half = x.dtype == torch.float16
+    calls = {
+        "quantize": lambda: ops.quantize_linear(x, scales, zeros), "fp_act": lambda: ops.linear_fp_act(x, w8, scale_a=0.02),
+        "deferred scaling": lambda: ops.linear_q4_1(x[:1], blocks, n, engine="gemv_dsq"),
+        "deferred scaling, early": lambda: ops.linear_q4_1(x[:1], blocks, n, engine="gemv_dsq", overlap_previous=True),
+        "warp MMA": lambda: ops.linear_q4_1(x[:few // 2], blocks, n, engine="gemv_mma"),
+        "warp MMA, early": lambda: ops.linear_q4_1(x[:few // 2], blocks, n, engine="gemv_mma", overlap_previous=True),
+        "CUDA cores": lambda: ops.linear_q4_1(x[:few], blocks, n, engine="gemv_simt"),
+        "rows": lambda: ops.linear_q4_1(x[:16], blocks, n, engine="rows"),
+        "rows, early": lambda: ops.linear_q4_1(x[:16], blocks, n, engine="rows", overlap_previous=True),
+        "two passes": lambda: ops.linear_q4_1(x, blocks, n, engine="gemm_two_pass"),
+    }
+    if half:
+        calls["fused"] = lambda: ops.linear_q4_1(x, blocks, n, engine="gemm")
+    return calls
+
+
+@pytest.mark.parametrize("producer", ["few rows, clusters", "few rows, tiles", "tile", "pair", "dense f16", "dense f16, pair", "rows",
+                                      "rows, f32", "rows, flagged"])
+def test_what_a_kernel_wrote_just_before(cuda_device, nnb200_lib, producer):
+    """Each call reads what the one before has written and the one after writes over it at once, with other values; calls
+    that need scratch get the one the call before them had."""
+    rng = np.random.default_rng(11)
+    torch.manual_seed(3)
+    xs, produce = _producers(rng, cuda_device)[producer]()
+    calls = _consumers(rng, cuda_device, produce(xs[0]))
+
+    def chain(after):
+        seen = []
+        for i, call in enumerate(calls.values()):
+            for step in range(2):
+                produce(xs[(i + step) % 3])
+                after()
+                seen.append(call())
+                after()
+        return seen
+
+    want = _same_with_and_without_waiting(chain)
+    for i in range(0, len(want), 2):   # the two inputs do not give the same, or nothing would show
+        assert not torch.equal(want[i], want[i + 1])

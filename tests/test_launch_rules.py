@@ -44,3 +44,19 @@ def test_tensor_memory_is_allocated_before_the_successor_may_start():
             kernel = text[at:kernel_end if kernel_end > 0 else len(text)]
             assert kernel.index("tmem_alloc(") < kernel.index("named_barrier_arrive(2, 64)"), name
             assert kernel.index("named_barrier_sync(2, 64)") < kernel.index("let_next_kernel_start()"), name
+
+
+def test_what_the_previous_kernel_may_still_write_is_read_coherently():
+    """A kernel that is resident before the previous one has completed must not read through the non-coherent path, nor
+    leave the compiler free to: a const __restrict__ pointer, an intrinsic that may move ahead of the wait."""
+    overlapped = 0
+    for name, text in _sources().items():
+        if name in ("ptx.cuh", "ptx_pair.cuh", "internal.cuh") or "previous_kernel_done()" not in text:
+            continue
+        assert "__ldg(" not in text and "global.nc" not in text, name
+        for at in (m.end() for m in re.finditer(r"__global__", text)):
+            signature = text[at:text.index("{", at)]
+            if "previous_kernel_done()" in _body(text, at):
+                overlapped += 1
+                assert not re.search(r"const [\w:]+\* __restrict__", signature), (name, signature)
+    assert overlapped >= 18
