@@ -558,6 +558,8 @@ gemm_i8_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             const bool n_ok = ch < tile_rows && n < n_total;
             const ChannelTerms ct = channel_terms<KIND>(ep, n, n_ok);
             uint32_t* mine = reinterpret_cast<uint32_t*>(stage_base) + ch;
+            const bool all_ok = __all_sync(0xFFFFFFFFu, n_ok);
+            const uint32_t never = static_cast<uint32_t>(parts) >> 16;   // 0, which the compiler does not know
             int row = 0, row_end = 1, store_end = 0, part = rank, part_step = 0;   // first pass: its own sums only, the others' CTAs may not have begun
 #pragma unroll 1
             for (int pass = 0; pass < 2; ++pass) {
@@ -608,7 +610,14 @@ gemm_i8_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                             v[j] += p < parts ? theirs[p][j] : 0u;
                         }
                     }
-                    finish_rows<KIND, 4>(ep, row_terms, v, r, store_end, n, n_ok, ct);
+                    int end = store_end;
+                    if (r + 4 > row_end || !all_ok) {
+                        // Rows or channels that are not stored: nothing else waits for their loads, and the CTA they come
+                        // from may leave after the barrier below.  Once the warp has met here they have come.
+                        const uint32_t seen = v[0] | v[1] | v[2] | v[3];
+                        end = __any_sync(0xFFFFFFFFu, (seen & never) != 0) ? 0 : store_end;
+                    }
+                    finish_rows<KIND, 4>(ep, row_terms, v, r, end, n, n_ok, ct);
                 }
             }
             __syncwarp();

@@ -60,3 +60,18 @@ def test_what_the_previous_kernel_may_still_write_is_read_coherently():
                 overlapped += 1
                 assert not re.search(r"const [\w:]+\* __restrict__", signature), (name, signature)
     assert overlapped >= 18
+
+
+def test_what_is_read_from_another_cta_has_come_before_it_may_leave():
+    """In the few-row engine's exchange the CTAs part at a barrier that orders no memory, so every load has to be waited
+    for: those of rows and channels that are not stored by a vote on their values."""
+    kernel = _sources()["gemm_i8_skinny.cu"]
+    kernel = kernel[kernel.index("gemm_i8_skinny_kernel(const"):]
+    loads, stores = kernel.index("theirs[p][j] = ld_shared_cluster_u32("), kernel.index("finish_rows<KIND, 4>(")
+    assert kernel.count("ld_shared_cluster_u32(") == 1
+    between = kernel[loads:stores]
+    at = between.index("if (r + 4 > row_end || !all_ok)")
+    vote = _body(between, at)
+    assert "v[0] | v[1] | v[2] | v[3]" in vote and re.search(r"end = __any_sync\(0xFFFFFFFFu, \(seen & never\) != 0\)", vote)
+    assert "all_ok = __all_sync(0xFFFFFFFFu, n_ok)" in kernel[:loads]
+    assert kernel[stores:].index("cluster_sync_all_relaxed()") > 0
