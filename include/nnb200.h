@@ -506,9 +506,11 @@ NNB200_API int nnb200_rank_barrier(int32_t* const* flags_by_rank, int32_t world,
 NNB200_API int nnb200_take_device_error(int32_t* code);
 
 /*
- * Exercises that mechanism without disturbing anything: launches one thread that waits, for
- * at most limit_cycles SM clock cycles (1 .. 2e8), on a barrier nothing arrives at.  The wait
- * runs out, the kernel records NNB200_DEVICE_ERROR_SELFTEST (7) in the error word and returns
+ * Exercises that mechanism without disturbing anything: launches one warp that waits on a
+ * barrier nothing arrives at, in each of the five forms of wait the kernels use, one after the
+ * other: the three that go by the clock for at most limit_cycles SM clock cycles each (1 .. 2e8),
+ * the others for a number of probes and until another role has given up.  All of them having
+ * run out, the kernel records NNB200_DEVICE_ERROR_SELFTEST (7) in the error word and returns
  * normally; the context stays usable.  The next nnb200_take_device_error reports the code.
  */
 #define NNB200_DEVICE_ERROR_SELFTEST 7

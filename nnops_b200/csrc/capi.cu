@@ -13,6 +13,7 @@
 #include "i8_realign.cuh"
 #include "internal.cuh"
 #include "ptx.cuh"
+#include "ptx_pair.cuh"
 #include "q4_1_rows_umma.cuh"
 
 namespace nnb200 {
@@ -295,20 +296,51 @@ size_t out_elem_bytes(int kind)
     return (kind == NNB200_OUT_S32 || kind == NNB200_OUT_F32) ? 4 : (kind == NNB200_OUT_F16 ? 2 : 1);
 }
 
-// Self-test of the bounded pipeline waits: one thread waits on a barrier nothing ever arrives
-// at.  The wait has to run out after `limit_cycles`, raise the CTA's abort flag and record
-// kErrSelfTest in the device's error word; the kernel then returns normally.
+// Self-test of the bounded pipeline waits: one warp waits on a barrier nothing ever arrives at, in every form of
+// wait the kernels use, one after the other.  Those that go by the clock run out after `limit_cycles`; the
+// converged ones after a number of probes, and at once where another role has aborted, keeping the code of the first
+// wait that failed.  All raise the abort flag.  If every one has done so, kErrSelfTest is recorded in the device's error
+// word; the kernel then returns normally.
 __global__ void wait_selftest_kernel(long long limit_cycles, int32_t* error_word)
 {
     __shared__ __align__(8) uint64_t bar;
     __shared__ int abort_flag;
-    if (threadIdx.x == 0) {
-        abort_flag = 0;
+    const bool first = threadIdx.x == 0;
+    bool all = true;
+    const auto lower_flag = [&]() {
+        __syncwarp();
+        if (first) {
+            abort_flag = 0;
+        }
+        __syncwarp();
+    };
+    if (first) {
         mbar_init(&bar, 1);
         mbar_init_fence();
-        if (!mbar_wait(&bar, 0, &abort_flag, limit_cycles)) {
-            atomicCAS(error_word, 0, kErrSelfTest);
-        }
+    }
+    lower_flag();
+    if (first) {
+        all = !mbar_wait(&bar, 0, &abort_flag, limit_cycles) && abort_flag == 1;
+    }
+    lower_flag();
+    if (first) {
+        all = all && !mbar_wait_cluster(&bar, 0, &abort_flag, limit_cycles) && abort_flag == 1;
+    }
+    const auto converged = [&](auto runs_out, auto full_limit) {
+        lower_flag();
+        uint32_t failed = 0, other = 0;
+        runs_out(failed);
+        const bool ran_out = warp_failure(failed) == kErrMmaWait && abort_flag == 1;
+        full_limit(failed);   // this role has failed before
+        full_limit(other);    // the abort flag is up
+        all = all && ran_out && failed == kErrMmaWait && other == kErrAccumWait;
+    };
+    converged([&](uint32_t& f) { mbar_wait_converged<kErrMmaWait, 100>(&bar, 0, &abort_flag, f); },
+              [&](uint32_t& f) { mbar_wait_converged<kErrAccumWait>(&bar, 0, &abort_flag, f); });
+    converged([&](uint32_t& f) { mbar_wait_converged_cluster<kErrMmaWait, 100>(&bar, 0, &abort_flag, f); },
+              [&](uint32_t& f) { mbar_wait_converged_cluster<kErrAccumWait>(&bar, 0, &abort_flag, f); });
+    if (first && all && !drain_ring(&bar, 1, 1, limit_cycles)) {
+        atomicCAS(error_word, 0, kErrSelfTest);
     }
 }
 

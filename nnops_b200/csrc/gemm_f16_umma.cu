@@ -265,7 +265,7 @@ gemm_f16_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     // The producer warp sets the barriers up and starts to load at once; the others meet at a barrier of
     // their own.  In both issuing roles the whole warp walks the loop, one elected lane issues, and no
     // branch depends on what a wait returned (see mbar_wait_converged).
-    uint32_t spent = 0;   // probes of this role's waits
+    uint32_t failed = 0;   // this role's first failed wait, see mbar_wait_converged
     int stage = 0;
     uint32_t phase = 0;
     if (role == 0) {
@@ -305,23 +305,23 @@ gemm_f16_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 
     if (role == 0) {
         // ---------------- TMA producer ----------------
-        uint32_t issued = 0;
+        uint32_t issued = 0;   // by this lane
         for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
             const TileCoord tc = tile_coord(tile, num_m, num_n, group_m);
             const int m0 = warp_uniform(tc.m_blk * kBlockM), n0 = warp_uniform(tc.n_blk * BN);
             // With split activations ([hi | lo] along K) the weights repeat every w_wrap_k, a multiple of the k-block.
             int wk = 0;
             for (int kb = 0; kb < num_kb; ++kb) {
-                mbar_wait_converged(&empty_bar[stage], phase ^ 1u, abort_flag, spent);
-                if (elect_one() && !wait_failed(spent)) {
+                mbar_wait_converged<kErrProducerWait>(&empty_bar[stage], phase ^ 1u, abort_flag, failed);
+                if (elect_one() && !wait_failed(failed)) {
                     uint8_t* a_dst = stage_base + stage * Cfg::kStageBytes;
                     mbar_expect_tx(&full_bar[stage], Cfg::kStageBytes);
+                    ++issued;
                     // x coordinates are in elements: kb * 64 halves = a multiple of 128 bytes.
                     tma_load_2d(a_dst, &map_a, &full_bar[stage], kb * kBlockK, m0);
                     tma_load_2d(a_dst + Cfg::kATileBytes, &map_w, &full_bar[stage], wk, n0);
                 }
                 __syncwarp();
-                issued += wait_failed(spent) ? 0u : 1u;
                 wk += kBlockK;
                 wk = wk == w_wrap_k ? 0 : wk;
                 if (++stage == kStages) {
@@ -330,12 +330,13 @@ gemm_f16_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 }
             }
         }
+        const uint32_t all_issued = __reduce_add_sync(0xFFFFFFFFu, issued);   // one lane has counted
         named_barrier_sync(2, 64);   // tensor memory is allocated
         let_next_kernel_start();
-        if (wait_failed(spent) && lane == 0) {
-            atomicCAS(error_word, 0, kErrProducerWait);
+        if (const uint32_t code = warp_failure(failed); code != 0 && lane == 0) {
+            atomicCAS(error_word, 0, static_cast<int32_t>(code));
             // Copies already issued still land in shared memory: the CTA must not exit underneath them.
-            if (!drain_ring(full_bar, kStages, issued)) {
+            if (!drain_ring(full_bar, kStages, all_issued)) {
                 atomicCAS(error_word, 0, kErrDrainWait);
             }
         }
@@ -349,12 +350,12 @@ gemm_f16_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++local_tile) {
             const int acc = local_tile & 1;
             const uint32_t acc_phase = (local_tile >> 1) & 1u;
-            mbar_wait_converged(&acc_empty_bar[acc], acc_phase ^ 1u, abort_flag, spent);
+            mbar_wait_converged<kErrAccumWait>(&acc_empty_bar[acc], acc_phase ^ 1u, abort_flag, failed);
             tc_fence_after_sync();
             const uint32_t d_tmem = tmem + static_cast<uint32_t>(acc * 256);
             uint32_t accumulate = 0;
             for (int kb = 0; kb < num_kb; ++kb) {
-                mbar_wait_converged(&full_bar[stage], phase, abort_flag, spent);
+                mbar_wait_converged<kErrMmaWait>(&full_bar[stage], phase, abort_flag, failed);
                 tc_fence_after_sync();
                 const uint64_t b_desc = a_desc + Cfg::kATileBytes / 16;
                 if (elect_one()) {
@@ -376,13 +377,13 @@ gemm_f16_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 }
             }
             if (elect_one()) {
-                umma_commit(&acc_full_bar[acc]);
+                umma_commit_unless(&acc_full_bar[acc], failed);
             }
             __syncwarp();
         }
-        if (wait_failed(spent)) {
+        if (const uint32_t code = warp_failure(failed); code != 0) {
             if (lane == 0) {
-                atomicCAS(error_word, 0, kErrMmaWait);
+                atomicCAS(error_word, 0, static_cast<int32_t>(code));
             }
             umma_settle_after_failure();
         }
@@ -513,7 +514,7 @@ gemm_f16_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     const uint32_t tmem_base = *tmem_slot;
 
     // Both issuing roles as in the single-CTA kernel: whole warp, one elected lane, waits nothing branches on.
-    uint32_t spent = 0;   // probes of this role's waits
+    uint32_t failed = 0;   // this role's first failed wait, see mbar_wait_converged
     int stage = 0;
     uint32_t phase = 0;
     if (role == 0) {
@@ -524,10 +525,10 @@ gemm_f16_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             const int n0 = warp_uniform(tc.n_blk * BN + static_cast<int>(rank) * (BN / 2));
             int wk = 0;   // repeats every w_wrap_k, a multiple of the k-block
             for (int kb = 0; kb < num_kb; kb += SUB) {
-                mbar_wait_converged_cluster(&empty_bar[stage], phase ^ 1u, abort_flag, spent);
+                mbar_wait_converged_cluster<kErrProducerWait>(&empty_bar[stage], phase ^ 1u, abort_flag, failed);
                 const int nsub = (num_kb - kb) < SUB ? (num_kb - kb) : SUB;
                 const uint32_t leader_full = map_to_cta(smem_u32(&full_bar[stage]), 0);
-                const bool issue = elect_one() && !wait_failed(spent);
+                const bool issue = elect_one() && !wait_failed(failed);
                 if (issue && rank == 0) {
                     mbar_expect_tx(&full_bar[stage], 2 * nsub * Cfg::kStageBytes);
                 }
@@ -551,8 +552,8 @@ gemm_f16_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             }
         }
         let_next_kernel_start();
-        if (wait_failed(spent) && lane == 0) {
-            atomicCAS(error_word, 0, kErrProducerWait);
+        if (const uint32_t code = warp_failure(failed); code != 0 && lane == 0) {
+            atomicCAS(error_word, 0, static_cast<int32_t>(code));
         }
         __syncwarp();
     } else if (role == 1) {
@@ -564,12 +565,12 @@ gemm_f16_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
         for (int tile = pair; rank == 0 && tile < num_tiles; tile += num_pairs, ++local_tile) {
             const int acc = local_tile & 1;
             const uint32_t acc_phase = (local_tile >> 1) & 1u;
-            mbar_wait_converged_cluster(&acc_empty_bar[acc], acc_phase ^ 1u, abort_flag, spent);
+            mbar_wait_converged_cluster<kErrAccumWait>(&acc_empty_bar[acc], acc_phase ^ 1u, abort_flag, failed);
             tc_fence_after_sync();
             const uint32_t d_tmem = tmem + static_cast<uint32_t>(acc * 256);
             uint32_t accumulate = 0;
             for (int kb = 0; kb < num_kb; kb += SUB) {
-                mbar_wait_converged_cluster(&full_bar[stage], phase, abort_flag, spent);
+                mbar_wait_converged_cluster<kErrMmaWait>(&full_bar[stage], phase, abort_flag, failed);
                 tc_fence_after_sync();
                 const int nsub = (num_kb - kb) < SUB ? (num_kb - kb) : SUB;
                 if (elect_one()) {
@@ -606,18 +607,18 @@ gemm_f16_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             }
             if (elect_one()) {
                 if constexpr (MC) {
-                    umma_commit_pair_mask(&acc_full_bar[acc], 3);
+                    umma_commit_pair_mask_unless(&acc_full_bar[acc], 3, failed);
                 } else {
                     const uint32_t f = smem_u32(&acc_full_bar[acc]);
-                    umma_commit_pair(map_to_cta(f, 0));
-                    umma_commit_pair(map_to_cta(f, 1));
+                    umma_commit_pair_unless(map_to_cta(f, 0), failed);
+                    umma_commit_pair_unless(map_to_cta(f, 1), failed);
                 }
             }
             __syncwarp();
         }
-        if (wait_failed(spent)) {
+        if (const uint32_t code = warp_failure(failed); code != 0) {
             if (lane == 0) {
-                atomicCAS(error_word, 0, kErrMmaWait);
+                atomicCAS(error_word, 0, static_cast<int32_t>(code));
             }
             umma_settle_after_failure();
         }

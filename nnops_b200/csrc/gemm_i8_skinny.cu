@@ -360,6 +360,11 @@ __device__ __forceinline__ uint32_t ld_shared_cluster_u32(uint32_t cluster_addr)
     return v;
 }
 
+__device__ __forceinline__ void st_shared_cluster_u32(uint32_t cluster_addr, uint32_t v)
+{
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
+}
+
 // How whole tiles are dealt to CTAs, or with parts > 1 the K blocks of a tile to the CTAs of a cluster: per_cta
 // each, one more for the first `longer`.
 struct Shares {
@@ -415,7 +420,7 @@ gemm_i8_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     // Like the MMA warp below: the whole warp walks the loop, one elected lane issues, and no branch
     // depends on what a wait returned.  Its loads need no barrier but the ring's, which it sets up itself, and
     // start before the CTA has met.
-    uint32_t spent = 0;   // probes of this role's waits
+    uint32_t failed = 0;   // this role's first failed wait, see mbar_wait_converged
     int stage = 0;
     uint32_t phase = 0;
     if (role == 0) {
@@ -455,31 +460,32 @@ gemm_i8_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     const uint32_t tmem_base = *tmem_slot;
 
     if (role == 0) {
-        uint32_t issued = 0;
+        uint32_t issued = 0;   // by this lane
         for (int si = 0; si < num_segments; ++si) {
             const Segment seg = segment_at(si);
             const int row = seg.tile * tile_rows;
             for (int kb = seg.kb0; kb < seg.kb1; ++kb) {
-                mbar_wait_converged(&empty_bar[stage], phase ^ 1u, abort_flag, spent);
-                if (elect_one() && !wait_failed(spent)) {
+                mbar_wait_converged<kErrProducerWait>(&empty_bar[stage], phase ^ 1u, abort_flag, failed);
+                if (elect_one() && !wait_failed(failed)) {
                     uint8_t* w_dst = stage_base + stage * Cfg::kStageBytes;
                     mbar_expect_tx(&full_bar[stage], static_cast<uint32_t>(tile_rows * kBlockKBytes + Cfg::kATileBytes));
+                    ++issued;
                     tma_load_2d(w_dst, &map_w, &full_bar[stage], kb * kBlockKBytes, row);
                     tma_load_2d(w_dst + Cfg::kWTileBytes, &map_a, &full_bar[stage], kb * kBlockKBytes, 0);
                 }
                 __syncwarp();
-                issued += wait_failed(spent) ? 0u : 1u;
                 if (++stage == kStages) {
                     stage = 0;
                     phase ^= 1u;
                 }
             }
         }
+        const uint32_t all_issued = __reduce_add_sync(0xFFFFFFFFu, issued);   // one lane has counted
         named_barrier_sync(2, 64);   // tensor memory is allocated
         let_next_kernel_start();
-        if (wait_failed(spent) && lane == 0) {
-            atomicCAS(error_word, 0, kErrProducerWait);
-            if (!drain_ring(full_bar, kStages, issued)) {
+        if (const uint32_t code = warp_failure(failed); code != 0 && lane == 0) {
+            atomicCAS(error_word, 0, static_cast<int32_t>(code));
+            if (!drain_ring(full_bar, kStages, all_issued)) {
                 atomicCAS(error_word, 0, kErrDrainWait);
             }
         }
@@ -502,12 +508,12 @@ gemm_i8_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             const Segment seg = segment_at(local_seg);
             const int acc = local_seg & 1;
             const uint32_t acc_phase = (local_seg >> 1) & 1u;
-            mbar_wait_converged(&acc_empty_bar[acc], acc_phase ^ 1u, abort_flag, spent);
+            mbar_wait_converged<kErrAccumWait>(&acc_empty_bar[acc], acc_phase ^ 1u, abort_flag, failed);
             tc_fence_after_sync();
             const uint32_t d_tmem = tmem + static_cast<uint32_t>(acc * MP);
             uint32_t accumulate = 0;
             for (int kb = seg.kb0; kb < seg.kb1; ++kb) {
-                mbar_wait_converged(&full_bar[stage], phase, abort_flag, spent);
+                mbar_wait_converged<kErrMmaWait>(&full_bar[stage], phase, abort_flag, failed);
                 tc_fence_after_sync();
                 const uint64_t a_desc = w_desc + Cfg::kWTileBytes / 16;  // its N operand: MP activation rows
                 if (elect_one()) {
@@ -528,13 +534,13 @@ gemm_i8_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 }
             }
             if (elect_one()) {
-                umma_commit(&acc_full_bar[acc]);
+                umma_commit_unless(&acc_full_bar[acc], failed);
             }
             __syncwarp();
         }
-        if (wait_failed(spent)) {
+        if (const uint32_t code = warp_failure(failed); code != 0) {
             if (lane == 0) {
-                atomicCAS(error_word, 0, kErrMmaWait);
+                atomicCAS(error_word, 0, static_cast<int32_t>(code));
             }
             umma_settle_after_failure();
         }
@@ -579,13 +585,19 @@ gemm_i8_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                                 mine[(r + j) * kBlockN] = v[j];
                             }
                         }
-                    } else if (lane == 0) {
-                        atomicCAS(error_word, 0, kErrEpilogueWait);
+                    } else {
+                        // This CTA has no sums (a role that gives up commits none): nobody in the cluster stores.
+                        if (lane == 0) {
+                            atomicCAS(error_word, 0, kErrEpilogueWait);
+                        }
+                        if (lane < parts) {
+                            st_shared_cluster_u32(map_to_cta(smem_u32(const_cast<const int*>(abort_flag)), static_cast<uint32_t>(lane)), 1u);
+                        }
                     }
                     __syncwarp();
                     cluster_sync_all();
                     row = rank * m_total / parts + group * 4;
-                    store_end = row_end = (rank + 1) * m_total / parts;
+                    store_end = row_end = *abort_flag != 0 ? row : (rank + 1) * m_total / parts;
                     part = 0;
                 }
 #pragma unroll 1

@@ -139,7 +139,7 @@ gemm_i8_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 
     // In both issuing roles the whole warp walks the loop, one elected lane issues, and no branch depends on
     // what a wait returned (see mbar_wait_converged).
-    uint32_t spent = 0;   // probes of this role's waits
+    uint32_t failed = 0;   // this role's first failed wait, see mbar_wait_converged
     int stage = 0;
     uint32_t phase = 0;
     if (role == 0) {
@@ -164,10 +164,10 @@ gemm_i8_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             }
             int kx = rot;
             for (int kb = 0; kb < num_kb; kb += SUB) {
-                mbar_wait_converged_cluster(&empty_bar[stage], phase ^ 1u, abort_flag, spent);
+                mbar_wait_converged_cluster<kErrProducerWait>(&empty_bar[stage], phase ^ 1u, abort_flag, failed);
                 const int nsub = (num_kb - kb) < SUB ? (num_kb - kb) : SUB;
                 const uint32_t leader_full = map_to_cta(smem_u32(&full_bar[stage]), 0);
-                const bool issue = elect_one() && !wait_failed(spent);
+                const bool issue = elect_one() && !wait_failed(failed);
                 if (issue && rank == 0) {
                     mbar_expect_tx(&full_bar[stage], 2 * nsub * Cfg::kStageBytes);
                 }
@@ -217,8 +217,8 @@ gemm_i8_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             }
         }
         let_next_kernel_start();
-        if (wait_failed(spent) && lane == 0) {
-            atomicCAS(error_word, 0, kErrProducerWait);
+        if (const uint32_t code = warp_failure(failed); code != 0 && lane == 0) {
+            atomicCAS(error_word, 0, static_cast<int32_t>(code));
         }
         __syncwarp();
     } else if (role == 1) {
@@ -237,12 +237,12 @@ gemm_i8_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         for (int tile = pair; rank == 0 && tile < num_tiles; tile += num_pairs, ++local_tile) {
             const int acc = local_tile & 1;
             const uint32_t acc_phase = (local_tile >> 1) & 1u;
-            mbar_wait_converged_cluster(&acc_empty_bar[acc], acc_phase ^ 1u, abort_flag, spent);
+            mbar_wait_converged_cluster<kErrAccumWait>(&acc_empty_bar[acc], acc_phase ^ 1u, abort_flag, failed);
             tc_fence_after_sync();
             const uint32_t d_tmem = tmem + static_cast<uint32_t>(acc * 256);
             uint32_t accumulate = 0;
             for (int kb = 0; kb < num_kb; kb += SUB) {
-                mbar_wait_converged_cluster(&full_bar[stage], phase, abort_flag, spent);
+                mbar_wait_converged_cluster<kErrMmaWait>(&full_bar[stage], phase, abort_flag, failed);
                 tc_fence_after_sync();
                 const int nsub = (num_kb - kb) < SUB ? (num_kb - kb) : SUB;
                 if (elect_one()) {
@@ -279,18 +279,18 @@ gemm_i8_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             }
             if (elect_one()) {
                 if constexpr (MC) {
-                    umma_commit_pair_mask(&acc_full_bar[acc], 3);
+                    umma_commit_pair_mask_unless(&acc_full_bar[acc], 3, failed);
                 } else {
                     const uint32_t f = smem_u32(&acc_full_bar[acc]);
-                    umma_commit_pair(map_to_cta(f, 0));
-                    umma_commit_pair(map_to_cta(f, 1));
+                    umma_commit_pair_unless(map_to_cta(f, 0), failed);
+                    umma_commit_pair_unless(map_to_cta(f, 1), failed);
                 }
             }
             __syncwarp();
         }
-        if (wait_failed(spent)) {
+        if (const uint32_t code = warp_failure(failed); code != 0) {
             if (lane == 0) {
-                atomicCAS(error_word, 0, kErrMmaWait);
+                atomicCAS(error_word, 0, static_cast<int32_t>(code));
             }
             umma_settle_after_failure();
         }

@@ -698,7 +698,7 @@ gemm_i8_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     // The producer warp sets the barriers up and starts to load at once: it needs nothing of the others, who
     // meet at a barrier of their own.
     constexpr uint32_t kThreads = tile_threads(KIND, PEERS);
-    uint32_t spent = 0;   // probes of this role's waits
+    uint32_t failed = 0;   // this role's first failed wait, see mbar_wait_converged
     int stage = 0;
     uint32_t phase = 0;
     if (role == 0) {
@@ -740,7 +740,7 @@ gemm_i8_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         // ---------------- TMA producer ----------------
         // The whole warp walks the loop, one elected lane issues, and no branch depends on what a wait
         // returned (see mbar_wait_converged); the same in the MMA warp.
-        uint32_t issued = 0;
+        uint32_t issued = 0;   // by this lane
         for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
             const TileCoord at = coord_of(tile);
             const int m_blk = warp_uniform(at.m_blk), n_blk = warp_uniform(at.n_blk);
@@ -761,11 +761,12 @@ gemm_i8_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             }
             int kb = rot;
             for (int step = 0; step < num_kb; ++step) {
-                mbar_wait_converged(&empty_bar[stage], phase ^ 1u, abort_flag, spent);
-                if (elect_one() && !wait_failed(spent)) {
+                mbar_wait_converged<kErrProducerWait>(&empty_bar[stage], phase ^ 1u, abort_flag, failed);
+                if (elect_one() && !wait_failed(failed)) {
                     uint8_t* a_dst = stage_base + stage * Cfg::kStageBytes;
                     uint8_t* b_dst = a_dst + Cfg::kATileBytes;
                     mbar_expect_tx(&full_bar[stage], Cfg::kStageBytes);
+                    ++issued;
                     if constexpr (CONV) {
                         // Patch (image, th, tw) shifted by the k-block's tap; 128 channels of it.
                         tma_load_4d(a_dst, &map_a, &full_bar[stage], conv.c_base + tap_c * kBlockKBytes,
@@ -811,7 +812,6 @@ gemm_i8_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     }
                 }
                 __syncwarp();
-                issued += wait_failed(spent) ? 0u : 1u;
                 if (++stage == kStages) {
                     stage = 0;
                     phase ^= 1u;
@@ -832,12 +832,13 @@ gemm_i8_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 }
             }
         }
+        const uint32_t all_issued = __reduce_add_sync(0xFFFFFFFFu, issued);   // one lane has counted
         named_barrier_sync(2, 64);   // tensor memory is allocated
         let_next_kernel_start();
-        if (wait_failed(spent) && lane == 0) {
-            atomicCAS(error_word, 0, kErrProducerWait);
+        if (const uint32_t code = warp_failure(failed); code != 0 && lane == 0) {
+            atomicCAS(error_word, 0, static_cast<int32_t>(code));
             // Copies already issued still land in shared memory: the CTA must not exit underneath them.
-            if (!drain_ring(full_bar, kStages, issued)) {
+            if (!drain_ring(full_bar, kStages, all_issued)) {
                 atomicCAS(error_word, 0, kErrDrainWait);
             }
         }
@@ -858,12 +859,12 @@ gemm_i8_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++local_tile) {
             const int acc = Cfg::kNSplit > 1 ? 0 : (local_tile & 1);
             const uint32_t acc_phase = Cfg::kNSplit > 1 ? (local_tile & 1u) : ((local_tile >> 1) & 1u);
-            mbar_wait_converged(&acc_empty_bar[acc], acc_phase ^ 1u, abort_flag, spent);
+            mbar_wait_converged<kErrAccumWait>(&acc_empty_bar[acc], acc_phase ^ 1u, abort_flag, failed);
             tc_fence_after_sync();
             const uint32_t d_tmem = tmem + static_cast<uint32_t>(acc * BN);
             uint32_t accumulate = 0;
             for (int kb = 0; kb < num_kb; ++kb) {
-                mbar_wait_converged(&full_bar[stage], phase, abort_flag, spent);
+                mbar_wait_converged<kErrMmaWait>(&full_bar[stage], phase, abort_flag, failed);
                 tc_fence_after_sync();
                 if (elect_one()) {
 #pragma unroll
@@ -892,13 +893,13 @@ gemm_i8_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 }
             }
             if (elect_one()) {
-                umma_commit(&acc_full_bar[acc]);  // accumulator complete
+                umma_commit_unless(&acc_full_bar[acc], failed);  // accumulator complete
             }
             __syncwarp();
         }
-        if (wait_failed(spent)) {
+        if (const uint32_t code = warp_failure(failed); code != 0) {
             if (lane == 0) {
-                atomicCAS(error_word, 0, kErrMmaWait);
+                atomicCAS(error_word, 0, static_cast<int32_t>(code));
             }
             umma_settle_after_failure();
         }

@@ -166,41 +166,57 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
 }
 
 // Wait of a whole warp that stays warp-uniform to the compiler: every lane polls, and nothing branches on
-// the outcome.  `spent` counts the probes of the wait under way (each suspends the warp for up to ~4 us)
-// and stays at the limit once a wait has run out or another role has aborted; later waits of the same
-// role then fall through at once, so a loop that goes on regardless still ends, in the time its own
-// instructions take.  The loops that issue tcgen05.mma are built on this: after a branch on a polled
+// the outcome.  `failed` is 0 and becomes CODE with the first wait of the role that finds the abort flag raised or has
+// probed PROBES times, which raises it; later waits of the same role then fall through after one probe, so a loop that
+// goes on regardless still ends, in the time its own instructions take.  Such a loop must not announce what it
+// has not done: see umma_commit_unless.
+//
+// The limit in time is the epilogue's: its warps wait for the accumulator with mbar_wait, by the clock, whenever an
+// issuing role waits for anything, and raise the flag; the count only makes sure that no wait depends on another role
+// alone (a probe of a barrier that is not ready returns after 2600 cycles: 13 s).  Reading the clock here as well, or a loop of more instructions than these, cost a batch of 32 products of
+// 512 x 128 x 512 2 to 6 % of its 6.5 us.
+//
+// The loops that issue tcgen05.mma are built on this: after a branch on a polled
 // value the compiler no longer knows the warp converged and hands the MMA its tensor-memory address and
 // descriptors register by register, and a suspend-time hint costs a hundred cycles on a barrier that is
 // ready.  Loop of one wait and four M128 x N32 x K32 MMAs (160 cycles of tensor pipe): 443 cycles with
 // mbar_wait_warp, 500 with one thread and mbar_wait, 185 with this; N128 (256 cycles): 467 / 500 / 262.
-constexpr uint32_t kWaitProbes = 500000;   // 2 s of suspended probes
+constexpr uint32_t kWaitProbes = 10'000'000;
 
-__device__ __forceinline__ void mbar_wait_converged(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t& spent)
+#define NNB200_WAIT_CONVERGED(PROBE)                                    \
+    asm volatile(                                                       \
+        "{\n\t"                                                         \
+        ".reg .pred p, q;\n\t"                                          \
+        ".reg .u32 f, n;\n\t"                                           \
+        "mov.u32 n, 0;\n\t"                                             \
+        "WAIT_LOOP:\n\t"                                                \
+        PROBE " p, [%1], %2;\n\t"                                       \
+        "@p bra WAIT_DONE;\n\t"                                         \
+        "ld.volatile.shared.u32 f, [%3];\n\t"                           \
+        "mad.lo.u32 n, f, %4, n;\n\t"                                   \
+        "add.u32 n, n, 1;\n\t"                                          \
+        "setp.lt.u32 q, n, %4;\n\t"                                     \
+        "@!q st.volatile.shared.u32 [%3], 1;\n\t"                       \
+        "@q bra WAIT_LOOP;\n\t"                                         \
+        "setp.eq.u32 p, %0, 0;\n\t"                                     \
+        "@p mov.u32 %0, %5;\n\t"                                        \
+        "WAIT_DONE:\n\t"                                                \
+        "}"                                                             \
+        : "+&r"(failed)                                                 \
+        : "r"(smem_u32(bar)), "r"(parity), "r"(smem_u32(const_cast<const int*>(abort_flag))), "n"(PROBES), "n"(CODE) \
+        : "memory")
+
+template <uint32_t CODE, uint32_t PROBES = kWaitProbes>
+__device__ __forceinline__ void mbar_wait_converged(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t& failed)
 {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p, q;\n\t"
-        ".reg .u32 f;\n\t"
-        "WAIT_LOOP:\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "@p bra WAIT_DONE;\n\t"
-        "ld.volatile.shared.u32 f, [%3];\n\t"
-        "mad.lo.u32 %0, f, %4, %0;\n\t"
-        "add.u32 %0, %0, 1;\n\t"
-        "setp.lt.u32 q, %0, %4;\n\t"
-        "@!q st.volatile.shared.u32 [%3], 1;\n\t"
-        "@q bra WAIT_LOOP;\n\t"
-        "WAIT_DONE:\n\t"
-        "setp.lt.u32 q, %0, %4;\n\t"
-        "selp.u32 %0, 0, %4, q;\n\t"
-        "}"
-        : "+&r"(spent)
-        : "r"(smem_u32(bar)), "r"(parity), "r"(smem_u32(const_cast<const int*>(abort_flag))), "r"(kWaitProbes)
-        : "memory");
+    NNB200_WAIT_CONVERGED("mbarrier.try_wait.parity.shared::cta.b64");
 }
 
-__device__ __forceinline__ bool wait_failed(uint32_t spent) { return spent >= kWaitProbes; }
+// Whether a wait of this lane has failed.
+__device__ __forceinline__ bool wait_failed(uint32_t failed) { return failed != 0; }
+
+// The same for the whole warp, after its loop: the code to record, or 0.
+__device__ __forceinline__ uint32_t warp_failure(uint32_t failed) { return __reduce_max_sync(0xFFFFFFFFu, failed); }
 
 // After a failed wait: the MMAs already issued are left the time to finish (a full queue is a few
 // microseconds) before the CTA gives its tensor memory back.
@@ -214,13 +230,13 @@ __device__ __forceinline__ void umma_settle_after_failure()
 // After the producer's wait failed: `issued` stages have been loaded in turn into `stages` slots, and what is in
 // flight still lands in shared memory; wait (bounded) for the last load of every slot.  False if one
 // did not land.
-__device__ __forceinline__ bool drain_ring(uint64_t* full_bar, int stages, uint32_t issued)
+__device__ __forceinline__ bool drain_ring(uint64_t* full_bar, int stages, uint32_t issued, long long limit_cycles = kWaitLimitCycles)
 {
     const long long t0 = clock64();
     const uint32_t first = issued > static_cast<uint32_t>(stages) ? issued - static_cast<uint32_t>(stages) : 0u;
     for (uint32_t i = first; i < issued; ++i) {
         while (!mbar_try_wait(&full_bar[i % static_cast<uint32_t>(stages)], (i / static_cast<uint32_t>(stages)) & 1u)) {
-            if (clock64() - t0 > kWaitLimitCycles) {
+            if (clock64() - t0 > limit_cycles) {
                 return false;
             }
         }
@@ -355,6 +371,20 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar)
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                      smem_u32(bar))
                  : "memory");
+}
+
+// The same unless a wait of this role has failed (see mbar_wait_converged): an accumulator that not every MMA has
+// summed into is not announced.  A predicate, as a branch on the outcome of a wait is what those loops avoid.
+__device__ __forceinline__ void umma_commit_unless(uint64_t* bar, uint32_t failed)
+{
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "setp.eq.u32 p, %1, 0;\n\t"
+        "@p tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
+        "}"
+        ::"r"(smem_u32(bar)), "r"(failed)
+        : "memory");
 }
 
 // Shared-memory matrix descriptor for a K-major operand tile written by TMA with the

@@ -85,7 +85,8 @@ __device__ __forceinline__ bool mbar_try_wait_cluster_suspend(uint64_t* bar, uin
 }
 
 // Bounded wait, as mbar_wait, with the cluster-scope probe.
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag)
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                                  long long limit_cycles = kWaitLimitCycles)
 {
     if (mbar_try_wait_cluster(bar, parity)) {
         return true;
@@ -100,7 +101,7 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
             if (*abort_flag != 0) {
                 return false;
             }
-            if (clock64() - t0 > kWaitLimitCycles) {
+            if (clock64() - t0 > limit_cycles) {
                 *abort_flag = 1;
                 return false;
             }
@@ -109,29 +110,10 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
 }
 
 // mbar_wait_converged with the cluster-scope probe.
-__device__ __forceinline__ void mbar_wait_converged_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
-                                                            uint32_t& spent)
+template <uint32_t CODE, uint32_t PROBES = kWaitProbes>
+__device__ __forceinline__ void mbar_wait_converged_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t& failed)
 {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p, q;\n\t"
-        ".reg .u32 f;\n\t"
-        "WAIT_LOOP:\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "@p bra WAIT_DONE;\n\t"
-        "ld.volatile.shared.u32 f, [%3];\n\t"
-        "mad.lo.u32 %0, f, %4, %0;\n\t"
-        "add.u32 %0, %0, 1;\n\t"
-        "setp.lt.u32 q, %0, %4;\n\t"
-        "@!q st.volatile.shared.u32 [%3], 1;\n\t"
-        "@q bra WAIT_LOOP;\n\t"
-        "WAIT_DONE:\n\t"
-        "setp.lt.u32 q, %0, %4;\n\t"
-        "selp.u32 %0, 0, %4, q;\n\t"
-        "}"
-        : "+&r"(spent)
-        : "r"(smem_u32(bar)), "r"(parity), "r"(smem_u32(const_cast<const int*>(abort_flag))), "r"(kWaitProbes)
-        : "memory");
+    NNB200_WAIT_CONVERGED("mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64");
 }
 
 // 2-D tiled load into THIS CTA's shared memory whose byte count is reported to the mbarrier at
@@ -218,6 +200,31 @@ __device__ __forceinline__ void umma_commit_pair_mask(uint64_t* bar, uint16_t ct
                      smem_u32(bar)),
                  "h"(cta_mask)
                  : "memory");
+}
+
+// Both unless a wait of this role has failed (see umma_commit_unless).
+__device__ __forceinline__ void umma_commit_pair_unless(uint32_t bar_cluster_addr, uint32_t failed)
+{
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "setp.eq.u32 p, %1, 0;\n\t"
+        "@p tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
+        "}"
+        ::"r"(bar_cluster_addr), "r"(failed)
+        : "memory");
+}
+
+__device__ __forceinline__ void umma_commit_pair_mask_unless(uint64_t* bar, uint16_t cta_mask, uint32_t failed)
+{
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "setp.eq.u32 p, %2, 0;\n\t"
+        "@p tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t"
+        "}"
+        ::"r"(smem_u32(bar)), "h"(cta_mask), "r"(failed)
+        : "memory");
 }
 
 }  // namespace nnb200

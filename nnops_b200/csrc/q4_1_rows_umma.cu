@@ -343,16 +343,16 @@ q4_1_rows_umma_kernel(const __grid_constant__ CUtensorMap map_a, const uint8_t* 
         const uint64_t ring_desc = umma_desc_sw128_kmajor(smem_u32(ring));
         const uint64_t slab_step = static_cast<uint64_t>(slab_bytes >> 4);
         const int my_units = warp_uniform(units);
-        uint32_t spent = 0;
+        uint32_t failed = 0;
         int stage = 0;
         uint32_t phase = 0, acc_phase = 1;
         for (int tile = warp_uniform(cluster); tile < num_tiles; tile += warp_uniform(clusters)) {
-            mbar_wait_converged(acc_empty, acc_phase, abort_flag, spent);
+            mbar_wait_converged<kErrAccumWait>(acc_empty, acc_phase, abort_flag, failed);
             tc_fence_after_sync();
             acc_phase ^= 1u;
             uint32_t accumulate = 0;
             for (int u = 0; u < my_units; ++u) {
-                mbar_wait_converged(&full_bar[stage], phase, abort_flag, spent);
+                mbar_wait_converged<kErrMmaWait>(&full_bar[stage], phase, abort_flag, failed);
                 tc_fence_after_sync();
                 const uint64_t b_desc = ring_desc + static_cast<uint64_t>((stage * stage_bytes) >> 4);
                 const uint32_t a_tmem = d_tmem + static_cast<uint32_t>(kAccCols + stage * Cfg::kUnitCols);
@@ -379,14 +379,14 @@ q4_1_rows_umma_kernel(const __grid_constant__ CUtensorMap map_a, const uint8_t* 
                 }
             }
             if (elect_one()) {
-                umma_commit(acc_full);
+                umma_commit_unless(acc_full, failed);
             }
             __syncwarp();
         }
         let_next_kernel_start();
-        if (wait_failed(spent)) {
+        if (const uint32_t code = warp_failure(failed); code != 0) {
             if (lane == 0) {
-                atomicCAS(error_word, 0, kErrMmaWait);
+                atomicCAS(error_word, 0, static_cast<int32_t>(code));
             }
             umma_settle_after_failure();
         }
