@@ -2,8 +2,9 @@
 
     python -m nnops_b200.build [--force] [--verbose]
 
-Output: nnops_b200/lib/libnnb200.so and torch_front.so, the tensor front end's compiled half (git-ignored; shipped to
-GPU machines as built files).  nvcc cross-compiles without a GPU.  -fmad=false keeps every f32 multiply and add separately
+Output: nnops_b200/lib/libnnb200.so, and torch_front.*.so, the tensor front end's compiled half for this interpreter's
+torch, where there is one with CUDA and a C++ compiler (git-ignored; shipped to GPU machines as built files).
+nvcc cross-compiles without a GPU.  -fmad=false keeps every f32 multiply and add separately
 rounded unless a kernel asks for an fma explicitly -- the int8 requantisation must match the
 CPU arithmetic bit for bit.
 """
@@ -11,8 +12,10 @@ from __future__ import annotations
 
 import os
 import re
+import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -20,7 +23,6 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB_DIR = PKG / "lib"
 LIB = LIB_DIR / "libnnb200.so"
-FRONT = LIB_DIR / "torch_front.so"
 FRONT_SRC = PKG / "host" / "torch_front.cpp"
 NVCC = os.environ.get("NNB200_NVCC", "/usr/local/cuda/bin/nvcc")
 CXX = os.environ.get("NNB200_CXX", "g++")
@@ -53,22 +55,28 @@ def _stale(out: Path, deps: list[Path]) -> bool:
     return any(d.stat().st_mtime > t for d in deps if d.exists())
 
 
-def build_front(force: bool = False) -> Path:
-    """host/torch_front.cpp against this interpreter's torch."""
-    if force or _stale(FRONT, [FRONT_SRC, PKG.parent / "include" / "nnb200.h"]):
-        import sysconfig
-
+def build_front(force: bool = False) -> Path | None:
+    """host/torch_front.cpp against this interpreter's torch; None, with nothing built, where that has no CUDA or there
+    is no compiler.  ops.py does without it."""
+    try:
         import torch
+    except ImportError:
+        return None
+    if torch.version.cuda is None or shutil.which(CXX) is None:
+        return None
+    from . import capi
+    out = capi.front_path()
+    if force or _stale(out, [FRONT_SRC, PKG.parent / "include" / "nnb200.h"]):
         root = Path(torch.__file__).resolve().parent
         include = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", sysconfig.get_paths()["include"],
                    Path(os.environ.get("CUDA_HOME", "/usr/local/cuda")) / "include"]
         r = subprocess.run([CXX, "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden",
                             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-isystem{i}" for i in include),
-                            str(FRONT_SRC), "-o", str(FRONT), f"-L{root / 'lib'}", f"-Wl,-rpath,{root / 'lib'}", "-ltorch_python",
+                            str(FRONT_SRC), "-o", str(out), f"-L{root / 'lib'}", f"-Wl,-rpath,{root / 'lib'}", "-ltorch_python",
                             "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10"], capture_output=True, text=True)
         if r.returncode != 0:
-            raise RuntimeError(f"g++ failed on {FRONT_SRC.name}:\n{r.stdout}\n{r.stderr}")
-    return FRONT
+            raise RuntimeError(f"{CXX} failed on {FRONT_SRC.name}:\n{r.stdout}\n{r.stderr}")
+    return out
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
@@ -88,15 +96,14 @@ def build(force: bool = False, verbose: bool = False) -> Path:
                 print(r.stderr)
         return obj
 
-    with ThreadPoolExecutor(max_workers=len(SOURCES) + 1) as ex:
-        front = ex.submit(build_front, force)
+    with ThreadPoolExecutor(max_workers=len(SOURCES)) as ex:
         objs = list(ex.map(compile_one, SOURCES))
-        front.result()
     if force or _stale(LIB, objs):
         r = subprocess.run([NVCC, "-shared", "-o", str(LIB), *map(str, objs)],
                            capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    build_front(force)
     return LIB
 
 

@@ -9,11 +9,11 @@ import ctypes as C
 import importlib.machinery
 import importlib.util
 import struct
+import sysconfig
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
 LIB_PATH = PKG / "lib" / "libnnb200.so"
-FRONT_PATH = PKG / "lib" / "torch_front.so"
 
 OK, INVALID_ARGUMENT, UNSUPPORTED, NOT_INITIALIZED, OUT_OF_MEMORY, INTERNAL = range(6)
 STATUS_NAMES = ["ok", "invalid_argument", "unsupported", "not_initialized", "out_of_memory", "internal"]
@@ -208,11 +208,19 @@ def lib() -> C.CDLL:
     return _lib
 
 
+def front_path() -> Path:
+    """Where the tensor front end's compiled half lies.  It is built against one torch and one interpreter, whose versions
+    are in its name: under another one it is not there, instead of misreading that one's tensors."""
+    import torch
+    return PKG / "lib" / f"torch_front.{sysconfig.get_config_var('SOABI')}-torch{torch.__version__}-cuda{torch.version.cuda}.so"
+
+
 def torch_front():
     """The compiled marshalling of the tensor front end (host/torch_front.cpp).  Raises if it has not been built."""
-    if not FRONT_PATH.exists():
-        raise RuntimeError(f"{FRONT_PATH} is missing: build it with `python -m nnops_b200.build`")
-    loader = importlib.machinery.ExtensionFileLoader("torch_front", str(FRONT_PATH))
+    path = front_path()
+    if not path.exists():
+        raise RuntimeError(f"{path} is missing: build it with `python -m nnops_b200.build`")
+    loader = importlib.machinery.ExtensionFileLoader("torch_front", str(path))
     module = importlib.util.module_from_spec(importlib.util.spec_from_loader("torch_front", loader))
     loader.exec_module(module)
     return module

@@ -6,6 +6,7 @@ from __future__ import annotations
 import ctypes as C
 import inspect
 import math
+import warnings
 
 import torch
 
@@ -14,16 +15,32 @@ from . import capi
 _native = None
 
 
+class _NoFront:
+    """Takes no call."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
 def _front():
     """host/torch_front.cpp, bound to the library capi has loaded: the usual calls without the interpreter.  Each
     of its functions answers None, with nothing done, to what is not one of those; the code below then does
-    the call, or says what is wrong with it."""
+    the call, or says what is wrong with it.  Where it is not built for this torch and interpreter, that code does
+    every call: the same kernels, some 10 us later."""
     global _native
     if _native is None:
-        front, lib = capi.torch_front(), capi.lib()
-        front.bind(*(C.cast(getattr(lib, name), C.c_void_p).value for name in (
+        lib = capi.lib()
+        try:
+            front = capi.torch_front()
+        except (RuntimeError, ImportError) as e:
+            warnings.warn(f"nnops_b200: every call goes through the interpreter: {e}", RuntimeWarning, stacklevel=3)
+            _native = _NoFront()
+            return _native
+        bound = front.bind(*(C.cast(getattr(lib, name), C.c_void_p).value for name in (
             "nnb200_gemm_i8_workspace_bytes", "nnb200_gemm_i8", "nnb200_q4_1_workspace_bytes", "nnb200_linear_q4_1",
             "nnb200_quantize_linear", "nnb200_dequantize_linear", "nnb200_conv2d_i8_workspace_bytes", "nnb200_conv2d_i8")), capi.check)
+        if bound is not True:
+            raise RuntimeError("torch_front is of another version than ops.py: rebuild it with `python -m nnops_b200.build --force`")
         _native = front
     return _native
 

@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from nnops_b200 import ops
+from nnops_b200 import capi, ops
 
 
 def _args(a, w, out, **kw):
@@ -50,3 +50,22 @@ def test_scratch_beyond_the_least_may_fail_to_be_had(nnb200_lib, monkeypatch, zp
     if zp_a:
         with pytest.raises(torch.OutOfMemoryError):
             _args((3, 2049), (5000, 2049), (3, 5000), zp_a=zp_a, keep=keep)
+
+
+def test_the_compiled_front_end_is_looked_up_by_torch_and_interpreter():
+    import sysconfig
+    import torch
+    name = capi.front_path().name
+    assert torch.__version__ in name and str(torch.version.cuda) in name and sysconfig.get_config_var("SOABI") in name
+
+
+def test_without_the_compiled_front_end_the_python_code_does_the_calls(nnb200_lib, monkeypatch, tmp_path):
+    """Not built, or built for another torch: a warning, once, and every function declines every call."""
+    for path, content in ((tmp_path / "missing.so", None), (tmp_path / "broken.so", b"not a library")):
+        if content is not None:
+            path.write_bytes(content)
+        monkeypatch.setattr(capi, "front_path", lambda: path)
+        monkeypatch.setattr(ops, "_native", None)
+        with pytest.warns(RuntimeWarning, match="through the interpreter"):
+            assert ops._front().gemm_i8(None, None, "s32", None, {}) is None
+        assert ops._native.conv2d_i8() is None
