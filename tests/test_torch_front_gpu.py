@@ -9,9 +9,25 @@ from nnops_b200 import capi, ops
 pytestmark = pytest.mark.gpu
 
 
-class _TakesNothing:
+class _Recorder:
+    """The compiled front end, noting of each call whether it took it."""
+
+    def __init__(self, front):
+        self.front, self.taken = front, []
+
     def __getattr__(self, name):
-        return lambda *args: None
+        def call(*args):
+            made = getattr(self.front, name)(*args)
+            self.taken.append((name, made is not None))
+            return made
+        return call
+
+
+# What the Python code does instead, and the calls of its own that the compiled code then takes or not.
+LEFT_TO_PYTHON = {
+    "numpy parameters": [("gemm_i8", False)], "engine, least scratch": [("gemm_i8", False)],
+    "quantize by one, from lists": [("quantize_linear", False)], "conv, zero points": [("conv2d_i8", False)], "conv, raw filter": [],
+}
 
 
 def _calls(dev):
@@ -62,9 +78,17 @@ def _calls(dev):
     "dequantize along 1", "fp_act", "fp_act, one scale", "fp_act, zero points", "fp_act, one zero point", "conv", "conv, zero points",
     "conv, raw filter"])
 def test_same_bytes_as_the_python_path(cuda_device, nnb200_lib, monkeypatch, name):
-    got = _calls(cuda_device)[name]().clone()
-    monkeypatch.setattr(ops, "_native", _TakesNothing())
-    want = _calls(cuda_device)[name]()
+    calls = _calls(cuda_device)
+    recorder = _Recorder(ops._front())
+    monkeypatch.setattr(ops, "_native", recorder)
+    got = calls[name]().clone()
+    if name in LEFT_TO_PYTHON:
+        assert recorder.taken == LEFT_TO_PYTHON[name]
+    else:
+        assert len(recorder.taken) == 1 and recorder.taken[0][1], recorder.taken
+    calls = _calls(cuda_device)   # the same inputs again
+    monkeypatch.setattr(ops, "_native", ops._NoFront())
+    want = calls[name]()
     assert got.dtype == want.dtype and got.shape == want.shape and torch.equal(got.view(torch.uint8), want.contiguous().view(torch.uint8))
 
 
