@@ -241,7 +241,14 @@ bool sharded_out(const nnb200_gemm_i8_args* a)
     return a->num_peer_outs != 0 || a->multicast_out != nullptr;
 }
 
-int pick_i8_engine(const nnb200_gemm_i8_args* a, const I8Problem& p)
+int64_t sm_count()
+{
+    const DeviceInfo* dev = current_device_info();
+    return dev != nullptr ? dev->sm_count : 148;
+}
+
+// By alignment, rows and channels alone.
+int pick_i8_engine_by_shape(const nnb200_gemm_i8_args* a, const I8Problem& p)
 {
     if (a->force_engine == NNB200_ENGINE_GENERIC) {
         return NNB200_ENGINE_GENERIC;
@@ -269,8 +276,7 @@ int pick_i8_engine(const nnb200_gemm_i8_args* a, const I8Problem& p)
     if (!sharded_out(a)) {
         const bool decode_ok = decode_i8_supported(p);
         const bool skinny_ok = skinny_i8_supported(p);
-        const DeviceInfo* dev = current_device_info();
-        const int64_t sms = dev != nullptr ? dev->sm_count : 148;
+        const int64_t sms = sm_count();
         const int64_t tiles128 = (p.n + 127) / 128;
         if (decode_ok && (p.m <= 8 || !skinny_ok || tiles128 <= 96)) {
             return NNB200_ENGINE_DECODE;
@@ -289,6 +295,18 @@ int pick_i8_engine(const nnb200_gemm_i8_args* a, const I8Problem& p)
         return NNB200_ENGINE_UMMA;
     }
     return NNB200_ENGINE_GENERIC;
+}
+
+// The engine of one product: the few-row engine, with K shared in clusters, takes part of what the shape alone gives
+// to two others.
+int pick_i8_engine(const nnb200_gemm_i8_args* a, const I8Problem& p)
+{
+    const int engine = pick_i8_engine_by_shape(a, p);
+    if (a->force_engine == NNB200_ENGINE_AUTO && !sharded_out(a) && (engine == NNB200_ENGINE_UMMA || engine == NNB200_ENGINE_DECODE) &&
+        skinny_i8_preferred(p, engine == NNB200_ENGINE_DECODE, sm_count())) {
+        return NNB200_ENGINE_SKINNY;
+    }
+    return engine;
 }
 
 size_t out_elem_bytes(int kind)
@@ -385,7 +403,7 @@ static I8SplitPlan i8_split_plan(const nnb200_gemm_i8_args* a)
         return plan;
     }
     const I8Problem p = problem_of(a, 0);
-    const int engine = pick_i8_engine(a, p);
+    const int engine = pick_i8_engine_by_shape(a, p);
     if (engine == NNB200_ENGINE_SKINNY) {
         plan.bytes = skinny_i8_split_bytes(p, *dev);
     } else if (engine == NNB200_ENGINE_UMMA && a->force_engine == NNB200_ENGINE_AUTO && p.m >= 17 && p.m <= 128) {
@@ -463,8 +481,7 @@ static bool i8_copies_pay(const nnb200_gemm_i8_args* a)
     if (a->a_stride_k != 1 || a->w_stride_k != 1) {
         return false;
     }
-    const DeviceInfo* dev = current_device_info();
-    const int64_t sms = dev != nullptr ? dev->sm_count : 148;
+    const int64_t sms = sm_count();
     const bool square_follows = a->m > 64 || (a->m > 16 && a->n <= 64 * sms);
     const int64_t tiles = ((a->m + 31) / 32) * ((a->n + 31) / 32);
     return (a->k > 96 && square_follows) || (a->k > 64 && tiles * ((a->k + 31) / 32) >= 12000) ||
@@ -553,17 +570,6 @@ static bool i8_align_in_workspace(const nnb200_gemm_i8_args* a, I8AlignPlan* pla
     return true;
 }
 
-int nnb200_gemm_i8_engine(const nnb200_gemm_i8_args* a)
-{
-    if (!valid_i8_args(a)) {
-        return -1;
-    }
-    if (a->m == 0 || a->n == 0 || a->batch == 0) {
-        return pick_i8_engine(a, problem_of(a, 0));
-    }
-    return i8_engine_with_workspace(a, 0, nullptr);
-}
-
 // Whether a batched call goes out as one launch of the tile kernel, and its strides.
 static bool i8_batched_call(const nnb200_gemm_i8_args* a, const DeviceInfo& dev, I8Batch* b)
 {
@@ -582,18 +588,34 @@ static bool i8_batched_call(const nnb200_gemm_i8_args* a, const DeviceInfo& dev,
     if (!apart || !umma_i8_batched_supported(problem_of(a, 0), *b, dev)) {
         return false;
     }
-    // Few rows alone run on the streaming engine, which spreads one product's channels 16 to a CTA and its K
-    // over the warps; a tile here walks all of K.  Until the launches add up that is the slower way.
-    // The estimates, in 10 ns, are fits to CUDA-graph timings of 15 layers at 1 to 16 rows (us, alone /
-    // batched: 2 x 1 x 2048 x 3968 7.1 / 12.6, 4 x 8 x 512 x 15360 26.9 / 35.1, 6 x 4 x 64 x 65536 98.8 / 134;
-    // 8 x 1 x 2048 x 3968 31.5 / 15.0, 2 x 8 x 16384 x 448 15.2 / 9.2, 8 x 8 x 4032 x 2048 33.1 / 12.3).
-    if (a->force_engine == NNB200_ENGINE_AUTO && pick_i8_engine(a, problem_of(a, 0)) == NNB200_ENGINE_DECODE) {
+    // Few rows alone run on engines that spread one product's channels and K over all SMs; a tile here walks all of
+    // K.  Until the launches add up that is the slower way.  The estimates, in 10 ns, are fits to CUDA-graph timings of
+    // 15 layers at 1 to 16 rows with each product on the streaming engine; with the engines of today (us, alone /
+    // batched): 2 x 1 x 2048 x 3968 9.1 / 11.6, 4 x 8 x 512 x 15360 21.6 / 20.7, 6 x 4 x 64 x 65536 60.5 / 75.3 stay
+    // alone, 8 x 1 x 2048 x 3968 36.9 / 17.5, 2 x 8 x 16384 x 448 8.7 / 9.2, 8 x 8 x 4032 x 2048 36.1 / 17.4 do not.
+    if (a->force_engine == NNB200_ENGINE_AUTO && pick_i8_engine_by_shape(a, problem_of(a, 0)) == NNB200_ENGINE_DECODE) {
         const double kb = static_cast<double>((a->k + 127) / 128);
         const double one = 230.0 + 0.01 * static_cast<double>(a->n) + 20.0 * static_cast<double>(a->m < 4 ? a->m : 4) +
                            (a->m <= 8 ? 2.4 : 5.2) * kb;
         return one * static_cast<double>(a->batch) > 550.0 + 28.0 * kb;
     }
     return true;
+}
+
+int nnb200_gemm_i8_engine(const nnb200_gemm_i8_args* a)
+{
+    if (!valid_i8_args(a)) {
+        return -1;
+    }
+    if (a->m == 0 || a->n == 0 || a->batch == 0) {
+        return pick_i8_engine(a, problem_of(a, 0));
+    }
+    const DeviceInfo* dev = current_device_info();
+    I8Batch batch;
+    if (a->batch > 1 && dev != nullptr && i8_batched_call(a, *dev, &batch)) {
+        return NNB200_ENGINE_UMMA;   // all products in one launch of its kernel
+    }
+    return i8_engine_with_workspace(a, 0, nullptr);
 }
 
 // One call's kernels.  `reserved`: bytes of the workspace between the sums and the optional
@@ -723,15 +745,7 @@ static int run_gemm_i8(const nnb200_gemm_i8_args* a, const DeviceInfo* dev, cuda
         if (batched) {
             return launch_gemm_i8_umma_batched(p, batch, ep, *dev, stream);
         }
-        int engine = a->batch == 1 ? engine0 : pick_i8_engine(a, p);
-        // The few-row engine with K shared in clusters takes part of what the rows and channels alone give to
-        // two others; nnb200_gemm_i8_engine keeps naming those.
-        if (a->force_engine == NNB200_ENGINE_AUTO && !sharded_out(a) &&
-            (engine == NNB200_ENGINE_UMMA || engine == NNB200_ENGINE_DECODE) &&
-            skinny_i8_preferred(p, engine == NNB200_ENGINE_DECODE, *dev)) {
-            engine = NNB200_ENGINE_SKINNY;
-        }
-        switch (engine) {
+        switch (a->batch == 1 ? engine0 : pick_i8_engine(a, p)) {
         case NNB200_ENGINE_UMMA: st = launch_gemm_i8_umma(p, ep, *dev, stream); break;
         case NNB200_ENGINE_NARROW: st = launch_gemm_i8_narrow(p, ep, *dev, stream); break;
         case NNB200_ENGINE_DECODE: st = launch_gemm_i8_decode(p, ep, *dev, stream); break;

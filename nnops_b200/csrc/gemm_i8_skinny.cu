@@ -823,6 +823,38 @@ unsigned long long next_split_tag()
     return t;
 }
 
+// Clusters of `parts` CTAs that the device holds at once; 0 where it cannot say.  Every variant of the kernel takes an
+// SM to itself, so one stands for all.
+int resident_clusters(const DeviceInfo& dev, int parts)
+{
+    static std::once_flag once[kMaxDevices];
+    static int resident[kMaxDevices][kMaxParts + 1];
+    std::call_once(once[dev.device], [&] {
+        auto kernel = gemm_i8_skinny_kernel<128, NNB200_OUT_F32>;
+        cudaLaunchConfig_t cfg = {};
+        cfg.blockDim = dim3(kNumThreads);
+        cfg.dynamicSmemBytes = SkinnyConfig<128>::kSmemBytes;
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.y = 1;
+        attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SkinnyConfig<128>::kSmemBytes) == cudaSuccess;
+        for (int c = 2; c <= kMaxParts && ok; ++c) {
+            attr.val.clusterDim.x = static_cast<unsigned>(c);
+            cfg.gridDim = dim3(static_cast<unsigned>(dev.sm_count / c * c));
+            int count = 0;
+            if (cudaOccupancyMaxActiveClusters(&count, kernel, &cfg) == cudaSuccess) {
+                resident[dev.device][c] = count;
+            } else {
+                (void)cudaGetLastError();   // no clusters of that many: the launch takes a smaller one
+            }
+        }
+    });
+    return resident[dev.device][parts];
+}
+
 // CTAs that share a tile's K, by way of their cluster: as many as leave every tile's cluster an SM per CTA.
 int cluster_parts(const I8Problem& p, const DeviceInfo& dev)
 {
@@ -831,6 +863,9 @@ int cluster_parts(const I8Problem& p, const DeviceInfo& dev)
     int64_t parts = dev.sm_count / tiles;
     parts = parts > kMaxParts ? kMaxParts : parts;
     parts = parts > num_kb / 4 ? num_kb / 4 : parts;
+    while (parts > 1 && resident_clusters(dev, static_cast<int>(parts)) < tiles) {
+        --parts;
+    }
     return parts > 1 ? static_cast<int>(parts) : 1;
 }
 
@@ -842,29 +877,8 @@ int launch_skinny_variant(const I8Problem& p, const I8Epilogue& ep, const Device
     auto kernel = gemm_i8_skinny_kernel<MP, KIND>;
     static std::once_flag once[kMaxDevices];
     static cudaError_t attr_err[kMaxDevices];
-    static int resident[kMaxDevices][kMaxParts + 1];   // clusters of that many CTAs the device holds at once
-    cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(kNumThreads);
-    cfg.dynamicSmemBytes = Cfg::kSmemBytes;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
     std::call_once(once[dev.device], [&] {
         attr_err[dev.device] = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
-        cfg.numAttrs = 1;
-        for (int c = 2; c <= kMaxParts && attr_err[dev.device] == cudaSuccess; ++c) {
-            attr.val.clusterDim.x = static_cast<unsigned>(c);
-            cfg.gridDim = dim3(static_cast<unsigned>(dev.sm_count / c * c));
-            int count = 0;
-            if (cudaOccupancyMaxActiveClusters(&count, kernel, &cfg) == cudaSuccess) {
-                resident[dev.device][c] = count;
-            } else {
-                (void)cudaGetLastError();   // no clusters of that many: the launch takes a smaller one
-            }
-        }
     });
     if (attr_err[dev.device] != cudaSuccess) {
         return NNB200_INTERNAL;
@@ -877,10 +891,7 @@ int launch_skinny_variant(const I8Problem& p, const I8Epilogue& ep, const Device
     // 10.3 / 10.0); with more, the activations that more CTAs load eat what the even weight stream gives (64 and
     // 128 rows lost 3 and 8 %).  Shared K evens the SMs out itself, and its scratch is laid out for 128.
     int tile_rows = kBlockN;
-    int parts = split_scratch != nullptr && knob(NNB200_KNOB_I8_SHARE_K) == 2 ? 1 : cluster_parts(p, dev);
-    while (parts > 1 && resident[dev.device][parts] < (n + kBlockN - 1) / kBlockN) {
-        --parts;
-    }
+    int parts = split_scratch != nullptr ? 1 : cluster_parts(p, dev);   // the scratch is offered where clusters do not serve
     const int waves = ((n + kBlockN - 1) / kBlockN + dev.sm_count - 1) / dev.sm_count;
     if (split_scratch == nullptr && parts == 1 && (waves > 1 || p.m <= 32)) {
         tile_rows = (n + waves * dev.sm_count - 1) / (waves * dev.sm_count);
@@ -942,6 +953,17 @@ bool skinny_i8_supported(const I8Problem& p)
            (p.n / kBlockN + 1) * (p.k / kBlockKBytes + 1) < (int64_t{1} << 29);   // units are counted in 32 bits
 }
 
+// Whether the busiest SM of a single wave of tiles sheds enough K blocks when all SMs share K: at least 30, plus 0.7 per
+// row above 12 (see skinny_i8_split_bytes).
+static bool sharing_sheds_enough(const I8Problem& p, int64_t sms)
+{
+    const int64_t tiles = (p.n + kBlockN - 1) / kBlockN;
+    const int64_t num_kb = (p.k + kBlockKBytes - 1) / kBlockKBytes;
+    const int64_t share = (tiles * num_kb + sms - 1) / sms;
+    const int64_t rows_over = p.m > 12 ? p.m - 12 : 0;
+    return (num_kb - share) * 10 >= 300 + 7 * rows_over;
+}
+
 // Whether a call that the square engine or the streaming engine (up to 16 rows) would get by its number of
 // rows and channels is better off here, on clusters that share K.  CUDA-graph timings, weights beyond L2,
 // here / square engine, us:
@@ -957,46 +979,47 @@ bool skinny_i8_supported(const I8Problem& p)
 //   N = 28672, 8192: 16 rows 40.0 / 56.8, one 38.0 / 40.9; 28672, 1024: one 7.7 / 12.3.  The one place past 6272
 //   channels where one row is better off there: too many tiles for clusters and too few for the SMs, with a
 //   long K (N = 11008: K = 1024 4.8 / 5.9, 4096 11.3 / 10.4; N = 14336, 4096 12.3 / 13.6).
-bool skinny_i8_preferred(const I8Problem& p, bool over_streaming, const DeviceInfo& dev)
+bool skinny_i8_preferred(const I8Problem& p, bool over_streaming, int64_t sms)
 {
     if (!skinny_i8_supported(p)) {
         return false;
     }
     const int64_t tiles = (p.n + kBlockN - 1) / kBlockN;
     if (over_streaming) {
-        const bool sparse = p.m == 1 && p.k > 2048 && tiles * 2 > dev.sm_count && tiles * 4 <= dev.sm_count * 3;
-        return (tiles * 3 > dev.sm_count && !sparse) || p.k >= 8192 || (p.m > 8 && p.n >= 1024 && p.k >= 4096);
+        const bool sparse = p.m == 1 && p.k > 2048 && tiles * 2 > sms && tiles * 4 <= sms * 3;
+        return (tiles * 3 > sms && !sparse) || p.k >= 8192 || (p.m > 8 && p.n >= 1024 && p.k >= 4096);
     }
     if (p.m <= 32) {
         return true;
     }
     if (p.m <= 64) {
-        return tiles * 3 <= dev.sm_count ? p.k >= 2048 : p.k >= 8192;
+        return tiles * 3 <= sms ? p.k >= 2048 : p.k >= 8192;
     }
-    return tiles * 4 <= dev.sm_count && p.k >= 4096;
+    // Past the middle only where K is long for the rows (clusters / square engine: 72 x 6400 x 16384 25.0 / 27.1, 72 x
+    // 9472 x 16384 32.4 / 32.9, 66 x 6400 x 12288 19.5 / 20.3).
+    return (tiles * 4 <= sms && p.k >= 4096) || (tiles * 2 <= sms && sharing_sheds_enough(p, sms));
 }
 
 // Scratch for the equal-share split of K over all SMs, or 0 when it would not pay.  Publishing a
 // part, counting in and collecting the others' parts is a chain of L2 round trips at the end of
 // the kernel, each well over a microsecond while every SM is streaming: about 6 us in all plus
-// ~0.1 us per activation row, against ~0.3 us per 128-byte K block that the busiest CTA no longer
-// has to stream.  Measured, 24 rows, whole tiles -> shared K (us):
-//   one wave of tiles:  N=4096,K=28672 70.1 -> 31.6;  N=4096,K=14336 38.5 -> 22.2;  N=8192,K=8192
-//   25.3 -> 22.2;  N=14336,K=8192 28.1 -> 29.5;  N=11008,K=4096 16.5 -> 18.3;
-// With several waves the alternative is equal tiles, which already give every SM the same bytes; what they
-// lose is a step a K block and wave, whether or not the tile is full.  Shared K / equal tiles, 24 and 64
-// rows (us), by waves of 128-channel tiles:
-//   1.03  N=19456,K=8192 34.5 / 42.2, 39.8 / 46.5       1.16  N=22016,K=8192 37.8 / 42.5, 42.9 / 47.2
-//   1.30  N=24576,K=8192 40.3 / 42.8, 45.7 / 47.4       1.51  N=28672,K=8192 45.7 / 44.4, 51.5 / 49.3
-//   1.51  N=28672,K=4096 26.9 / 26.0, 34.0 / 30.6       1.51  N=28672,K=16384 80.4 / 80.7, 87.1 / 87.8
-//   1.69  N=32000,K=8192 51.6 / 47.9, 58.5 / 53.4       2.27  N=43008,K=8192 63.4 / 62.5, 70.5 / 68.7
-// (The line for several waves was drawn against 128-channel tiles, 52.0 -> 47.6 at N=28672,K=8192.  Against
-// equal ones it would lie nearer 7/10 full: from there to 9/10 shared K is 0 to 10 % the slower form.)
-// Hence: with one wave, share when the busiest CTA sheds at least 30 K blocks, plus 0.7 per row
+// ~0.1 us per activation row, against the K blocks that the busiest CTA no longer has to stream.  Measured, shared K /
+// without, 24 and 64 rows (us):
+//   one wave of tiles:
+//         N=9600,K=8192 20.4 / 17.2, 24.8 / 18.5          N=9600,K=16384 36.6 / 30.8, 41.8 / 33.2
+//         N=11008,K=8192 22.4 / 19.1, 27.1 / 20.7         N=11008,K=16384 36.8 / 33.7, 42.6 / 36.4
+//         N=12288,K=28672 61.5 / 56.6, 67.4 / 59.6        N=16384,K=16384 49.5 / 44.8, 54.8 / 47.8
+//   several, where the alternative is equal tiles, by waves of 128-channel tiles:
+//   1.03  N=19456,K=8192 33.0 / 31.5, 37.5 / 35.3         1.16  N=22016,K=8192 35.3 / 33.6, 39.4 / 37.5
+//   1.30  N=24576,K=8192 38.4 / 36.7, 42.7 / 40.4         1.51  N=28672,K=8192 43.4 / 40.8, 48.2 / 44.5
+//   1.51  N=28672,K=4096 25.3 / 22.9, 29.5 / 25.2         1.51  N=28672,K=16384 77.8 / 74.5, 82.6 / 80.0
+//   1.69  N=32000,K=8192 47.6 / 44.9, 52.2 / 48.9         2.27  N=43008,K=8192 59.3 / 58.8, 63.7 / 63.0
+// So none of these gains.  The lines below are older: they were drawn when a K block took the issuing warps 525 cycles
+// (0.3 us for the busiest CTA; N=8192, K=8192 25.3 / 22.2 the other way round) and have not been drawn again.
+// With one wave, share when the busiest CTA sheds at least 30 K blocks, plus 0.7 per row
 // above 12; with several waves, when the last one is less than 9/10 full, a share is at least 48
 // K blocks and there are at most 64 rows.
-// A caller that brings the scratch where clusters share K gets those all the same (4096 x 14336, 24 rows: 21.3 us
-// on the scratch, 13.3 in clusters; the offer stays, engines are named by it).
+// None where clusters share K (4096 x 14336, 24 rows: 21.3 us on the scratch, 13.3 in clusters).
 // Knob I8_SHARE_K = 0 turns this split off; 2 offers it from 8 K blocks per SM and prefers it (measurement, tests).
 size_t skinny_i8_split_bytes(const I8Problem& p, const DeviceInfo& dev)
 {
@@ -1017,9 +1040,11 @@ size_t skinny_i8_split_bytes(const I8Problem& p, const DeviceInfo& dev)
         return 0;  // whole tiles already fill the SMs, or there is next to nothing to share
     }
     if (mode != '2') {
+        if (cluster_parts(p, dev) > 1) {
+            return 0;
+        }
         if (waves == 1) {
-            const int64_t rows_over = p.m > 12 ? p.m - 12 : 0;
-            if ((num_kb - share) * 10 < 300 + 7 * rows_over) {
+            if (!sharing_sheds_enough(p, sms)) {
                 return 0;
             }
         } else if (share < 48 || p.m > 64) {

@@ -160,7 +160,7 @@ int launch_gemm_i8_skinny(const I8Problem& p, const I8Epilogue& ep, const Device
                           cudaStream_t stream);
 size_t skinny_i8_split_bytes(const I8Problem& p, const DeviceInfo& dev);
 bool skinny_i8_supported(const I8Problem& p);
-bool skinny_i8_preferred(const I8Problem& p, bool over_streaming, const DeviceInfo& dev);
+bool skinny_i8_preferred(const I8Problem& p, bool over_streaming, int64_t sms);
 
 // R_a[m] = sum_k A[m][k] and R_w[n] = sum_k W[n][k] into int32 scratch; r_w == nullptr skips the
 // sweep over W (the caller has the sums already).

@@ -96,3 +96,25 @@ def test_q4_gemv_knob_comes_before_the_weights_in_tensor_memory(nnb200_lib, knob
     assert (engine(4, True), engine(4, False), engine(1, True)) == (6, 6, 6)
     knobs("q4_gemv", 1)
     assert (engine(4, True), engine(4, False), engine(1, True)) == (7, 7, 4)
+
+
+@pytest.mark.parametrize("m,n,k,engine", [
+    # from the streaming engine (up to 16 rows): by tiles per SM, by K, from 9 rows by both
+    (1, 6272, 512, "decode"), (1, 6273, 512, "skinny"), (8, 6272, 4096, "decode"), (8, 6273, 4096, "skinny"),
+    (1, 64, 8128, "decode"), (1, 64, 8192, "skinny"), (8, 1024, 4096, "decode"), (9, 1024, 4096, "skinny"), (9, 1023, 4096, "decode"),
+    (9, 1024, 4032, "decode"), (16, 6272, 512, "decode"), (16, 6273, 512, "skinny"),
+    # one row of a long K where tiles are too many for clusters and too few for the SMs stays there
+    (1, 9472, 4096, "skinny"), (1, 9473, 4096, "decode"), (1, 9473, 2048, "skinny"), (2, 9473, 4096, "skinny"),
+    (1, 14208, 4096, "decode"), (1, 14209, 4096, "skinny"),
+    # from the square engine: up to 32 rows, up to 64 with a long K, beyond with few channels too
+    (17, 64, 64, "skinny"), (32, 9472, 512, "skinny"), (33, 4096, 2032, "umma"), (33, 6272, 2048, "skinny"), (33, 6273, 2048, "umma"),
+    (64, 6273, 8176, "umma"), (64, 9472, 8192, "skinny"), (64, 9473, 512, "skinny"),
+    (65, 4736, 4080, "umma"), (65, 4736, 4096, "skinny"), (65, 4737, 4096, "umma"), (128, 4736, 4096, "skinny"), (129, 4096, 8192, "umma"),
+    (89, 6400, 16384, "skinny"), (90, 6400, 16384, "umma"), (72, 9472, 16384, "umma"), (72, 9472, 32768, "skinny")])
+def test_few_rows_engine_by_tiles_and_k(nnb200_lib, m, n, k, engine):
+    """Both sides of each line of the rule, for 148 SMs; the query answers what the call runs on."""
+    from nnops_b200 import capi
+    a = _i8(nnb200_lib, m, n, k)
+    assert capi.ENGINE_NAMES[nnb200_lib.nnb200_gemm_i8_engine(C.byref(a))] == engine
+    a.force_engine = capi.ENGINES["umma"]
+    assert capi.ENGINE_NAMES[nnb200_lib.nnb200_gemm_i8_engine(C.byref(a))] == "umma"

@@ -1,5 +1,7 @@
 """The few-row engine on layers with few channels: clusters of CTAs share a tile's K and add up their sums through
 distributed shared memory.  Byte for byte against the oracle at the edges of rows, channels, K shares and cluster sizes."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -51,6 +53,9 @@ def test_clusters_share_k(cuda_device, nnb200_lib, m, shape):
 def test_calls_routed_to_clusters(cuda_device, nnb200_lib, shape):
     """The smallest K of each row of the rule, one row to a handful, and a call with only the minimum workspace."""
     m, n, k = shape
+    args = capi.GemmI8Args(a=4096, w=4096, out=4096, m=m, n=n, k=k, a_stride_m=k, a_stride_k=1, w_stride_n=k, w_stride_k=1, ldc=n, batch=1,
+                           scale_a_scalar=1.0, scale_w_scalar=1.0, out_scale=1.0)
+    assert capi.ENGINE_NAMES[nnb200_lib.nnb200_gemm_i8_engine(ctypes.byref(args))] == "skinny"
     _case(cuda_device, m, n, k, "f16", engine="auto", seed=m + k)
     a = torch.randint(-127, 128, (m, k), dtype=torch.int8, device=cuda_device)
     w = torch.randint(-127, 128, (n, k), dtype=torch.int8, device=cuda_device)

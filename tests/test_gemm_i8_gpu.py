@@ -6,6 +6,8 @@ byte for byte; ragged M/N/K tails, odd N, per-token / per-channel parameters, al
 destinations, both operand poses, batch broadcast -- plus pitched views with canary bytes,
 which the reference leaves untested.
 """
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -42,8 +44,6 @@ def _run_case(dev, m, n, k, *, out_kind="s32", a_unsigned=False, relu=False, bia
         assert ops.gemm_i8_engine(ta, tw, o, engine=engine, **common) == expect_engine
     if expect_shared_k is not None:
         # The scratch for sharing K among the SMs is what the full workspace has over the minimum.
-        import ctypes
-        from nnops_b200 import capi
         o = torch.empty((m, n), dtype=ops._OUT_TORCH[out_kind], device=dev)
         probe = ops.gemm_i8_args(ta, tw, o, engine=engine, min_workspace=True, **common)
         full = capi.lib().nnb200_gemm_i8_workspace_bytes(ctypes.byref(probe))
@@ -167,20 +167,20 @@ def test_skinny_engine_shared_k_not_offered_when_tiles_fill_the_sms(cuda_device,
               expect_engine="skinny", expect_shared_k=False)
 
 
-@pytest.mark.parametrize("case", [(8, 28672, 1024, "decode"), (12, 4096, 1024, "decode"), (16, 12288, 512, "decode"),
-                                  (12, 14336, 512, "skinny"), (16, 28672, 512, "skinny"), (24, 4096, 1024, "umma"),
-                                  (100, 9472, 512, "umma"), (24, 11008, 512, "skinny"), (64, 28672, 512, "skinny"),
-                                  (100, 11008, 512, "skinny"), (100, 28672, 512, "umma"), (129, 11008, 512, "umma"),
-                                  (12, 4096, 28672, "skinny"), (8, 4096, 28672, "decode")])
+@pytest.mark.parametrize("case", [(8, 28672, 1024, "skinny"), (8, 4096, 4096, "decode"), (12, 4096, 1024, "decode"),
+                                  (16, 12288, 512, "skinny"), (12, 14336, 512, "skinny"), (16, 28672, 512, "skinny"),
+                                  (24, 4096, 1024, "skinny"), (64, 4096, 1024, "umma"), (100, 9472, 512, "umma"), (24, 11008, 512, "skinny"),
+                                  (64, 28672, 512, "skinny"), (100, 11008, 512, "skinny"), (100, 28672, 512, "umma"),
+                                  (129, 11008, 512, "umma"), (12, 4096, 28672, "skinny"), (8, 4096, 28672, "skinny")])
 def test_few_row_engine_choice(cuda_device, nnb200_lib, case):
     """The measured crossovers between the streaming engine, weights-as-rows and the square engine."""
     m, n, k, want = case
     _run_case(cuda_device, m, n, k, out_kind="s8", per_channel=True, out_scale=30.0, expect_engine=want, seed=m + n)
 
 
-def test_narrow_layer_with_long_k_depends_on_the_workspace(cuda_device, nnb200_lib):
-    """4096 channels, K = 14336, 24 rows: with the full workspace the weights-as-rows engine
-    shares K among all SMs; with the minimum one the call stays on the square engine.  Same bytes."""
+def test_narrow_layer_with_long_k_needs_no_workspace(cuda_device, nnb200_lib):
+    """4096 channels, K = 14336, 24 rows: clusters of the weights-as-rows engine share K, and no scratch is asked for
+    that they would not read.  Same bytes as the square engine's, and with K shared through scratch."""
     m, n, k = 24, 4096, 14336
     rng = np.random.default_rng(77)
     a = torch.from_numpy(rng.integers(-127, 128, (m, k), dtype=np.int8)).to(cuda_device)
@@ -188,12 +188,24 @@ def test_narrow_layer_with_long_k_depends_on_the_workspace(cuda_device, nnb200_l
     sw = rng.uniform(0.001, 0.02, n).astype(np.float32)
     kw = dict(out_kind="s8", scale_a=0.02, scale_w=sw, out_scale=150.0, relu=True)
     o = torch.empty((m, n), dtype=torch.int8, device=cuda_device)
-    assert ops.gemm_i8_engine(a, w, o, **kw) == "skinny"
-    assert ops.gemm_i8_engine(a, w, o, min_workspace=True, **kw) == "umma"
-    full = ops.gemm_i8(a, w, **kw).cpu().numpy()
-    least = ops.gemm_i8(a, w, min_workspace=True, **kw).cpu().numpy()
+    for least in (False, True):
+        assert ops.gemm_i8_engine(a, w, o, min_workspace=least, **kw) == "skinny"
+    args = ops.gemm_i8_args(a, w, o, **kw)
+    assert args.workspace_bytes == 0 and capi.lib().nnb200_gemm_i8_workspace_bytes(ctypes.byref(args)) == 0
     want = oracle.gemm_i8(a.cpu().numpy(), w.cpu().numpy(), **kw)
-    assert np.array_equal(full, want) and np.array_equal(least, want)
+    for engine in ("auto", "umma"):
+        assert np.array_equal(ops.gemm_i8(a, w, engine=engine, **kw).cpu().numpy(), want)
+
+
+def test_a_batch_in_one_launch_is_named_by_its_kernel(cuda_device, nnb200_lib):
+    """32 products of 512 x 128 x 512 in one launch; 2 of 8 rows go out one by one, on the engine each would get alone."""
+    i8 = lambda *s: torch.ones(s, dtype=torch.int8, device=cuda_device)
+    o = lambda *s: torch.empty(s, dtype=torch.int32, device=cuda_device)
+    for batch, m, n, k, engine, launches in [(32, 512, 128, 512, "umma", 1), (2, 8, 512, 4096, "decode", 2)]:
+        a, w, out = i8(batch, m, k), i8(batch, n, k), o(batch, m, n)
+        assert ops.gemm_i8_engine(a, w, out, out_kind="s32") == engine
+        before = nnb200_lib.nnb200_launch_count()
+        assert bool((ops.gemm_i8(a, w, out=out) == k).all()) and nnb200_lib.nnb200_launch_count() - before == launches
 
 
 def test_skinny_engine_small_m_on_request(cuda_device, nnb200_lib):
