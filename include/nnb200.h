@@ -300,9 +300,8 @@ NNB200_API int nnb200_measure_i8_mma_peak(int32_t iters, int32_t pattern, double
 NNB200_API int nnb200_set_knob(int knob, int value);
 NNB200_API int nnb200_get_knob(int knob);
 
-/* Which engine nnb200_gemm_i8 would run for these arguments (NNB200_ENGINE_*), the workspace the
- * block carries included: with enough of it some few-row calls move to the weights-as-rows engine.
- * A batch that goes out as one launch is NNB200_ENGINE_UMMA.
+/* Which engine nnb200_gemm_i8 would run for these arguments (NNB200_ENGINE_*).  The workspace the
+ * block carries does not matter.  A batch that goes out as one launch is NNB200_ENGINE_UMMA.
  * The answer is for the operands as they lie: a call that this says is NNB200_ENGINE_GENERIC, with the
  * workspace nnb200_gemm_i8_workspace_bytes asks for, first copies the operands that the tensor-core
  * engines cannot address into aligned rows and then runs the engine of the copies. */

@@ -383,41 +383,24 @@ size_t nnb200_gemm_i8_min_workspace_bytes(const nnb200_gemm_i8_args* a)
     return static_cast<size_t>(a->batch) * (ra + rw);
 }
 
-// Scratch that lets the few-row tensor-core engine share K evenly among all SMs (optional), and
-// whether having it changes the engine: on a layer with so few channels that the square engine
-// was chosen for its narrow tiles (17..128 rows), weights-as-rows with shared K is faster still
-// when K is long (N=4096, K=14336, 24 rows: 24.4 against 35.9 us) -- but only with the scratch.
-struct I8SplitPlan {
-    size_t bytes;         // scratch wanted beyond the required minimum (0 = no use for it)
-    bool switches_engine; // with the scratch the call runs on the weights-as-rows engine instead
-};
-
-static I8SplitPlan i8_split_plan(const nnb200_gemm_i8_args* a)
+// Scratch beyond the required minimum that lets the few-row engine share K evenly among all SMs (optional); 0 where the
+// call has no use for it.
+static size_t i8_split_bytes(const nnb200_gemm_i8_args* a)
 {
-    I8SplitPlan plan{0, false};
     if (a->batch != 1 || sharded_out(a)) {
-        return plan;
+        return 0;
     }
     const DeviceInfo* dev = current_device_info();
-    if (dev == nullptr) {
-        return plan;
-    }
     const I8Problem p = problem_of(a, 0);
-    const int engine = pick_i8_engine_by_shape(a, p);
-    if (engine == NNB200_ENGINE_SKINNY) {
-        plan.bytes = skinny_i8_split_bytes(p, *dev);
-    } else if (engine == NNB200_ENGINE_UMMA && a->force_engine == NNB200_ENGINE_AUTO && p.m >= 17 && p.m <= 128) {
-        plan.bytes = skinny_i8_split_bytes(p, *dev);  // 0 unless weights-as-rows is supported and the split pays
-        plan.switches_engine = plan.bytes > 0;
-    } else if (engine == NNB200_ENGINE_DECODE && a->force_engine == NNB200_ENGINE_AUTO && p.m > 8 &&
-               p.n * p.k >= (int64_t{80} << 20)) {
-        // 9..16 rows on a layer of modest width: the streaming engine costs ~0.23 us per MB of weights,
-        // weights-as-rows with shared K ~0.16 us per MB plus 5 us more up front; from about 80 MB the
-        // latter wins (N=4096, K=28672, 12 rows: 30.5 against 33.6 us).
-        plan.bytes = skinny_i8_split_bytes(p, *dev);
-        plan.switches_engine = plan.bytes > 0;
+    if (dev == nullptr || pick_i8_engine(a, p) != NNB200_ENGINE_SKINNY) {
+        return 0;
     }
-    return plan;
+    // Where the shape alone would have the streaming engine: from about 80 MB of weights, for 9 to 16 rows (a line drawn
+    // between that engine's ~0.23 us per MB and shared K's ~0.16 plus 5 us up front).
+    if (pick_i8_engine_by_shape(a, p) == NNB200_ENGINE_DECODE && (p.m <= 8 || p.n * p.k < (int64_t{80} << 20))) {
+        return 0;
+    }
+    return skinny_i8_split_bytes(p, *dev);
 }
 
 // The part of the caller's workspace, past the first `required` bytes, that serves the split, or null when it is absent, too small or misaligned.
@@ -428,20 +411,6 @@ static void* i8_split_scratch(const nnb200_gemm_i8_args* a, size_t required, siz
         return nullptr;
     }
     return static_cast<uint8_t*>(a->workspace) + required;
-}
-
-// Engine of batch element 0 given the workspace the block carries.
-static int i8_engine_with_workspace(const nnb200_gemm_i8_args* a, size_t reserved, void** split_scratch)
-{
-    const I8SplitPlan plan = i8_split_plan(a);
-    void* scratch = i8_split_scratch(a, nnb200_gemm_i8_min_workspace_bytes(a) + reserved, plan.bytes);
-    if (split_scratch != nullptr) {
-        *split_scratch = scratch;
-    }
-    if (plan.switches_engine && scratch != nullptr) {
-        return NNB200_ENGINE_SKINNY;
-    }
-    return pick_i8_engine(a, problem_of(a, 0));
 }
 
 // Realigned copies of the operands, for calls that alone their base or row pitch keeps off the
@@ -547,7 +516,7 @@ size_t nnb200_gemm_i8_workspace_bytes(const nnb200_gemm_i8_args* a)
     }
     const size_t least = nnb200_gemm_i8_min_workspace_bytes(a);
     const I8AlignPlan align = i8_align_plan(a, plan_scratch_stand_in());
-    return least + align.copy_bytes + i8_split_plan(align.copy_bytes > 0 ? &align.aligned : a).bytes;
+    return least + align.copy_bytes + i8_split_bytes(align.copy_bytes > 0 ? &align.aligned : a);
 }
 
 // Whether the workspace has room for realigned copies where the call wants them; if so *q is the
@@ -615,7 +584,7 @@ int nnb200_gemm_i8_engine(const nnb200_gemm_i8_args* a)
     if (a->batch > 1 && dev != nullptr && i8_batched_call(a, *dev, &batch)) {
         return NNB200_ENGINE_UMMA;   // all products in one launch of its kernel
     }
-    return i8_engine_with_workspace(a, 0, nullptr);
+    return pick_i8_engine(a, problem_of(a, 0));
 }
 
 // One call's kernels.  `reserved`: bytes of the workspace between the sums and the optional
@@ -625,10 +594,8 @@ static int run_gemm_i8(const nnb200_gemm_i8_args* a, const DeviceInfo* dev, cuda
                        bool ra_done, bool rw_done)
 {
     const bool comp = needs_compensation(a);
-    // The rest of the workspace, when there is enough of it, lets the few-row engine share K
-    // among the SMs (and on narrow layers with a long K makes it the engine of choice).
-    void* split_scratch = nullptr;
-    const int engine0 = i8_engine_with_workspace(a, reserved, &split_scratch);
+    // The rest of the workspace, when there is enough of it, lets the few-row engine share K among the SMs.
+    void* split_scratch = i8_split_scratch(a, nnb200_gemm_i8_min_workspace_bytes(a) + reserved, i8_split_bytes(a));
     const size_t ra_bytes = (static_cast<size_t>(a->m) * 4 + 255) & ~size_t(255);
     const size_t rw_bytes = (static_cast<size_t>(a->n) * 4 + 255) & ~size_t(255);
 
@@ -664,7 +631,7 @@ static int run_gemm_i8(const nnb200_gemm_i8_args* a, const DeviceInfo* dev, cuda
     // Launchability of every batch element is settled before the first launch, so that a
     // refusal leaves the outputs untouched: the generic engine's grid has 65535 rows of 32.
     for (int64_t b = 0; !batched && b < a->batch; ++b) {
-        const int e = a->batch == 1 ? engine0 : pick_i8_engine(a, problem_of(a, b));
+        const int e = pick_i8_engine(a, problem_of(a, b));
         if (e == NNB200_ENGINE_GENERIC && (a->m + 31) / 32 > 65535) {
             return NNB200_UNSUPPORTED;
         }
@@ -745,7 +712,7 @@ static int run_gemm_i8(const nnb200_gemm_i8_args* a, const DeviceInfo* dev, cuda
         if (batched) {
             return launch_gemm_i8_umma_batched(p, batch, ep, *dev, stream);
         }
-        switch (a->batch == 1 ? engine0 : pick_i8_engine(a, p)) {
+        switch (pick_i8_engine(a, p)) {
         case NNB200_ENGINE_UMMA: st = launch_gemm_i8_umma(p, ep, *dev, stream); break;
         case NNB200_ENGINE_NARROW: st = launch_gemm_i8_narrow(p, ep, *dev, stream); break;
         case NNB200_ENGINE_DECODE: st = launch_gemm_i8_decode(p, ep, *dev, stream); break;
