@@ -248,7 +248,7 @@ int64_t sm_count()
 }
 
 // By alignment, rows and channels alone.
-int pick_i8_engine_by_shape(const nnb200_gemm_i8_args* a, const I8Problem& p)
+int pick_i8_engine_by_shape(const nnb200_gemm_i8_args* a, const I8Problem& p, int64_t sms)
 {
     if (a->force_engine == NNB200_ENGINE_GENERIC) {
         return NNB200_ENGINE_GENERIC;
@@ -276,7 +276,6 @@ int pick_i8_engine_by_shape(const nnb200_gemm_i8_args* a, const I8Problem& p)
     if (!sharded_out(a)) {
         const bool decode_ok = decode_i8_supported(p);
         const bool skinny_ok = skinny_i8_supported(p);
-        const int64_t sms = sm_count();
         const int64_t tiles128 = (p.n + 127) / 128;
         if (decode_ok && (p.m <= 8 || !skinny_ok || tiles128 <= 96)) {
             return NNB200_ENGINE_DECODE;
@@ -301,9 +300,10 @@ int pick_i8_engine_by_shape(const nnb200_gemm_i8_args* a, const I8Problem& p)
 // to two others.
 int pick_i8_engine(const nnb200_gemm_i8_args* a, const I8Problem& p)
 {
-    const int engine = pick_i8_engine_by_shape(a, p);
+    const int64_t sms = sm_count();
+    const int engine = pick_i8_engine_by_shape(a, p, sms);
     if (a->force_engine == NNB200_ENGINE_AUTO && !sharded_out(a) && (engine == NNB200_ENGINE_UMMA || engine == NNB200_ENGINE_DECODE) &&
-        skinny_i8_preferred(p, engine == NNB200_ENGINE_DECODE, sm_count())) {
+        skinny_i8_preferred(p, engine == NNB200_ENGINE_DECODE, sms)) {
         return NNB200_ENGINE_SKINNY;
     }
     return engine;
@@ -383,21 +383,21 @@ size_t nnb200_gemm_i8_min_workspace_bytes(const nnb200_gemm_i8_args* a)
     return static_cast<size_t>(a->batch) * (ra + rw);
 }
 
-// Scratch beyond the required minimum that lets the few-row engine share K evenly among all SMs (optional); 0 where the
-// call has no use for it.
-static size_t i8_split_bytes(const nnb200_gemm_i8_args* a)
+// Scratch beyond the required minimum that lets the few-row engine, if that is the call's, share K evenly among all SMs
+// (optional); 0 where the call has no use for it.
+static size_t i8_split_bytes(const nnb200_gemm_i8_args* a, int engine)
 {
-    if (a->batch != 1 || sharded_out(a)) {
+    if (engine != NNB200_ENGINE_SKINNY || a->batch != 1 || sharded_out(a)) {
         return 0;
     }
     const DeviceInfo* dev = current_device_info();
-    const I8Problem p = problem_of(a, 0);
-    if (dev == nullptr || pick_i8_engine(a, p) != NNB200_ENGINE_SKINNY) {
+    if (dev == nullptr) {
         return 0;
     }
     // Where the shape alone would have the streaming engine: from about 80 MB of weights, for 9 to 16 rows (a line drawn
     // between that engine's ~0.23 us per MB and shared K's ~0.16 plus 5 us up front).
-    if (pick_i8_engine_by_shape(a, p) == NNB200_ENGINE_DECODE && (p.m <= 8 || p.n * p.k < (int64_t{80} << 20))) {
+    const I8Problem p = problem_of(a, 0);
+    if ((p.m <= 8 || p.n * p.k < (int64_t{80} << 20)) && pick_i8_engine_by_shape(a, p, dev->sm_count) == NNB200_ENGINE_DECODE) {
         return 0;
     }
     return skinny_i8_split_bytes(p, *dev);
@@ -465,9 +465,10 @@ static I8AlignPlan i8_align_plan(const nnb200_gemm_i8_args* a, uint8_t* scratch)
         a->k > INT32_MAX || !i8_copies_pay(a)) {
         return plan;
     }
+    const int64_t sms = sm_count();
     for (int64_t b = 0; b < (a->batch < 2 ? 1 : 2); ++b) {
         // Element 0 tells for base and pitch, element 1 for the batch strides.
-        if (pick_i8_engine(a, problem_of(a, b)) == NNB200_ENGINE_GENERIC) {
+        if (pick_i8_engine_by_shape(a, problem_of(a, b), sms) == NNB200_ENGINE_GENERIC) {
             plan.copy_bytes = 1;
         }
     }
@@ -516,7 +517,8 @@ size_t nnb200_gemm_i8_workspace_bytes(const nnb200_gemm_i8_args* a)
     }
     const size_t least = nnb200_gemm_i8_min_workspace_bytes(a);
     const I8AlignPlan align = i8_align_plan(a, plan_scratch_stand_in());
-    return least + align.copy_bytes + i8_split_bytes(align.copy_bytes > 0 ? &align.aligned : a);
+    const nnb200_gemm_i8_args* q = align.copy_bytes > 0 ? &align.aligned : a;
+    return least + align.copy_bytes + i8_split_bytes(q, pick_i8_engine(q, problem_of(q, 0)));
 }
 
 // Whether the workspace has room for realigned copies where the call wants them; if so *q is the
@@ -562,7 +564,7 @@ static bool i8_batched_call(const nnb200_gemm_i8_args* a, const DeviceInfo& dev,
     // 15 layers at 1 to 16 rows with each product on the streaming engine; with the engines of today (us, alone /
     // batched): 2 x 1 x 2048 x 3968 9.1 / 11.6, 4 x 8 x 512 x 15360 21.6 / 20.7, 6 x 4 x 64 x 65536 60.5 / 75.3 stay
     // alone, 8 x 1 x 2048 x 3968 36.9 / 17.5, 2 x 8 x 16384 x 448 8.7 / 9.2, 8 x 8 x 4032 x 2048 36.1 / 17.4 do not.
-    if (a->force_engine == NNB200_ENGINE_AUTO && pick_i8_engine_by_shape(a, problem_of(a, 0)) == NNB200_ENGINE_DECODE) {
+    if (a->force_engine == NNB200_ENGINE_AUTO && pick_i8_engine_by_shape(a, problem_of(a, 0), dev.sm_count) == NNB200_ENGINE_DECODE) {
         const double kb = static_cast<double>((a->k + 127) / 128);
         const double one = 230.0 + 0.01 * static_cast<double>(a->n) + 20.0 * static_cast<double>(a->m < 4 ? a->m : 4) +
                            (a->m <= 8 ? 2.4 : 5.2) * kb;
@@ -595,7 +597,8 @@ static int run_gemm_i8(const nnb200_gemm_i8_args* a, const DeviceInfo* dev, cuda
 {
     const bool comp = needs_compensation(a);
     // The rest of the workspace, when there is enough of it, lets the few-row engine share K among the SMs.
-    void* split_scratch = i8_split_scratch(a, nnb200_gemm_i8_min_workspace_bytes(a) + reserved, i8_split_bytes(a));
+    const int engine0 = pick_i8_engine(a, problem_of(a, 0));
+    void* split_scratch = i8_split_scratch(a, nnb200_gemm_i8_min_workspace_bytes(a) + reserved, i8_split_bytes(a, engine0));
     const size_t ra_bytes = (static_cast<size_t>(a->m) * 4 + 255) & ~size_t(255);
     const size_t rw_bytes = (static_cast<size_t>(a->n) * 4 + 255) & ~size_t(255);
 
@@ -631,7 +634,7 @@ static int run_gemm_i8(const nnb200_gemm_i8_args* a, const DeviceInfo* dev, cuda
     // Launchability of every batch element is settled before the first launch, so that a
     // refusal leaves the outputs untouched: the generic engine's grid has 65535 rows of 32.
     for (int64_t b = 0; !batched && b < a->batch; ++b) {
-        const int e = pick_i8_engine(a, problem_of(a, b));
+        const int e = b == 0 ? engine0 : pick_i8_engine(a, problem_of(a, b));
         if (e == NNB200_ENGINE_GENERIC && (a->m + 31) / 32 > 65535) {
             return NNB200_UNSUPPORTED;
         }
@@ -712,7 +715,7 @@ static int run_gemm_i8(const nnb200_gemm_i8_args* a, const DeviceInfo* dev, cuda
         if (batched) {
             return launch_gemm_i8_umma_batched(p, batch, ep, *dev, stream);
         }
-        switch (pick_i8_engine(a, p)) {
+        switch (b == 0 ? engine0 : pick_i8_engine(a, p)) {
         case NNB200_ENGINE_UMMA: st = launch_gemm_i8_umma(p, ep, *dev, stream); break;
         case NNB200_ENGINE_NARROW: st = launch_gemm_i8_narrow(p, ep, *dev, stream); break;
         case NNB200_ENGINE_DECODE: st = launch_gemm_i8_decode(p, ep, *dev, stream); break;
