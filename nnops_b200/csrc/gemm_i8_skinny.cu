@@ -622,14 +622,13 @@ gemm_i8_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                             v[j] += p < parts ? theirs[p][j] : 0u;
                         }
                     }
-                    int end = store_end;
+                    finish_rows<KIND, 4>(ep, row_terms, v, r, store_end, n, n_ok, ct);
                     if (r + 4 > row_end || !all_ok) {
                         // Rows or channels that are not stored: nothing else waits for their loads, and the CTA they come
                         // from may leave after the barrier below.  Once the warp has met here they have come.
                         const uint32_t seen = v[0] | v[1] | v[2] | v[3];
-                        end = __any_sync(0xFFFFFFFFu, (seen & never) != 0) ? 0 : store_end;
+                        row_end = __any_sync(0xFFFFFFFFu, (seen & never) != 0) ? 0 : row_end;
                     }
-                    finish_rows<KIND, 4>(ep, row_terms, v, r, end, n, n_ok, ct);
                 }
             }
             __syncwarp();

@@ -68,10 +68,9 @@ def test_what_is_read_from_another_cta_has_come_before_it_may_leave():
     kernel = _sources()["gemm_i8_skinny.cu"]
     kernel = kernel[kernel.index("gemm_i8_skinny_kernel(const"):]
     loads, stores = kernel.index("theirs[p][j] = ld_shared_cluster_u32("), kernel.index("finish_rows<KIND, 4>(")
-    assert kernel.count("ld_shared_cluster_u32(") == 1
-    between = kernel[loads:stores]
-    at = between.index("if (r + 4 > row_end || !all_ok)")
-    vote = _body(between, at)
-    assert "v[0] | v[1] | v[2] | v[3]" in vote and re.search(r"end = __any_sync\(0xFFFFFFFFu, \(seen & never\) != 0\)", vote)
+    parting = kernel.index("cluster_sync_all_relaxed()", stores)
+    assert kernel.count("ld_shared_cluster_u32(") == 1 and loads < stores < parting
+    after = kernel[stores:parting]
+    vote = _body(after, after.index("if (r + 4 > row_end || !all_ok)"))
+    assert "v[0] | v[1] | v[2] | v[3]" in vote and re.search(r"row_end = __any_sync\(0xFFFFFFFFu, \(seen & never\) != 0\)", vote)
     assert "all_ok = __all_sync(0xFFFFFFFFu, n_ok)" in kernel[:loads]
-    assert kernel[stores:].index("cluster_sync_all_relaxed()") > 0
