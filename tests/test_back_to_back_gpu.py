@@ -148,3 +148,59 @@ def test_what_a_kernel_wrote_just_before(cuda_device, nnb200_lib, producer):
     want = _same_with_and_without_waiting(chain)
     for i in range(0, len(want), 2):   # the two inputs do not give the same, or nothing would show
         assert not torch.equal(want[i], want[i + 1])
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_forks_and_joins(cuda_device, nnb200_lib, captured):
+    """Calls on two streams that wait for each other by events, eager and in a CUDA graph: a kernel that may overlap the one
+    before it in its stream still comes after what its stream has waited for."""
+    rng = np.random.default_rng(5)
+    w1, w2, wide = _s8(rng, cuda_device, 2048, 1024), _s8(rng, cuda_device, 1024, 2048), _s8(rng, cuda_device, 6144, 1024)
+    blocks = torch.from_numpy(synth.q4_1_weights(rng, 2048, 1024)).to(cuda_device)
+    x0 = _s8(rng, cuda_device, 300, 1024)
+    outs = {n: torch.empty(s, dtype=t, device=cuda_device) for n, s, t in [
+        ("a", (300, 2048), torch.int8), ("b", (16, 2048), torch.int8), ("c", (300, 1024), torch.int8), ("d", (16, 1024), torch.int8),
+        ("e", (16, 2048), torch.float16), ("f", (300, 6144), torch.int8)]}
+    x = torch.empty_like(x0)
+    half = torch.empty((16, 1024), dtype=torch.float16, device=cuda_device)
+    scale, zp = torch.full((300,), 0.02, device=cuda_device), torch.zeros(300, dtype=torch.int8, device=cuda_device)
+    side = torch.cuda.Stream()
+    kw = dict(out_kind="s8", out_scale=20.0, scale_w=0.01)
+
+    def work():
+        main = torch.cuda.current_stream()
+        for _ in range(3):
+            ops.gemm_i8(x, w1, out=outs["a"], engine="umma", **kw)
+            side.wait_stream(main)
+            with torch.cuda.stream(side):
+                ops.gemm_i8(outs["a"][:16, :1024], w1, out=outs["b"], engine="skinny", **kw)     # reads what main wrote
+                ops.dequantize_linear(outs["b"][:, :1024].contiguous(), scale[:16], zp[:16], out=half)
+                ops.linear_q4_1(half, blocks, 1024, out=outs["e"], engine="rows")
+            ops.gemm_i8(outs["a"], w2, out=outs["c"], engine="umma", **kw)
+            main.wait_stream(side)
+            ops.gemm_i8(outs["b"], w2, out=outs["d"], engine="skinny", **kw)      # behind c on main, reads what side wrote
+            ops.gemm_i8(outs["c"], wide, out=outs["f"], engine="umma", **kw)
+            x[:16].copy_(outs["d"])
+            x[16:].copy_(outs["c"][16:])
+
+    def serial():
+        x.copy_(x0)
+        work()
+        torch.cuda.synchronize()
+        return {n: t.clone() for n, t in outs.items()}
+
+    want = serial()
+    for _ in range(3):
+        x.copy_(x0)
+        for t in outs.values():
+            t.zero_()
+        if captured:
+            torch.cuda.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                work()
+            graph.replay()
+        else:
+            work()
+        torch.cuda.synchronize()
+        assert all(torch.equal(outs[n].view(torch.uint8), want[n].view(torch.uint8)) for n in outs)
